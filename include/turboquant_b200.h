@@ -95,8 +95,8 @@ int tq_packed_row_bytes(int D, int bits);
 int tq_build_codebook(const float* centroids, int bits, float* block);
 
 /* Tensor-core operand image of a (D, D) row-major fp32 matrix m [dev]: two fp16 pieces
- * (m = hi + lo), K-major, 128-byte swizzled, tq_rotation_image_bytes(D) bytes (0 when D
- * has no tensor-core path; only D = 128 has one).  Built once per compressor.
+ * (m = hi + lo) and three bf16 pieces, K-major, 128-byte swizzled, tq_rotation_image_bytes(D) bytes
+ * (0 when D has no tensor-core path; D = 64 and 128 have one).  Built once per compressor.
  * For TqQuantizeJob pass m = Pi; for TqDequantizeJob pass m = Pi^T.
  * Replaces nothing in the reference (a constant of this implementation).       */
 size_t tq_rotation_image_bytes(int D);
@@ -128,7 +128,7 @@ typedef struct {
   void* idx_out;          /* [dev] (B*H*S, row) contiguous                                   */
   uint16_t* norms_out;    /* [dev] fp16 bit patterns (B*H*S); may be NULL when normalize==0  */
   const void* rotation_image; /* [dev] optional: tq_prepare_rotation_image(Pi) output.  With it, head_dim
-                             128, 16-bit x, normalize=1 and TQ_IDX_PACKED the job runs on the tensor
+                             64 or 128, 16-bit x, normalize=1 and TQ_IDX_PACKED the job runs on the tensor
                              cores; NULL keeps it on the FP32 path                              */
 } TqQuantizeJob;
 
@@ -153,7 +153,7 @@ typedef struct {
   const float* rotation;  /* [dev] Pi, (D, D) row-major fp32: x_hat = c[idx] @ rotation      */
   const float* codebook;  /* [dev] codebook block                                            */
   const void* rotation_image; /* [dev] optional: tq_prepare_rotation_image(Pi^T) output; with it, head_dim
-                             128 and TQ_IDX_PACKED with norms run on the tensor cores            */
+                             64 or 128 and TQ_IDX_PACKED with norms run on the tensor cores            */
 } TqDequantizeJob;
 
 /* Replaces: MSECompressor.decompress turboquant/compressors_v3.py:83-105; with a

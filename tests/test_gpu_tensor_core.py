@@ -17,6 +17,7 @@ from parity_helpers import check_indices, check_norms, check_recon_16bit, mismat
 
 import turboquant as tq
 from turboquant import _native as N
+from turboquant import _ops
 from turboquant import batched
 
 pytestmark = pytest.mark.gpu
@@ -209,3 +210,49 @@ def test_index_rows_at_a_16_byte_offset_equal_the_aligned_ones(bits):
     assert torch.equal(got, want)
     assert bool((raw[:16] == 0xA5).all()) and bool((raw[16 + want.numel():] == 0xA5).all())
     assert g == N.packed_row_bytes(128, bits) and N.lib().tq_last_device_status() == 0
+
+
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 255, 256, 257, 700])
+def test_head_dim_64_round_trip(rows, dtype, bits):
+    """A tile is 256 vectors: edges of its two halves, several tiles, odd lengths, a view and a strided output."""
+    base = O.synthetic_kv((2, 3, rows + 3, 64), dtype, seed=50 * bits + rows)
+    x = base[:, :, 2:rows + 2]
+    comp = tq.MSECompressor(64, bits, seed=80 + bits, device=DEV)
+    assert comp._img_q is not None
+    c = comp.compress(base.to(DEV)[:, :, 2:rows + 2])
+    cent, bnd = O.lloyd_max(64, bits)
+    norms, _ = check_indices(c["idx_bytes"], x.contiguous(), comp.Pi.cpu(), cent, bnd, bits, 64)
+    check_norms(c["vec_norms"], norms)
+    want = _simt(lambda: comp.decompress(c))
+    out = torch.full((2, 3, rows + 8, 64), -7.0, dtype=dtype, device=DEV)
+    job, _keep = comp.decompress_job(c, out[:, :, 1:rows + 1])
+    _ops.run_dequantize([job], DEV)
+    full = comp.decompress(c)
+    torch.cuda.synchronize()
+    assert N.lib().tq_last_device_status() == 0
+    # three passes of fp16 pieces: 2^-21 of the sum of magnitudes, at most 8 times the largest value
+    assert float((full - want).abs().max()) <= 2.0 ** -18 * float(want.abs().max())
+    # so the 16-bit output is the FP32 kernel's up to one step where that value lies on a rounding edge
+    got, ref = out[:, :, 1:rows + 1].float(), want.to(dtype).float()
+    step = 2.0 ** (-10 if dtype == torch.float16 else -7)
+    assert bool(((got - ref).abs() <= step * ref.abs() + 2.0 ** -18 * float(want.abs().max())).all())
+    assert float((got != ref).float().mean()) <= 0.01 if dtype == torch.bfloat16 else True
+    assert bool((out[:, :, 0] == -7).all()) and bool((out[:, :, rows + 1:] == -7).all())
+
+
+def test_head_dim_64_keeps_infinite_and_nan_norms():
+    for dtype in (torch.float16, torch.bfloat16):
+        x = O.synthetic_kv((1, 2, 300, 64), dtype, seed=5)
+        x[0, 0, 3] = 0
+        x[0, 0, 9, 5] = float("nan")
+        x[0, 1, 140, 17] = float("inf")
+        x[0, 1, 299, 1] = float("-inf")
+        comp = tq.MSECompressor(64, 4, seed=42, device=DEV)
+        xg = x.to(DEV)
+        c, ref = comp.compress(xg), _simt(lambda: comp.compress(xg))
+        for h, s in ((0, 3), (0, 9), (1, 140), (1, 299)):
+            assert torch.equal(c["idx_bytes"][0, h, s], ref["idx_bytes"][0, h, s])
+            a, b = c["vec_norms"][0, h, s], ref["vec_norms"][0, h, s]
+            assert bool(a.isnan()) == bool(b.isnan()) and (bool(a.isnan()) or bool(a == b))

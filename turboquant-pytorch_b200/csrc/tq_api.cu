@@ -320,7 +320,7 @@ int tq_quantize(const TqQuantizeJob* jobs, int n_jobs, void* stream) {
     int rc;
     if (tq::umma_quantize_eligible(jobs[i])) {
       int k = i + 1;
-      while (k < n_jobs && jobs[k].x_dtype == jobs[i].x_dtype && tq::umma_quantize_eligible(jobs[k])) ++k;
+      while (k < n_jobs && jobs[k].x_dtype == jobs[i].x_dtype && jobs[k].D == jobs[i].D && tq::umma_quantize_eligible(jobs[k])) ++k;
       rc = tq::umma_quantize(jobs + i, k - i, (cudaStream_t)stream);
       i = k;
     } else {
@@ -352,7 +352,7 @@ int tq_dequantize(const TqDequantizeJob* jobs, int n_jobs, void* stream) {
     if (tq::umma_dequantize_eligible(jobs[i])) {
       const bool out32 = jobs[i].out_dtype == TQ_F32;
       int k = i + 1;
-      while (k < n_jobs && (jobs[k].out_dtype == TQ_F32) == out32 && tq::umma_dequantize_eligible(jobs[k])) ++k;
+      while (k < n_jobs && (jobs[k].out_dtype == TQ_F32) == out32 && jobs[k].D == jobs[i].D && tq::umma_dequantize_eligible(jobs[k])) ++k;
       rc = tq::umma_dequantize(jobs + i, k - i, (cudaStream_t)stream);
       i = k;
     } else {

@@ -142,10 +142,10 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
   return lo | (hi << 32);
 }
 
-__device__ __forceinline__ uint32_t idesc_f16(bool bf16) {
-  // D = fp32, A and B both fp16 or both bf16, K-major, N = 128, M = 128
+__device__ __forceinline__ uint32_t idesc_f16(bool bf16, uint32_t n = 128u) {
+  // D = fp32, A and B both fp16 or both bf16, K-major, N = n, M = 128
   const uint32_t fmt = bf16 ? 1u : 0u;
-  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {

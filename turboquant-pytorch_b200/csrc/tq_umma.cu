@@ -1,5 +1,5 @@
-// Tensor-core (tcgen05 / TMEM / TMA) kernels for the headline shape: head_dim 128,
-// 16-bit vectors, packed indices.
+// Tensor-core (tcgen05 / TMEM / TMA) kernels for 16-bit vectors of head_dim 128 (the headline shape) or 64 and
+// packed indices.  What follows describes head_dim 128; see kTileVecs for head_dim 64.
 //
 // quantize: a persistent, warp-specialised CTA per SM walks a contiguous range of
 // 128-vector tiles that may span several jobs (layers, K or V):
@@ -22,8 +22,10 @@
 #include <cuda.h>
 
 #include <atomic>
+#include <cstddef>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "tq_common.cuh"
@@ -40,8 +42,17 @@ constexpr int kEpiWarps = 16;
 constexpr int kThreads = 64 + kEpiWarps * 32;          // 576
 constexpr uint32_t kTileBytes = kTileRows * kDim * 2;  // 32768
 constexpr uint32_t kHalfBytes = kTileBytes / 2;        // one 64-column box
-constexpr uint32_t kImageBytes = 5 * kTileBytes;       // fp16 hi, lo; then bf16 p0, p1, p2
+// A tile is 32 KB of 16-bit values: 128 vectors of head_dim 128 (its two 64-column boxes are the k-halves of one
+// operand) or 256 vectors of head_dim 64 (the boxes are two operands of 128 vectors; each has its own 64 columns of
+// the tile's accumulator).  Ring, accumulator and staging sizes are then the same for both.
+// Head_dim 64 ran on the FP32 kernels before, which are bound by their fused multiply-adds: 124 us to quantise and 80 us to
+// rebuild one (2, 8, 4875, 64) bf16 tensor; compress_kv + decompress_kv of such a layer (K4/V3) went from 376 to 108 us,
+// most of which is the host's.
+template <int D> constexpr int kTileVecs = (int)(kTileBytes / 2) / D;
+template <int D> constexpr uint32_t kImagePiece = (uint32_t)(D * D * 2);                 // one piece of a rotation image
+constexpr int tile_vecs_of(int D) { return (int)(kTileBytes / 2) / D; }
 constexpr int kMaxJobs = 96;
+constexpr int kFewJobs = 8;
 constexpr int kMaxCtas = 192;                          // upper bound of the grid (one CTA per SM)
 
 // Timing-only switches that skip parts of the kernels exist only in builds made with
@@ -53,13 +64,14 @@ constexpr int kMaxCtas = 192;                          // upper bound of the gri
 #endif
 
 // shared memory map (offsets from a 1024-byte aligned base)
-template <bool BF16, bool WIDE = false>
+template <bool BF16, bool WIDE = false, int D = kDim>
 struct Cfg {
   // x-tile ring: launches with wide codes give one stage to the look-up tables (their tiles take 1.7-2.5 us,
   // enough for a load to land with one tile of look-ahead less)
   static constexpr int kStages = (BF16 ? 3 : 4) - (WIDE ? 1 : 0);
   static constexpr int kPieces = BF16 ? 3 : 2;
-  static constexpr uint32_t kPieceOff = BF16 ? 2 * kTileBytes : 0;            // offset of the pieces in the image
+  static constexpr uint32_t kPieceBytes = kImagePiece<D>;
+  static constexpr uint32_t kPieceOff = BF16 ? 2 * kPieceBytes : 0;           // offset of the pieces in the image
   static constexpr uint32_t kOffA = 0;
   static constexpr uint32_t kOffPi = kOffA + kStages * kTileBytes;
   // Narrow launches: 256 thresholds (fp32) per epilogue warpgroup.  Launches with wide codes: ONE set of
@@ -67,7 +79,7 @@ struct Cfg {
   // entry stored once per lane so that random look-ups never collide in the banks:
   //   thresholds * 2^40 of 7/8-bit codes:        256 x 32 x 4 bytes   (6-bit codes: 64 x 32 x 4 bytes, same place),
   //   candidate index per cell of t (7/8 bits): 1025 x 32 x 1 byte    (four lanes share a word)
-  static constexpr uint32_t kOffThr = kOffPi + kPieces * kTileBytes;
+  static constexpr uint32_t kOffThr = kOffPi + kPieces * kPieceBytes;
   static constexpr uint32_t kThrRegion = 1024;
   static constexpr uint32_t kOffCells = kOffThr + 32768;
   static constexpr uint32_t kOffBar = WIDE ? kOffCells + 32800 : kOffThr + 4 * kThrRegion;
@@ -76,11 +88,13 @@ struct Cfg {
 static_assert(Cfg<false, true>::kSmemBytes <= 232448 && Cfg<true, true>::kSmemBytes <= 232448, "shared memory budget");
 
 struct alignas(64) UmmaQuantJob {
-  CUtensorMap tmap;          // (D, S, H, B) view of x, box 64 x 128 x 1 x 1, 128-byte swizzle
+  CUtensorMap tmap;          // (D, S, H, B) view of x, box 64 x 128 x 1 x 1, 128-byte swizzle (two boxes per tile)
   const void* image;         // rotation image: hi piece then lo piece, swizzled K-major
   const float* codebook;
   uint8_t* idx_out;
   uint16_t* norms_out;
+  const uint16_t* x;         // the vectors once more (x_norm)
+  int64_t xs_b, xs_h, xs_s;  // and their strides in elements
   int64_t S;
   int32_t H;
   int32_t tiles_per_slab;
@@ -90,7 +104,11 @@ struct alignas(64) UmmaQuantJob {
   int32_t pad_;
 };
 
-struct UmmaQuantBatch {
+// J: room for jobs.  The whole struct travels as the kernel's parameter, and a launch costs the host 3 us with 4 KB
+// of parameters and 5.8 us with 24 KB, so calls of few jobs (one layer's K and V) launch a kernel with the small form,
+// which is a prefix of the large one.
+template <int J>
+struct UmmaQuantBatchOf {
   int32_t n_jobs;
   int32_t total_tiles;
   int32_t* status;           // device status word (may be null)
@@ -98,8 +116,9 @@ struct UmmaQuantBatch {
                              // 32 half loads, 64 no loads, 256 / 512 skip the quantise / norm sweep
   int32_t pad_[3];
   int32_t cta_begin[kMaxCtas + 1];   // CTA c owns tiles [cta_begin[c], cta_begin[c + 1]): equal estimated cost, not equal count
-  UmmaQuantJob jobs[kMaxJobs];
+  UmmaQuantJob jobs[J];
 };
+using UmmaQuantBatch = UmmaQuantBatchOf<kMaxJobs>;
 
 static_assert(sizeof(UmmaQuantBatch) < 32000, "kernel parameter space");
 
@@ -121,7 +140,8 @@ struct QuantJobView {
   const CUtensorMap* tmap = nullptr;
 };
 // true when `tile` belongs to another job than the cached one (tiles only grow within a role)
-__device__ __forceinline__ bool view_advance(const UmmaQuantBatch& b, int tile, QuantJobView& v) {
+template <int D, int J>
+__device__ __forceinline__ bool view_advance(const UmmaQuantBatchOf<J>& b, int tile, QuantJobView& v) {
   if (v.j >= 0 && tile < v.end) return false;
   int j = v.j < 0 ? 0 : v.j;
   while (j + 1 < b.n_jobs && tile >= b.jobs[j + 1].tile_begin) ++j;
@@ -132,7 +152,7 @@ __device__ __forceinline__ bool view_advance(const UmmaQuantBatch& b, int tile, 
   v.tps = job.tiles_per_slab;
   v.H = job.H;
   v.bits = job.bits;
-  v.g = kDim / (8 / job.bits);
+  v.g = D / (8 / job.bits);
   v.S = job.S;
   v.idx_out = job.idx_out;
   v.norms_out = job.norms_out;
@@ -145,14 +165,14 @@ __device__ __forceinline__ bool view_advance(const UmmaQuantBatch& b, int tile, 
 // ---------------------------------------------------------------- epilogue
 // One thread owns one vector (registers = coordinates).
 // Generic (binary search) quantise sweep for codebooks without a search shortcut.  A thread
-// owns all 128 coordinates of one vector; tmem_acc points at its first column.
-template <int BITS>
+// owns all D coordinates of one vector; tmem_acc points at its first column.
+template <int BITS, int D>
 __device__ __forceinline__ void quant_row_generic(uint32_t tmem_acc, float inv, const float* thr, uint8_t* idx_half,
                                                   bool valid) {
   constexpr int IPB = 8 / BITS;
   constexpr int BYTES_PER_CHUNK = 32 / IPB;     // packed bytes per 32 coordinates
 #pragma unroll 1
-  for (int c = 0; c < 4; ++c) {
+  for (int c = 0; c < D / 32; ++c) {
     float v[32];
     tmem_ld32(tmem_acc + c * 32, v);
     uint32_t words[BYTES_PER_CHUNK / 4 > 0 ? BYTES_PER_CHUNK / 4 : 1];
@@ -189,18 +209,31 @@ __device__ __forceinline__ void quant_row_generic(uint32_t tmem_acc, float inv, 
 
 // Codebooks without a verified shortcut (none of the Lloyd-Max codebooks): out of line, so that its
 // registers and code do not weigh on the paths that run.
+template <int D>
 __device__ __noinline__ void quant_row_search(int bits, uint32_t tacc, float inv, const float* thr, uint8_t* idx_row,
                                               bool valid) {
   switch (bits) {
-    case 1: quant_row_generic<1>(tacc, inv, thr, idx_row, valid); break;
-    case 2: quant_row_generic<2>(tacc, inv, thr, idx_row, valid); break;
-    case 3: quant_row_generic<3>(tacc, inv, thr, idx_row, valid); break;
-    case 4: quant_row_generic<4>(tacc, inv, thr, idx_row, valid); break;
-    case 5: quant_row_generic<5>(tacc, inv, thr, idx_row, valid); break;
-    case 6: quant_row_generic<6>(tacc, inv, thr, idx_row, valid); break;
-    case 7: quant_row_generic<7>(tacc, inv, thr, idx_row, valid); break;
-    default: quant_row_generic<8>(tacc, inv, thr, idx_row, valid); break;
+    case 1: quant_row_generic<1, D>(tacc, inv, thr, idx_row, valid); break;
+    case 2: quant_row_generic<2, D>(tacc, inv, thr, idx_row, valid); break;
+    case 3: quant_row_generic<3, D>(tacc, inv, thr, idx_row, valid); break;
+    case 4: quant_row_generic<4, D>(tacc, inv, thr, idx_row, valid); break;
+    case 5: quant_row_generic<5, D>(tacc, inv, thr, idx_row, valid); break;
+    case 6: quant_row_generic<6, D>(tacc, inv, thr, idx_row, valid); break;
+    case 7: quant_row_generic<7, D>(tacc, inv, thr, idx_row, valid); break;
+    default: quant_row_generic<8, D>(tacc, inv, thr, idx_row, valid); break;
   }
+}
+
+// Norm of a vector from its own coordinates.  The rotated row of a vector with an infinity is NaN throughout (the
+// pieces of Pi meet it with both signs) while its norm is infinite; such rows come here.  Out of line: cold.
+template <bool BF16, int D>
+__device__ __noinline__ float x_norm(const uint16_t* x) {
+  float ssq = 0.f;
+  for (int k = 0; k < D; ++k) {
+    const float v = BF16 ? __uint_as_float((uint32_t)__ldg(x + k) << 16) : __half2float(__ushort_as_half(__ldg(x + k)));
+    ssq = fmaf(v, v, ssq);
+  }
+  return __fsqrt_rn(ssq);
 }
 
 // Search shortcut (see the codebook block): one cubic, one lane look-up of the candidate
@@ -331,17 +364,18 @@ __device__ __forceinline__ unsigned long long ssq_chunk(const uint32_t (&raw)[CH
   return ssq2;
 }
 
-// A thread owns one vector: eight 16-column steps per sweep.  Two register buffers
+// A thread owns one vector: D / 16 steps of 16 columns per sweep.  Two register buffers
 // alternate so that a TMEM load is always in flight behind the math; the loops stay rolled
 // (two inlined copies of the step body, one per buffer).
+template <int D>
 __device__ __forceinline__ float ssq_row_fast(uint32_t tacc, uint32_t (&a)[16], uint32_t (&b)[16]) {
   unsigned long long ssq2 = pack2(0.f, 0.f);
   tmem_issue16(tacc, a);
 #pragma unroll 1
-  for (int c = 0; c < 8; c += 2) {
+  for (int c = 0; c < D / 16; c += 2) {
     tmem_wait16(a); tmem_issue16(tacc + (c + 1) * 16, b);
     ssq2 = ssq_chunk<16>(a, ssq2);
-    tmem_wait16(b); tmem_issue16(tacc + ((c + 2) & 7) * 16, a);      // wraps to step 0 for the second sweep
+    tmem_wait16(b); tmem_issue16(tacc + ((c + 2) & (D / 16 - 1)) * 16, a);      // wraps to step 0 for the second sweep
     ssq2 = ssq_chunk<16>(b, ssq2);
   }
   float lo, hi;
@@ -349,51 +383,51 @@ __device__ __forceinline__ float ssq_row_fast(uint32_t tacc, uint32_t (&a)[16], 
   return lo + hi;   // step 0 is in flight into `a`
 }
 
-template <int BITS, bool LDS = false, bool LINEAR = false>
+template <int D, int BITS, bool LDS = false, bool LINEAR = false>
 __device__ __forceinline__ void quant_row_fast(uint32_t tacc, uint32_t (&a)[16], uint32_t (&b)[16], const Shortcut& sc,
                                                uint8_t* idx_row, bool valid, uint32_t thr_addr = 0u) {
   constexpr int BYTES = 16 / (8 / BITS);
   if constexpr (BYTES == 16) {                   // one-byte codes: 32 coordinates leave as one store
     const bool wide = (reinterpret_cast<uintptr_t>(idx_row) & 31u) == 0;
 #pragma unroll 1
-    for (int c = 0; c < 8; c += 2) {
+    for (int c = 0; c < D / 16; c += 2) {
       uint32_t wa[4], wb[4];
       tmem_wait16(a); tmem_issue16(tacc + (c + 1) * 16, b);
       quant_chunk_words<BITS, 16, LDS, LINEAR>(a, sc, thr_addr, wa);
       tmem_wait16(b);
-      if (c + 2 < 8) tmem_issue16(tacc + (c + 2) * 16, a);
+      if (c + 2 < D / 16) tmem_issue16(tacc + (c + 2) * 16, a);
       quant_chunk_words<BITS, 16, LDS, LINEAR>(b, sc, thr_addr, wb);
       if (valid) store_index_pair(idx_row + c * 16, wa, wb, wide);
     }
   } else if constexpr (BYTES == 8) {             // 3- and 4-bit codes: a round (32 coordinates) leaves as one 16-byte store
 #pragma unroll 1
-    for (int c = 0; c < 8; c += 2) {
+    for (int c = 0; c < D / 16; c += 2) {
       uint32_t wa[2], wb[2];
       tmem_wait16(a); tmem_issue16(tacc + (c + 1) * 16, b);
       quant_chunk_words<BITS, 16, LDS, LINEAR>(a, sc, thr_addr, wa);
       tmem_wait16(b);
-      if (c + 2 < 8) tmem_issue16(tacc + (c + 2) * 16, a);
+      if (c + 2 < D / 16) tmem_issue16(tacc + (c + 2) * 16, a);
       quant_chunk_words<BITS, 16, LDS, LINEAR>(b, sc, thr_addr, wb);
       if (valid) *reinterpret_cast<uint4*>(idx_row + c * 8) = make_uint4(wa[0], wa[1], wb[0], wb[1]);
     }
   } else if constexpr (BYTES == 4) {             // 2-bit codes: a round leaves as one 8-byte store
 #pragma unroll 1
-    for (int c = 0; c < 8; c += 2) {
+    for (int c = 0; c < D / 16; c += 2) {
       uint32_t wa[1], wb[1];
       tmem_wait16(a); tmem_issue16(tacc + (c + 1) * 16, b);
       quant_chunk_words<BITS, 16, LDS, LINEAR>(a, sc, thr_addr, wa);
       tmem_wait16(b);
-      if (c + 2 < 8) tmem_issue16(tacc + (c + 2) * 16, a);
+      if (c + 2 < D / 16) tmem_issue16(tacc + (c + 2) * 16, a);
       quant_chunk_words<BITS, 16, LDS, LINEAR>(b, sc, thr_addr, wb);
       if (valid) *reinterpret_cast<uint2*>(idx_row + c * 4) = make_uint2(wa[0], wb[0]);
     }
   } else {
 #pragma unroll 1
-    for (int c = 0; c < 8; c += 2) {
+    for (int c = 0; c < D / 16; c += 2) {
       tmem_wait16(a); tmem_issue16(tacc + (c + 1) * 16, b);
       quant_chunk_fast<BITS, 16, LDS, LINEAR>(a, sc, idx_row + c * BYTES, valid, thr_addr);
       tmem_wait16(b);
-      if (c + 2 < 8) tmem_issue16(tacc + (c + 2) * 16, a);
+      if (c + 2 < D / 16) tmem_issue16(tacc + (c + 2) * 16, a);
       quant_chunk_fast<BITS, 16, LDS, LINEAR>(b, sc, idx_row + (c + 1) * BYTES, valid, thr_addr);
     }
   }
@@ -424,16 +458,17 @@ __device__ __forceinline__ void quant_chunk_cells(const uint32_t (&raw)[16], con
   }
 }
 
+template <int D>
 __device__ __forceinline__ void quant_row_cells(uint32_t tacc, uint32_t (&a)[16], uint32_t (&b)[16], const Shortcut& sc,
                                                 uint32_t cells_lane, uint32_t thr_lane, uint8_t* idx_row, bool valid) {
   const bool wide = (reinterpret_cast<uintptr_t>(idx_row) & 31u) == 0;
 #pragma unroll 1
-  for (int c = 0; c < 8; c += 2) {
+  for (int c = 0; c < D / 16; c += 2) {
     uint32_t wa[4], wb[4];
     tmem_wait16(a); tmem_issue16(tacc + (c + 1) * 16, b);
     quant_chunk_cells(a, sc, cells_lane, thr_lane, wa);
     tmem_wait16(b);
-    if (c + 2 < 8) tmem_issue16(tacc + (c + 2) * 16, a);
+    if (c + 2 < D / 16) tmem_issue16(tacc + (c + 2) * 16, a);
     quant_chunk_cells(b, sc, cells_lane, thr_lane, wb);
     if (valid) store_index_pair(idx_row + c * 16, wa, wb, wide);
   }
@@ -441,13 +476,14 @@ __device__ __forceinline__ void quant_row_cells(uint32_t tacc, uint32_t (&a)[16]
 
 // Rest of a role's walk after one of its waits ran out: only the two named barriers of every job
 // change, so that the other warps of the group never wait for this one.  Out of line: cold.
-__device__ __noinline__ void walk_job_barriers(const UmmaQuantBatch& batch, int job_index, int t0, int i, int step,
+template <int D, int J>
+__device__ __noinline__ void walk_job_barriers(const UmmaQuantBatchOf<J>& batch, int job_index, int t0, int i, int step,
                                                int n_local, int bar_id, int threads) {
   QuantJobView job;
   job.j = job_index;
   job.end = (job_index + 1 < batch.n_jobs) ? batch.jobs[job_index + 1].tile_begin : batch.total_tiles;
   for (i += step; i < n_local; i += step)
-    if (view_advance(batch, t0 + i, job)) {
+    if (view_advance<D>(batch, t0 + i, job)) {
       asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(threads) : "memory");
       asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(threads) : "memory");
     }
@@ -455,9 +491,10 @@ __device__ __noinline__ void walk_job_barriers(const UmmaQuantBatch& batch, int 
 
 // WIDE: the launch holds a job with codes of 6 bits or more; the narrow instantiation carries none of
 // the wide-code paths (its epilogue loop is sensitive to code size).
-template <bool BF16, bool WIDE>
-__global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_constant__ UmmaQuantBatch batch) {
-  using C = Cfg<BF16, WIDE>;
+template <bool BF16, bool WIDE, int D, int J>
+__global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_constant__ UmmaQuantBatchOf<J> batch) {
+  static_assert(D == 128 || D == 64, "one or two vectors per accumulator row");
+  using C = Cfg<BF16, WIDE, D>;
   constexpr int kStages = C::kStages;
   constexpr int kPieces = C::kPieces;
   constexpr uint32_t kOffA = C::kOffA, kOffPi = C::kOffPi, kOffThr = C::kOffThr, kOffBar = C::kOffBar;
@@ -505,13 +542,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
       QuantJobView job;
       for (int i = 0; i < n_local && ok; ++i) {
         const int t = t0 + i;
-        if (view_advance(batch, t, job)) {
+        if (view_advance<D>(batch, t, job)) {
           if (pi_loads > 0) ok = mbar_wait(bar_pifree, (uint32_t)((pi_loads - 1) & 1), abort_flag);
           if (!ok) break;
-          mbar_arrive_expect_tx(bar_pifull, kPieces * kTileBytes);
+          mbar_arrive_expect_tx(bar_pifull, kPieces * C::kPieceBytes);
           const uint8_t* img = reinterpret_cast<const uint8_t*>(job.image) + C::kPieceOff;
 #pragma unroll
-          for (int p = 0; p < kPieces; ++p) bulk_load(pi_smem + p * kTileBytes, img + p * kTileBytes, kTileBytes, bar_pifull);
+          for (int p = 0; p < kPieces; ++p)
+            bulk_load(pi_smem + p * C::kPieceBytes, img + p * C::kPieceBytes, C::kPieceBytes, bar_pifull);
           ++pi_loads;
         }
         const int s = i % kStages;
@@ -522,7 +560,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
         }
         const int lt = t - job.begin;
         const int slab = lt / job.tps;
-        const int row0 = (lt - slab * job.tps) * kTileRows;
+        const int row0 = (lt - slab * job.tps) * kTileVecs<D>;
         const int bb = slab / job.H, hh = slab - bb * job.H;
         if (TQ_ABL(batch, 64)) {
           mbar_arrive(bar_full + 8 * s);
@@ -532,7 +570,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
         } else {
           mbar_arrive_expect_tx(bar_full + 8 * s, kTileBytes);
           tma_load_4d(a_smem + s * kTileBytes, job.tmap, 0, row0, hh, bb, bar_full + 8 * s);
-          tma_load_4d(a_smem + s * kTileBytes + kHalfBytes, job.tmap, 64, row0, hh, bb, bar_full + 8 * s);
+          // head_dim 64: the second box starts 128 vectors on, past the end of a short slab at worst (zero fill)
+          tma_load_4d(a_smem + s * kTileBytes + kHalfBytes, job.tmap, D == 128 ? 64 : 0, D == 128 ? row0 : row0 + kTileRows, hh,
+                      bb, bar_full + 8 * s);
         }
       }
       if (!ok) {
@@ -555,11 +595,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
       int pi_uses = 0;
       bool ok = true;
       QuantJobView job;
-      const uint32_t idesc = idesc_f16(BF16);
+      const uint32_t idesc = idesc_f16(BF16, D);
       const uint64_t b_base = smem_desc_sw128(pi_smem);
       for (int i = 0; i < n_local && ok; ++i) {
         const int t = t0 + i;
-        if (view_advance(batch, t, job)) {
+        if (view_advance<D>(batch, t, job)) {
           ok = mbar_wait(bar_pifull, (uint32_t)(pi_uses & 1), abort_flag);
           ++pi_uses;
         }
@@ -578,13 +618,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
         if (elect_one()) {
           if (!TQ_ABL(batch, 4)) {
 #pragma unroll
-            for (int piece = 0; piece < kPieces; ++piece) {
+            for (int h = 0; h < 128 / D; ++h) {        // head_dim 64: the two operands of a tile, 64 columns each
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                constexpr uint32_t kUnit = 16;
-                const uint64_t koff = (uint64_t)(((k >> 2) * kHalfBytes + (k & 3) * 32) / kUnit);
-                const uint64_t poff = (uint64_t)((piece * kTileBytes) / kUnit);
-                umma_f16(d_tmem, a_base + koff, b_base + poff + koff, idesc, (piece | k) != 0 ? 1u : 0u);
+              for (int piece = 0; piece < kPieces; ++piece) {
+#pragma unroll
+                for (int k = 0; k < D / 16; ++k) {
+                  constexpr uint32_t kUnit = 16;
+                  const uint64_t koff = (uint64_t)(((k >> 2) * kHalfBytes + (k & 3) * 32) / kUnit);
+                  const uint64_t hoff = (uint64_t)(h * kHalfBytes / kUnit);
+                  const uint64_t poff = (uint64_t)((piece * C::kPieceBytes) / kUnit);
+                  umma_f16(d_tmem + h * 64, a_base + hoff + koff, b_base + poff + koff, idesc, (piece | k) != 0 ? 1u : 0u);
+                }
               }
             }
           }
@@ -650,7 +694,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
     int i = wg;
     for (; i < n_local; i += 4) {
       const int t = t0 + i;
-      if (view_advance(batch, t, job)) {
+      if (view_advance<D>(batch, t, job)) {
         if constexpr (WIDE) {
           build_tables_up_to(job.j);
           mode = (int)__ldg(job.codebook + 512);
@@ -678,51 +722,61 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
       tc_fence_after();
       const int lt = t - job.begin;
       const int slab = lt / job.tps;
-      const int64_t s_row = (int64_t)(lt - slab * job.tps) * kTileRows + row;
-      const bool valid = s_row < job.S && !TQ_ABL(batch, 1);
-      const int64_t n = (int64_t)slab * job.S + s_row;
-      const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(wg * 128);
-      uint8_t* idx_row = job.idx_out + n * (int64_t)job.g;
-      if (!TQ_ABL(batch, 2)) {
-        uint32_t ra[16], rb[16];
-        float ssq;
-        if (TQ_ABL(batch, 512)) { ssq = 1.0f; tmem_issue16(tacc, ra); }
-        else ssq = ssq_row_fast(tacc, ra, rb);
-        const float norm = __fsqrt_rn(ssq);
-        const float inv = __fdiv_rn(1.0f, norm + 1e-8f);
-        if (valid) job.norms_out[n] = __half_as_ushort(__float2half_rn(norm));
-        sc.s_inv = sc.s * inv;
-        sc.h_inv = 1099511627776.0f * inv;            // 2^40: exact scaling
-        if (TQ_ABL(batch, 256)) {
-          tmem_wait16(ra);
-        } else if (WIDE && mode == 2) {
-          if constexpr (WIDE)
-            quant_row_cells(tacc, ra, rb, sc, base + C::kOffCells + (uint32_t)lane - 32u * 0x4B000000u,
-                            base + C::kOffThr + 4u * (uint32_t)lane, idx_row, valid);
-        } else if (WIDE && fast_lds) {
-          if constexpr (WIDE)
-            quant_row_fast<6, true>(tacc, ra, rb, sc, idx_row, valid, base + C::kOffThr + 4u * (uint32_t)lane - 128u * 0x4B000000u);
-        } else if (fast) {
-          switch (job.bits) {
-            case 1:
-              if (linear) quant_row_fast<1, false, true>(tacc, ra, rb, sc, idx_row, valid);
-              else quant_row_fast<1>(tacc, ra, rb, sc, idx_row, valid);
-              break;
-            case 2:
-              if (linear) quant_row_fast<2, false, true>(tacc, ra, rb, sc, idx_row, valid);
-              else quant_row_fast<2>(tacc, ra, rb, sc, idx_row, valid);
-              break;
-            case 3:
-              if (linear) quant_row_fast<3, false, true>(tacc, ra, rb, sc, idx_row, valid);
-              else quant_row_fast<3>(tacc, ra, rb, sc, idx_row, valid);
-              break;
-            case 4: quant_row_fast<4>(tacc, ra, rb, sc, idx_row, valid); break;
-            default: quant_row_fast<5>(tacc, ra, rb, sc, idx_row, valid); break;
+#pragma unroll 1
+      for (int h = 0; h < 128 / D; ++h) {          // head_dim 64: vectors `row` and `row + 128` of the tile
+        const int64_t s_row = (int64_t)(lt - slab * job.tps) * kTileVecs<D> + h * kTileRows + row;
+        const bool valid = s_row < job.S && !TQ_ABL(batch, 1);
+        const int64_t n = (int64_t)slab * job.S + s_row;
+        const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(wg * 128 + h * 64);
+        uint8_t* idx_row = job.idx_out + n * (int64_t)job.g;
+        if (!TQ_ABL(batch, 2)) {
+          uint32_t ra[16], rb[16];
+          float ssq;
+          if (TQ_ABL(batch, 512)) { ssq = 1.0f; tmem_issue16(tacc, ra); }
+          else ssq = ssq_row_fast<D>(tacc, ra, rb);
+          float norm = __fsqrt_rn(ssq);
+          if constexpr (D == 64) {
+            if (!(ssq == ssq) && valid) {
+              const UmmaQuantJob& full = batch.jobs[job.j];
+              const int bb = slab / job.H, hh = slab - bb * job.H;
+              norm = x_norm<BF16, D>(full.x + bb * full.xs_b + hh * full.xs_h + s_row * full.xs_s);
+            }
           }
-        } else {
-          tmem_wait16(ra);                       // the norm sweep left a load in flight
-          // wide launches have no plain threshold table in shared memory: the search reads the codebook block
-          quant_row_search(job.bits, tacc, inv, WIDE ? job.codebook + kThresholdOff : thr, idx_row, valid);
+          const float inv = __fdiv_rn(1.0f, norm + 1e-8f);
+          if (valid) job.norms_out[n] = __half_as_ushort(__float2half_rn(norm));
+          sc.s_inv = sc.s * inv;
+          sc.h_inv = 1099511627776.0f * inv;            // 2^40: exact scaling
+          if (TQ_ABL(batch, 256)) {
+            tmem_wait16(ra);
+          } else if (WIDE && mode == 2) {
+            if constexpr (WIDE)
+              quant_row_cells<D>(tacc, ra, rb, sc, base + C::kOffCells + (uint32_t)lane - 32u * 0x4B000000u,
+                              base + C::kOffThr + 4u * (uint32_t)lane, idx_row, valid);
+          } else if (WIDE && fast_lds) {
+            if constexpr (WIDE)
+              quant_row_fast<D, 6, true>(tacc, ra, rb, sc, idx_row, valid, base + C::kOffThr + 4u * (uint32_t)lane - 128u * 0x4B000000u);
+          } else if (fast) {
+            switch (job.bits) {
+              case 1:
+                if (linear) quant_row_fast<D, 1, false, true>(tacc, ra, rb, sc, idx_row, valid);
+                else quant_row_fast<D, 1>(tacc, ra, rb, sc, idx_row, valid);
+                break;
+              case 2:
+                if (linear) quant_row_fast<D, 2, false, true>(tacc, ra, rb, sc, idx_row, valid);
+                else quant_row_fast<D, 2>(tacc, ra, rb, sc, idx_row, valid);
+                break;
+              case 3:
+                if (linear) quant_row_fast<D, 3, false, true>(tacc, ra, rb, sc, idx_row, valid);
+                else quant_row_fast<D, 3>(tacc, ra, rb, sc, idx_row, valid);
+                break;
+              case 4: quant_row_fast<D, 4>(tacc, ra, rb, sc, idx_row, valid); break;
+              default: quant_row_fast<D, 5>(tacc, ra, rb, sc, idx_row, valid); break;
+            }
+          } else {
+            tmem_wait16(ra);                       // the norm sweep left a load in flight
+            // wide launches have no plain threshold table in shared memory: the search reads the codebook block
+            quant_row_search<D>(job.bits, tacc, inv, WIDE ? job.codebook + kThresholdOff : thr, idx_row, valid);
+          }
         }
       }
       tc_fence_before();
@@ -736,7 +790,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
     if constexpr (WIDE) {
       build_tables_up_to(last_job);              // the rest of the CTA's job sequence: barriers for the others
     } else {
-      if (!ok) walk_job_barriers(batch, job.j, t0, i, 4, n_local, wg + 1, 128);
+      if (!ok) walk_job_barriers<D>(batch, job.j, t0, i, 4, n_local, wg + 1, 128);
     }
   }
   tc_fence_before();
@@ -772,15 +826,17 @@ struct alignas(64) UmmaDeqJob {
   int32_t pad_;
 };
 constexpr int kMaxDeqJobs = 96;
-struct UmmaDeqBatch {
+template <int J>
+struct UmmaDeqBatchOf {
   int32_t n_jobs;
   int32_t total_tiles;
   int32_t* status;
   int32_t ablate;            // -DTQ_ABLATION builds only (TQ_ABLATE): 1 skip stores, 2 skip expansion, 4 skip MMA, 8 skip the drain arithmetic
   int32_t pad_[3];
   int32_t cta_begin[kMaxCtas + 1];   // tiles [cta_begin[c], cta_begin[c + 1]) belong to CTA c (equal estimated cost)
-  UmmaDeqJob jobs[kMaxDeqJobs];
+  UmmaDeqJob jobs[J];
 };
+using UmmaDeqBatch = UmmaDeqBatchOf<kMaxDeqJobs>;
 static_assert(sizeof(UmmaDeqBatch) < 32000, "kernel parameter space");
 
 // Decoupled pipeline: producer (bulk copies of packed tiles) -> 8 expander warps (packed
@@ -789,23 +845,26 @@ static_assert(sizeof(UmmaDeqBatch) < 32000, "kernel parameter space");
 // load latency, expansion, tensor work and stores all overlap across tiles.
 // NARROW: every job of the launch has codes of at most 4 bits, so a packed tile is at most
 // 8 KB; the space saved buys a deeper packed ring and a third operand stage.
-template <bool OUT32, bool NARROW>
+// ROWS: three passes over two centroid pieces and row stores straight from the accumulators: fp32 outputs, and every
+// output at head_dim 64, where a 16-bit row is one full 128-byte line.
+template <bool ROWS, bool NARROW, int D = kDim>
 struct DCfg {
-  static constexpr int kPk = NARROW ? 4 : (OUT32 ? 2 : 3); // packed-tile ring
-  static constexpr int kNA = (NARROW && !OUT32) ? 3 : 2;   // operand ring
+  static constexpr int kPk = NARROW ? 4 : (ROWS ? 2 : 3); // packed-tile ring
+  static constexpr int kNA = (NARROW && !ROWS) ? 3 : 2;   // operand ring
   static constexpr int kNT = 4;                            // TMEM accumulators
-  static constexpr int kPiecesA = OUT32 ? 2 : 1;
-  static constexpr int kPiecesB = OUT32 ? 2 : 1;
+  static constexpr int kPiecesA = ROWS ? 2 : 1;
+  static constexpr int kPiecesB = ROWS ? 2 : 1;
+  static constexpr uint32_t kPieceBytes = kImagePiece<D>;
   static constexpr int kExpWarps = 8, kDrainWarps = 8;
   static constexpr int kThreadsD = 64 + 32 * (kExpWarps + kDrainWarps);     // 576
-  static constexpr uint32_t kPkBytes = NARROW ? 8192 : 16384;   // 128 rows x up to 64 / 128 packed bytes
+  static constexpr uint32_t kPkBytes = NARROW ? 8192 : 16384;   // 16384 coordinates of a tile: up to 64 / 128 packed bytes per 128
   static constexpr uint32_t kOffA = 0;
   static constexpr uint32_t kOffPi = kOffA + kNA * kPiecesA * kTileBytes;
-  static constexpr uint32_t kOffPk = kOffPi + kPiecesB * kTileBytes;
+  static constexpr uint32_t kOffPk = kOffPi + kPiecesB * kPieceBytes;
   static constexpr uint32_t kOffStage = kOffPk + kPk * kPkBytes;           // 16-bit outputs: one tile per drain group
   // 16-bit outputs of wide codes: replicated look-up table (see expand_half_wide16), 16 KB
-  static constexpr bool kWide16 = !OUT32 && !NARROW;
-  static constexpr uint32_t kOffLut16 = kOffStage + (OUT32 ? 0u : 2u * kTileBytes);
+  static constexpr bool kWide16 = !ROWS && !NARROW;
+  static constexpr uint32_t kOffLut16 = kOffStage + (ROWS ? 0u : 2u * kTileBytes);
   static constexpr uint32_t kOffBar = kOffLut16 + (kWide16 ? 16384u : 0u);
   static constexpr uint32_t kSmemBytes = kOffBar + 256 + 1024;
 };
@@ -826,7 +885,8 @@ struct DeqJobView {
   void* out = nullptr;
   const CUtensorMap* out_map = nullptr;
 };
-__device__ __forceinline__ bool view_advance(const UmmaDeqBatch& b, int tile, DeqJobView& v) {
+template <int D, int J>
+__device__ __forceinline__ bool view_advance(const UmmaDeqBatchOf<J>& b, int tile, DeqJobView& v) {
   if (v.j >= 0 && tile < v.end) return false;
   int j = v.j < 0 ? 0 : v.j;
   while (j + 1 < b.n_jobs && tile >= b.jobs[j + 1].tile_begin) ++j;
@@ -837,7 +897,7 @@ __device__ __forceinline__ bool view_advance(const UmmaDeqBatch& b, int tile, De
   v.tps = job.tiles_per_slab;
   v.H = job.H;
   v.bits = job.bits;
-  v.g = kDim / (8 / job.bits);
+  v.g = D / (8 / job.bits);
   v.out_dtype = job.out_dtype;
   v.S = job.S; v.os_b = job.os_b; v.os_h = job.os_h; v.os_s = job.os_s;
   v.idx = job.idx;
@@ -853,18 +913,18 @@ __device__ __forceinline__ bool view_advance(const UmmaDeqBatch& b, int tile, De
 
 // The TMEM load is warp-collective: every lane of the warp must come through here, rows
 // past the end of a slab included; `valid` only guards the stores.
-template <int ODT>
+template <int ODT, int D>
 __device__ __forceinline__ void drain_row(uint32_t tacc, float nv, void* out_row, bool valid) {
   uint32_t a[16], b[16];
   tmem_issue16(tacc, a);
 #pragma unroll 1
-  for (int c = 0; c < 8; c += 2) {
+  for (int c = 0; c < D / 16; c += 2) {
 #pragma unroll
     for (int hb = 0; hb < 2; ++hb) {
       uint32_t (&cur)[16] = hb ? b : a;
       uint32_t (&nxt)[16] = hb ? a : b;
       tmem_wait16(cur);
-      if (c + hb + 1 < 8) tmem_issue16(tacc + (c + hb + 1) * 16, nxt);
+      if (c + hb + 1 < D / 16) tmem_issue16(tacc + (c + hb + 1) * 16, nxt);
       if (valid) {
         float v[16];
 #pragma unroll
@@ -935,9 +995,10 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t sr
                : "memory");
 }
 
-template <bool OUT32, bool NARROW>
-__global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequantize(const __grid_constant__ UmmaDeqBatch batch) {
-  using C = DCfg<OUT32, NARROW>;
+template <bool ROWS, bool NARROW, int D, int J>
+__global__ void __launch_bounds__(DCfg<ROWS, NARROW, D>::kThreadsD, 1) k_umma_dequantize(const __grid_constant__ UmmaDeqBatchOf<J> batch) {
+  static_assert(D == 128 || (D == 64 && ROWS), "head_dim 64 has no staged form");
+  using C = DCfg<ROWS, NARROW, D>;
   constexpr int kPk = C::kPk, kNA = C::kNA, kNT = C::kNT;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -986,13 +1047,14 @@ __global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequ
       DeqJobView job;
       for (int i = 0; i < n_local && ok; ++i) {
         const int t = t0 + i;
-        if (view_advance(batch, t, job)) {
+        if (view_advance<D>(batch, t, job)) {
           if (pi_loads > 0) ok = mbar_wait(bar_pifree, (uint32_t)((pi_loads - 1) & 1), abort_flag);
           if (!ok) break;
-          mbar_arrive_expect_tx(bar_pifull, C::kPiecesB * kTileBytes);
+          mbar_arrive_expect_tx(bar_pifull, C::kPiecesB * C::kPieceBytes);
           const uint8_t* img = reinterpret_cast<const uint8_t*>(job.image);
 #pragma unroll
-          for (int p = 0; p < C::kPiecesB; ++p) bulk_load(pi_smem + p * kTileBytes, img + p * kTileBytes, kTileBytes, bar_pifull);
+          for (int p = 0; p < C::kPiecesB; ++p)
+            bulk_load(pi_smem + p * C::kPieceBytes, img + p * C::kPieceBytes, C::kPieceBytes, bar_pifull);
           ++pi_loads;
         }
         const int s = i % kPk;
@@ -1000,8 +1062,8 @@ __global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequ
         if (!ok) break;
         const int lt = t - job.begin;
         const int slab = lt / job.tps;
-        const int64_t s0 = (int64_t)(lt - slab * job.tps) * kTileRows;
-        const int64_t rows = (job.S - s0) < kTileRows ? (job.S - s0) : kTileRows;
+        const int64_t s0 = (int64_t)(lt - slab * job.tps) * kTileVecs<D>;
+        const int64_t rows = (job.S - s0) < kTileVecs<D> ? (job.S - s0) : kTileVecs<D>;
         const int g = job.g;
         const uint32_t bytes = (uint32_t)(rows * g);
         mbar_arrive_expect_tx(bar_pkfull + 8 * s, bytes);
@@ -1023,11 +1085,11 @@ __global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequ
     if (lane == 0) {
       int pi_uses = 0;
       bool ok = true;
-      const uint32_t idesc = idesc_f16(false);
+      const uint32_t idesc = idesc_f16(false, D);
       DeqJobView job;
       for (int i = 0; i < n_local && ok; ++i) {
         const int t = t0 + i;
-        if (view_advance(batch, t, job)) {
+        if (view_advance<D>(batch, t, job)) {
           ok = mbar_wait(bar_pifull, (uint32_t)(pi_uses & 1), abort_flag);
           if (!ok) break;
           ++pi_uses;
@@ -1041,17 +1103,21 @@ __global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequ
         const uint32_t d_tmem = tmem_base + (uint32_t)(b * 128);
         const uint64_t a_base = smem_desc_sw128(a_smem + a * C::kPiecesA * kTileBytes);
         const uint64_t b_base = smem_desc_sw128(pi_smem);
-        constexpr int kPasses = OUT32 ? 3 : 1;      // hi.hi [, lo.hi, hi.lo]
+        constexpr int kPasses = ROWS ? 3 : 1;      // hi.hi [, lo.hi, hi.lo]
         if (!TQ_ABL(batch, 4)) {
 #pragma unroll
-          for (int pass = 0; pass < kPasses; ++pass) {
+          for (int h = 0; h < 128 / D; ++h) {          // head_dim 64: the two operands of a tile, 64 columns each
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              // descriptor = per-tile base + compile-time offset in 16-byte units
-              const uint64_t koff = (uint64_t)(((k >> 2) * kHalfBytes + (k & 3) * 32) / 16);
-              const uint64_t pa = (uint64_t)(((pass == 1) ? kTileBytes : 0u) / 16);
-              const uint64_t pb = (uint64_t)(((pass == 2) ? kTileBytes : 0u) / 16);
-              umma_f16(d_tmem, a_base + pa + koff, b_base + pb + koff, idesc, (pass | k) != 0 ? 1u : 0u);
+            for (int pass = 0; pass < kPasses; ++pass) {
+#pragma unroll
+              for (int k = 0; k < D / 16; ++k) {
+                // descriptor = per-tile base + compile-time offset in 16-byte units
+                const uint64_t koff = (uint64_t)(((k >> 2) * kHalfBytes + (k & 3) * 32) / 16);
+                const uint64_t hoff = (uint64_t)(h * kHalfBytes / 16);
+                const uint64_t pa = (uint64_t)(((pass == 1) ? kTileBytes : 0u) / 16);
+                const uint64_t pb = (uint64_t)(((pass == 2) ? C::kPieceBytes : 0u) / 16);
+                umma_f16(d_tmem + h * 64, a_base + hoff + pa + koff, b_base + pb + koff, idesc, (pass | k) != 0 ? 1u : 0u);
+              }
             }
           }
         }
@@ -1077,7 +1143,7 @@ __global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequ
     int i = 0;
     for (; i < n_local; ++i) {
       const int t = t0 + i;
-      if (view_advance(batch, t, job)) {
+      if (view_advance<D>(batch, t, job)) {
         asm volatile("bar.sync 1, 256;" ::: "memory");       // everyone is past the previous tile's look-ups
         const float c = __ldg(job.codebook + kCentroidOff + et);
         const __half h = __float2half_rn(c);
@@ -1109,10 +1175,12 @@ __global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequ
       if (!ok) break;
       const int lt = t - job.begin;
       const int slab = lt / job.tps;
-      const int64_t s_row = (int64_t)(lt - slab * job.tps) * kTileRows + row;
+      // `half` is a k-half of the vector `row` (head_dim 128) or one of the vectors `row` and `row + 128` (head_dim 64):
+      // 64 coordinates and the same 128-byte operand row either way
+      const int64_t s_row = (int64_t)(lt - slab * job.tps) * kTileVecs<D> + (D == 128 ? 0 : half * kTileRows) + row;
       if (s_row < job.S && !TQ_ABL(batch, 2)) {
         const int g = job.g;
-        const uint32_t src = pk_smem + s * C::kPkBytes + (uint32_t)(row * g + half * (g >> 1));
+        const uint32_t src = pk_smem + s * C::kPkBytes + (uint32_t)(D == 128 ? row * g + half * (g >> 1) : (half * kTileRows + row) * g);
         const uint32_t a_stage = a_smem + a * C::kPiecesA * kTileBytes;
         switch (job.bits) {
           case 1: expand_half<1, C::kPiecesA>(src, lut, a_stage, row, half); break;
@@ -1147,7 +1215,7 @@ __global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequ
         if (batch.status != nullptr) atomicCAS(batch.status, 0, (6 << 16) | (int)blockIdx.x);
       }
       for (++i; i < n_local; ++i)
-        if (view_advance(batch, t0 + i, job)) {
+        if (view_advance<D>(batch, t0 + i, job)) {
           asm volatile("bar.sync 1, 256;" ::: "memory");
           asm volatile("bar.sync 1, 256;" ::: "memory");
         }
@@ -1166,23 +1234,32 @@ __global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequ
     int i = wg;
     for (; i < n_local; i += 2) {
       const int t = t0 + i;
-      view_advance(batch, t, job);
+      view_advance<D>(batch, t, job);
       const int lt = t - job.begin;
       const int slab = lt / job.tps;
-      const int s0 = (lt - slab * job.tps) * kTileRows;
+      const int s0 = (lt - slab * job.tps) * kTileVecs<D>;
       const int64_t s_row = (int64_t)s0 + row;
       const bool valid = s_row < job.S;
       const int64_t n = (int64_t)slab * job.S + s_row;
       const float nv = valid ? __half2float(__ushort_as_half(__ldg(job.norms + n))) : 0.f;   // in flight during the wait
+      const bool valid2 = D == 64 && s_row + kTileRows < job.S;                               // head_dim 64: the second vector
+      const float nv2 = valid2 ? __half2float(__ushort_as_half(__ldg(job.norms + n + kTileRows))) : 0.f;
       const int bb = slab / job.H, hh = slab - bb * job.H;
       const int b = i % kNT;
       ok = __all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * b, (uint32_t)((i / kNT) & 1), abort_flag));
       if (!ok) break;
       tc_fence_after();
       const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * 128);
-      if constexpr (OUT32) {
+      if constexpr (ROWS) {
         const int64_t off = (int64_t)bb * job.os_b + (int64_t)hh * job.os_h + s_row * job.os_s;
-        drain_row<TQ_F32>(tacc, nv, reinterpret_cast<float*>(job.out) + off, valid);
+        auto drain = [&](auto odt, auto* out) {
+          constexpr int ODT = decltype(odt)::value;
+          drain_row<ODT, D>(tacc, nv, out + off, valid);
+          if constexpr (D == 64) drain_row<ODT, D>(tacc + 64, nv2, out + off + kTileRows * job.os_s, valid2);
+        };
+        if (D == 128 || job.out_dtype == TQ_F32) drain(std::integral_constant<int, TQ_F32>{}, reinterpret_cast<float*>(job.out));
+        else if (job.out_dtype == TQ_F16) drain(std::integral_constant<int, TQ_F16>{}, reinterpret_cast<uint16_t*>(job.out));
+        else drain(std::integral_constant<int, TQ_BF16>{}, reinterpret_cast<uint16_t*>(job.out));
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_tempty + 8 * b);
@@ -1206,14 +1283,14 @@ __global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequ
         }
       }
     }
-    if constexpr (!OUT32) {
+    if constexpr (!ROWS) {
       if (!ok)                                     // keep the group's two barriers per tile complete
         for (; i < n_local; i += 2) {
           asm volatile("bar.sync %0, 128;" ::"r"(wg + 2) : "memory");
           bar_red_and(wg + 2, 128, false);
         }
     }
-    if constexpr (!OUT32) {
+    if constexpr (!ROWS) {
       if (wg_tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // all stores done before exit
     }
     if (!ok && lane == 0) {
@@ -1232,10 +1309,10 @@ __global__ void __launch_bounds__(DCfg<OUT32, NARROW>::kThreadsD, 1) k_umma_dequ
 // ---------------------------------------------------------------- rotation image
 // image[piece][khalf][row n][64 cols], rows of 128 bytes, 16-byte chunk c stored at c ^ (n & 7).
 // Pieces 0-1: fp16 hi / lo (m = hi + lo, lo in fp16 subnormals).  Pieces 2-4: bf16 p0 + p1 + p2.
-__global__ void k_rotation_image(const float* __restrict__ m, uint16_t* __restrict__ image) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;     // over 128 x 128
-  if (idx >= kDim * kDim) return;
-  const int n = idx / kDim, k = idx % kDim;
+__global__ void k_rotation_image(const float* __restrict__ m, int D, uint16_t* __restrict__ image) {
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;     // over D x D
+  if (idx >= D * D) return;
+  const int n = idx / D, k = idx % D;
   const float v = m[idx];
   const __half hi = __float2half_rn(v);
   const __half lo = __float2half_rn(v - __half2float(hi));
@@ -1245,8 +1322,8 @@ __global__ void k_rotation_image(const float* __restrict__ m, uint16_t* __restri
   const __nv_bfloat16 p2 = __float2bfloat16_rn(r1 - __bfloat162float(p1));
   const int khalf = k >> 6, kk = k & 63;
   const int chunk = (kk >> 3) ^ (n & 7);
-  const int off = khalf * (kTileRows * 64) + n * 64 + chunk * 8 + (kk & 7);
-  const int piece = kTileRows * kDim;
+  const int off = khalf * (D * 64) + n * 64 + chunk * 8 + (kk & 7);
+  const int piece = D * D;
   image[off] = __half_as_ushort(hi);
   image[piece + off] = __half_as_ushort(lo);
   image[2 * piece + off] = __bfloat16_as_ushort(p0);
@@ -1328,11 +1405,14 @@ TensorMapEncodeFn tensor_map_encoder() {
   return reinterpret_cast<TensorMapEncodeFn>(p);
 }
 
-size_t umma_rotation_image_bytes(int D) { return D == kDim ? (size_t)kImageBytes : 0; }
+static bool tc_dim(int D) { return D == 128 || D == 64; }
+
+// fp16 hi, lo; then bf16 p0, p1, p2
+size_t umma_rotation_image_bytes(int D) { return tc_dim(D) ? (size_t)5 * D * D * 2 : 0; }
 
 int umma_prepare_rotation_image(const float* m, int D, void* image, cudaStream_t st) {
-  if (D != kDim) return TQ_EDIM;
-  k_rotation_image<<<(kDim * kDim + 255) / 256, 256, 0, st>>>(m, reinterpret_cast<uint16_t*>(image));
+  if (!tc_dim(D)) return TQ_EDIM;
+  k_rotation_image<<<(D * D + 255) / 256, 256, 0, st>>>(m, D, reinterpret_cast<uint16_t*>(image));
   return check_launch();
 }
 
@@ -1366,18 +1446,30 @@ static LaunchSlot<Batch>& pick_slot(LaunchSlot<Batch> (&slots)[kLaunchSlots], un
   return slots[victim];
 }
 
+// Launches `kern` with the first sizeof(P) bytes of the launch description.
+template <typename P, typename Batch, typename K>
+static int launch_prefix(K kern, const Batch& batch, int grid, int threads, uint32_t smem, bool set_attr, cudaStream_t st) {
+  if (set_attr) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
+  }
+  static_assert(sizeof(P) <= sizeof(Batch) && offsetof(P, jobs) == offsetof(Batch, jobs), "a prefix");
+  kern<<<grid, threads, smem, st>>>(reinterpret_cast<const P&>(batch));
+  return TQ_OK;
+}
+
 bool umma_quantize_eligible(const TqQuantizeJob& j) {
   if (force_simt()) return false;
-  if (j.rotation_image == nullptr || j.D != kDim || j.normalize != 1 || j.idx_mode != TQ_IDX_PACKED) return false;
+  if (j.rotation_image == nullptr || !tc_dim(j.D) || j.normalize != 1 || j.idx_mode != TQ_IDX_PACKED) return false;
   if (j.x_dtype != TQ_F16 && j.x_dtype != TQ_BF16) return false;
   if (j.B <= 0 || j.H <= 0 || j.S <= 0) return false;
   if (j.B > 65535 || j.H > 65535 || j.S > (int64_t)1 << 30) return false;
   if (((uintptr_t)j.x & 15u) || ((uintptr_t)j.idx_out & 15u) || ((uintptr_t)j.rotation_image & 15u)) return false;
-  if ((j.S > 1 && (j.stride_s % 8 != 0 || j.stride_s < kDim)) || (j.H > 1 && j.stride_h % 8 != 0) ||
+  if ((j.S > 1 && (j.stride_s % 8 != 0 || j.stride_s < j.D)) || (j.H > 1 && j.stride_h % 8 != 0) ||
       (j.B > 1 && j.stride_b % 8 != 0))
     return false;
   if (j.stride_s < 0 || j.stride_h < 0 || j.stride_b < 0) return false;
-  const int64_t tiles = j.B * j.H * ((j.S + kTileRows - 1) / kTileRows);
+  const int64_t tiles = j.B * j.H * ((j.S + tile_vecs_of(j.D) - 1) / tile_vecs_of(j.D));
   return tiles < ((int64_t)1 << 30);
 }
 
@@ -1400,6 +1492,7 @@ int umma_quantize(const TqQuantizeJob* jobs, int n_jobs, cudaStream_t st) {
   int& last_ablate = slot.ablate;
   int& last_grid = slot.grid;
   last_dev = -1;                                 // invalid until this call has rebuilt or reused the batch
+  const int D = jobs[0].D;
   int done = 0;
   while (done < n_jobs) {
     const int take = (n_jobs - done) < kMaxJobs ? (n_jobs - done) : kMaxJobs;
@@ -1409,14 +1502,14 @@ int umma_quantize(const TqQuantizeJob* jobs, int n_jobs, cudaStream_t st) {
     for (int i = 0; i < take && !reuse; ++i) {
       const TqQuantizeJob& j = jobs[done + i];
       UmmaQuantJob& u = batch.jobs[i];
-      const int64_t tps = (j.S + kTileRows - 1) / kTileRows;
+      const int64_t tps = (j.S + tile_vecs_of(D) - 1) / tile_vecs_of(D);
       job_tiles[i] = tps * j.B * j.H;
       job_weight[i] = quantize_tile_weight(j.bits, j.x_dtype == TQ_BF16);
       // size-1 dimensions get a harmless stride; TMA wants multiples of 16 bytes
-      const int64_t ss = j.S > 1 ? j.stride_s : kDim;
+      const int64_t ss = j.S > 1 ? j.stride_s : D;
       const int64_t sh = j.H > 1 ? j.stride_h : ss * j.S;
       const int64_t sb = j.B > 1 ? j.stride_b : (sh > ss ? sh : ss) * (j.H > 1 ? j.H : j.S);
-      cuuint64_t dims[4] = {(cuuint64_t)kDim, (cuuint64_t)j.S, (cuuint64_t)j.H, (cuuint64_t)j.B};
+      cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)j.S, (cuuint64_t)j.H, (cuuint64_t)j.B};
       cuuint64_t strides[3] = {(cuuint64_t)ss * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
       cuuint32_t box[4] = {64, (cuuint32_t)kTileRows, 1, 1};
       cuuint32_t estr[4] = {1, 1, 1, 1};
@@ -1428,6 +1521,8 @@ int umma_quantize(const TqQuantizeJob* jobs, int n_jobs, cudaStream_t st) {
       u.codebook = j.codebook;
       u.idx_out = reinterpret_cast<uint8_t*>(j.idx_out);
       u.norms_out = j.norms_out;
+      u.x = reinterpret_cast<const uint16_t*>(j.x);
+      u.xs_b = j.stride_b; u.xs_h = j.stride_h; u.xs_s = j.stride_s;
       u.S = j.S;
       u.H = (int32_t)j.H;
       u.tiles_per_slab = (int32_t)tps;
@@ -1442,8 +1537,6 @@ int umma_quantize(const TqQuantizeJob* jobs, int n_jobs, cudaStream_t st) {
     const bool bf16 = jobs[done].x_dtype == TQ_BF16;
     bool wide = false;
     for (int i = 0; i < take; ++i) wide = wide || jobs[done + i].bits > 5;
-    const uint32_t smem = bf16 ? (wide ? Cfg<true, true>::kSmemBytes : Cfg<true, false>::kSmemBytes)
-                               : (wide ? Cfg<false, true>::kSmemBytes : Cfg<false, false>::kSmemBytes);
     if (!reuse) {
       batch.n_jobs = take;
       batch.total_tiles = (int32_t)tile_cursor;
@@ -1457,19 +1550,20 @@ int umma_quantize(const TqQuantizeJob* jobs, int n_jobs, cudaStream_t st) {
       grid = (int)(tile_cursor < sms ? tile_cursor : sms);
       partition_tiles(job_tiles, job_weight, take, grid, batch.cta_begin);
     }
-    auto launch = [&](auto kern) -> int {
-      if (!reuse) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
-      }
-      kern<<<grid, kThreads, smem, st>>>(batch);
-      return TQ_OK;
+    auto launch_dim = [&](auto few, auto many, uint32_t smem) -> int {
+      if (take <= kFewJobs) return launch_prefix<UmmaQuantBatchOf<kFewJobs>>(few, batch, grid, kThreads, smem, !reuse, st);
+      return launch_prefix<UmmaQuantBatch>(many, batch, grid, kThreads, smem, !reuse, st);
+    };
+    auto launch = [&](auto b, auto w) -> int {
+      constexpr bool B16 = decltype(b)::value, W = decltype(w)::value;
+      if (D == 64) return launch_dim(k_umma_quantize<B16, W, 64, kFewJobs>, k_umma_quantize<B16, W, 64, kMaxJobs>, Cfg<B16, W, 64>::kSmemBytes);
+      return launch_dim(k_umma_quantize<B16, W, 128, kFewJobs>, k_umma_quantize<B16, W, 128, kMaxJobs>, Cfg<B16, W, 128>::kSmemBytes);
     };
     int lrc;
-    if (bf16 && wide) lrc = launch(k_umma_quantize<true, true>);
-    else if (bf16) lrc = launch(k_umma_quantize<true, false>);
-    else if (wide) lrc = launch(k_umma_quantize<false, true>);
-    else lrc = launch(k_umma_quantize<false, false>);
+    if (bf16 && wide) lrc = launch(std::true_type{}, std::true_type{});
+    else if (bf16) lrc = launch(std::true_type{}, std::false_type{});
+    else if (wide) lrc = launch(std::false_type{}, std::true_type{});
+    else lrc = launch(std::false_type{}, std::false_type{});
     if (lrc != TQ_OK) return lrc;
     int rc = check_launch();
     if (rc != TQ_OK) return rc;
@@ -1486,14 +1580,15 @@ int umma_quantize(const TqQuantizeJob* jobs, int n_jobs, cudaStream_t st) {
 
 bool umma_dequantize_eligible(const TqDequantizeJob& j) {
   if (force_simt()) return false;
-  if (j.rotation_image == nullptr || j.D != kDim || j.idx_mode != TQ_IDX_PACKED || j.norms == nullptr) return false;
+  if (j.rotation_image == nullptr || !tc_dim(j.D) || j.idx_mode != TQ_IDX_PACKED || j.norms == nullptr) return false;
+  if (j.D == 64 && j.bits == 1) return false;          // 8-byte rows: a bulk copy moves multiples of 16 bytes
   if (j.B <= 0 || j.H <= 0 || j.S <= 0) return false;
   if (((uintptr_t)j.idx & 15u) || ((uintptr_t)j.out & 15u) || ((uintptr_t)j.rotation_image & 15u)) return false;
   const int64_t q = j.out_dtype == TQ_F32 ? 4 : 8;     // elements per 16 bytes
   if (j.ostride_s % q != 0 || j.ostride_h % q != 0 || j.ostride_b % q != 0) return false;
   if (j.ostride_s < 0 || j.ostride_h < 0 || j.ostride_b < 0) return false;
-  if (j.out_dtype != TQ_F32 && (j.B > 65535 || j.H > 65535 || (j.S > 1 && j.ostride_s < kDim))) return false;
-  const int64_t tiles = j.B * j.H * ((j.S + kTileRows - 1) / kTileRows);
+  if (j.out_dtype != TQ_F32 && (j.B > 65535 || j.H > 65535 || (j.S > 1 && j.ostride_s < j.D))) return false;
+  const int64_t tiles = j.B * j.H * ((j.S + tile_vecs_of(j.D) - 1) / tile_vecs_of(j.D));
   return tiles < ((int64_t)1 << 30);
 }
 
@@ -1515,6 +1610,7 @@ int umma_dequantize(const TqDequantizeJob* jobs, int n_jobs, cudaStream_t st) {
   int& last_ablate = slot.ablate;
   int& last_grid = slot.grid;
   last_dev = -1;
+  const int D = jobs[0].D;
   int done = 0;
   while (done < n_jobs) {
     const int take = (n_jobs - done) < kMaxDeqJobs ? (n_jobs - done) : kMaxDeqJobs;
@@ -1524,14 +1620,14 @@ int umma_dequantize(const TqDequantizeJob* jobs, int n_jobs, cudaStream_t st) {
     for (int i = 0; i < take && !reuse; ++i) {
       const TqDequantizeJob& j = jobs[done + i];
       UmmaDeqJob& u = batch.jobs[i];
-      const int64_t tps = (j.S + kTileRows - 1) / kTileRows;
+      const int64_t tps = (j.S + tile_vecs_of(D) - 1) / tile_vecs_of(D);
       job_tiles[i] = tps * j.B * j.H;
       job_weight[i] = dequantize_tile_weight(j.bits, j.out_dtype == TQ_F32);
-      if (j.out_dtype != TQ_F32) {
-        const int64_t ss = j.S > 1 ? j.ostride_s : kDim;
+      if (j.out_dtype != TQ_F32 && D == 128) {
+        const int64_t ss = j.S > 1 ? j.ostride_s : D;
         const int64_t sh = j.H > 1 ? j.ostride_h : ss * j.S;
         const int64_t sb = j.B > 1 ? j.ostride_b : (sh > ss ? sh : ss) * (j.H > 1 ? j.H : j.S);
-        cuuint64_t dims[4] = {(cuuint64_t)kDim, (cuuint64_t)j.S, (cuuint64_t)j.H, (cuuint64_t)j.B};
+        cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)j.S, (cuuint64_t)j.H, (cuuint64_t)j.B};
         cuuint64_t strides[3] = {(cuuint64_t)ss * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
         cuuint32_t box[4] = {64, (cuuint32_t)kTileRows, 1, 1};
         cuuint32_t estr[4] = {1, 1, 1, 1};
@@ -1573,19 +1669,22 @@ int umma_dequantize(const TqDequantizeJob* jobs, int n_jobs, cudaStream_t st) {
     const bool out32 = jobs[done].out_dtype == TQ_F32;
     bool narrow = true;
     for (int i = 0; i < take; ++i) narrow = narrow && jobs[done + i].bits <= 4;
-    auto launch = [&](auto kern, uint32_t smem, int threads) -> int {
-      if (!reuse) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
-      }
-      kern<<<grid, threads, smem, st>>>(batch);
-      return TQ_OK;
+    auto launch = [&](auto rows, auto nar, auto dim) -> int {
+      constexpr bool R = decltype(rows)::value, NW = decltype(nar)::value;
+      constexpr int DD = decltype(dim)::value;
+      using C = DCfg<R, NW, DD>;
+      if (take <= kFewJobs)
+        return launch_prefix<UmmaDeqBatchOf<kFewJobs>>(k_umma_dequantize<R, NW, DD, kFewJobs>, batch, grid, C::kThreadsD, C::kSmemBytes, !reuse, st);
+      return launch_prefix<UmmaDeqBatch>(k_umma_dequantize<R, NW, DD, kMaxDeqJobs>, batch, grid, C::kThreadsD, C::kSmemBytes, !reuse, st);
     };
+    const std::true_type yes;
+    const std::false_type no;
+    const std::integral_constant<int, 128> d128;
+    const std::integral_constant<int, 64> d64;
     int lrc;
-    if (out32 && narrow) lrc = launch(k_umma_dequantize<true, true>, DCfg<true, true>::kSmemBytes, DCfg<true, true>::kThreadsD);
-    else if (out32) lrc = launch(k_umma_dequantize<true, false>, DCfg<true, false>::kSmemBytes, DCfg<true, false>::kThreadsD);
-    else if (narrow) lrc = launch(k_umma_dequantize<false, true>, DCfg<false, true>::kSmemBytes, DCfg<false, true>::kThreadsD);
-    else lrc = launch(k_umma_dequantize<false, false>, DCfg<false, false>::kSmemBytes, DCfg<false, false>::kThreadsD);
+    if (D == 64) lrc = narrow ? launch(yes, yes, d64) : launch(yes, no, d64);
+    else if (out32) lrc = narrow ? launch(yes, yes, d128) : launch(yes, no, d128);
+    else lrc = narrow ? launch(no, yes, d128) : launch(no, no, d128);
     if (lrc != TQ_OK) return lrc;
     int rc = check_launch();
     if (rc != TQ_OK) return rc;
