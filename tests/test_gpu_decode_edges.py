@@ -1,0 +1,61 @@
+"""Decode attention: block counts, windows without 16-byte rows, and the least scratch the entry point takes."""
+
+import pytest
+import torch
+
+import tq_oracle as O
+
+import turboquant as tq
+from turboquant import _native as N
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _gen(seed):
+    return torch.Generator(device=DEV).manual_seed(seed)
+
+
+def _attend(codec, q, ck, cv):
+    parts = []
+    for side, comp in ((ck, codec.key_compressor), (cv, codec.val_compressor)):
+        c = comp.centroids.double()
+        B, H, S, D = side["compressed"]["shape"]
+        idx = torch.from_numpy(O.unpack_indices(side["compressed"]["idx_bytes"].cpu().numpy().reshape(B * H * S, -1), comp.bits, D))
+        back = (c[idx.to(DEV).long()] @ comp.Pi.double()).reshape(B, H, S, D) * side["compressed"]["vec_norms"].double().unsqueeze(-1)
+        parts.append(torch.cat([back, side["fp16"].double()], dim=2))
+    k, v = (p.repeat_interleave(q.shape[1] // p.shape[1], 1) for p in parts)
+    return ((q.double() @ k.transpose(-1, -2)) * q.shape[-1] ** -0.5).softmax(-1) @ v
+
+
+@pytest.mark.parametrize("window", [0, 1, 63, 65, 200])
+@pytest.mark.parametrize("packed", [1, 255, 257, 5000])
+@pytest.mark.parametrize("bits", [(4, 2), (8, 8)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_decode_attention_blocks_and_windows(window, packed, bits, dtype, monkeypatch):
+    codec = tq.TurboQuantV3(128, key_bits=bits[0], value_bits=bits[1], residual_window=window, layer_idx=9, n_layers=32,
+                            protected_layers=0, device=DEV)
+    keys, vals = (O.synthetic_kv((1, 2, packed + window, 128), dtype, seed=s).to(DEV) for s in (packed, packed + 1))
+    q = torch.randn(1, 6, 1, 128, generator=_gen(7), device=DEV)
+    ck, cv = codec.compress_kv(keys, vals)
+    want = _attend(codec, q, ck, cv)
+    wide = codec.decode_attention(q, ck, cv)
+    assert float((wide.double() - want).abs().max() / want.abs().max()) <= 1e-5
+    # rows of 129 elements: no 16-byte loads from the window
+    for side in (ck, cv):
+        odd = torch.zeros(1, 2, window, 129, dtype=dtype, device=DEV)
+        odd[..., 1:] = side["fp16"]
+        side["fp16"] = odd[..., 1:]
+    got = codec.decode_attention(q, ck, cv)
+    assert float((got.double() - want).abs().max() / want.abs().max()) <= 1e-5
+    # the least scratch that the entry point takes: one partial per 2048 keys
+    L = N.lib()
+    rows = 6
+    least = (rows * 128 * 4 + 255) // 256 * 256 + rows * max(1, -(-packed // 2048)) * 130 * 4
+    assert L.tq_decode_attention_workspace_bytes(1, 6, 1, packed) >= least
+    monkeypatch.setattr(L, "tq_decode_attention_workspace_bytes", lambda *a: least)
+    got = codec.decode_attention(q, ck, cv)
+    assert float((got.double() - want).abs().max() / want.abs().max()) <= 1e-5
+    monkeypatch.setattr(L, "tq_decode_attention_workspace_bytes", lambda *a: least - 4)
+    with pytest.raises(ValueError):
+        codec.decode_attention(q, ck, cv)

@@ -423,7 +423,7 @@ int tq_score_packed(const TqScoreJob* job, void* stream) {
 
 size_t tq_decode_attention_workspace_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk) {
   if (B < 0 || Hq < 0 || Sq < 0 || Sk < 0) return 0;
-  return tq::decode_attention_workspace(B, Hq, Sq, Sk, 2048);
+  return tq::decode_attention_workspace_wanted(B, Hq, Sq, Sk);
 }
 
 int tq_decode_attention(const TqDecodeAttnJob* job, void* stream) {

@@ -349,7 +349,7 @@ struct DecodeParams {
 constexpr int kPartStride = 130;
 
 template <int KBITS, int VBITS>
-__global__ void __launch_bounds__(kThreads, 1) k_decode_attn(DecodeParams P) {
+__global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
   constexpr int GK = Packed<KBITS>::G, KW = Packed<KBITS>::CW;
   constexpr int GV = PackedV<VBITS>::G, VW = PackedV<VBITS>::CW;
   __shared__ __align__(1024) uint32_t lut_k[256];
@@ -544,6 +544,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_attn(DecodeParams P) {
 
 // One CTA per query row: merge the partials of the packed tokens, add the 16-bit window tokens (their logits use
 // the UNROTATED query), normalise, and rotate back:  out = (acc / L) Pi_v + sum_w p_w v_w / L.
+// Nothing here is large (a few hundred KB for all rows); what it costs is the number of memory latencies in a row.
+// So every phase spreads its loads over all 16 warps, a few independent 16-byte loads per thread, and the rows of
+// Pi_v are fetched before the first barrier.
+// 32 query rows, 16 partials and 128 window tokens each: 59 us as one warp per 32 tokens and a loop over rows of Pi_v, 9 us so.
 struct FinishParams {
   const void* q; int q_dtype;
   const float* part; int nblk;
@@ -554,83 +558,163 @@ struct FinishParams {
   float scale;
   float* out;
 };
+constexpr int kFinWarps = 16;
+constexpr int kFinThreads = 32 * kFinWarps;
 
-template <int QDT, int WDT>
-__global__ void __launch_bounds__(128) k_decode_finish(FinishParams F) {
-  __shared__ float sh_q[kDimA], sh_acc[kDimA], sh_red[4];
-  __shared__ float sh_m, sh_l;
+// N consecutive elements as fp32; VEC: the address is a multiple of 16 bytes (of 8 for four 16-bit elements)
+template <int DT, int N, bool VEC>
+__device__ __forceinline__ void load_run(const void* p, int64_t off, float (&v)[N]) {
+  if constexpr (!VEC) {
+#pragma unroll
+    for (int e = 0; e < N; ++e) v[e] = load_elem<DT>(p, off + e);
+  } else if constexpr (DT == TQ_F32) {
+#pragma unroll
+    for (int e = 0; e < N; e += 4) {
+      const float4 f = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + off + e));
+      v[e] = f.x; v[e + 1] = f.y; v[e + 2] = f.z; v[e + 3] = f.w;
+    }
+  } else {
+    uint32_t w[N / 2];
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(p) + off;
+    if constexpr (N == 4) {
+      const uint2 u = __ldg(reinterpret_cast<const uint2*>(src));
+      w[0] = u.x; w[1] = u.y;
+    } else {
+#pragma unroll
+      for (int e = 0; e < N / 8; ++e) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>(src) + e);
+        w[4 * e] = u.x; w[4 * e + 1] = u.y; w[4 * e + 2] = u.z; w[4 * e + 3] = u.w;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < N / 2; ++e) {
+      if constexpr (DT == TQ_F16) {
+        const __half2 h = *reinterpret_cast<const __half2*>(&w[e]);
+        v[2 * e] = __low2float(h); v[2 * e + 1] = __high2float(h);
+      } else {
+        v[2 * e] = __uint_as_float(w[e] << 16); v[2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u);
+      }
+    }
+  }
+}
+
+template <int QDT, int WDT, bool VEC>
+__global__ void __launch_bounds__(kFinThreads) k_decode_finish(FinishParams F) {
+  __shared__ float sh_q[kDimA], sh_acc[kDimA], sh_m[kFinWarps], sh_l[kFinWarps];
+  __shared__ __align__(16) float sh_part[kFinWarps][kDimA];
   extern __shared__ float sh_w[];                 // window logits, then probabilities: W floats
   const int64_t row = blockIdx.x;
-  const int64_t sq = row % F.Sq, hq = (row / F.Sq) % F.Hq, b = row / (F.Sq * F.Hq);
+  const int64_t hq = (row / F.Sq) % F.Hq, b = row / (F.Sq * F.Hq);
   const int64_t hkv = hq / (F.Hq / F.Hkv);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  (void)sq;
-  sh_q[tid] = load_elem<QDT>(F.q, row * kDimA + tid);
+  // rows 8 warp .. 8 warp + 7 of Pi_v, columns 4 lane .. 4 lane + 3
+  constexpr int kRot = kDimA / kFinWarps;
+  float rot[kRot][4];
+#pragma unroll
+  for (int u = 0; u < kRot; ++u)
+    load_run<TQ_F32, 4, VEC>(F.v_rotation, (int64_t)(kRot * warp + u) * kDimA + 4 * lane, rot[u]);
+  if (tid < kDimA) sh_q[tid] = load_elem<QDT>(F.q, row * kDimA + tid);
   __syncthreads();
-  // window logits
+  // window logits: eight lanes per token, 16 coordinates each
   const int64_t wbase = b * F.ws_b + hkv * F.ws_h;
-  float wmax = -INFINITY;
-  for (int64_t w = warp; w < F.W; w += 4) {
+  float m = -INFINITY;
+  const int sub = tid & 7;
+#pragma unroll 2
+  for (int64_t w0 = 0; w0 < F.W; w0 += kFinThreads / 8) {
+    const int64_t w = w0 + (tid >> 3);
     float d = 0.f;
-    for (int j = lane; j < kDimA; j += 32) d = fmaf(sh_q[j], load_elem<WDT>(F.k_window, wbase + w * F.ws_s + j), d);
-    d = warp_sum(d) * F.scale;
-    if (lane == 0) sh_w[w] = d;
-    wmax = fmaxf(wmax, d);
+    if (w < F.W) {
+      float kv[16];
+      load_run<WDT, 16, VEC>(F.k_window, wbase + w * F.ws_s + 16 * sub, kv);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) d = fmaf(sh_q[16 * sub + e], kv[e], d);
+    }
+    d += __shfl_xor_sync(0xffffffffu, d, 4);
+    d += __shfl_xor_sync(0xffffffffu, d, 2);
+    d += __shfl_xor_sync(0xffffffffu, d, 1);
+    d *= F.scale;
+    if (w < F.W) {
+      if (sub == 0) sh_w[w] = d;
+      m = fmaxf(m, d);
+    }
   }
   // global maximum over the partials and the window
-  float m = wmax;
+  const float* parts = F.part + row * F.nblk * kPartStride;
   if (F.Sk > 0)
-    for (int i = tid; i < F.nblk; i += 128) m = fmaxf(m, F.part[(row * F.nblk + i) * kPartStride]);
+    for (int i = tid; i < F.nblk; i += kFinThreads) m = fmaxf(m, parts[(int64_t)i * kPartStride]);
   m = warp_max(m);
-  if (lane == 0) sh_red[warp] = m;
+  if (lane == 0) sh_m[warp] = m;
   __syncthreads();
-  m = fmaxf(fmaxf(sh_red[0], sh_red[1]), fmaxf(sh_red[2], sh_red[3]));
-  __syncthreads();
-  // rotated-domain accumulator and sum of the packed part; thread = coordinate
-  float acc = 0.f, lsum = 0.f;
+  m = sh_m[0];
+#pragma unroll
+  for (int u = 1; u < kFinWarps; ++u) m = fmaxf(m, sh_m[u]);
+  // window probabilities, and the rotated-domain sums of this warp's partials (lane = four coordinates)
+  float lsum = 0.f;
+  for (int64_t w = tid; w < F.W; w += kFinThreads) {
+    const float pw = __expf(sh_w[w] - m);
+    sh_w[w] = pw;
+    lsum += pw;
+  }
+  lsum = warp_sum(lsum);                          // of the warp's window tokens, the same in every lane
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
   if (F.Sk > 0) {
-    // eight partials per round: their loads are independent and in flight together (a loop that tests each
-    // partial's maximum before loading the next spends one memory latency per partial)
-    constexpr int kBatch = 8;
-    for (int i0 = 0; i0 < F.nblk; i0 += kBatch) {
-      float pm[kBatch], ps[kBatch], pv[kBatch];
+    constexpr int kBatch = 4;                     // partials in flight per warp
+    for (int i0 = warp; i0 < F.nblk; i0 += kBatch * kFinWarps) {
+      float2 ms[kBatch], lo[kBatch], hi[kBatch];
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
-        const int i = i0 + u < F.nblk ? i0 + u : F.nblk - 1;
-        const float* pp = F.part + (row * F.nblk + i) * kPartStride;
-        pm[u] = i0 + u < F.nblk ? pp[0] : -INFINITY;
-        ps[u] = pp[1];
-        pv[u] = pp[2 + tid];
+        const int i = i0 + u * kFinWarps;
+        const float2* pp = reinterpret_cast<const float2*>(parts + (int64_t)(i < F.nblk ? i : i0) * kPartStride);
+        ms[u] = pp[0];
+        if (i >= F.nblk) ms[u].x = -INFINITY;
+        lo[u] = pp[1 + 2 * lane];
+        hi[u] = pp[2 + 2 * lane];
       }
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
-        if (pm[u] != -INFINITY) {
-          const float f = __expf(pm[u] - m);
-          acc += pv[u] * f;
-          lsum += ps[u] * f;
+        if (ms[u].x != -INFINITY) {
+          const float f = __expf(ms[u].x - m);
+          acc[0] += lo[u].x * f; acc[1] += lo[u].y * f; acc[2] += hi[u].x * f; acc[3] += hi[u].y * f;
+          lsum += ms[u].y * f;
         }
       }
     }
   }
-  sh_acc[tid] = acc;
-  // window probabilities
-  float wl = 0.f;
-  for (int64_t w = tid; w < F.W; w += 128) {
-    const float pw = __expf(sh_w[w] - m);
-    sh_w[w] = pw;
-    wl += pw;
-  }
-  wl = warp_sum(wl);
-  if (lane == 0) sh_red[warp] = wl;
+  *reinterpret_cast<float4*>(&sh_part[warp][4 * lane]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  if (lane == 0) sh_l[warp] = lsum;
   __syncthreads();
-  const float total = lsum + sh_red[0] + sh_red[1] + sh_red[2] + sh_red[3];
-  // out[tid] = sum_j acc[j] Pi_v[j][tid] + sum_w p_w v_w[tid]
-  float o = 0.f;
-#pragma unroll 16
-  for (int j = 0; j < kDimA; ++j) o = fmaf(sh_acc[j], __ldg(F.v_rotation + j * kDimA + tid), o);
-  for (int64_t w = 0; w < F.W; ++w) o = fmaf(sh_w[w], load_elem<WDT>(F.v_window, wbase + w * F.ws_s + tid), o);
-  F.out[row * kDimA + tid] = o / total;
-  (void)sh_m; (void)sh_l;
+  if (tid < kDimA) {
+    float a = 0.f;
+#pragma unroll
+    for (int u = 0; u < kFinWarps; ++u) a += sh_part[u][tid];
+    sh_acc[tid] = a;
+  }
+  // this warp's window tokens while the sums settle: o += p_w v_w
+  float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+  for (int64_t w = warp; w < F.W; w += kFinWarps) {
+    float vv[4];
+    load_run<WDT, 4, VEC>(F.v_window, wbase + w * F.ws_s + 4 * lane, vv);
+    const float pw = sh_w[w];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = fmaf(pw, vv[e], o[e]);
+  }
+  __syncthreads();
+  // o += acc @ Pi_v over this warp's eight rows of Pi_v
+#pragma unroll
+  for (int u = 0; u < kRot; ++u) {
+    const float a = sh_acc[kRot * warp + u];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = fmaf(a, rot[u][e], o[e]);
+  }
+  *reinterpret_cast<float4*>(&sh_part[warp][4 * lane]) = make_float4(o[0], o[1], o[2], o[3]);
+  __syncthreads();
+  if (tid < kDimA) {
+    float sum = 0.f, total = 0.f;
+#pragma unroll
+    for (int u = 0; u < kFinWarps; ++u) { sum += sh_part[u][tid]; total += sh_l[u]; }
+    F.out[row * kDimA + tid] = sum / total;
+  }
 }
 
 }  // namespace
@@ -682,11 +766,51 @@ static int device_sm_count() {
   return n;
 }
 
+// Blocks of keys per (batch, KV head): fewer keys per CTA fill the chip sooner, and every CTA pays a fixed cost
+// (table, query pieces, first loads, folding its warps) worth about kFixedKeys keys of its loop.  The count with the
+// smallest  waves x (keys per CTA + kFixedKeys)  is taken, at most `most` (what the scratch holds) and never blocks
+// of fewer than kDecodeMinKeys keys (two rounds of the CTA's eight warps).
+// 8 KV heads x 32640 tokens, K4/V2: 36 us as 128 CTAs of 2048 keys with one CTA per SM, 30 us as 296 CTAs with two.
+constexpr int kDecodeMinKeys = 256;
+static int decode_blocks(int64_t units, int64_t Sk, int64_t most, int slots) {
+  constexpr int64_t kFixedKeys = 256;
+  int64_t cap = (Sk + kDecodeMinKeys - 1) / kDecodeMinKeys;
+  if (cap > most) cap = most;
+  if (cap > 1024) cap = 1024;
+  int64_t best = 1, best_cost = -1;
+  for (int64_t nblk = 1; nblk <= cap; ++nblk) {
+    const int64_t kpb = ((Sk + nblk - 1) / nblk + 15) / 16 * 16;
+    const int64_t cost = ((units * nblk + slots - 1) / slots) * (kpb + kFixedKeys);
+    if (best_cost < 0 || cost < best_cost) { best = nblk; best_cost = cost; }
+  }
+  return (int)best;
+}
+
+// Scratch the entry point asks for: room for the blocks of one full wave (two CTAs per SM) at one unit, as long as
+// the partials stay within 16 MB; never less than decode_attention_workspace(), which every caller brings.
+size_t decode_attention_workspace_wanted(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk) {
+  const size_t least = decode_attention_workspace(B, Hq, Sq, Sk, 2048);
+  const int64_t rows = B * Hq * Sq;
+  if (rows <= 0 || Sk <= 0) return least;
+  int64_t nblk = (Sk + kDecodeMinKeys - 1) / kDecodeMinKeys;
+  if (nblk > 320) nblk = 320;
+  const int64_t fit = ((int64_t)16 << 20) / (rows * kPartStride * (int64_t)sizeof(float));
+  if (nblk > fit) nblk = fit;
+  const size_t q = ((size_t)rows * kDimA * sizeof(float) + 255) / 256 * 256;
+  const size_t want = q + (size_t)rows * (nblk > 0 ? nblk : 1) * kPartStride * sizeof(float);
+  return want > least ? want : least;
+}
+
 int decode_attention(const TqDecodeAttnJob& job, cudaStream_t st) {
-  constexpr int kMinKeysPerBlock = 2048;          // decode_attention_workspace() sizes the partials for this
-  const int kKeysPerBlock = wave_keys_per_block(job.B * job.Hkv, job.Sk, kMinKeysPerBlock, device_sm_count());
   const int64_t rows = job.B * job.Hq * job.Sq;
-  const int nblk = job.Sk > 0 ? (int)((job.Sk + kKeysPerBlock - 1) / kKeysPerBlock) : 1;
+  int nblk = 1, kKeysPerBlock = 16;
+  if (job.Sk > 0) {
+    const size_t q = ((size_t)rows * kDimA * sizeof(float) + 255) / 256 * 256;
+    const int64_t most = (int64_t)((job.workspace_bytes - q) / ((size_t)rows * kPartStride * sizeof(float)));
+    nblk = decode_blocks(job.B * job.Hkv, job.Sk, most, 2 * device_sm_count());
+    kKeysPerBlock = (int)(((job.Sk + nblk - 1) / nblk + 15) / 16 * 16);
+    nblk = (int)((job.Sk + kKeysPerBlock - 1) / kKeysPerBlock);
+  }
   float* qrot = reinterpret_cast<float*>(job.workspace);
   const size_t qbytes = ((size_t)rows * kDimA * sizeof(float) + 255) / 256 * 256;
   float* part = reinterpret_cast<float*>(reinterpret_cast<char*>(job.workspace) + qbytes);
@@ -726,15 +850,26 @@ int decode_attention(const TqDecodeAttnJob& job, cudaStream_t st) {
   F.scale = job.scale;
   F.out = job.out;
   const size_t smem = (size_t)(F.W > 0 ? F.W : 1) * sizeof(float);
-  auto launch = [&](auto kern) {
-    kern<<<(unsigned)rows, 128, smem, st>>>(F);
-  };
   const int wdt = F.W > 0 ? job.window_dtype : TQ_F16;
-#define TQ_FIN(QD, WD) launch(k_decode_finish<QD, WD>)
+  // 16-byte loads where every row of the windows and of Pi_v starts on such a boundary
+  const int64_t per16 = wdt == TQ_F32 ? 4 : 8;
+  const bool vec = (((uintptr_t)F.k_window | (uintptr_t)F.v_window | (uintptr_t)F.v_rotation) & 15u) == 0 &&
+                   (F.ws_b % per16 == 0 && F.ws_h % per16 == 0 && F.ws_s % per16 == 0);
+  cudaError_t attr = cudaSuccess;
+  auto launch = [&](auto vec_kernel, auto any_kernel) {
+    auto kern = vec ? vec_kernel : any_kernel;
+    if (smem > 36 * 1024) {                        // with its 10 KB of static shared memory past the default limit
+      attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (attr != cudaSuccess) return;
+    }
+    kern<<<(unsigned)rows, kFinThreads, smem, st>>>(F);
+  };
+#define TQ_FIN(QD, WD) launch(k_decode_finish<QD, WD, true>, k_decode_finish<QD, WD, false>)
   if (job.q_dtype == TQ_F32) { if (wdt == TQ_F16) TQ_FIN(TQ_F32, TQ_F16); else if (wdt == TQ_BF16) TQ_FIN(TQ_F32, TQ_BF16); else TQ_FIN(TQ_F32, TQ_F32); }
   else if (job.q_dtype == TQ_F16) { if (wdt == TQ_F16) TQ_FIN(TQ_F16, TQ_F16); else if (wdt == TQ_BF16) TQ_FIN(TQ_F16, TQ_BF16); else TQ_FIN(TQ_F16, TQ_F32); }
   else { if (wdt == TQ_F16) TQ_FIN(TQ_BF16, TQ_F16); else if (wdt == TQ_BF16) TQ_FIN(TQ_BF16, TQ_BF16); else TQ_FIN(TQ_BF16, TQ_F32); }
 #undef TQ_FIN
+  if (attr != cudaSuccess) { note_cuda_error((int)attr); return TQ_ELAUNCH; }
   return check_launch();
 }
 

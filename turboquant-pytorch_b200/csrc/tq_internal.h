@@ -40,6 +40,7 @@ int mma_score_keys_per_block(const TqScoreJob& job, int min_keys);
 
 // decode attention on packed keys and packed values (tq_attn_mma.cu)
 size_t decode_attention_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int keys_per_block);
+size_t decode_attention_workspace_wanted(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk);
 int decode_attention(const TqDecodeAttnJob& job, cudaStream_t st);
 
 // packed MSE+QJL storage and scores from it (tq_qjl_packed.cu)
