@@ -112,6 +112,34 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   tmem_wait16(r);
 }
 
+// The 32 bytes of one vector's row that an epilogue step produces or reads.  A warp's access touches 32 rows, that is 32
+// lines, whatever its width, and the load/store unit takes them one at a time: that was the whole cost of stages 1
+// and 2 (eight 16-byte accesses per step are 33 000 of the 36 000 clocks that stage 2 took per tile), so a row's 32
+// bytes go as one access (262144 vectors of head_dim 256: stages 183 + 264 + 87 us before, 154 + 195 + 81 us so).  `wide`
+// is false where a caller's buffer starts on an odd multiple of 16 bytes.
+__device__ __forceinline__ void store_row32(void* dst, const uint32_t (&v)[8], bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+  } else {
+    uint4* d = reinterpret_cast<uint4*>(dst);
+    d[0] = make_uint4(v[0], v[1], v[2], v[3]);
+    d[1] = make_uint4(v[4], v[5], v[6], v[7]);
+  }
+}
+__device__ __forceinline__ void load_row32(const void* src, uint32_t (&v)[8], bool wide) {
+  if (wide) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]),
+                 "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(src));
+  } else {
+    const uint4* s = reinterpret_cast<const uint4*>(src);
+    const uint4 a = __ldg(s), b = __ldg(s + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  }
+}
+
 template <int D, int STAGE>
 __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __grid_constant__ V2Stage p) {
   using C = VCfg<D>;
@@ -389,25 +417,26 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
               ph[j] = __byte_perm(w[2 * j], w[2 * j + 1], 0x5410);
               pl[j] = __byte_perm(w[2 * j], w[2 * j + 1], 0x7632);
             }
-            uint4* dh = reinterpret_cast<uint4*>(p.p_hi + row * D + col0 + c * 16);
-            uint4* dl = reinterpret_cast<uint4*>(p.p_lo + row * D + col0 + c * 16);
-            dh[0] = make_uint4(ph[0], ph[1], ph[2], ph[3]); dh[1] = make_uint4(ph[4], ph[5], ph[6], ph[7]);
-            dl[0] = make_uint4(pl[0], pl[1], pl[2], pl[3]); dl[1] = make_uint4(pl[4], pl[5], pl[6], pl[7]);
+            store_row32(p.p_hi + row * D + col0 + c * 16, ph, true);
+            store_row32(p.p_lo + row * D + col0 + c * 16, pl, true);
           }
         }
       } else if constexpr (STAGE == 2) {
         const float nv = valid ? p.norms[row] : 0.f;
         float ssq = 0.f;
         // the vector's own 16-coordinate pieces are fetched one step ahead of their use
-        const uint4* xrow = reinterpret_cast<const uint4*>(p.x + (valid ? row : 0) * D + col0);
-        uint4 nx0 = __ldg(xrow), nx1 = __ldg(xrow + 1);
+        const uint16_t* xrow = p.x + (valid ? row : 0) * D + col0;
+        const bool x_wide = ((uintptr_t)p.x & 31u) == 0, k_wide = ((uintptr_t)p.k_mse_out & 31u) == 0;
+        uint32_t xn[8];
+        load_row32(xrow, xn, x_wide);
 #pragma unroll 1
         for (int c = 0; c < 8; ++c) {
-          const uint4 x0 = nx0, x1 = nx1;
-          if (c + 1 < 8) { nx0 = __ldg(xrow + 2 * (c + 1)); nx1 = __ldg(xrow + 2 * (c + 1) + 1); }
+          uint32_t xw[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) xw[j] = xn[j];
+          if (c + 1 < 8) load_row32(xrow + 16 * (c + 1), xn, x_wide);
           tmem_ld16(tacc + c * 16, v);
           if (valid) {
-            const uint32_t xw[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
             uint32_t kq[8], rh[8], rl[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -423,14 +452,9 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
               const __half2 ll = __floats2half2_rn(r0 - __low2float(hh), r1 - __high2float(hh));
               rl[j] = *reinterpret_cast<const uint32_t*>(&ll);
             }
-            uint4* dh = reinterpret_cast<uint4*>(p.p_hi + row * D + col0 + c * 16);
-            uint4* dl = reinterpret_cast<uint4*>(p.p_lo + row * D + col0 + c * 16);
-            if (p.k_mse_out != nullptr) {
-              uint4* dk = reinterpret_cast<uint4*>(p.k_mse_out + row * D + col0 + c * 16);
-              dk[0] = make_uint4(kq[0], kq[1], kq[2], kq[3]); dk[1] = make_uint4(kq[4], kq[5], kq[6], kq[7]);
-            }
-            dh[0] = make_uint4(rh[0], rh[1], rh[2], rh[3]); dh[1] = make_uint4(rh[4], rh[5], rh[6], rh[7]);
-            dl[0] = make_uint4(rl[0], rl[1], rl[2], rl[3]); dl[1] = make_uint4(rl[4], rl[5], rl[6], rl[7]);
+            if (p.k_mse_out != nullptr) store_row32(p.k_mse_out + row * D + col0 + c * 16, kq, k_wide);
+            store_row32(p.p_hi + row * D + col0 + c * 16, rh, true);
+            store_row32(p.p_lo + row * D + col0 + c * 16, rl, true);
           }
         }
         if constexpr (NBLK == 2) {
@@ -442,28 +466,34 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
         }
         if (valid && blk == 0) p.rnorm_out[row] = __half_as_ushort(__float2half_rn(__fsqrt_rn(ssq)));
       } else {
+        const bool s_wide = ((uintptr_t)p.signs_out & 31u) == 0;
 #pragma unroll 1
-        for (int c = 0; c < 8; ++c) {
-          tmem_ld16(tacc + c * 16, v);
+        for (int c = 0; c < 8; c += 2) {
+          uint32_t v2[16];
+          tmem_issue16(tacc + c * 16, v);
+          tmem_issue16(tacc + (c + 1) * 16, v2);
+          tmem_wait16(v);
+          tmem_wait16(v2);
           if (valid && p.signs_out != nullptr) {
-            uint32_t sw[4];
+            uint32_t sw[8];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < 8; ++j) {
               uint32_t x = 0u;
 #pragma unroll
               for (int b = 0; b < 4; ++b) {
-                const uint32_t s8 = __uint_as_float(v[4 * j + b]) >= 0.f ? 0x01u : 0xFFu;
+                const uint32_t s8 = __uint_as_float(j < 4 ? v[4 * j + b] : v2[4 * (j - 4) + b]) >= 0.f ? 0x01u : 0xFFu;
                 x |= s8 << (8 * b);
               }
               sw[j] = x;
             }
-            *reinterpret_cast<uint4*>(p.signs_out + row * D + col0 + c * 16) = make_uint4(sw[0], sw[1], sw[2], sw[3]);
+            store_row32(p.signs_out + row * D + col0 + c * 16, sw, s_wide);
           }
           if (valid && p.sign_bits_out != nullptr) {
             uint32_t o = 0u;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) o |= (__uint_as_float(v[e]) >= 0.f ? 1u : 0u) << (8 * (e >> 3) + 7 - (e & 7));
-            *reinterpret_cast<uint16_t*>(p.sign_bits_out + row * (D / 8) + (col0 + c * 16) / 8) = (uint16_t)o;
+            for (int e = 0; e < 32; ++e)
+              o |= (__uint_as_float(e < 16 ? v[e] : v2[e - 16]) >= 0.f ? 1u : 0u) << (8 * (e >> 3) + 7 - (e & 7));
+            *reinterpret_cast<uint32_t*>(p.sign_bits_out + row * (D / 8) + (col0 + c * 16) / 8) = o;
           }
         }
       }
