@@ -16,60 +16,97 @@
 
 namespace tq {
 
-constexpr int TM = 64;    // vectors per tile
+constexpr int TM = 64;    // vectors per tile of the large form (RI = 4)
 constexpr int KC = 16;    // k rows of B staged per step
 constexpr int NT = 256;   // threads per CTA
 constexpr int BPAD = 4;
+constexpr int BST = 3;    // stages of the ring that B travels through
 
 enum { B_KN = 0, B_NK = 1 };
 
 __host__ __device__ inline int lda_for(int K) { return round_up(K, KC) + 4; }
 __host__ __device__ inline int ldb_for(int N) { return round_up(N, 64) + BPAD; }
+// floats of shared memory for the ring of a contraction with 64 * nj columns
+__host__ __device__ inline int b_ring_floats(int nj) { return BST * KC * (64 * nj + BPAD); }
 
-// acc[ri][4*j+c] += sum_k As[(ty*4+ri)*lda + k] * B[k][tx*4 + 64*j + c]
-// B is global, fp32, either [K][N] row-major with row stride ldg (B_KN) or
-// [N][K] row-major with row stride ldg (B_NK).  Columns >= N and rows >= K read
-// as zero.  As must hold zeros in columns [K, round_up(K,16)).
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool ok) {
+  const int bytes = ok ? 4 : 0;                          // 0: the word is filled with zero, nothing is read
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool ok) {
+  const int bytes = ok ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+// One k-chunk of B (rows k0 .. k0 + KC) into ring stage k0 / KC % BST, as one group of asynchronous copies.  A chunk
+// past the end of B commits an empty group, so that groups and chunks keep step.
 template <int NJ, int BL>
-__device__ __forceinline__ void tile_gemm(const float* As, int lda, int K, const float* __restrict__ Bg, int64_t ldg,
-                                          int N, float* Bs, float (&acc)[4][4 * NJ]) {
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int npad = 64 * NJ;
-  const int ldb = npad + BPAD;
-  const int kpad = round_up(K, KC);
-  for (int k0 = 0; k0 < kpad; k0 += KC) {
-    __syncthreads();
-    if constexpr (BL == B_KN) {
-      for (int e = tid; e < KC * npad; e += NT) {
-        int kk = e / npad, n = e - kk * npad;
-        int k = k0 + kk;
-        float v = 0.f;
-        if (k < K && n < N) v = __ldg(Bg + (int64_t)k * ldg + n);
-        Bs[kk * ldb + n] = v;
+__device__ __forceinline__ void b_stage(int k0, int K, const float* __restrict__ Bg, int64_t ldg, int N, float* ring) {
+  constexpr int npad = 64 * NJ;
+  constexpr int ldb = npad + BPAD;
+  float* Bs = ring + (k0 / KC) % BST * (KC * ldb);
+  if (k0 < round_up(K, KC)) {
+    if (BL == B_KN && (N & 3) == 0 && (ldg & 3) == 0 && ((uintptr_t)Bg & 15u) == 0) {
+      for (int e = threadIdx.x; e < KC * (npad / 4); e += NT) {
+        const int kk = e / (npad / 4), n = 4 * (e - kk * (npad / 4));
+        const int k = k0 + kk;
+        const bool ok = k < K && n < N;
+        cp_async16(Bs + kk * ldb + n, ok ? Bg + (int64_t)k * ldg + n : Bg, ok);
       }
     } else {
-      for (int e = tid; e < KC * npad; e += NT) {
-        int n = e / KC, kk = e - n * KC;
-        int k = k0 + kk;
-        float v = 0.f;
-        if (k < K && n < N) v = __ldg(Bg + (int64_t)n * ldg + k);
-        Bs[kk * ldb + n] = v;
+      for (int e = threadIdx.x; e < KC * npad; e += NT) {
+        const int kk = BL == B_KN ? e / npad : e % KC, n = BL == B_KN ? e % npad : e / KC;
+        const int k = k0 + kk;
+        const bool ok = k < K && n < N;
+        const float* src = BL == B_KN ? Bg + (int64_t)k * ldg + n : Bg + (int64_t)n * ldg + k;
+        cp_async4(Bs + kk * ldb + n, ok ? src : Bg, ok);
       }
     }
-    __syncthreads();
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// The first BST - 1 chunks of B: issued before whatever the kernel does ahead of the contraction, so that their
+// latency runs beside it.  The previous contraction's readers must be past their last barrier.
+template <int NJ, int BL>
+__device__ __forceinline__ void b_begin(int K, const float* __restrict__ Bg, int64_t ldg, int N, float* ring) {
+#pragma unroll
+  for (int c = 0; c < BST - 1; ++c) b_stage<NJ, BL>(c * KC, K, Bg, ldg, N, ring);
+}
+
+// acc[ri][4*j+c] += sum_k As[(ty*RI+ri)*lda + k] * B[k][tx*4 + 64*j + c]
+// B is global, fp32, either [K][N] row-major with row stride ldg (B_KN) or
+// [N][K] row-major with row stride ldg (B_NK).  Columns >= N and rows >= K read
+// as zero.  As must hold zeros in columns [K, round_up(K,16)).  b_begin() with the same B comes first.
+//
+// B goes through a ring of three chunks of 16 rows by asynchronous copies: one barrier per chunk, and a chunk's L2
+// latency passes under the two before it (staged through registers with two barriers, each chunk cost that latency:
+// 40 us for 4096 vectors of head_dim 128 on 64 SMs).  Every output is one chain of fused multiply-adds in
+// ascending k, whatever RI is.
+template <int RI, int NJ, int BL>
+__device__ __forceinline__ void tile_gemm(const float* As, int lda, int K, const float* __restrict__ Bg, int64_t ldg,
+                                          int N, float* ring, float (&acc)[RI][4 * NJ]) {
+  const int tid = threadIdx.x;
+  const int tx = tid & 15, ty = tid >> 4;
+  constexpr int ldb = 64 * NJ + BPAD;
+  const int kpad = round_up(K, KC);
+  for (int k0 = 0; k0 < kpad; k0 += KC) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(BST - 2) : "memory");
+    __syncthreads();                            // chunk k0 is there for everyone; the stage of chunk k0 - KC is free
+    b_stage<NJ, BL>(k0 + (BST - 1) * KC, K, Bg, ldg, N, ring);
+    const float* Bs = ring + (k0 / KC) % BST * (KC * ldb);
 #pragma unroll
     for (int kk = 0; kk < KC; kk += 4) {
-      float4 a[4];
+      float4 a[RI];
 #pragma unroll
-      for (int ri = 0; ri < 4; ++ri) a[ri] = *reinterpret_cast<const float4*>(As + (ty * 4 + ri) * lda + k0 + kk);
+      for (int ri = 0; ri < RI; ++ri) a[ri] = *reinterpret_cast<const float4*>(As + (ty * RI + ri) * lda + k0 + kk);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         float4 b[NJ];
 #pragma unroll
         for (int j = 0; j < NJ; ++j) b[j] = *reinterpret_cast<const float4*>(Bs + (kk + u) * ldb + tx * 4 + 64 * j);
 #pragma unroll
-        for (int ri = 0; ri < 4; ++ri) {
+        for (int ri = 0; ri < RI; ++ri) {
           float av = (u == 0) ? a[ri].x : (u == 1) ? a[ri].y : (u == 2) ? a[ri].z : a[ri].w;
 #pragma unroll
           for (int j = 0; j < NJ; ++j) {
@@ -82,54 +119,75 @@ __device__ __forceinline__ void tile_gemm(const float* As, int lda, int K, const
       }
     }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");     // only empty groups are left
 }
 
-template <int NJ>
-__device__ __forceinline__ void zero_acc(float (&acc)[4][4 * NJ]) {
+template <int RI, int NJ>
+__device__ __forceinline__ void zero_acc(float (&acc)[RI][4 * NJ]) {
 #pragma unroll
-  for (int ri = 0; ri < 4; ++ri)
+  for (int ri = 0; ri < RI; ++ri)
 #pragma unroll
     for (int c = 0; c < 4 * NJ; ++c) acc[ri][c] = 0.f;
 }
 
 // registers -> Cs[r*ldc + n] for n < ncols (a multiple of 4, at most ldc); caller syncs around it
-template <int NJ>
-__device__ __forceinline__ void acc_to_smem(const float (&acc)[4][4 * NJ], float* Cs, int ldc, int ncols) {
+template <int RI, int NJ>
+__device__ __forceinline__ void acc_to_smem(const float (&acc)[RI][4 * NJ], float* Cs, int ldc, int ncols) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
-  for (int ri = 0; ri < 4; ++ri)
+  for (int ri = 0; ri < RI; ++ri)
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
       const int col = tx * 4 + 64 * j;
       if (col < ncols)
-        *reinterpret_cast<float4*>(Cs + (ty * 4 + ri) * ldc + col) =
+        *reinterpret_cast<float4*>(Cs + (ty * RI + ri) * ldc + col) =
             make_float4(acc[ri][4 * j], acc[ri][4 * j + 1], acc[ri][4 * j + 2], acc[ri][4 * j + 3]);
     }
 }
 
 // Load a tile of vectors as fp32 into Xs (zero padded to kpad columns, zero rows
 // past n_total); per-row L2 norms into nrm[] when wanted.
-template <int XDT>
+// A warp loads two of its rows at a time, so that up to eight of a lane's loads are in flight.
+template <int XDT, int RI>
 __device__ __forceinline__ void load_tile_rows(const void* x, int64_t row0, int64_t n_total, int D, int64_t H, int64_t S,
                                                int64_t sb, int64_t sh, int64_t ss, float* Xs, int ld, float* nrm) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kpad = round_up(D, KC);
-  for (int r = warp; r < TM; r += NT / 32) {
-    int64_t n = row0 + r;
-    float ssq = 0.f;
-    if (n < n_total) {
-      int64_t off = vec_offset(n, H, S, sb, sh, ss);
-      for (int k = lane; k < kpad; k += 32) {
-        float v = (k < D) ? load_elem<XDT>(x, off + k) : 0.f;
-        Xs[r * ld + k] = v;
-        ssq = fmaf(v, v, ssq);
-      }
-    } else {
-      for (int k = lane; k < kpad; k += 32) Xs[r * ld + k] = 0.f;
+#pragma unroll
+  for (int r0 = warp; r0 < 16 * RI; r0 += 2 * (NT / 32)) {
+    float ssq[2] = {0.f, 0.f};
+    int64_t off[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t n = row0 + r0 + h * (NT / 32);
+      off[h] = n < n_total ? vec_offset(n, H, S, sb, sh, ss) : -1;
+    }
+    for (int k0 = 0; k0 < kpad; k0 += 128) {
+      float v[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int k = k0 + 32 * u + lane;
+          v[h][u] = (off[h] >= 0 && k < D) ? load_elem<XDT>(x, off[h] + k) : 0.f;
+        }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int k = k0 + 32 * u + lane;
+          if (k < kpad) {
+            Xs[(r0 + h * (NT / 32)) * ld + k] = v[h][u];
+            ssq[h] = fmaf(v[h][u], v[h][u], ssq[h]);
+          }
+        }
     }
     if (nrm != nullptr) {
-      ssq = warp_sum(ssq);
-      if (lane == 0) nrm[r] = __fsqrt_rn(ssq);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float s = warp_sum(ssq[h]);
+        if (lane == 0) nrm[r0 + h * (NT / 32)] = __fsqrt_rn(s);
+      }
     }
   }
 }
@@ -196,14 +254,15 @@ __global__ void __launch_bounds__(NT) k_quantize_rotated(const float* __restrict
 // ---------------------------------------------------------------------------
 // K1: norm + rotate + quantise + pack
 // ---------------------------------------------------------------------------
-template <int XDT, int NJ>
+template <int XDT, int NJ, int RI>
 __global__ void __launch_bounds__(NT) k_quantize(TqQuantizeJob job) {
+  constexpr int TM = 16 * RI;                   // vectors per tile
   extern __shared__ __align__(16) float smem[];
   const int D = job.D;
   const int lda = lda_for(D);
   float* As = smem;
   float* Bs = As + TM * lda;
-  float* cent_s = Bs + KC * (64 * NJ + BPAD);
+  float* cent_s = Bs + b_ring_floats(NJ);
   float* thr_s = cent_s + 256;
   float* nrm = thr_s + 256;
   load_codebook(job.codebook, cent_s, thr_s);
@@ -214,7 +273,8 @@ __global__ void __launch_bounds__(NT) k_quantize(TqQuantizeJob job) {
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t row0 = tile * TM;
     __syncthreads();
-    load_tile_rows<XDT>(job.x, row0, n_total, D, job.H, job.S, job.stride_b, job.stride_h, job.stride_s, As, lda,
+    b_begin<NJ, B_KN>(D, job.rotation_t, D, D, Bs);
+    load_tile_rows<XDT, RI>(job.x, row0, n_total, D, job.H, job.S, job.stride_b, job.stride_h, job.stride_s, As, lda,
                         job.normalize ? nrm : nullptr);
     if (job.normalize) {
       __syncwarp();
@@ -226,11 +286,11 @@ __global__ void __launch_bounds__(NT) k_quantize(TqQuantizeJob job) {
         for (int k = lane; k < kpad; k += 32) As[r * lda + k] = __fdiv_rn(As[r * lda + k], den);
       }
     }
-    float acc[4][4 * NJ];
-    zero_acc<NJ>(acc);
-    tile_gemm<NJ, B_KN>(As, lda, D, job.rotation_t, D, D, Bs, acc);
+    float acc[RI][4 * NJ];
+    zero_acc<RI, NJ>(acc);
+    tile_gemm<RI, NJ, B_KN>(As, lda, D, job.rotation_t, D, D, Bs, acc);
     __syncthreads();
-    acc_to_smem<NJ>(acc, As, lda, kpad);
+    acc_to_smem<RI, NJ>(acc, As, lda, kpad);
     __syncthreads();
     for (int r = warp; r < TM; r += NT / 32) {
       int64_t n = row0 + r;
@@ -242,14 +302,15 @@ __global__ void __launch_bounds__(NT) k_quantize(TqQuantizeJob job) {
 // ---------------------------------------------------------------------------
 // K2: unpack + lookup + inverse rotation + rescale
 // ---------------------------------------------------------------------------
-template <int ODT, int NJ>
+template <int ODT, int NJ, int RI>
 __global__ void __launch_bounds__(NT) k_dequantize(TqDequantizeJob job) {
+  constexpr int TM = 16 * RI;                   // vectors per tile
   extern __shared__ __align__(16) float smem[];
   const int D = job.D;
   const int lda = lda_for(D);
   float* As = smem;
   float* Bs = As + TM * lda;
-  float* cent_s = Bs + KC * (64 * NJ + BPAD);
+  float* cent_s = Bs + b_ring_floats(NJ);
   float* thr_s = cent_s + 256;
   load_codebook(job.codebook, cent_s, thr_s);
   const int64_t n_total = job.B * job.H * job.S;
@@ -260,20 +321,23 @@ __global__ void __launch_bounds__(NT) k_dequantize(TqDequantizeJob job) {
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t row0 = tile * TM;
     __syncthreads();
+    b_begin<NJ, B_KN>(D, job.rotation, D, D, Bs);
+#pragma unroll 4
     for (int r = warp; r < TM; r += NT / 32) {
       int64_t n = row0 + r;
+#pragma unroll 4
       for (int c = lane; c < kpad; c += 32) {
         float v = 0.f;
         if (n < n_total && c < D) v = cent_s[fetch_index(job.idx, job.idx_mode, n, c, D, job.bits)];
         As[r * lda + c] = v;
       }
     }
-    float acc[4][4 * NJ];
-    zero_acc<NJ>(acc);
-    tile_gemm<NJ, B_KN>(As, lda, D, job.rotation, D, D, Bs, acc);
+    float acc[RI][4 * NJ];
+    zero_acc<RI, NJ>(acc);
+    tile_gemm<RI, NJ, B_KN>(As, lda, D, job.rotation, D, D, Bs, acc);
 #pragma unroll
-    for (int ri = 0; ri < 4; ++ri) {
-      int64_t n = row0 + ty * 4 + ri;
+    for (int ri = 0; ri < RI; ++ri) {
+      int64_t n = row0 + ty * RI + ri;
       if (n >= n_total) continue;
       float nv = (job.norms != nullptr) ? __half2float(__ushort_as_half(job.norms[n])) : 1.f;
       int64_t off = vec_offset(n, job.H, job.S, job.ostride_b, job.ostride_h, job.ostride_s);
@@ -306,10 +370,11 @@ __global__ void __launch_bounds__(NT) k_project(const void* x, int64_t n_total, 
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t row0 = tile * TM;
     __syncthreads();
-    load_tile_rows<XDT>(x, row0, n_total, K, 1, n_total, 0, 0, K, As, lda, nullptr);
+    b_begin<NJ, B_KN>(K, m, N, N, Bs);
+    load_tile_rows<XDT, 4>(x, row0, n_total, K, 1, n_total, 0, 0, K, As, lda, nullptr);
     float acc[4][4 * NJ];
-    zero_acc<NJ>(acc);
-    tile_gemm<NJ, B_KN>(As, lda, K, m, N, N, Bs, acc);
+    zero_acc<4, NJ>(acc);
+    tile_gemm<4, NJ, B_KN>(As, lda, K, m, N, N, Bs, acc);
 #pragma unroll
     for (int ri = 0; ri < 4; ++ri) {
       int64_t n = row0 + ty * 4 + ri;
@@ -690,8 +755,9 @@ __global__ void __launch_bounds__(NT) k_softmax_finish(const float* __restrict__
 // ---------------------------------------------------------------------------
 // K4: MSE stage + QJL signs on one resident tile
 // ---------------------------------------------------------------------------
-template <int XDT, int NJ, int NJM>
+template <int XDT, int NJ, int NJM, int RI>
 __global__ void __launch_bounds__(NT) k_qjl_compress(TqQjlCompressJob job) {
+  constexpr int TM = 16 * RI;                   // vectors per tile
   extern __shared__ __align__(16) float smem[];
   const int D = job.D, M = job.M;
   const int lda = lda_for(D);
@@ -699,7 +765,7 @@ __global__ void __launch_bounds__(NT) k_qjl_compress(TqQjlCompressJob job) {
   float* Xs = smem;
   float* As = Xs + TM * lda;
   float* Bs = As + TM * lda;
-  float* cent_s = Bs + KC * (64 * NJB + BPAD);
+  float* cent_s = Bs + b_ring_floats(NJB);
   float* thr_s = cent_s + 256;
   float* nrm = thr_s + 256;
   load_codebook(job.codebook, cent_s, thr_s);
@@ -712,7 +778,8 @@ __global__ void __launch_bounds__(NT) k_qjl_compress(TqQjlCompressJob job) {
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t row0 = tile * TM;
     __syncthreads();
-    load_tile_rows<XDT>(job.x, row0, n_total, D, job.H, job.S, job.stride_b, job.stride_h, job.stride_s, Xs, lda,
+    b_begin<NJ, B_KN>(D, job.rotation_t, D, D, Bs);
+    load_tile_rows<XDT, RI>(job.x, row0, n_total, D, job.H, job.S, job.stride_b, job.stride_h, job.stride_s, Xs, lda,
                         job.normalize ? nrm : nullptr);
     __syncwarp();
     for (int r = warp; r < TM; r += NT / 32) {
@@ -721,11 +788,12 @@ __global__ void __launch_bounds__(NT) k_qjl_compress(TqQjlCompressJob job) {
         As[r * lda + k] = job.normalize ? __fdiv_rn(Xs[r * lda + k], den) : Xs[r * lda + k];
     }
     {
-      float acc[4][4 * NJ];
-      zero_acc<NJ>(acc);
-      tile_gemm<NJ, B_KN>(As, lda, D, job.rotation_t, D, D, Bs, acc);
+      float acc[RI][4 * NJ];
+      zero_acc<RI, NJ>(acc);
+      tile_gemm<RI, NJ, B_KN>(As, lda, D, job.rotation_t, D, D, Bs, acc);
       __syncthreads();
-      acc_to_smem<NJ>(acc, As, lda, kpad);
+      b_begin<NJ, B_KN>(D, job.rotation, D, D, Bs);
+      acc_to_smem<RI, NJ>(acc, As, lda, kpad);
     }
     __syncthreads();
     // quantise in place: As <- centroid of the nearest level
@@ -745,14 +813,15 @@ __global__ void __launch_bounds__(NT) k_qjl_compress(TqQjlCompressJob job) {
       }
     }
     {
-      float acc[4][4 * NJ];
-      zero_acc<NJ>(acc);
-      tile_gemm<NJ, B_KN>(As, lda, D, job.rotation, D, D, Bs, acc);
+      float acc[RI][4 * NJ];
+      zero_acc<RI, NJ>(acc);
+      tile_gemm<RI, NJ, B_KN>(As, lda, D, job.rotation, D, D, Bs, acc);
       __syncthreads();
+      b_begin<NJM, B_KN>(D, job.qjl_t, M, M, Bs);
       // k_mse (fp32) -> optional fp16 output; residual = x - k_mse back into As
 #pragma unroll
-      for (int ri = 0; ri < 4; ++ri) {
-        int r = ty * 4 + ri;
+      for (int ri = 0; ri < RI; ++ri) {
+        int r = ty * RI + ri;
         int64_t n = row0 + r;
         float nv = job.normalize ? nrm[r] : 1.f;
 #pragma unroll
@@ -784,12 +853,12 @@ __global__ void __launch_bounds__(NT) k_qjl_compress(TqQjlCompressJob job) {
       }
     }
     {
-      float acc[4][4 * NJM];
-      zero_acc<NJM>(acc);
-      tile_gemm<NJM, B_KN>(As, lda, D, job.qjl_t, M, M, Bs, acc);
+      float acc[RI][4 * NJM];
+      zero_acc<RI, NJM>(acc);
+      tile_gemm<RI, NJM, B_KN>(As, lda, D, job.qjl_t, M, M, Bs, acc);
 #pragma unroll
-      for (int ri = 0; ri < 4; ++ri) {
-        int64_t n = row0 + ty * 4 + ri;
+      for (int ri = 0; ri < RI; ++ri) {
+        int64_t n = row0 + ty * RI + ri;
         if (n >= n_total) continue;
 #pragma unroll
         for (int j = 0; j < NJM; ++j)
@@ -822,7 +891,7 @@ __global__ void __launch_bounds__(NT) k_qjl_scores(TqQjlScoreJob job, const floa
   const int lda = lda_for(D);
   float* As = smem;
   float* Bs = As + TM * lda;
-  float* Cs = Bs + KC * (64 * NJ + BPAD);   // [64*NJ][TM+1]
+  float* Cs = Bs + b_ring_floats(NJ);   // [64*NJ][TM+1]
   const int ldc = TM + 1;
   const int64_t key_tiles = (job.Sk + TM - 1) / TM;
   const int64_t total = job.BH * key_tiles;
@@ -837,8 +906,8 @@ __global__ void __launch_bounds__(NT) k_qjl_scores(TqQjlScoreJob job, const floa
     for (int q0 = 0; q0 < job.Sq; q0 += 64 * NJ) {
       const int nq = (int)min((int64_t)(64 * NJ), job.Sq - q0);
       float acc1[4][4 * NJ], acc2[4][4 * NJ];
-      zero_acc<NJ>(acc1);
-      zero_acc<NJ>(acc2);
+      zero_acc<4, NJ>(acc1);
+      zero_acc<4, NJ>(acc2);
       __syncthreads();
       for (int r = warp; r < TM; r += NT / 32) {
         int64_t s = s0 + r;
@@ -846,18 +915,18 @@ __global__ void __launch_bounds__(NT) k_qjl_scores(TqQjlScoreJob job, const floa
           As[r * lda + k] = (s < job.Sk && k < D) ? __half2float(__ushort_as_half(km[s * D + k])) : 0.f;
       }
       // queries as B in [N][K] layout, converted to fp32 on the fly for 16-bit q
-      if constexpr (QDT == TQ_F32) {
-        tile_gemm<NJ, B_NK>(As, lda, D, reinterpret_cast<const float*>(job.q) + (bh * job.Sq + q0) * D, D, nq, Bs, acc1);
-      } else {
-        // 16-bit queries were upcast into the workspace behind qproj by the host wrapper
-        tile_gemm<NJ, B_NK>(As, lda, D, qproj + (job.BH * job.Sq + bh * job.Sq + q0) * D, D, nq, Bs, acc1);
-      }
+      // (16-bit queries were upcast into the workspace behind qproj by the host wrapper)
+      const float* qf = QDT == TQ_F32 ? reinterpret_cast<const float*>(job.q) + (bh * job.Sq + q0) * D
+                                      : qproj + (job.BH * job.Sq + bh * job.Sq + q0) * D;
+      b_begin<NJ, B_NK>(D, qf, D, nq, Bs);
+      tile_gemm<4, NJ, B_NK>(As, lda, D, qf, D, nq, Bs, acc1);
       __syncthreads();
       for (int r = warp; r < TM; r += NT / 32) {
         int64_t s = s0 + r;
         for (int k = lane; k < kpad; k += 32) As[r * lda + k] = (s < job.Sk && k < D) ? (float)sg[s * D + k] : 0.f;
       }
-      tile_gemm<NJ, B_NK>(As, lda, D, qproj + (bh * job.Sq + q0) * D, D, nq, Bs, acc2);
+      b_begin<NJ, B_NK>(D, qproj + (bh * job.Sq + q0) * D, D, nq, Bs);
+      tile_gemm<4, NJ, B_NK>(As, lda, D, qproj + (bh * job.Sq + q0) * D, D, nq, Bs, acc2);
       __syncthreads();
 #pragma unroll
       for (int ri = 0; ri < 4; ++ri) {
@@ -908,6 +977,68 @@ __global__ void __launch_bounds__(NT) k_prod_inner(const float* __restrict__ y, 
   }
 }
 
+// One query against every vector: <y, c[idx] Pi> = <y Pi^T, c[idx]>, so the query is rotated once instead of every
+// vector being rotated back.  k_query_rotate computes yr = y Pi^T and sy = y S^T.
+__global__ void __launch_bounds__(NT) k_query_rotate(const float* __restrict__ y, int D, int M, const float* __restrict__ rotation,
+                                                    const float* __restrict__ qjl_t, float* yr, float* sy) {
+  __shared__ float ys[TQ_MAX_DIM];
+  __shared__ float part[NT / 32][33];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int k = threadIdx.x; k < D; k += NT) ys[k] = y[k];
+  __syncthreads();
+  const int row_blocks = (D + 7) / 8;
+  if ((int)blockIdx.x < row_blocks) {                 // a warp per row of Pi
+    const int j = blockIdx.x * 8 + warp;
+    float t = 0.f;
+    if (j < D)
+      for (int k = lane; k < D; k += 32) t = fmaf(ys[k], __ldg(rotation + (int64_t)j * D + k), t);
+    t = warp_sum(t);
+    if (lane == 0 && j < D) yr[j] = t;
+  } else {                                            // 32 columns of S^T, its rows split over the warps
+    const int m = ((int)blockIdx.x - row_blocks) * 32 + lane;
+    float t = 0.f;
+    if (m < M)
+#pragma unroll 8
+      for (int k = warp; k < D; k += NT / 32) t = fmaf(ys[k], __ldg(qjl_t + (int64_t)k * M + m), t);
+    part[warp][lane] = t;
+    __syncthreads();
+    if (warp == 0 && m < M) {
+      float a = 0.f;
+#pragma unroll
+      for (int w = 0; w < NT / 32; ++w) a += part[w][lane];
+      sy[m] = a;
+    }
+  }
+}
+
+// out[n] = <yr, c[idx_n]> + (rnorm_n * corr) * <sy, signs_n>: a warp per vector, bound by reading the 8-byte indices and
+// 4-byte signs once.  8192 vectors of head_dim 128: 52 us as dequantise, projection and row products, 8 us so.
+__global__ void __launch_bounds__(NT) k_prod_inner_one(const int64_t* __restrict__ idx, const float* __restrict__ signs,
+                                                      const float* __restrict__ rnorm, int64_t n, int D, int M,
+                                                      const float* __restrict__ cb, const float* __restrict__ yr,
+                                                      const float* __restrict__ sy, float corr, float* out) {
+  __shared__ float cent_s[256];
+  __shared__ float yr_s[TQ_MAX_DIM], sy_s[TQ_MAX_DIM];
+  for (int i = threadIdx.x; i < 256; i += NT) {
+    cent_s[i] = __ldg(cb + kCentroidOff + i);
+    if (i < D) yr_s[i] = yr[i];
+    if (i < M) sy_s[i] = sy[i];
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t wstride = (int64_t)gridDim.x * (NT / 32);
+  for (int64_t r = (int64_t)blockIdx.x * (NT / 32) + warp; r < n; r += wstride) {
+    float t1 = 0.f, ip = 0.f;
+#pragma unroll 4
+    for (int k = lane; k < D; k += 32) t1 = fmaf(yr_s[k], cent_s[(int)(__ldg(idx + r * D + k) & 255)], t1);
+#pragma unroll 4
+    for (int k = lane; k < M; k += 32) ip = fmaf(sy_s[k], __ldg(signs + r * M + k), ip);
+    t1 = warp_sum(t1);
+    ip = warp_sum(ip);
+    if (lane == 0) out[r] = t1 + (rnorm[r] * corr) * ip;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
@@ -947,6 +1078,12 @@ static int set_smem(K kernel, size_t bytes) {
 
 static inline int nj_for(int n) { return (n + 63) / 64; }
 
+// Vectors per tile: 64 (RI = 4) reads the matrix once for more vectors, 32 (RI = 2) gives twice the CTAs and half the
+// work behind each barrier.  Below two tiles of 64 per SM the chip is not full either way and the small tile wins.
+// With the ring, head_dim 128 in fp32: 4096 vectors quantised in 40 -> 19 us; 8192 vectors quantised in 32 -> 22 us, rebuilt in
+// 37 -> 26 us, MSE + QJL compressed in 78 -> 50 us (single launches, cold caches).
+static inline bool small_tiles(int64_t n) { return n < (int64_t)2 * TM * sm_count(); }
+
 #define TQ_DISPATCH_NJ(nj, ...)                              \
   switch (nj) {                                              \
     case 1: { constexpr int NJ_ = 1; __VA_ARGS__; } break;   \
@@ -974,11 +1111,13 @@ int simt_quantize(const TqQuantizeJob& job, cudaStream_t st) {
   const int64_t n = job.B * job.H * job.S;
   if (n == 0) return TQ_OK;
   const int nj = nj_for(job.D);
-  const size_t smem = sizeof(float) * (TM * lda_for(job.D) + KC * (64 * nj + BPAD) + 512 + TM);
-  const int grid = grid_for((n + TM - 1) / TM, 2);
+  const bool small = small_tiles(n);
+  const int tm = small ? TM / 2 : TM;
+  const size_t smem = sizeof(float) * (tm * lda_for(job.D) + b_ring_floats(nj) + 512 + tm);
+  const int grid = grid_for((n + tm - 1) / tm, 2);
   int rc = TQ_OK;
   TQ_DISPATCH_DT(job.x_dtype, TQ_DISPATCH_NJ(nj, {
-    auto kern = k_quantize<DT_, NJ_>;
+    auto kern = small ? k_quantize<DT_, NJ_, 2> : k_quantize<DT_, NJ_, 4>;
     rc = set_smem(kern, smem);
     if (rc == TQ_OK) kern<<<grid, NT, smem, st>>>(job);
   }));
@@ -989,11 +1128,13 @@ int simt_dequantize(const TqDequantizeJob& job, cudaStream_t st) {
   const int64_t n = job.B * job.H * job.S;
   if (n == 0) return TQ_OK;
   const int nj = nj_for(job.D);
-  const size_t smem = sizeof(float) * (TM * lda_for(job.D) + KC * (64 * nj + BPAD) + 512);
-  const int grid = grid_for((n + TM - 1) / TM, 2);
+  const bool small = small_tiles(n);
+  const int tm = small ? TM / 2 : TM;
+  const size_t smem = sizeof(float) * (tm * lda_for(job.D) + b_ring_floats(nj) + 512);
+  const int grid = grid_for((n + tm - 1) / tm, 2);
   int rc = TQ_OK;
   TQ_DISPATCH_DT(job.out_dtype, TQ_DISPATCH_NJ(nj, {
-    auto kern = k_dequantize<DT_, NJ_>;
+    auto kern = small ? k_dequantize<DT_, NJ_, 2> : k_dequantize<DT_, NJ_, 4>;
     rc = set_smem(kern, smem);
     if (rc == TQ_OK) kern<<<grid, NT, smem, st>>>(job);
   }));
@@ -1012,7 +1153,7 @@ int simt_project(const void* x, int x_dtype, int64_t n, int K, const float* m, i
     return check_launch();
   }
   const int nj = nj_for(N);
-  const size_t smem = sizeof(float) * (TM * lda_for(K) + KC * (64 * nj + BPAD));
+  const size_t smem = sizeof(float) * (TM * lda_for(K) + b_ring_floats(nj));
   const int grid = grid_for((n + TM - 1) / TM, 2);
   int rc = TQ_OK;
   TQ_DISPATCH_DT(x_dtype, TQ_DISPATCH_NJ(nj, {
@@ -1076,12 +1217,14 @@ int simt_qjl_compress(const TqQjlCompressJob& job, cudaStream_t st) {
   if (n == 0) return TQ_OK;
   const int nj = nj_for(job.D), njm = nj_for(job.M);
   const int njb = nj > njm ? nj : njm;
-  const size_t smem = sizeof(float) * (2 * TM * lda_for(job.D) + KC * (64 * njb + BPAD) + 512 + TM);
-  const int grid = grid_for((n + TM - 1) / TM, 1);
+  const bool small = small_tiles(n);
+  const int tm = small ? TM / 2 : TM;
+  const size_t smem = sizeof(float) * (2 * tm * lda_for(job.D) + b_ring_floats(njb) + 512 + tm);
+  const int grid = grid_for((n + tm - 1) / tm, small ? 2 : 1);
   int rc = TQ_OK;
   // the projection width shares the head_dim's tile class unless it is wider
   TQ_DISPATCH_DT(job.x_dtype, TQ_DISPATCH_NJ(njb, {
-    auto kern = k_qjl_compress<DT_, NJ_, NJ_>;
+    auto kern = small ? k_qjl_compress<DT_, NJ_, NJ_, 2> : k_qjl_compress<DT_, NJ_, NJ_, 4>;
     rc = set_smem(kern, smem);
     if (rc == TQ_OK) kern<<<grid, NT, smem, st>>>(job);
   }));
@@ -1120,7 +1263,7 @@ int simt_qjl_scores(const TqQjlScoreJob& job, cudaStream_t st) {
   if (rc != TQ_OK) return rc;
   const float* qproj = qproj_c;
   const int nj = nj_for((int)(job.Sq < 256 ? job.Sq : 256));
-  const size_t smem = sizeof(float) * (TM * lda_for(job.D) + KC * (64 * nj + BPAD) + 64 * nj * (TM + 1));
+  const size_t smem = sizeof(float) * (TM * lda_for(job.D) + b_ring_floats(nj) + 64 * nj * (TM + 1));
   const int64_t tiles = job.BH * ((job.Sk + TM - 1) / TM);
   const int grid = grid_for(tiles, 1);
   const float corr = (float)(1.2533141373155001 / (double)job.D);   // sqrt(pi/2) / m with m = D
@@ -1144,8 +1287,18 @@ int simt_prod_inner_product(const float* y, int64_t ny, const int64_t* idx, cons
                             int64_t n, int D, int M, const float* rotation, const float* codebook, const float* qjl_t,
                             float* out, void* workspace, cudaStream_t st) {
   if (n == 0) return TQ_OK;
+  const float corr = (float)(1.2533141373155001 / (double)M);
   float* xhat = reinterpret_cast<float*>(workspace);
   float* sy = xhat + n * 256;
+  if (ny == 1) {
+    float* yr = xhat;
+    k_query_rotate<<<(unsigned)((D + 7) / 8 + (M + 31) / 32), NT, 0, st>>>(y, D, M, rotation, qjl_t, yr, sy);
+    int rc = check_launch();
+    if (rc != TQ_OK) return rc;
+    const int grid = grid_for((n + NT / 32 - 1) / (NT / 32), 8);
+    k_prod_inner_one<<<grid, NT, 0, st>>>(idx, signs, rnorm, n, D, M, codebook, yr, sy, corr, out);
+    return check_launch();
+  }
   TqDequantizeJob dj{};
   dj.idx = idx; dj.norms = nullptr; dj.idx_mode = TQ_IDX_I64; dj.D = D; dj.bits = 8; dj.out_dtype = TQ_F32;
   dj.B = 1; dj.H = 1; dj.S = n; dj.out = xhat; dj.ostride_b = 0; dj.ostride_h = 0; dj.ostride_s = D;
@@ -1154,7 +1307,6 @@ int simt_prod_inner_product(const float* y, int64_t ny, const int64_t* idx, cons
   if (rc != TQ_OK) return rc;
   rc = simt_project(y, TQ_F32, ny, D, qjl_t, M, sy, st);
   if (rc != TQ_OK) return rc;
-  const float corr = (float)(1.2533141373155001 / (double)M);
   int grid = grid_for((n + NT / 32 - 1) / (NT / 32), 8);
   k_prod_inner<<<grid, NT, 0, st>>>(y, ny, xhat, sy, signs, rnorm, n, D, M, corr, out);
   return check_launch();
