@@ -525,11 +525,7 @@ int tq_qjl_scores(const TqQjlScoreJob* job, void* stream) {
   if (tq::umma_qjl_scores_eligible(*job)) {
     const size_t img = tq::umma_qjl_scores_image_bytes(job->BH, job->Sq, job->D);
     if (job->workspace_bytes < simt_ws + img) return TQ_EWORKSPACE;
-    const float* qf = nullptr;
-    const float* qproj = nullptr;
-    int rc = tq::simt_qjl_queries(*job, &qf, &qproj, (cudaStream_t)stream);
-    if (rc != TQ_OK) return rc;
-    return tq::umma_qjl_scores(*job, qf, qproj, reinterpret_cast<char*>(job->workspace) + simt_ws, (cudaStream_t)stream);
+    return tq::umma_qjl_scores(*job, reinterpret_cast<char*>(job->workspace) + simt_ws, (cudaStream_t)stream);
   }
   return tq::simt_qjl_scores(*job, (cudaStream_t)stream);
 }

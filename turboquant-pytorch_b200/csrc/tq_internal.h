@@ -75,7 +75,8 @@ int umma_v2_device_status();
 // tensor-core asymmetric scores of the MSE+QJL representation (tq_qjl_umma.cu)
 bool umma_qjl_scores_eligible(const TqQjlScoreJob& job);
 size_t umma_qjl_scores_image_bytes(int64_t BH, int64_t Sq, int D);
-int umma_qjl_scores(const TqQjlScoreJob& job, const float* qf, const float* qproj, void* images, cudaStream_t st);
+int umma_qjl_scores(const TqQjlScoreJob& job, void* images, cudaStream_t st);
+int simt_qjl_query_operand(const TqQjlScoreJob& job, void* images, cudaStream_t st);
 int umma_qjl_device_status();
 
 }  // namespace tq

@@ -86,35 +86,6 @@ __device__ __forceinline__ uint32_t idesc_f16_n(uint32_t n) {
   return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
-// Query image of one unit: row n = query q0 + n of head bh (zero past Sq), contraction index
-// j < D -> Q[n][j], j >= D -> corr * (S Q)[n][j - D]; value = hi + lo in fp16.  Stored as
-// [piece][chunk][row n][64 columns], rows of 128 bytes, 16-byte chunk c at c ^ (n & 7).
-constexpr int kImageSplit = 16;               // blocks per unit in the image kernel
-template <int D>
-__global__ void k_qjl_query_image(const float* __restrict__ qf, const float* __restrict__ qproj, float corr, int64_t Sq,
-                                  int n_qblocks, uint8_t* __restrict__ images) {
-  constexpr int kChunks = QCfg<D>::kChunks;
-  const int unit = blockIdx.x / kImageSplit, part = blockIdx.x % kImageSplit;
-  const int64_t bh = unit / n_qblocks;
-  const int q0 = (unit % n_qblocks) * kQ;
-  uint16_t* img = reinterpret_cast<uint16_t*>(images + (size_t)unit * QCfg<D>::kImageBytes);
-  constexpr int kPer = kQ * 2 * D / kImageSplit;
-  for (int e = part * kPer + threadIdx.x; e < (part + 1) * kPer; e += blockDim.x) {
-    const int n = e / (2 * D), j = e % (2 * D);
-    float v = 0.f;
-    if (q0 + n < Sq) {
-      const int64_t row = bh * Sq + q0 + n;
-      v = j < D ? qf[row * D + j] : corr * qproj[row * D + (j - D)];
-    }
-    const __half hi = __float2half_rn(v);
-    const __half lo = __float2half_rn(v - __half2float(hi));
-    const int chunk = j / 64, c = (j % 64) / 8, w = j % 8;
-    const size_t off = (size_t)chunk * (kChunkB / 2) + (size_t)n * 64 + (size_t)((c ^ (n & 7)) * 8 + w);
-    img[off] = __half_as_ushort(hi);
-    img[(size_t)kChunks * (kChunkB / 2) + off] = __half_as_ushort(lo);
-  }
-}
-
 template <int D>
 __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_constant__ QjlBatch batch) {
   using C = QCfg<D>;
@@ -378,7 +349,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
 }
 
 template <int D>
-int launch(const TqQjlScoreJob& job, const float* qf, const float* qproj, uint8_t* images, cudaStream_t st) {
+int launch(const TqQjlScoreJob& job, uint8_t* images, cudaStream_t st) {
   TensorMapEncodeFn enc = tensor_map_encoder();
   if (enc == nullptr) return TQ_ELAUNCH;
   static thread_local QjlBatch batch;
@@ -400,9 +371,7 @@ int launch(const TqQjlScoreJob& job, const float* qf, const float* qproj, uint8_
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { note_cuda_error(100000 + (int)r); return TQ_ELAUNCH; }
-  const float corr = (float)(1.2533141373155001 / (double)D);   // sqrt(pi/2) / m with m = D
-  k_qjl_query_image<D><<<(unsigned)(units * kImageSplit), 256, 0, st>>>(qf, qproj, corr, job.Sq, n_qblocks, images);
-  int rc = check_launch();
+  int rc = simt_qjl_query_operand(job, images, st);
   if (rc != TQ_OK) return rc;
   batch.rnorm = job.rnorm;
   batch.images = images;
@@ -444,10 +413,10 @@ size_t umma_qjl_scores_image_bytes(int64_t BH, int64_t Sq, int D) {
   return (size_t)units * (D == 256 ? QCfg<256>::kImageBytes : QCfg<128>::kImageBytes) + 1024;
 }
 
-// qf: the queries as fp32 (BH, Sq, D); qproj: S-projected queries (BH, Sq, D); images: scratch
-int umma_qjl_scores(const TqQjlScoreJob& job, const float* qf, const float* qproj, void* images, cudaStream_t st) {
+// images: scratch for the query operands
+int umma_qjl_scores(const TqQjlScoreJob& job, void* images, cudaStream_t st) {
   uint8_t* img = reinterpret_cast<uint8_t*>(((uintptr_t)images + 1023u) & ~(uintptr_t)1023u);
-  return job.D == 256 ? launch<256>(job, qf, qproj, img, st) : launch<128>(job, qf, qproj, img, st);
+  return job.D == 256 ? launch<256>(job, img, st) : launch<128>(job, img, st);
 }
 
 int umma_qjl_device_status() {

@@ -952,6 +952,53 @@ __global__ void __launch_bounds__(NT) k_qjl_scores(TqQjlScoreJob job, const floa
   }
 }
 
+// Query operand of the tensor-core score kernel (tq_qjl_umma.cu), head_dim a multiple of 64: per unit (head, block of
+// 64 queries) the rows [Q | corr * Q S^T] as fp16 pieces hi + lo, laid out [piece][chunk of 64 columns][row][64], rows of
+// 128 bytes with 16-byte chunk c at c ^ (row & 7); rows past Sq are zero.  A CTA takes 32 rows and 64 columns: the
+// projection (one sequential chain per output, as tq_project), then the query's own columns and the projected ones.
+// 1024 queries of head_dim 256 took 27 us as projection, upcast and image kernels (the projection read the whole matrix
+// for every four rows).
+template <int QDT>
+__global__ void __launch_bounds__(NT) k_qjl_query_operand(const void* q, int D, int64_t Sq, int n_qblocks,
+                                                         const float* __restrict__ qjl_t, float corr, uint8_t* __restrict__ images) {
+  constexpr int RI = 2, ROWS = 16 * RI;
+  extern __shared__ __align__(16) float smem[];
+  const int lda = lda_for(D);
+  float* As = smem;
+  float* Bs = As + ROWS * lda;
+  const int chunks = D / 64;
+  const int cb = blockIdx.x % chunks, half = (blockIdx.x / chunks) & 1, unit = blockIdx.x / (2 * chunks);
+  const int64_t bh = unit / n_qblocks;
+  const int64_t q0 = (int64_t)(unit % n_qblocks) * 64 + half * ROWS;       // first query of this CTA, of head bh
+  b_begin<1, B_KN>(D, qjl_t + cb * 64, D, 64, Bs);
+  // rows past the end of this head read as zero, so the row limit is the head's own end
+  load_tile_rows<QDT, RI>(q, bh * Sq + q0, (bh + 1) * Sq, D, 1, (bh + 1) * Sq, 0, 0, D, As, lda, nullptr);
+  float acc[RI][4];
+  zero_acc<RI, 1>(acc);
+  tile_gemm<RI, 1, B_KN>(As, lda, D, qjl_t + cb * 64, D, 64, Bs, acc);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const size_t piece = (size_t)2 * chunks * 64 * 64;                       // elements of one piece
+  uint16_t* img = reinterpret_cast<uint16_t*>(images) + (size_t)unit * 2 * piece;
+#pragma unroll
+  for (int ri = 0; ri < RI; ++ri) {
+    const int r = ty * RI + ri, n = half * ROWS + r;
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {                                 // the query's columns, then the projected ones
+      uint16_t hi[4], lo[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float v = part == 0 ? As[r * lda + cb * 64 + 4 * tx + c] : corr * acc[ri][c];
+        const __half h = __float2half_rn(v);
+        hi[c] = __half_as_ushort(h);
+        lo[c] = __half_as_ushort(__float2half_rn(v - __half2float(h)));
+      }
+      const size_t off = (size_t)(part * chunks + cb) * (64 * 64) + (size_t)n * 64 + (size_t)((((4 * tx) >> 3) ^ (n & 7)) * 8 + ((4 * tx) & 7));
+      *reinterpret_cast<uint2*>(img + off) = make_uint2(hi[0] | ((uint32_t)hi[1] << 16), hi[2] | ((uint32_t)hi[3] << 16));
+      *reinterpret_cast<uint2*>(img + piece + off) = make_uint2(lo[0] | ((uint32_t)lo[1] << 16), lo[2] | ((uint32_t)lo[3] << 16));
+    }
+  }
+}
+
 // upcast a 16-bit tensor to fp32
 template <int XDT>
 __global__ void k_upcast(const void* x, int64_t n, float* out) {
@@ -1233,6 +1280,20 @@ int simt_qjl_compress(const TqQjlCompressJob& job, cudaStream_t st) {
 
 size_t simt_qjl_scores_workspace(int64_t BH, int64_t Sq, int D) {
   return (size_t)2 * BH * Sq * D * sizeof(float);   // projected queries + room for upcast queries
+}
+
+int simt_qjl_query_operand(const TqQjlScoreJob& job, void* images, cudaStream_t st) {
+  const int n_qblocks = (int)((job.Sq + 63) / 64);
+  const int64_t blocks = job.BH * n_qblocks * 2 * (job.D / 64);
+  const size_t smem = sizeof(float) * (32 * lda_for(job.D) + b_ring_floats(1));
+  const float corr = (float)(1.2533141373155001 / (double)job.D);   // sqrt(pi/2) / m with m = D
+  int rc = TQ_OK;
+  TQ_DISPATCH_DT(job.q_dtype, {
+    auto kern = k_qjl_query_operand<DT_>;
+    rc = set_smem(kern, smem);
+    if (rc == TQ_OK) kern<<<(unsigned)blocks, NT, smem, st>>>(job.q, job.D, job.Sq, n_qblocks, job.qjl_t, corr, reinterpret_cast<uint8_t*>(images));
+  });
+  return rc != TQ_OK ? rc : check_launch();
 }
 
 int simt_qjl_queries(const TqQjlScoreJob& job, const float** qf_out, const float** qproj_out, cudaStream_t st) {
