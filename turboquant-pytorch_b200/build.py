@@ -21,6 +21,8 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "turboquant", "libturboquant_b200.so")
 SOURCES = ["tq_api.cu", "tq_simt.cu", "tq_umma.cu", "tq_qjl_umma.cu", "tq_v2_umma.cu", "tq_score_static.cu", "tq_copy.cu", "tq_attn_mma.cu", "tq_qjl_packed.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+HOST_SRC = os.path.join(CSRC, "tq_host.cpp")
+HOST_OUT = os.path.join(HERE, "turboquant", "_tq_host.so")
 
 
 def nvcc_path() -> str:
@@ -42,12 +44,34 @@ def stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_host(force: bool = False) -> str:
+    """Compile the Python extension that fills in and submits the jobs (no kernels in it)."""
+    deps = [HOST_SRC, os.path.join(HERE, "..", "include", "turboquant_b200.h")]
+    if not force and os.path.exists(HOST_OUT) and all(os.path.getmtime(d) <= os.path.getmtime(HOST_OUT) for d in deps):
+        return HOST_OUT
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(os.path.abspath(torch.__file__))
+    cuda = os.path.join(os.path.dirname(nvcc_path()), "..", "include")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-I" + sysconfig.get_paths()["include"],
+           "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-I" + cuda, "-o", HOST_OUT, HOST_SRC, "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           "-ltorch_python"]
+    print(" ".join(cmd), flush=True)
+    subprocess.check_call(cmd)
+    return HOST_OUT
+
+
 def build(force: bool = False, verbose: bool = False, ablate: bool = False, out: str = OUT, defines=()) -> str:
     """Compile the library.  `ablate` adds -DTQ_ABLATION: the timing-only switches that skip parts of the
     tensor-core kernels (environment variable TQ_ABLATE) exist only in such a build; give it its own `out`
     path and load it through TURBOQUANT_B200_LIB, never as the in-tree library."""
     if ablate and os.path.abspath(out) == os.path.abspath(OUT):
         raise ValueError("an ablation build must not replace the in-tree library: pass --out")
+    if out == OUT:
+        build_host(force)
     if not force and out == OUT and not stale():
         return OUT
     # --fmad=false: products that the reference rounds before adding (k_mse before the

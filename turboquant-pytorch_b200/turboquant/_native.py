@@ -156,6 +156,26 @@ def lib():
     return L
 
 
+_host = None
+
+
+def host():
+    """The extension that does the per-call host work for plain CUDA tensors (csrc/tq_host.cpp), bound to lib()."""
+    global _host
+    if _host is None:
+        L = lib()
+        try:
+            from . import _tq_host as H
+        except ImportError as e:
+            raise RuntimeError(f"{os.path.join(_HERE, '_tq_host.so')} is missing or does not load ({e}): build it with "
+                               "`python turboquant-pytorch_b200/build.py`.") from e
+        H.bind(*(C.cast(getattr(L, n), C.c_void_p).value for n in
+                 ("tq_quantize", "tq_dequantize", "tq_copy_rows", "tq_qjl_compress", "tq_qjl_compress_workspace_bytes",
+                  "tq_prod_inner_product")), check)
+        _host = H
+    return _host
+
+
 def check(rc: int, what: str):
     """Map a TQ_E* code to the Python exception a caller of the reference would expect."""
     if rc == 0:

@@ -240,6 +240,17 @@ def qjl_compress(x: torch.Tensor, pi: torch.Tensor, pi_t: torch.Tensor, codebook
     """MSE stage + QJL signs for a (B,H,S,D) tensor.  Returns (k_mse|None, idx|None, signs (n,M), rnorm (n,)), and
     the fp32 vector norms (n,) as a fifth value with want_vec_norms."""
     N.require_cuda(x, "qjl_compress")
+    form = -1
+    if not want_vec_norms:
+        if normalize and want_k_mse and idx_mode is None and not signs_fp32 and not rnorm_fp32:
+            form = 0
+        elif not normalize and not want_k_mse and idx_mode == N.IDX_I64 and signs_fp32 and rnorm_fp32:
+            form = 2
+    if form >= 0:
+        done = N.host().qjl_compress(x, pi, pi_t, codebook, qjl_t, bits, form)
+        if done is not None:
+            first, signs, rnorm = done
+            return (first, None, signs, rnorm) if form == 0 else (None, first, signs, rnorm)
     B, H, S, D = x.shape
     x, sb, sh, ss = N.bhs_strides(x)
     n = B * H * S
@@ -280,6 +291,9 @@ def qjl_compress_packed(x: torch.Tensor, pi: torch.Tensor, pi_t: torch.Tensor, c
     rows from its epilogues; inputs it does not take go through the unpacked outputs and tq_pack_mse_qjl."""
     N.require_cuda(x, "qjl_compress")
     B, H, S, D = x.shape
+    done = N.host().qjl_compress(x, pi, pi_t, codebook, qjl_t, bits, 1)
+    if done is not None:
+        return done
     n = B * H * S
     dev = x.device
     L = N.lib()
@@ -381,6 +395,9 @@ def prod_inner_product(y: torch.Tensor, idx: torch.Tensor, signs: torch.Tensor, 
                        codebook: torch.Tensor, qjl_t: torch.Tensor) -> torch.Tensor:
     """Row-paired estimator; y is (n, D) or a single row (1, D)."""
     N.require_cuda(idx, "prod_inner_product")
+    done = N.host().prod_inner(y, idx, signs, rnorm, pi, codebook, qjl_t)
+    if done is not None:
+        return done
     n, D = idx.shape
     M = signs.shape[1]
     y = y.float().contiguous()

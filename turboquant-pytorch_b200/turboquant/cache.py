@@ -168,16 +168,29 @@ class V3Cache(_Base):
                                  dstride_b=buf.stride(0), dstride_h=buf.stride(1), dstride_s=buf.stride(2))
         base = [(st.k.data_ptr(), st.v.data_ptr()) for st in sts]
         cap = min(min(st.k.shape[2], st.v.shape[2]) for st in sts)
+        # the same for the native form of step(), which keeps its own copy of the job arrays
+        native = N.host().step_plan(bytes(q), bytes(d), bytes(c), row_bytes, [x for pair in base for x in pair],
+                                    (L, B, H, D, cap, self.residual_window, D * eb, N.dtype_code(like), like.device.index))
         return {"L": L, "B": B, "H": H, "D": D, "eb": eb, "dtype": like.dtype, "device": like.device, "q": q, "d": d, "c": c,
-                "row_bytes": row_bytes, "base": base, "cap": cap, "tok_bytes": D * eb}
+                "row_bytes": row_bytes, "base": base, "cap": cap, "tok_bytes": D * eb, "native": native, "states": sts,
+                "window": self.residual_window}
 
-    @torch.no_grad()
     def step(self, key_states: Sequence[torch.Tensor], value_states: Sequence[torch.Tensor], return_views: bool = True):
         """One step for layers 0..L-1 at once: append key_states[l] / value_states[l] ((B, H, S_new, D) each) to
         layer l, quantise what left the window and put its reconstruction in place.  Three library calls in all.
 
         Returns [(keys, values)] per layer as update() would (views of the persistent buffers), or None with
         return_views=False.  Falls back to per-layer update() calls while layers are being created or grown."""
+        p = self._step_plan
+        if p is not None and p["native"] is not None and p["L"] == len(key_states) and p["window"] == self.residual_window:
+            done = N.host().step(p["native"], p["states"], key_states, value_states, return_views)
+            if done is not None:
+                return done if return_views else None
+        return self._step_general(key_states, value_states, return_views)
+
+    @torch.no_grad()
+    def _step_general(self, key_states, value_states, return_views):
+        """step() in Python: the first call, calls that create or grow layers, and inputs the native form does not take."""
         L = len(key_states)
         k0 = key_states[0]
         B, H, S_new, D = k0.shape

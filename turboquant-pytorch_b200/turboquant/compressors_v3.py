@@ -56,16 +56,30 @@ class MSECompressor:
         return _ops.dequantize_job(compressed["idx_bytes"], compressed["vec_norms"], compressed["shape"], self.Pi,
                                    self._cb, self.bits, N.IDX_PACKED, out, image=self._img_d)
 
-    @torch.no_grad()
     def compress(self, states: torch.Tensor) -> dict:
         """(B, H, S, D) -> {"idx_bytes" uint8 (B,H,S,G), "vec_norms" fp16 (B,H,S), "shape", "idx_pad"}."""
+        if states.is_cuda:
+            result = N.host().compress(self, states)
+            if result is not None:
+                return result
+        return self._compress_general(states)
+
+    @torch.no_grad()
+    def _compress_general(self, states: torch.Tensor) -> dict:
         job, result, _keep = self.compress_job(states)
         _ops.run_quantize([job], states.device)
         return result
 
-    @torch.no_grad()
     def decompress(self, compressed: dict) -> torch.Tensor:
         """Back to an fp32 (B, H, S, D) tensor."""
+        if compressed["idx_bytes"].is_cuda:
+            out = N.host().decompress(self, compressed)
+            if out is not None:
+                return out
+        return self._decompress_general(compressed)
+
+    @torch.no_grad()
+    def _decompress_general(self, compressed: dict) -> torch.Tensor:
         B, H, S, D = compressed["shape"]
         out = torch.empty((B, H, S, D), dtype=torch.float32, device=compressed["idx_bytes"].device)
         job, _keep = self.decompress_job(compressed, out)
@@ -125,8 +139,15 @@ class TurboQuantV3:
         cv = {"compressed": rv, "fp16": values[:, :, cut:, :], "shape": (B, H, S, D), "split_at": cut}
         return [jk, jv], (ck, cv), (keep_k, keep_v)
 
-    @torch.no_grad()
     def compress_kv(self, keys: torch.Tensor, values: torch.Tensor):
+        if keys.is_cuda:
+            result = N.host().compress_kv(self.key_compressor, self.val_compressor, keys, values, self.residual_window)
+            if result is not None:
+                return result
+        return self._compress_kv_general(keys, values)
+
+    @torch.no_grad()
+    def _compress_kv_general(self, keys: torch.Tensor, values: torch.Tensor):
         jobs, result, _keep = self.compress_jobs(keys, values)
         if jobs:
             _ops.run_quantize(jobs, keys.device)
@@ -148,10 +169,17 @@ class TurboQuantV3:
             outs.append(full)
         return jobs, tuple(outs), keep
 
-    @torch.no_grad()
     def decompress_kv(self, compressed_k: dict, compressed_v: dict):
         if compressed_k["compressed"] is None:
             return compressed_k["fp16"], compressed_v["fp16"]
+        if compressed_k["fp16"].is_cuda:
+            result = N.host().decompress_kv(self.key_compressor, self.val_compressor, compressed_k, compressed_v)
+            if result is not None:
+                return result
+        return self._decompress_kv_general(compressed_k, compressed_v)
+
+    @torch.no_grad()
+    def _decompress_kv_general(self, compressed_k: dict, compressed_v: dict):
         jobs, outs, _keep = self.decompress_jobs(compressed_k, compressed_v)
         _ops.run_dequantize(jobs, outs[0].device)
         return outs

@@ -79,12 +79,20 @@ class TurboQuantMSE(nn.Module):
         return _ops.project(y, self.Pi)
 
     def quantize(self, x: torch.Tensor) -> torch.Tensor:
+        if x.is_cuda:
+            out = N.host().quantize_rows(x, self._pi_t, self._cb, self.bits, self.d)
+            if out is not None:
+                return out
         flat = x.reshape(1, 1, -1, self.d)
         job, idx, _norms, keep = _ops.quantize_job(flat, self._pi_t, self._cb, self.bits, False, N.IDX_I64)
         _ops.run_quantize([job], x.device)
         return idx.reshape(x.shape)
 
     def dequantize(self, indices: torch.Tensor) -> torch.Tensor:
+        if indices.is_cuda:
+            out = N.host().dequantize_rows(indices, self.Pi, self._cb, self.bits, self.d)
+            if out is not None:
+                return out
         n = indices.numel() // self.d
         out = torch.empty((1, 1, n, self.d), dtype=torch.float32, device=indices.device)
         job, keep = _ops.dequantize_job(indices.reshape(n, self.d), None, (1, 1, n, self.d), self.Pi, self._cb,
