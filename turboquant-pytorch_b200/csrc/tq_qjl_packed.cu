@@ -22,8 +22,6 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kQB = 64;                        // queries per CTA
-constexpr int kNT = kQB / 8;                   // 8-query tiles
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                           uint32_t b1) {
@@ -125,8 +123,12 @@ struct PackedScoreParams {
 // word (((nt * 2 KS + ks) * 32 + lane) * 4 + r), r = {hi k0, hi k1, lo k0, lo k1}: the B registers of
 // 8-query tile nt, k-step ks (first KS steps: q Pi^T, then coef * S q), for lane (n = lane / 4, t = lane % 4)
 // coordinates D/4 * t + 4 ks' + {0, 1} (k0) and + {2, 3} (k1).
-template <int BITS, int D>
-__global__ void __launch_bounds__(kThreads, 1) k_qjl_score_packed(PackedScoreParams P) {
+// NT: tiles of 8 queries that a CTA computes, 2 (up to 16 queries) or 8: with eight tiles for 16 queries three quarters of the
+// MMAs were padding.  8 heads x 4096 keys of head_dim 128, 16 queries: compress + scores 87 -> 63 us, with one launch for both
+// projections and one for the three operand images.
+template <int BITS, int D, int NT>
+__global__ void __launch_bounds__(kThreads, NT <= 2 ? 2 : 1) k_qjl_score_packed(PackedScoreParams P) {
+  constexpr int kNT = NT, kQB = 8 * NT;
   using C = PK<BITS, D>;
   constexpr int KS = C::KS, CW = C::CW, SW = C::SW, DQ = C::DQ;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -264,7 +266,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_qjl_score_packed(PackedScorePar
   (void)sgn; (void)img_base;
 }
 
-template <int D>
+template <int D, int NT>
 int launch_packed(const PackedScoreParams& P, int bits, unsigned grid, size_t smem, cudaStream_t st) {
   auto go = [&](auto kern) -> int {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -273,14 +275,14 @@ int launch_packed(const PackedScoreParams& P, int bits, unsigned grid, size_t sm
     return check_launch();
   };
   switch (bits) {
-    case 1: return go(k_qjl_score_packed<1, D>);
-    case 2: return go(k_qjl_score_packed<2, D>);
-    case 3: return go(k_qjl_score_packed<3, D>);
-    case 4: return go(k_qjl_score_packed<4, D>);
-    case 5: return go(k_qjl_score_packed<5, D>);
-    case 6: return go(k_qjl_score_packed<6, D>);
-    case 7: return go(k_qjl_score_packed<7, D>);
-    default: return go(k_qjl_score_packed<8, D>);
+    case 1: return go(k_qjl_score_packed<1, D, NT>);
+    case 2: return go(k_qjl_score_packed<2, D, NT>);
+    case 3: return go(k_qjl_score_packed<3, D, NT>);
+    case 4: return go(k_qjl_score_packed<4, D, NT>);
+    case 5: return go(k_qjl_score_packed<5, D, NT>);
+    case 6: return go(k_qjl_score_packed<6, D, NT>);
+    case 7: return go(k_qjl_score_packed<7, D, NT>);
+    default: return go(k_qjl_score_packed<8, D, NT>);
   }
 }
 
@@ -307,10 +309,10 @@ int qjl_scores_packed(const TqQjlPackedScoreJob& job, cudaStream_t st) {
   const size_t one = ((size_t)rows * D * sizeof(float) + 255) / 256 * 256;
   float* qrot = reinterpret_cast<float*>(job.workspace);
   float* qproj = reinterpret_cast<float*>(reinterpret_cast<char*>(job.workspace) + one);
-  int rc = simt_project(job.q, job.q_dtype, rows, D, job.rotation_t, D, qrot, st);
+  int rc = simt_project_two(job.q, job.q_dtype, rows, D, job.rotation_t, job.qjl_t, qrot, qproj, st);
   if (rc != TQ_OK) return rc;
-  rc = simt_project(job.q, job.q_dtype, rows, D, job.qjl_t, D, qproj, st);
-  if (rc != TQ_OK) return rc;
+  const bool few = job.Sq <= 16;
+  const int nt = few ? 2 : 8, qb = 8 * nt;
   PackedScoreParams P;
   P.qrot = qrot; P.qproj = qproj;
   P.idx = job.idx_packed; P.sign_bits = job.sign_bits; P.vec_norms = job.vec_norms; P.rnorm = job.rnorm;
@@ -318,20 +320,21 @@ int qjl_scores_packed(const TqQjlPackedScoreJob& job, cudaStream_t st) {
   P.scores = job.scores;
   P.BH = job.BH; P.Sq = job.Sq; P.Sk = job.Sk;
   P.coef = 1.2533141373155003f / (float)D;            // sqrt(pi / 2) / m, m = D rows of S
-  P.n_qblocks = (int)((job.Sq + kQB - 1) / kQB);
+  P.n_qblocks = (int)((job.Sq + qb - 1) / qb);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // enough key splits to fill the GPU, at least 256 keys each
   int64_t units = job.BH * P.n_qblocks;
-  int64_t want = (2 * sms + units - 1) / units;
-  int64_t max_split = (job.Sk + 255) / 256;
+  int64_t want = ((few ? 4 : 2) * sms + units - 1) / units;
+  int64_t max_split = few ? (job.Sk + 127) / 128 : (job.Sk + 255) / 256;
   if (want > max_split) want = max_split;
   if (want < 1) want = 1;
   P.n_ksplit = (int)want;
   const unsigned grid = (unsigned)(units * P.n_ksplit);
-  const size_t smem = 2048 + (size_t)kNT * 2 * (D / 16) * 32 * 16 + 1024;
-  return D == 128 ? launch_packed<128>(P, job.bits, grid, smem, st) : launch_packed<256>(P, job.bits, grid, smem, st);
+  const size_t smem = 2048 + (size_t)nt * 2 * (D / 16) * 32 * 16 + 1024;
+  if (few) return D == 128 ? launch_packed<128, 2>(P, job.bits, grid, smem, st) : launch_packed<256, 2>(P, job.bits, grid, smem, st);
+  return D == 128 ? launch_packed<128, 8>(P, job.bits, grid, smem, st) : launch_packed<256, 8>(P, job.bits, grid, smem, st);
 }
 
 }  // namespace tq

@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(NT) k_score_packed(TqScoreJob job, const float
 // output coordinate, the same sequential-k fma order as the tiled contraction.  A matrix
 // element is loaded once and used for all RPB rows of the block.
 template <int XDT, int RPB>
-__global__ void k_project_rows(const void* x, int64_t n, int K, const float* __restrict__ m, int N, float* out) {
+__device__ __forceinline__ void project_rows(const void* x, int64_t n, int K, const float* __restrict__ m, int N, float* out) {
   __shared__ float xs[RPB][TQ_MAX_DIM];
   const int64_t row0 = (int64_t)blockIdx.x * RPB;
 #pragma unroll
@@ -546,6 +546,16 @@ __global__ void k_project_rows(const void* x, int64_t n, int K, const float* __r
     for (int r = 0; r < RPB; ++r)
       if (row0 + r < n) out[(row0 + r) * N + col] = acc[r];
   }
+}
+
+template <int XDT, int RPB>
+__global__ void k_project_rows(const void* x, int64_t n, int K, const float* __restrict__ m, int N, float* out) {
+  project_rows<XDT, RPB>(x, n, K, m, N, out);
+}
+// the same rows by two matrices: blockIdx.y picks one
+template <int XDT>
+__global__ void k_project_rows_two(const void* x, int64_t n, int D, const float* m0, const float* m1, float* out0, float* out1) {
+  project_rows<XDT, 1>(x, n, D, blockIdx.y ? m1 : m0, D, blockIdx.y ? out1 : out0);
 }
 
 // head_dim 128 specialisation: a thread owns whole keys (two at a time, 64 keys per warp and
@@ -1209,6 +1219,19 @@ int simt_project(const void* x, int x_dtype, int64_t n, int K, const float* m, i
     if (rc == TQ_OK) kern<<<grid, NT, smem, st>>>(x, n, K, m, N, out);
   }));
   return rc != TQ_OK ? rc : check_launch();
+}
+
+// Two projections of the same rows (head_dim square matrices) in one launch, or in two where the rows are many.
+int simt_project_two(const void* x, int x_dtype, int64_t n, int D, const float* m0, const float* m1, float* out0, float* out1,
+                     cudaStream_t st) {
+  if (n == 0) return TQ_OK;
+  if (n <= 512) {
+    const int threads = D <= 128 ? 128 : 256;
+    TQ_DISPATCH_DT(x_dtype, (k_project_rows_two<DT_><<<dim3((unsigned)n, 2), threads, 0, st>>>(x, n, D, m0, m1, out0, out1)));
+    return check_launch();
+  }
+  const int rc = simt_project(x, x_dtype, n, D, m0, D, out0, st);
+  return rc != TQ_OK ? rc : simt_project(x, x_dtype, n, D, m1, D, out1, st);
 }
 
 size_t simt_score_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int D) {

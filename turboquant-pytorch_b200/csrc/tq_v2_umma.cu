@@ -91,13 +91,19 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 // Operand image of a D x D matrix B (rows = output columns n, columns = contraction index k):
 // value hi + lo in fp16, [piece][kc][nb][row n % 128][64 columns], rows of 128 bytes, 16-byte
 // chunk c at c ^ (row & 7).  B[n][k] = src[n * ld_n + k * ld_k].
+// blockIdx.y = the operand: Pi (B[n][k] = Pi[n][k]), Pi^T (Pi[k][n]) and S (qjl_t[k][n]), one image after the other; three
+// launches of a microsecond's work cost 9 us a call.
 template <int D>
-__global__ void k_v2_operand_image(const float* __restrict__ src, int64_t ld_n, int64_t ld_k, uint8_t* __restrict__ image) {
+__global__ void k_v2_operand_image(const float* __restrict__ rotation, const float* __restrict__ qjl_t, int64_t M,
+                                  uint8_t* __restrict__ images) {
   constexpr int KC = VCfg<D>::KC, NBLK = VCfg<D>::NBLK;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= D * D) return;
+  const float* src = blockIdx.y == 2 ? qjl_t : rotation;
+  const int64_t ld_n = blockIdx.y == 0 ? D : 1, ld_k = blockIdx.y == 0 ? 1 : blockIdx.y == 1 ? D : M;
+  uint8_t* image = images + (size_t)blockIdx.y * VCfg<D>::kImageBytes;
   const int n = e / D, k = e % D;
-  const float v = src[(int64_t)n * ld_n + (int64_t)k * ld_k];
+  const float v = __ldg(src + (int64_t)n * ld_n + (int64_t)k * ld_k);
   const __half hi = __float2half_rn(v);
   const __half lo = __float2half_rn(v - __half2float(hi));
   const int kc = k / 64, nb = n / 128, rr = n % 128, c = (k % 64) / 8, w = k % 8;
@@ -321,6 +327,18 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
     for (int i = slot; i < n_local && ok; i += 2) {
       const int64_t row = (int64_t)(t0 + i) * kRowsT + rloc;
       const bool valid = row < p.n;
+      // stage 2: the vector's norm and its first coordinates are in flight while the tile's contraction runs
+      // (together with TMEM loads that run behind the arithmetic: 496 -> 483 us for the call above)
+      const uint16_t* xrow = p.x + (valid ? row : 0) * D + blk * 128;
+      const bool x_wide = ((uintptr_t)p.x & 31u) == 0;
+      constexpr int kAhead = 3;                   // steps of 16 coordinates in flight
+      uint32_t xn[kAhead][8];
+      float nv = 0.f;
+      if constexpr (STAGE == 2) {
+        nv = valid ? p.norms[row] : 0.f;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) load_row32(xrow + 16 * u, xn[u], x_wide);
+      }
       // The exit decision is made uniform before anything collective: per warp (the TMEM loads are
       // warp-collective) and, where the two warpgroups of a tile later meet at a named barrier (stage 2,
       // head_dim 256), over those 256 threads, so that nobody waits at that barrier for a warp that left.
@@ -334,11 +352,18 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
       uint32_t v[16];
       if constexpr (STAGE == 1) {
         float ssq = 0.f;                         // the norm needs every column: both warpgroups sweep the whole row
+        uint32_t v2[16];                         // two buffers: a TMEM load is in flight behind the arithmetic
+        tmem_issue16(tile_acc, v);
 #pragma unroll 1
-        for (int c = 0; c < D / 16; ++c) {
-          tmem_ld16(tile_acc + c * 16, v);
+        for (int c = 0; c < D / 16; c += 2) {
+          tmem_wait16(v);
+          tmem_issue16(tile_acc + (c + 1) * 16, v2);
 #pragma unroll
           for (int e = 0; e < 16; ++e) ssq = fmaf(__uint_as_float(v[e]), __uint_as_float(v[e]), ssq);
+          tmem_wait16(v2);
+          tmem_issue16(c + 2 < D / 16 ? tile_acc + (c + 2) * 16 : tacc, v);      // after the last step: step 0 of the sweep below
+#pragma unroll
+          for (int e = 0; e < 16; ++e) ssq = fmaf(__uint_as_float(v2[e]), __uint_as_float(v2[e]), ssq);
         }
         const float norm = __fsqrt_rn(ssq);
         const float inv = __fdiv_rn(1.0f, norm + 1e-8f);
@@ -346,7 +371,7 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
         const int bits = p.bits;
 #pragma unroll 1
         for (int c = 0; c < 8; ++c) {
-          tmem_ld16(tacc + c * 16, v);
+          tmem_wait16(v);
           uint32_t w[16];
           uint32_t ib[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
@@ -377,6 +402,7 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
             w[e] = lut_s[idx];
             ib[e >> 2] |= (uint32_t)idx << (8 * (e & 3));
           }
+          if (c + 1 < 8) tmem_issue16(tacc + (c + 1) * 16, v);
           if (valid && p.idx_u8_out != nullptr)
             *reinterpret_cast<uint4*>(p.idx_u8_out + row * D + col0 + c * 16) = make_uint4(ib[0], ib[1], ib[2], ib[3]);
           if (valid && p.idx_packed_out != nullptr) {
@@ -422,20 +448,20 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
           }
         }
       } else if constexpr (STAGE == 2) {
-        const float nv = valid ? p.norms[row] : 0.f;
         float ssq = 0.f;
-        // the vector's own 16-coordinate pieces are fetched one step ahead of their use
-        const uint16_t* xrow = p.x + (valid ? row : 0) * D + col0;
-        const bool x_wide = ((uintptr_t)p.x & 31u) == 0, k_wide = ((uintptr_t)p.k_mse_out & 31u) == 0;
-        uint32_t xn[8];
-        load_row32(xrow, xn, x_wide);
+        const bool k_wide = ((uintptr_t)p.k_mse_out & 31u) == 0;
+        tmem_issue16(tacc, v);
 #pragma unroll 1
         for (int c = 0; c < 8; ++c) {
           uint32_t xw[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) xw[j] = xn[j];
-          if (c + 1 < 8) load_row32(xrow + 16 * (c + 1), xn, x_wide);
-          tmem_ld16(tacc + c * 16, v);
+          for (int j = 0; j < 8; ++j) {
+            xw[j] = xn[0][j];
+#pragma unroll
+            for (int u = 0; u + 1 < kAhead; ++u) xn[u][j] = xn[u + 1][j];
+          }
+          if (c + kAhead < 8) load_row32(xrow + 16 * (c + kAhead), xn[kAhead - 1], x_wide);
+          tmem_wait16(v);
           if (valid) {
             uint32_t kq[8], rh[8], rl[8];
 #pragma unroll
@@ -456,6 +482,7 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
             store_row32(p.p_hi + row * D + col0 + c * 16, rh, true);
             store_row32(p.p_lo + row * D + col0 + c * 16, rl, true);
           }
+          if (c + 1 < 8) tmem_issue16(tacc + (c + 1) * 16, v);
         }
         if constexpr (NBLK == 2) {
           // the residual norm spans both blocks: the upper block's warpgroup hands its partial sum over
@@ -553,9 +580,7 @@ int run(const TqQjlCompressJob& job, cudaStream_t st) {
   uint16_t* p_lo = reinterpret_cast<uint16_t*>(ws + 3 * img + piece);
   float* norms = reinterpret_cast<float*>(ws + 3 * img + 2 * piece);
   const int ib = (D * D + 255) / 256;
-  k_v2_operand_image<D><<<ib, 256, 0, st>>>(job.rotation, D, 1, img1);      // B[n][k] = Pi[n][k]
-  k_v2_operand_image<D><<<ib, 256, 0, st>>>(job.rotation, 1, D, img2);      // B[j][n] = Pi[n][j]
-  k_v2_operand_image<D><<<ib, 256, 0, st>>>(job.qjl_t, 1, job.M, img3);     // B[m][j] = S[m][j] = qjl_t[j][m]
+  k_v2_operand_image<D><<<dim3(ib, 3), 256, 0, st>>>(job.rotation, job.qjl_t, job.M, img1);
   int rc = check_launch();
   if (rc != TQ_OK) return rc;
   static thread_local V2Stage p;
