@@ -13,12 +13,17 @@
 //     order its terms are visited, so the coordinates are assigned to k-steps in the order that makes a
 //     thread's operand elements come from its own contiguous bytes: k-step ks, thread t covers coordinates
 //     32 t + 4 ks + 0..3 (the query operand uses the same order);
-//   * two MMAs per k-step (centroid pieces hi, lo) into ONE accumulator: column g collects
-//     (c_hi + c_lo).q_hi, column g + 4 collects (c_hi + c_lo).q_lo; their sum is the fp32-accurate logit
-//     (all four cross terms), one shuffle away.
+//   * a table entry (hi | lo << 16) IS an operand register: a register holds two neighbouring k, and these two are
+//     the pieces of ONE coordinate, with the query value of that coordinate in both of the other operand's places.
+//     Packing the high pieces of two coordinates into one register and the low pieces into another took a byte
+//     permute per coordinate and gave the same number of MMAs;
+//   * column g collects (c_hi + c_lo).q_hi, column g + 4 collects (c_hi + c_lo).q_lo; their sum is the fp32-accurate
+//     logit (all four cross terms), one shuffle away.
 // The softmax partials per block of keys and the finishing pass are those of the FP32 path.
 
 #include <atomic>
+#include <cfloat>
+#include <type_traits>
 
 #include "tq_common.cuh"
 #include "tq_internal.h"
@@ -118,26 +123,17 @@ struct WordAddr {
   }
 };
 
-// key operand of k-step ks for both centroid pieces: the thread's local coordinates 4 ks .. 4 ks + 3
+// table entries (hi | lo << 16) of the thread's local coordinates 4 ks .. 4 ks + 3
 template <int BITS>
-__device__ __forceinline__ void key_fragment(const uint32_t (&w)[Packed<BITS>::CW], int ks, uint32_t lut_base,
-                                             uint32_t (&bh)[2], uint32_t (&bl)[2]) {
+__device__ __forceinline__ void key_entries(const uint32_t (&w)[Packed<BITS>::CW], int ks, uint32_t lut_base, uint32_t (&e)[4]) {
   constexpr int CPW = 4 * Packed<BITS>::IPB;    // coordinates per word: 4 (wide codes) .. 32 (1 bit)
   const int u0 = 4 * ks;
   const WordAddr<BITS> wa(w[u0 / CPW], lut_base);
-  uint32_t e[4];
 #pragma unroll
   for (int p = 0; p < 4; ++p) e[p] = lds_u32(wa((u0 + p) % CPW));
-  bh[0] = __byte_perm(e[0], e[1], 0x5410); bl[0] = __byte_perm(e[0], e[1], 0x7632);
-  bh[1] = __byte_perm(e[2], e[3], 0x5410); bl[1] = __byte_perm(e[2], e[3], 0x7632);
 }
 
 // (max, sum of exp) running pair
-__device__ __forceinline__ void stat_add(float& m, float& s, float l) {
-  const float nm = fmaxf(m, l);
-  if (nm != -INFINITY) s = s * __expf(m - nm) + __expf(l - nm);
-  m = nm;
-}
 __device__ __forceinline__ void stat_merge(float& m, float& s, float m2, float s2) {
   const float nm = fmaxf(m, m2);
   if (nm != -INFINITY) s = (m == -INFINITY ? 0.f : s * __expf(m - nm)) + (m2 == -INFINITY ? 0.f : s2 * __expf(m2 - nm));
@@ -145,50 +141,99 @@ __device__ __forceinline__ void stat_merge(float& m, float& s, float m2, float s
 }
 
 // Query operand of one pass: column n = lane / 4 of the 8-column operand is row r0 + (n & 3) of the rotated
-// queries, as its high piece (n < 4) or low piece (n >= 4); thread t holds coordinates 32 t + 4 ks + 0..3.
+// queries, as its high piece (n < 4) or low piece (n >= 4); thread t holds coordinates 32 t + 4 ks + 0..3, each value in
+// both halves of its register.
 __device__ __forceinline__ void query_fragments(const float* __restrict__ qrot, int64_t row, bool row_ok, int lane,
-                                                uint32_t (&bq)[8][2]) {
+                                                uint32_t (&bq)[8][4]) {
   const int t = lane & 3;
   const bool low = (lane >> 2) >= 4;
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row_ok) v = __ldg(reinterpret_cast<const float4*>(qrot + row * kDimA + 32 * t + 4 * ks));
-    uint32_t h0, l0, h1, l1;
-    split2(v.x, v.y, h0, l0);
-    split2(v.z, v.w, h1, l1);
-    bq[ks][0] = low ? l0 : h0;
-    bq[ks][1] = low ? l1 : h1;
+    const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const __half h = __float2half_rn(f[p]);
+      const __half piece = low ? __float2half_rn(f[p] - __half2float(h)) : h;
+      bq[ks][p] = (uint32_t)__half_as_ushort(piece) * 0x00010001u;
+    }
   }
 }
 
-// 16 keys x 4 query rows: c[0..1] = key gid, c[2..3] = key gid + 8, columns (2t, 2t + 1) of [q_hi | q_lo].
+// The same for eight query rows per pass: column n is row r0 + n, high pieces in bh, low pieces in bl; a register holds
+// two coordinates and is widened at its use (both values in both halves would be 64 registers).
+__device__ __forceinline__ void query_fragments8(const float* __restrict__ qrot, int64_t row, bool row_ok, int lane,
+                                                 uint32_t (&bh)[8][2], uint32_t (&bl)[8][2]) {
+  const int t = lane & 3;
+#pragma unroll
+  for (int ks = 0; ks < 8; ++ks) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row_ok) v = __ldg(reinterpret_cast<const float4*>(qrot + row * kDimA + 32 * t + 4 * ks));
+    split2(v.x, v.y, bh[ks][0], bl[ks][0]);
+    split2(v.z, v.w, bh[ks][1], bl[ks][1]);
+  }
+}
 template <int BITS>
-__device__ __forceinline__ void score_block(const uint32_t (&w0)[Packed<BITS>::CW], const uint32_t (&w1)[Packed<BITS>::CW],
-                                            const uint32_t (&bq)[8][2], uint32_t lut_base, float (&c)[4]) {
+__device__ __forceinline__ void score_block8(const uint32_t (&w0)[Packed<BITS>::CW], const uint32_t (&w1)[Packed<BITS>::CW],
+                                             const uint32_t (&bh)[8][2], const uint32_t (&bl)[8][2], uint32_t lut_base, float (&c)[4]) {
+  float d[4] = {0.f, 0.f, 0.f, 0.f};
   c[0] = c[1] = c[2] = c[3] = 0.f;
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) {
-    uint32_t h0[2], l0[2], h1[2], l1[2];
-    key_fragment<BITS>(w0, ks, lut_base, h0, l0);
-    key_fragment<BITS>(w1, ks, lut_base, h1, l1);
-    mma_16816(c, h0[0], h1[0], h0[1], h1[1], bq[ks][0], bq[ks][1]);
-    mma_16816(c, l0[0], l1[0], l0[1], l1[1], bq[ks][0], bq[ks][1]);
+    uint32_t e[4], f[4];
+    key_entries<BITS>(w0, ks, lut_base, e);
+    key_entries<BITS>(w1, ks, lut_base, f);
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      mma_16816(c, e[2 * p], f[2 * p], e[2 * p + 1], f[2 * p + 1], __byte_perm(bh[ks][p], 0u, 0x1010), __byte_perm(bh[ks][p], 0u, 0x3232));
+      mma_16816(d, e[2 * p], f[2 * p], e[2 * p + 1], f[2 * p + 1], __byte_perm(bl[ks][p], 0u, 0x1010), __byte_perm(bl[ks][p], 0u, 0x3232));
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) c[j] += d[j];
+}
+
+// 16 keys x 4 query rows: c[0..1] = key gid, c[2..3] = key gid + 8, columns (2t, 2t + 1) of [q_hi | q_lo].
+// Two accumulators, so that neighbouring MMAs do not wait for one another.
+template <int BITS>
+__device__ __forceinline__ void score_block(const uint32_t (&w0)[Packed<BITS>::CW], const uint32_t (&w1)[Packed<BITS>::CW],
+                                            const uint32_t (&bq)[8][4], uint32_t lut_base, float (&c)[4]) {
+  float d[4] = {0.f, 0.f, 0.f, 0.f};
+  c[0] = c[1] = c[2] = c[3] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < 8; ++ks) {
+    uint32_t e[4], f[4];
+    key_entries<BITS>(w0, ks, lut_base, e);
+    key_entries<BITS>(w1, ks, lut_base, f);
+    mma_16816(c, e[0], f[0], e[1], f[1], bq[ks][0], bq[ks][1]);
+    mma_16816(d, e[2], f[2], e[3], f[3], bq[ks][2], bq[ks][3]);
   }
   // column g + 4 (low query piece) lives two lanes away: afterwards lanes t and t ^ 2 both hold the full sums
 #pragma unroll
-  for (int j = 0; j < 4; ++j) c[j] += __shfl_xor_sync(0xffffffffu, c[j], 2);
+  for (int j = 0; j < 4; ++j) {
+    c[j] += d[j];
+    c[j] += __shfl_xor_sync(0xffffffffu, c[j], 2);
+  }
 }
 
 // grid: B * Hkv * nblk CTAs, each over keys_per_block keys of one KV head; stats as in the FP32 path:
 // stats[(row * nblk + blk) * 2 + {0, 1}] = (max, sum of exp(l - max)) of the block's keys.
-template <int BITS>
+// Two CTAs per SM: three (80 registers) spill, 70 us against 65 for the call below.
+// 8 KV heads x 131072 4-bit keys, 32 query heads: the call, with projection and softmax, 75 us with packed pieces, one
+// accumulator and a rescaled sum for every logit, 65 us as it is.
+// 8 KV heads x 65536 4-bit keys with 8 query rows per KV head: 65 -> 43 us for the call, with 16 rows 117 -> 78 us.
+//
+// ROWS: query rows per pass over the keys.  With eight a lane finishes keys gid and gid + 8 for rows 2t, 2t + 1 and the
+// look-ups of a key serve twice the rows; four rows put their low pieces into the other four columns instead.
+template <int BITS, int ROWS>
 __global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const float* __restrict__ qrot, float* stats, int nblk,
                                                         int keys_per_block) {
   constexpr int G = Packed<BITS>::G;
   constexpr int CW = Packed<BITS>::CW;
   __shared__ __align__(1024) uint32_t lut[256];
-  __shared__ float red_m[kWarps][kRows], red_s[kWarps][kRows];
+  constexpr bool kEight = ROWS == 8;
+  __shared__ float red_m[kWarps][ROWS], red_s[kWarps][ROWS];
   {
     const float c = __ldg(job.codebook + kCentroidOff + threadIdx.x);
     const __half h = __float2half_rn(c);
@@ -202,72 +247,93 @@ __global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const
   const int rep = (int)(job.Hq / job.Hkv);
   const int R = rep * (int)job.Sq;
   const int64_t s_begin = (int64_t)blk * keys_per_block;
-  const int64_t s_end = min(s_begin + (int64_t)keys_per_block, job.Sk);
-  const uint8_t* keys = job.idx_bytes + bh * job.Sk * G;
-  const uint16_t* norms = job.norms + bh * job.Sk;
+  const int n_keys = (int)min((int64_t)keys_per_block, job.Sk - s_begin);      // of this CTA; keys below count from s_begin
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, t = lane & 3;
+  const int my = gid + (!kEight && t >= 2 ? 8 : 0);     // the (first) key of a block whose logits this lane finishes
+  const uint8_t* keys = job.idx_bytes + (bh * job.Sk + s_begin) * G + t * Packed<BITS>::CB;
+  const uint16_t* norms = job.norms + bh * job.Sk + s_begin;
   __syncthreads();
   auto global_row = [&](int r) -> int64_t {
     const int64_t hq = hkv * rep + r / job.Sq, sq = r % job.Sq;
     return (b * job.Hq + hq) * job.Sq + sq;
   };
-  for (int r0 = 0; r0 < R; r0 += kRows) {
-    uint32_t bq[8][2];
-    {
+  for (int r0 = 0; r0 < R; r0 += ROWS) {
+    uint32_t bq[kEight ? 1 : 8][4], bh[kEight ? 8 : 1][2], bl[kEight ? 8 : 1][2];
+    if constexpr (kEight) {
+      const int r = r0 + gid;
+      query_fragments8(qrot, r < R ? global_row(r) : 0, r < R, lane, bh, bl);
+    } else {
       const int r = r0 + (gid & 3);
       query_fragments(qrot, r < R ? global_row(r) : 0, r < R, lane, bq);
     }
-    // after the shuffle in score_block this lane finishes ONE key (gid for t < 2, gid + 8 otherwise) and the
+    // four rows: after the shuffle in score_block this lane finishes ONE key (gid for t < 2, gid + 8 otherwise) and the
     // two query rows r0 + 2 (t & 1) + {0, 1}
-    const int ra = r0 + 2 * (t & 1);
+    const int ra = r0 + 2 * (kEight ? t : t & 1);
     const bool ok_a = ra < R, ok_b = ra + 1 < R;
-    const int64_t row_a = ok_a ? global_row(ra) : 0, row_b = ok_b ? global_row(ra + 1) : 0;
-    float m_a = -INFINITY, s_a = 0.f, m_b = -INFINITY, s_b = 0.f;
+    float* out_a = job.logits + (ok_a ? global_row(ra) : 0) * job.Sk + s_begin;
+    float* out_b = job.logits + (ok_b ? global_row(ra + 1) : 0) * job.Sk + s_begin;
+    // running (max, sum of exp(l - max)) of the two rows over this lane's keys.  The maximum starts at the lowest finite
+    // value, so that logits of -inf add exp(-inf) = 0; it moves about ln(n) times in n keys.
+    float m_a = -FLT_MAX, s_a = 0.f, m_b = -FLT_MAX, s_b = 0.f;
     // the packed quarter rows and the norm of the NEXT block of 16 keys are in flight while this one is scored
     uint32_t w0[CW], w1[CW], n0[CW], n1[CW];
-    uint16_t nv_bits = 0, nn_bits = 0;
-    auto fetch = [&](int64_t kb, uint32_t (&a0)[CW], uint32_t (&a1)[CW], uint16_t& nb) {
-      const int64_t k_lo = kb + gid, k_hi = kb + 8 + gid;
-      load_quarter<BITS>(keys + (k_lo < s_end ? k_lo : s_begin) * G, t, a0);
-      load_quarter<BITS>(keys + (k_hi < s_end ? k_hi : s_begin) * G, t, a1);
-      const int64_t key = t < 2 ? k_lo : k_hi;
-      nb = __ldg(norms + (key < s_end ? key : s_begin));
+    uint32_t nv_bits = 0, nn_bits = 0;          // norm of key `my`; eight rows: that of the key 8 further in the high half
+    auto fetch = [&](int kb, uint32_t (&a0)[CW], uint32_t (&a1)[CW], uint32_t& nb) {
+      load_quarter<BITS>(keys + (int64_t)min(kb + gid, n_keys - 1) * G, 0, a0);
+      load_quarter<BITS>(keys + (int64_t)min(kb + 8 + gid, n_keys - 1) * G, 0, a1);
+      nb = __ldg(norms + min(kb + my, n_keys - 1));
+      if constexpr (kEight) nb |= (uint32_t)__ldg(norms + min(kb + my + 8, n_keys - 1)) << 16;
     };
-    int64_t kb = s_begin + warp * 16;
-    if (kb < s_end) fetch(kb, w0, w1, nv_bits);
-    for (; kb < s_end; kb += kWarps * 16) {
-      const int64_t kn = kb + kWarps * 16;
-      if (kn < s_end) fetch(kn, n0, n1, nn_bits);
-      float c[4];
-      score_block<BITS>(w0, w1, bq, lut_base, c);
-      const int64_t key = (t < 2 ? kb : kb + 8) + gid;
-      if (key < s_end) {
-        const float nv = __half2float(__ushort_as_half(nv_bits)) * job.scale;
-        const float la = (t < 2 ? c[0] : c[2]) * nv, lb = (t < 2 ? c[1] : c[3]) * nv;
-        if (ok_a) job.logits[row_a * job.Sk + key] = la;
-        if (ok_b) job.logits[row_b * job.Sk + key] = lb;
-        if (stats != nullptr) { stat_add(m_a, s_a, la); stat_add(m_b, s_b, lb); }
+    auto finish_key = [&](int key, float ca, float cb, uint32_t nb) {
+      if (key < n_keys) {
+        const float nv = __half2float(__ushort_as_half((uint16_t)nb)) * job.scale;
+        const float la = ca * nv, lb = cb * nv;
+        if (ok_a) out_a[key] = la;
+        if (ok_b) out_b[key] = lb;
+        if (la > m_a) { s_a *= __expf(m_a - la); m_a = la; }
+        if (lb > m_b) { s_b *= __expf(m_b - lb); m_b = lb; }
+        s_a += __expf(la - m_a);
+        s_b += __expf(lb - m_b);
       }
-#pragma unroll
-      for (int k = 0; k < CW; ++k) { w0[k] = n0[k]; w1[k] = n1[k]; }
-      nv_bits = nn_bits;
+    };
+    auto score = [&](const uint32_t (&a0)[CW], const uint32_t (&a1)[CW], int kb, uint32_t nb) {
+      float c[4];
+      if constexpr (kEight) {
+        score_block8<BITS>(a0, a1, bh, bl, lut_base, c);
+        finish_key(kb + my, c[0], c[1], nb & 0xFFFFu);
+        finish_key(kb + my + 8, c[2], c[3], nb >> 16);
+      } else {
+        score_block<BITS>(a0, a1, bq, lut_base, c);
+        finish_key(kb + my, t < 2 ? c[0] : c[2], t < 2 ? c[1] : c[3], nb);
+      }
+    };
+    int kb = warp * 16;
+    if (kb < n_keys) fetch(kb, w0, w1, nv_bits);
+    for (; kb < n_keys; kb += 2 * kWarps * 16) {              // two blocks a round: the buffers swap without copies
+      const int k1 = kb + kWarps * 16, k2 = k1 + kWarps * 16;
+      if (k1 < n_keys) fetch(k1, n0, n1, nn_bits);
+      score(w0, w1, kb, nv_bits);
+      if (k1 < n_keys) {
+        if (k2 < n_keys) fetch(k2, w0, w1, nv_bits);
+        score(n0, n1, k1, nn_bits);
+      }
     }
     if (stats != nullptr) {
-      // lanes that share (t & 1) share the two rows: fold over the other lane bits, then over the warps
+      // lanes that share t (four rows: t & 1) share the two rows: fold over the other lane bits, then over the warps
 #pragma unroll
-      for (int o = 2; o <= 16; o <<= 1) {
+      for (int o = kEight ? 4 : 2; o <= 16; o <<= 1) {
         const float m2 = __shfl_xor_sync(0xffffffffu, m_a, o), s2 = __shfl_xor_sync(0xffffffffu, s_a, o);
         stat_merge(m_a, s_a, m2, s2);
         const float m3 = __shfl_xor_sync(0xffffffffu, m_b, o), s3 = __shfl_xor_sync(0xffffffffu, s_b, o);
         stat_merge(m_b, s_b, m3, s3);
       }
-      if (lane < 2) {
+      if (lane < ROWS / 2) {
         red_m[warp][2 * lane] = m_a; red_s[warp][2 * lane] = s_a;
         red_m[warp][2 * lane + 1] = m_b; red_s[warp][2 * lane + 1] = s_b;
       }
       __syncthreads();
-      if (threadIdx.x < kRows && r0 + (int)threadIdx.x < R) {
+      if (threadIdx.x < ROWS && r0 + (int)threadIdx.x < R) {
         float m = -INFINITY, s = 0.f;
         for (int wv = 0; wv < kWarps; ++wv) stat_merge(m, s, red_m[wv][threadIdx.x], red_s[wv][threadIdx.x]);
         const int64_t orow = global_row(r0 + threadIdx.x);
@@ -385,7 +451,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
     return (b * P.Hq + hq) * P.Sq + sq;
   };
   for (int r0 = 0; r0 < R; r0 += kRows) {
-    uint32_t bq[8][2];
+    uint32_t bq[8][4];
     {
       const int r = r0 + (gid & 3);
       query_fragments(P.qrot, r < R ? global_row(r) : 0, r < R, lane, bq);
@@ -461,6 +527,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
       }
       const uint32_t pb0 = movmatrix_trans(x0);               // keys 2t, 2t+1  x column gid
       const uint32_t pb1 = movmatrix_trans(x1);               // keys 2t+8, 2t+9 x column gid
+      const uint32_t p0 = __byte_perm(pb0, 0u, 0x1010), p1 = __byte_perm(pb0, 0u, 0x3232);     // each value in both halves
+      const uint32_t p2 = __byte_perm(pb1, 0u, 0x1010), p3 = __byte_perm(pb1, 0u, 0x3232);
       // rescale the accumulators when a maximum moved (columns 2t, 2t+1 are this lane's two rows in both halves)
       if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
 #pragma unroll
@@ -477,13 +545,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
           e[q][0] = value_entry<VBITS>(vw[q], 2 * mb, lutv);
           e[q][1] = value_entry<VBITS>(vw[q], 2 * mb + 1, lutv);
         }
-        // A registers: (row gid, keys 2t, 2t+1), (row gid + 8, keys 2t, 2t+1), (row gid, keys 2t+8, 2t+9), (row gid + 8, ...)
-        const uint32_t ah0 = __byte_perm(e[0][0], e[1][0], 0x5410), ah1 = __byte_perm(e[0][1], e[1][1], 0x5410);
-        const uint32_t ah2 = __byte_perm(e[2][0], e[3][0], 0x5410), ah3 = __byte_perm(e[2][1], e[3][1], 0x5410);
-        const uint32_t al0 = __byte_perm(e[0][0], e[1][0], 0x7632), al1 = __byte_perm(e[0][1], e[1][1], 0x7632);
-        const uint32_t al2 = __byte_perm(e[2][0], e[3][0], 0x7632), al3 = __byte_perm(e[2][1], e[3][1], 0x7632);
-        mma_16816(acc[mb], ah0, ah1, ah2, ah3, pb0, pb1);
-        mma_16816(acc[mb], al0, al1, al2, al3, pb0, pb1);
+        // an entry is the operand's two neighbouring k, the pieces of one value; rows gid, gid + 8 are the two coordinates,
+        // the k pairs t, t + 4 the keys 2t, 2t + 1 (first MMA) and 2t + 8, 2t + 9 (second)
+        mma_16816(acc[mb], e[0][0], e[0][1], e[1][0], e[1][1], p0, p1);
+        mma_16816(acc[mb], e[2][0], e[2][1], e[3][0], e[3][1], p2, p3);
       }
 #pragma unroll
       for (int k = 0; k < KW; ++k) { w0[k] = n0[k]; w1[k] = n1[k]; }
@@ -885,15 +950,21 @@ int mma_score_keys_per_block(const TqScoreJob& job, int min_keys) {
 
 int mma_score_packed(const TqScoreJob& job, const float* qrot, float* stats, int nblk, int keys_per_block, cudaStream_t st) {
   const int64_t blocks = job.B * job.Hkv * nblk;
+  const bool eight = job.Hq / job.Hkv * job.Sq > 4;      // more than four query rows per KV head: one pass serves eight
+  auto go = [&](auto bits) {
+    constexpr int BITS = decltype(bits)::value;
+    if (eight) k_score_mma<BITS, 8><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block);
+    else k_score_mma<BITS, 4><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block);
+  };
   switch (job.bits) {
-    case 1: k_score_mma<1><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block); break;
-    case 2: k_score_mma<2><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block); break;
-    case 3: k_score_mma<3><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block); break;
-    case 4: k_score_mma<4><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block); break;
-    case 5: k_score_mma<5><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block); break;
-    case 6: k_score_mma<6><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block); break;
-    case 7: k_score_mma<7><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block); break;
-    default: k_score_mma<8><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block); break;
+    case 1: go(std::integral_constant<int, 1>{}); break;
+    case 2: go(std::integral_constant<int, 2>{}); break;
+    case 3: go(std::integral_constant<int, 3>{}); break;
+    case 4: go(std::integral_constant<int, 4>{}); break;
+    case 5: go(std::integral_constant<int, 5>{}); break;
+    case 6: go(std::integral_constant<int, 6>{}); break;
+    case 7: go(std::integral_constant<int, 7>{}); break;
+    default: go(std::integral_constant<int, 8>{}); break;
   }
   return check_launch();
 }
