@@ -313,6 +313,7 @@ int tq_quantize(const TqQuantizeJob* jobs, int n_jobs, void* stream) {
     if (j.x == nullptr || j.rotation_t == nullptr || j.codebook == nullptr || j.idx_out == nullptr) return TQ_ENULL;
     if (j.normalize && j.norms_out == nullptr) return TQ_ENULL;
   }
+  if (tq::few_quantize_eligible(jobs, n_jobs)) return tq::few_quantize(jobs, n_jobs, (cudaStream_t)stream);
   // maximal runs of tensor-core-eligible jobs go out as one persistent launch each
   int i = 0;
   while (i < n_jobs) {
@@ -345,6 +346,7 @@ int tq_dequantize(const TqDequantizeJob* jobs, int n_jobs, void* stream) {
     if (j.B * j.H * j.S == 0) continue;
     if (j.idx == nullptr || j.rotation == nullptr || j.codebook == nullptr || j.out == nullptr) return TQ_ENULL;
   }
+  if (tq::few_dequantize_eligible(jobs, n_jobs)) return tq::few_dequantize(jobs, n_jobs, (cudaStream_t)stream);
   int i = 0;
   while (i < n_jobs) {
     if (jobs[i].B * jobs[i].H * jobs[i].S == 0) { ++i; continue; }

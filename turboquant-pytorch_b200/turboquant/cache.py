@@ -24,6 +24,7 @@ is the per-layer form the transformers attention modules call.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
@@ -76,6 +77,7 @@ class V3Cache(_Base):
         self.initial_capacity = initial_capacity
         self._layers: Dict[int, _Layer] = {}
         self._step_plan = None
+        self._step_log: List[tuple] = []               # native steps whose packed rows are not in the layers' lists yet
 
     # ------------------------------------------------------------------ layers and buffers
     def _layer(self, layer_idx: int, head_dim: int, device) -> _Layer:
@@ -126,6 +128,7 @@ class V3Cache(_Base):
         st.total = need
         n_c = self._leaving(st, need)
         if n_c > 0:
+            self._file_steps()
             lo, hi = st.compressed, st.compressed + n_c
             view_k, view_v = st.k[:, :, lo:hi], st.v[:, :, lo:hi]
             kc, vc = st.codec.key_compressor, st.codec.val_compressor
@@ -183,7 +186,7 @@ class V3Cache(_Base):
         return_views=False.  Falls back to per-layer update() calls while layers are being created or grown."""
         p = self._step_plan
         if p is not None and p["native"] is not None and p["L"] == len(key_states) and p["window"] == self.residual_window:
-            done = N.host().step(p["native"], p["states"], key_states, value_states, return_views)
+            done = N.host().step(p["native"], p["states"], key_states, value_states, return_views, self._step_log)
             if done is not None:
                 return done if return_views else None
         return self._step_general(key_states, value_states, return_views)
@@ -191,6 +194,7 @@ class V3Cache(_Base):
     @torch.no_grad()
     def _step_general(self, key_states, value_states, return_views):
         """step() in Python: the first call, calls that create or grow layers, and inputs the native form does not take."""
+        self._file_steps()
         L = len(key_states)
         k0 = key_states[0]
         B, H, S_new, D = k0.shape
@@ -270,6 +274,18 @@ class V3Cache(_Base):
         return f"{comp} compressed, {total - comp} fp16, {total} total"
 
     # ------------------------------------------------------------------ beyond the reference
+    def _file_steps(self):
+        """Moves what the native steps recorded into the layers' lists of packed rows."""
+        if not self._step_log:
+            return
+        for store, blob in self._step_log:
+            r = struct.unpack(f"{len(blob) // 8}q", blob)
+            L = len(r) // 6
+            for l in range(L):
+                if r[L + l]:
+                    self._layers[l].packed.append((r[l], r[L + l], store, r[2 * L + 4 * l:2 * L + 4 * l + 4]))
+        self._step_log.clear()
+
     def _chunk_tensors(self, st: _Layer, entry):
         """(first token, n, k idx, k norms, v idx, v norms) of one compressed-store entry, as (B, H, n, ...) tensors."""
         if len(entry) == 6:
@@ -287,6 +303,7 @@ class V3Cache(_Base):
 
     def packed_chunks(self, layer_idx: int):
         """The compressed store of a layer: lists of MSECompressor dicts for keys and values, in token order."""
+        self._file_steps()
         st = self._layers[layer_idx]
         B, H, _, D = st.k.shape
         cks, cvs = [], []
