@@ -5,8 +5,9 @@
 // hi + lo (lo reaches into fp16 subnormals), so products match an fp32 matmul to ~2^-21:
 //
 //   stage 1  y = x Pi^T            A = x (exact fp16), B = Pi hi/lo.  Epilogue: ||y|| = ||x||, scale,
-//                                  nearest centroid by exact thresholds, centroid pieces hi/lo -> scratch
-//   stage 2  k = (c Pi) ||x||      A = centroid pieces, B = Pi^T hi/lo (hi.hi + lo.hi + hi.lo).  Epilogue:
+//                                  nearest centroid by exact thresholds, one index byte per coordinate -> scratch
+//   stage 2  k = (c Pi) ||x||      A = centroid pieces, which expander warps write into the operand ring from the
+//                                  index bytes, B = Pi^T hi/lo (hi.hi + lo.hi + hi.lo).  Epilogue:
 //                                  k_mse (fp16 out), residual r = x - k, ||r|| (out), residual pieces -> scratch
 //   stage 3  p = r S^T             A = residual pieces, B = S hi/lo.  Epilogue: signs (int8 out)
 //
@@ -36,6 +37,8 @@ namespace {
 constexpr int kRowsT = 128;                    // vectors per tile (MMA M)
 constexpr uint32_t kChunk = 128 * 128;         // 128 rows x 64 fp16 = 16 KB (an A chunk or a B chunk)
 constexpr int kNB = 4;                         // B ring stages
+constexpr uint32_t kRawChunk = 128 * 64;       // index bytes of a k-chunk: 128 rows x 64
+constexpr int kExpandThreads = 64;             // stage 2: two expander warps, thread = two rows
 
 template <int D>
 struct VCfg {
@@ -43,14 +46,16 @@ struct VCfg {
   static constexpr int NBLK = D / 128;         // blocks of 128 output columns
   // A: two k-chunk slots per piece (chunk kc lands in slot kc & 1 and is released as soon as its MMAs are done), so
   // that the B ring can hold stages of ALL output columns: one MMA of N = D per k-step instead of one per block of
-  // 128 columns (an MMA takes ~127 clocks whatever its N, so N = 256 halves the tensor time at head_dim 256)
+  // 128 columns, which reads the A operand once (M = 128 takes 65 clocks at N = 128 and 129 at N = 256)
   static constexpr int kASlots = 2;
   static constexpr uint32_t kBStage = NBLK * kChunk;                     // one k-chunk of B for all D output columns
   static constexpr uint32_t kOffA = 0;                                   // [piece 2][slot 2] chunks
   static constexpr uint32_t kOffB = kOffA + 2u * kASlots * kChunk;       // ring
-  static constexpr uint32_t kOffTab = kOffB + kNB * kBStage;             // thresholds, centroid piece pairs, cell table, partial sums
+  static constexpr uint32_t kOffRaw = kOffB + kNB * kBStage;             // stage 2: index bytes of two k-chunks
+  static constexpr uint32_t kOffTab = kOffRaw + 2u * kRawChunk;          // thresholds, centroid piece pairs, cell table, partial sums
   static constexpr uint32_t kOffBar = kOffTab + 6144;
   static constexpr int kThreads = 64 + 2 * NBLK * 128;                   // two tiles in flight, one warpgroup per 128 columns
+  static constexpr int threads(int stage) { return kThreads + (stage == 2 ? kExpandThreads : 0); }
   static constexpr uint32_t kUsedBytes = kOffBar + 256;
   static constexpr uint32_t kSmemBytes = kUsedBytes + 1024;
   static constexpr uint32_t kImageBytes = 2u * KC * NBLK * kChunk;       // [piece][kc][nb] chunks of one operand
@@ -64,7 +69,9 @@ struct V2Stage {
   const uint8_t* b_image;    // [piece][kc][nb][128 rows x 128 bytes swizzled]
   const float* codebook;     // stage 1
   const uint16_t* x;         // stage 2: the original vectors (n, D) fp16
-  uint16_t* p_hi;            // scratch (n, D): centroid pieces after stage 1, residual pieces after stage 2
+  uint16_t* p_hi;            // scratch (n, D): after stage 1 (156 -> 124 us for the call below with one byte per coordinate
+                             // instead of four of centroid pieces) the first D bytes of a row are the vector's index bytes, after
+                             // stage 2 (which reads a tile's bytes before it writes the tile's rows) the residual's pieces
   uint16_t* p_lo;
   float* norms;              // scratch (n): ||x||
   uint8_t* idx_u8_out;       // stage 1: optional, one index per byte (n, D)
@@ -103,7 +110,10 @@ __global__ void k_v2_operand_image(const float* __restrict__ rotation, const flo
   const int64_t ld_n = blockIdx.y == 0 ? D : 1, ld_k = blockIdx.y == 0 ? 1 : blockIdx.y == 1 ? D : M;
   uint8_t* image = images + (size_t)blockIdx.y * VCfg<D>::kImageBytes;
   const int n = e / D, k = e % D;
-  const float v = __ldg(src + (int64_t)n * ld_n + (int64_t)k * ld_k);
+  // operand row (= accumulator column) n of Pi^T holds output column 16 t + 2 r + j of its 64, where n = 8 r + 2 t + j: the
+  // stage's TMEM loads give thread t of a quad the accumulator columns 8 r + 2 t + {0, 1}, which are then 16 in a row
+  const int col = blockIdx.y == 1 ? (n & ~63) + 16 * ((n >> 1) & 3) + 2 * ((n >> 3) & 7) + (n & 1) : n;
+  const float v = __ldg(src + (int64_t)col * ld_n + (int64_t)k * ld_k);
   const __half hi = __float2half_rn(v);
   const __half lo = __float2half_rn(v - __half2float(hi));
   const int kc = k / 64, nb = n / 128, rr = n % 128, c = (k % 64) / 8, w = k % 8;
@@ -111,11 +121,6 @@ __global__ void k_v2_operand_image(const float* __restrict__ rotation, const flo
   uint16_t* img = reinterpret_cast<uint16_t*>(image);
   img[off] = __half_as_ushort(hi);
   img[(size_t)KC * NBLK * (kChunk / 2) + off] = __half_as_ushort(lo);
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  tmem_issue16(taddr, r);
-  tmem_wait16(r);
 }
 
 // The 32 bytes of one vector's row that an epilogue step produces or reads.  A warp's access touches 32 rows, that is 32
@@ -146,8 +151,31 @@ __device__ __forceinline__ void load_row32(const void* src, uint32_t (&v)[8], bo
   }
 }
 
+// 16 rows x 64 accumulator columns of this warp's lanes: registers 4 r + {0, 1} are row lane / 4, columns 8 r + 2 (lane % 4) +
+// {0, 1}, registers 4 r + {2, 3} the same of row lane / 4 + 8
+__device__ __forceinline__ void tmem_ld_quads(uint32_t taddr, uint32_t (&r)[32]) {
+  __syncwarp();
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                 "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]),
+                 "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]),
+                 "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+               :
+               : "memory");
+}
+
 template <int D, int STAGE>
-__global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __grid_constant__ V2Stage p) {
+__global__ void __launch_bounds__(VCfg<D>::kThreads + (STAGE == 2 ? kExpandThreads : 0), 1) k_umma_v2_stage(const __grid_constant__ V2Stage p) {
   using C = VCfg<D>;
   constexpr int KC = C::KC, NBLK = C::NBLK;
   constexpr int PA = STAGE == 1 ? 1 : 2;       // pieces of A
@@ -175,6 +203,9 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
   const uint32_t bar_bempty = bar_bfull + 8 * kNB;          // [kNB] MMA commit -> producer
   const uint32_t bar_tfull = bar_bempty + 8 * kNB;          // [2] MMA commit -> epilogue
   const uint32_t bar_tempty = bar_tfull + 16;               // [2] epilogue (4 arrivals) -> MMA
+  const uint32_t bar_rfull = bar_tempty + 16;               // [2] stage 2: TMA -> expanders (index bytes)
+  const uint32_t bar_rempty = bar_rfull + 16;               // [2] stage 2: expanders -> producer
+  const uint32_t raw_smem = base + C::kOffRaw;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + C::kOffBar + 200);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + C::kOffBar + 208);
 
@@ -185,13 +216,14 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
   const int n_local = t1 - t0;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < C::kASlots; ++i) { mbar_init(bar_afull + 8 * i, 1); mbar_init(bar_aempty + 8 * i, 1); }
+    for (int i = 0; i < C::kASlots; ++i) { mbar_init(bar_afull + 8 * i, STAGE == 2 ? kExpandThreads : 1); mbar_init(bar_aempty + 8 * i, 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(bar_rfull + 8 * i, 1); mbar_init(bar_rempty + 8 * i, kExpandThreads); }
     for (int i = 0; i < kNB; ++i) { mbar_init(bar_bfull + 8 * i, 1); mbar_init(bar_bempty + 8 * i, 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(bar_tfull + 8 * i, 1); mbar_init(bar_tempty + 8 * i, 4 * NBLK); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if constexpr (STAGE == 1) {
+  if constexpr (STAGE != 3) {
     if (threadIdx.x >= 64 && threadIdx.x < 64 + 256) {
       const int e = threadIdx.x - 64;
       thr_s[e] = __ldg(p.codebook + kThresholdOff + e);
@@ -218,11 +250,18 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
         const int row0 = (t0 + i) * kRowsT;
         for (int kc = 0; kc < KC && ok; ++kc, ++ac) {
           const int as = ac % C::kASlots;
-          ok = mbar_wait(bar_aempty + 8 * as, (uint32_t)(((ac / C::kASlots) & 1) ^ 1), abort_flag);
-          if (!ok) break;
-          mbar_arrive_expect_tx(bar_afull + 8 * as, PA * kChunk);
-          tma_load_2d(a_smem + as * kChunk, &p.a_hi_map, kc * 64, row0, bar_afull + 8 * as);
-          if constexpr (PA == 2) tma_load_2d(a_smem + (C::kASlots + as) * kChunk, &p.a_lo_map, kc * 64, row0, bar_afull + 8 * as);
+          if constexpr (STAGE == 2) {                       // the operand itself is written by the expanders
+            ok = mbar_wait(bar_rempty + 8 * as, (uint32_t)(((ac / C::kASlots) & 1) ^ 1), abort_flag);
+            if (!ok) break;
+            mbar_arrive_expect_tx(bar_rfull + 8 * as, kRawChunk);
+            tma_load_2d(raw_smem + as * kRawChunk, &p.a_hi_map, kc * 64, row0, bar_rfull + 8 * as);
+          } else {
+            ok = mbar_wait(bar_aempty + 8 * as, (uint32_t)(((ac / C::kASlots) & 1) ^ 1), abort_flag);
+            if (!ok) break;
+            mbar_arrive_expect_tx(bar_afull + 8 * as, PA * kChunk);
+            tma_load_2d(a_smem + as * kChunk, &p.a_hi_map, kc * 64, row0, bar_afull + 8 * as);
+            if constexpr (PA == 2) tma_load_2d(a_smem + (C::kASlots + as) * kChunk, &p.a_lo_map, kc * 64, row0, bar_afull + 8 * as);
+          }
           for (int pb = 0; pb < 2; ++pb) {
             const int s = bc % kNB;
             ok = mbar_wait(bar_bempty + 8 * s, (uint32_t)(((bc / kNB) & 1) ^ 1), abort_flag);
@@ -240,7 +279,7 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
       // none of this CTA's own copies may still be in flight when it exits
       for (int k = 0; k < C::kASlots && k < ac; ++k) {
         const int j = ac - 1 - k;
-        mbar_wait(bar_afull + 8 * (j % C::kASlots), (uint32_t)((j / C::kASlots) & 1), abort_flag);
+        mbar_wait((STAGE == 2 ? bar_rfull : bar_afull) + 8 * (j % C::kASlots), (uint32_t)((j / C::kASlots) & 1), abort_flag);
       }
       for (int k = 0; k < kNB && k < bc; ++k) {
         const int j = bc - 1 - k;
@@ -305,6 +344,59 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
       *abort_flag = 1;
       if (p.status != nullptr) atomicCAS(p.status, 0, (STAGE << 20) | (2 << 16) | (int)blockIdx.x);
     }
+  } else if (STAGE == 2 && warp >= C::kThreads / 32) {
+    // ------------------------------------------------------------ expanders (stage 2): index bytes of a k-chunk -> centroid
+    // pieces hi and lo in operand layout, thread = two rows.  The thread walks its four 16-byte pieces in an order XOR-ed with
+    // `g`, a linear map of the row's bits 1 and 2 for which the map and its sum with the identity are both one-to-one:
+    // the eight rows of a quarter warp then read eight different bank groups of the raw chunk and write eight different
+    // ones of the operand.
+    const uint32_t lut = smem_u32(lut_s);
+    bool ok = true;
+    int ac = 0;
+    for (int i = 0; i < n_local && ok; ++i) {
+      for (int kc = 0; kc < KC && ok; ++kc, ++ac) {
+        const int as = ac % C::kASlots;
+        const uint32_t parity = (uint32_t)((ac / C::kASlots) & 1);
+        ok = mbar_wait(bar_rfull + 8 * as, parity, abort_flag) && mbar_wait(bar_aempty + 8 * as, parity ^ 1u, abort_flag);
+        if (!ok) break;
+#pragma unroll 1
+        for (int row = threadIdx.x - C::kThreads; row < kRowsT; row += kExpandThreads) {
+        const uint32_t r1 = (uint32_t)(row >> 1) & 1u, r2 = (uint32_t)(row >> 2) & 1u;
+        const uint32_t g = ((r2 ^ r1) << 1) | r2;
+        const uint32_t src = raw_smem + as * kRawChunk + (uint32_t)row * 64u;
+        const uint32_t dst = a_smem + as * kChunk + (uint32_t)row * 128u;
+#pragma unroll
+        for (uint32_t c = 0; c < 4; ++c) {
+          const uint32_t cc = c ^ g;
+          const uint4 x = ld_shared_v4(src + cc * 16u);
+          const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (uint32_t h = 0; h < 2; ++h) {                // 8 coordinates: one 16-byte operand chunk per piece
+            uint32_t e[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const uint32_t w = xw[2 * h + (u >> 2)];
+              const int sh = 8 * (u & 3);
+              const uint32_t off = sh == 0 ? ((w << 2) & 0x3FCu) : ((w >> (sh - 2)) & 0x3FCu);
+              asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e[u]) : "r"(lut + off));
+            }
+            const uint32_t at = dst + (((2u * cc + h) ^ (uint32_t)(row & 7)) << 4);
+            st_shared_v4(at, __byte_perm(e[0], e[1], 0x5410), __byte_perm(e[2], e[3], 0x5410), __byte_perm(e[4], e[5], 0x5410),
+                         __byte_perm(e[6], e[7], 0x5410));
+            st_shared_v4(at + C::kASlots * kChunk, __byte_perm(e[0], e[1], 0x7632), __byte_perm(e[2], e[3], 0x7632),
+                         __byte_perm(e[4], e[5], 0x7632), __byte_perm(e[6], e[7], 0x7632));
+          }
+        }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // operand writes -> visible to the tensor core
+        mbar_arrive(bar_afull + 8 * as);
+        mbar_arrive(bar_rempty + 8 * as);
+      }
+    }
+    if (!ok) {
+      *abort_flag = 1;
+      if (p.status != nullptr) atomicCAS(p.status, 0, (STAGE << 20) | (4 << 16) | (int)blockIdx.x);
+    }
   } else {
     // ------------------------------------------------------------ epilogue: per tile in flight one warpgroup per block
     // of 128 output columns, thread = vector
@@ -327,17 +419,17 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
     for (int i = slot; i < n_local && ok; i += 2) {
       const int64_t row = (int64_t)(t0 + i) * kRowsT + rloc;
       const bool valid = row < p.n;
-      // stage 2: the vector's norm and its first coordinates are in flight while the tile's contraction runs
-      // (together with TMEM loads that run behind the arithmetic: 496 -> 483 us for the call above)
-      const uint16_t* xrow = p.x + (valid ? row : 0) * D + blk * 128;
+      // stage 2: a quad of lanes holds 64 columns of a row, 16 each, so that its accesses to x, k_mse and the pieces are whole
+      // 128-byte lines (see below).  The norms and the first coordinates are in flight while the tile's contraction runs.
+      const int quad = lane & 3, r8 = lane >> 2;
+      const int64_t qrow = (int64_t)(t0 + i) * kRowsT + quarter * 32 + r8;        // rows qrow + {0, 8, 16, 24}
       const bool x_wide = ((uintptr_t)p.x & 31u) == 0;
-      constexpr int kAhead = 3;                   // steps of 16 coordinates in flight
-      uint32_t xn[kAhead][8];
-      float nv = 0.f;
+      uint32_t xn[8];
+      float nv4[4];
       if constexpr (STAGE == 2) {
-        nv = valid ? p.norms[row] : 0.f;
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) load_row32(xrow + 16 * u, xn[u], x_wide);
+        for (int u = 0; u < 4; ++u) nv4[u] = qrow + 8 * u < p.n ? p.norms[qrow + 8 * u] : 0.f;
+        load_row32(p.x + (qrow < p.n ? qrow : 0) * D + blk * 128 + 16 * quad, xn, x_wide);
       }
       // The exit decision is made uniform before anything collective: per warp (the TMEM loads are
       // warp-collective) and, where the two warpgroups of a tile later meet at a named barrier (stage 2,
@@ -369,10 +461,10 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
         const float inv = __fdiv_rn(1.0f, norm + 1e-8f);
         if (valid && blk == 0) p.norms[row] = norm;
         const int bits = p.bits;
+        uint32_t ib0[4] = {0u, 0u, 0u, 0u};       // index bytes of the even step
 #pragma unroll 1
         for (int c = 0; c < 8; ++c) {
           tmem_wait16(v);
-          uint32_t w[16];
           uint32_t ib[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
@@ -399,7 +491,6 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
               }
               idx = lo;
             }
-            w[e] = lut_s[idx];
             ib[e >> 2] |= (uint32_t)idx << (8 * (e & 3));
           }
           if (c + 1 < 8) tmem_issue16(tacc + (c + 1) * 16, v);
@@ -436,62 +527,81 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __
               *reinterpret_cast<uint16_t*>(dst) = (uint16_t)o;
             }
           }
-          if (valid) {
-            uint32_t ph[8], pl[8];
+          if ((c & 1) == 0) {                     // two steps leave as one access
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              ph[j] = __byte_perm(w[2 * j], w[2 * j + 1], 0x5410);
-              pl[j] = __byte_perm(w[2 * j], w[2 * j + 1], 0x7632);
-            }
-            store_row32(p.p_hi + row * D + col0 + c * 16, ph, true);
-            store_row32(p.p_lo + row * D + col0 + c * 16, pl, true);
+            for (int j = 0; j < 4; ++j) ib0[j] = ib[j];
+          } else if (valid) {
+            const uint32_t both[8] = {ib0[0], ib0[1], ib0[2], ib0[3], ib[0], ib[1], ib[2], ib[3]};
+            store_row32(reinterpret_cast<uint8_t*>(p.p_hi + row * D) + col0 + (c - 1) * 16, both, true);
           }
         }
       } else if constexpr (STAGE == 2) {
-        float ssq = 0.f;
+        // Rows x 32 bytes per access cost the load/store unit a slot per row (see store_row32), and the operand traffic of the
+        // MMAs and the expanders runs through the same data path: thread = row took 199 us here for the call above, of
+        // which 16 400 of 26 600 clocks per tile were such slots.  tcgen05.ld.16x256b spreads a row over a quad of lanes
+        // instead: thread (r8, quad) gets rows r8 and r8 + 8 of 16, 16 columns each, and a warp's access is 8 lines: 133 us.
         const bool k_wide = ((uintptr_t)p.k_mse_out & 31u) == 0;
-        tmem_issue16(tacc, v);
-#pragma unroll 1
-        for (int c = 0; c < 8; ++c) {
-          uint32_t xw[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            xw[j] = xn[0][j];
+        for (int rg = 0; rg < 2; ++rg) {            // 16 rows
+          float sq[2] = {0.f, 0.f};
 #pragma unroll
-            for (int u = 0; u + 1 < kAhead; ++u) xn[u][j] = xn[u + 1][j];
-          }
-          if (c + kAhead < 8) load_row32(xrow + 16 * (c + kAhead), xn[kAhead - 1], x_wide);
-          tmem_wait16(v);
-          if (valid) {
-            uint32_t kq[8], rh[8], rl[8];
+          for (int cg = 0; cg < 2; ++cg) {          // 64 columns
+            uint32_t a[32];
+            tmem_ld_quads(tacc + ((uint32_t)(rg * 16) << 16) + (uint32_t)(cg * 64), a);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float k0 = __uint_as_float(v[2 * j]) * nv, k1 = __uint_as_float(v[2 * j + 1]) * nv;
-              const __half2 xh = *reinterpret_cast<const __half2*>(&xw[j]);
-              const float r0 = __low2float(xh) - k0, r1 = __high2float(xh) - k1;
-              ssq = fmaf(r0, r0, ssq);
-              ssq = fmaf(r1, r1, ssq);
-              const __half2 kh = __floats2half2_rn(k0, k1);
-              kq[j] = *reinterpret_cast<const uint32_t*>(&kh);
-              const __half2 hh = __floats2half2_rn(r0, r1);
-              rh[j] = *reinterpret_cast<const uint32_t*>(&hh);
-              const __half2 ll = __floats2half2_rn(r0 - __low2float(hh), r1 - __high2float(hh));
-              rl[j] = *reinterpret_cast<const uint32_t*>(&ll);
+            for (int hh = 0; hh < 2; ++hh) {
+              const int64_t r = qrow + 16 * rg + 8 * hh;
+              const int64_t at = r * D + col0 + 64 * cg + 16 * quad;
+              uint32_t xw[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) xw[j] = xn[j];
+              const int nxt = 4 * rg + 2 * cg + hh + 1;                // the next (rg, cg, hh)
+              if (nxt < 8) {
+                const int64_t rn = qrow + 16 * (nxt >> 2) + 8 * (nxt & 1);
+                load_row32(p.x + (rn < p.n ? rn : 0) * D + col0 + 64 * ((nxt >> 1) & 1) + 16 * quad, xn, x_wide);
+              }
+              if (r < p.n) {
+                const float nv = nv4[2 * rg + hh];
+                uint32_t kq[8], rh[8], rl[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  const float k0 = __uint_as_float(a[4 * j + 2 * hh]) * nv, k1 = __uint_as_float(a[4 * j + 2 * hh + 1]) * nv;
+                  const __half2 xh = *reinterpret_cast<const __half2*>(&xw[j]);
+                  const float r0 = __low2float(xh) - k0, r1 = __high2float(xh) - k1;
+                  sq[hh] = fmaf(r0, r0, sq[hh]);
+                  sq[hh] = fmaf(r1, r1, sq[hh]);
+                  const __half2 kh = __floats2half2_rn(k0, k1);
+                  kq[j] = *reinterpret_cast<const uint32_t*>(&kh);
+                  const __half2 h2 = __floats2half2_rn(r0, r1);
+                  rh[j] = *reinterpret_cast<const uint32_t*>(&h2);
+                  const __half2 l2 = __floats2half2_rn(r0 - __low2float(h2), r1 - __high2float(h2));
+                  rl[j] = *reinterpret_cast<const uint32_t*>(&l2);
+                }
+                if (p.k_mse_out != nullptr) store_row32(p.k_mse_out + at, kq, k_wide);
+                store_row32(p.p_hi + at, rh, true);
+                store_row32(p.p_lo + at, rl, true);
+              }
             }
-            if (p.k_mse_out != nullptr) store_row32(p.k_mse_out + row * D + col0 + c * 16, kq, k_wide);
-            store_row32(p.p_hi + row * D + col0 + c * 16, rh, true);
-            store_row32(p.p_lo + row * D + col0 + c * 16, rl, true);
           }
-          if (c + 1 < 8) tmem_issue16(tacc + (c + 1) * 16, v);
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {          // the quad's four parts of a row
+            sq[hh] += __shfl_xor_sync(0xffffffffu, sq[hh], 1);
+            sq[hh] += __shfl_xor_sync(0xffffffffu, sq[hh], 2);
+            const int64_t r = qrow + 16 * rg + 8 * hh;
+            if constexpr (NBLK == 2) {
+              // the residual norm spans both blocks: each warpgroup leaves its part
+              if (quad == 0) part_s[(slot * 2 + blk) * 128 + quarter * 32 + r8 + 16 * rg + 8 * hh] = sq[hh];
+            } else {
+              if (quad == 0 && r < p.n) p.rnorm_out[r] = __half_as_ushort(__float2half_rn(__fsqrt_rn(sq[hh])));
+            }
+          }
         }
         if constexpr (NBLK == 2) {
-          // the residual norm spans both blocks: the upper block's warpgroup hands its partial sum over
-          if (blk == 1) part_s[slot * 128 + rloc] = ssq;
           asm volatile("bar.sync %0, 256;" ::"r"(1 + slot) : "memory");
-          if (blk == 0) ssq += part_s[slot * 128 + rloc];
+          if (blk == 0 && valid)
+            p.rnorm_out[row] = __half_as_ushort(__float2half_rn(__fsqrt_rn(part_s[slot * 2 * 128 + rloc] + part_s[(slot * 2 + 1) * 128 + rloc])));
           asm volatile("bar.sync %0, 256;" ::"r"(1 + slot) : "memory");     // part_s is reused by the next tile
         }
-        if (valid && blk == 0) p.rnorm_out[row] = __half_as_ushort(__float2half_rn(__fsqrt_rn(ssq)));
       } else {
         const bool s_wide = ((uintptr_t)p.signs_out & 31u) == 0;
 #pragma unroll 1
@@ -553,12 +663,25 @@ int encode_rows(TensorMapEncodeFn enc, CUtensorMap* map, const void* ptr, int64_
   return TQ_OK;
 }
 
+// index bytes: n rows of D bytes, 2 D bytes apart
+int encode_index_rows(TensorMapEncodeFn enc, CUtensorMap* map, const void* ptr, int64_t n, int D) {
+  cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)n};
+  cuuint64_t strides[1] = {(cuuint64_t)D * 2};
+  cuuint32_t box[2] = {64, (cuuint32_t)kRowsT};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { note_cuda_error(100000 + (int)r); return TQ_ELAUNCH; }
+  return TQ_OK;
+}
+
 template <int D, int STAGE>
 int launch_stage(const V2Stage& p, int grid, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k_umma_v2_stage<D, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)VCfg<D>::kSmemBytes);
   if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
-  k_umma_v2_stage<D, STAGE><<<grid, VCfg<D>::kThreads, VCfg<D>::kSmemBytes, st>>>(p);
+  k_umma_v2_stage<D, STAGE><<<grid, VCfg<D>::threads(STAGE), VCfg<D>::kSmemBytes, st>>>(p);
   return check_launch();
 }
 
@@ -610,11 +733,13 @@ int run(const TqQjlCompressJob& job, cudaStream_t st) {
   p.a_lo_map = p.a_hi_map;
   p.b_image = img1;
   if ((rc = launch_stage<D, 1>(p, grid, st)) != TQ_OK) return rc;
-  // stages 2 and 3: A = the piece arrays
-  if ((rc = encode_rows(enc, &p.a_hi_map, p_hi, n, D)) != TQ_OK) return rc;
-  if ((rc = encode_rows(enc, &p.a_lo_map, p_lo, n, D)) != TQ_OK) return rc;
+  // stage 2: A from the index bytes at the head of the rows of p_hi
+  if ((rc = encode_index_rows(enc, &p.a_hi_map, p_hi, n, D)) != TQ_OK) return rc;
   p.b_image = img2;
   if ((rc = launch_stage<D, 2>(p, grid, st)) != TQ_OK) return rc;
+  // stage 3: A = the piece arrays
+  if ((rc = encode_rows(enc, &p.a_hi_map, p_hi, n, D)) != TQ_OK) return rc;
+  if ((rc = encode_rows(enc, &p.a_lo_map, p_lo, n, D)) != TQ_OK) return rc;
   p.b_image = img3;
   return launch_stage<D, 3>(p, grid, st);
 }
