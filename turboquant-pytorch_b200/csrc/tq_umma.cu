@@ -911,10 +911,24 @@ __device__ __forceinline__ bool view_advance(const UmmaDeqBatchOf<J>& b, int til
 
 #include "tq_tc_expand.cuh"
 
+// 32 bytes of a row, as one access where the rows start on 32-byte boundaries: a warp's store touches 32 rows and takes 32
+// slots of the load/store unit whatever its width.  16-byte stores: 19 us for the rebuild of 156 000 vectors of head_dim 64, 17 so.
+__device__ __forceinline__ void store_32_bytes(void* dst, const uint32_t* v, bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+  } else {
+    uint4* o = reinterpret_cast<uint4*>(dst);
+    o[0] = make_uint4(v[0], v[1], v[2], v[3]);
+    o[1] = make_uint4(v[4], v[5], v[6], v[7]);
+  }
+}
+
 // The TMEM load is warp-collective: every lane of the warp must come through here, rows
 // past the end of a slab included; `valid` only guards the stores.
 template <int ODT, int D>
-__device__ __forceinline__ void drain_row(uint32_t tacc, float nv, void* out_row, bool valid) {
+__device__ __forceinline__ void drain_row(uint32_t tacc, float nv, void* out_row, bool valid, bool wide) {
   uint32_t a[16], b[16];
   tmem_issue16(tacc, a);
 #pragma unroll 1
@@ -930,9 +944,12 @@ __device__ __forceinline__ void drain_row(uint32_t tacc, float nv, void* out_row
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(cur[e]) * nv;
         if constexpr (ODT == TQ_F32) {
-          float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(out_row) + (c + hb) * 16);
+          uint32_t w[16];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) o[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+          for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(v[e]);
+          float* o = reinterpret_cast<float*>(out_row) + (c + hb) * 16;
+          store_32_bytes(o, w, wide);
+          store_32_bytes(o + 8, w + 8, wide);
         } else {
           uint32_t pk[8];
 #pragma unroll
@@ -945,9 +962,7 @@ __device__ __forceinline__ void drain_row(uint32_t tacc, float nv, void* out_row
               pk[e] = *reinterpret_cast<uint32_t*>(&h);
             }
           }
-          uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(out_row) + (c + hb) * 16);
-          o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-          o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+          store_32_bytes(reinterpret_cast<uint16_t*>(out_row) + (c + hb) * 16, pk, wide);
         }
       }
     }
@@ -1254,8 +1269,9 @@ __global__ void __launch_bounds__(DCfg<ROWS, NARROW, D>::kThreadsD, 1) k_umma_de
         const int64_t off = (int64_t)bb * job.os_b + (int64_t)hh * job.os_h + s_row * job.os_s;
         auto drain = [&](auto odt, auto* out) {
           constexpr int ODT = decltype(odt)::value;
-          drain_row<ODT, D>(tacc, nv, out + off, valid);
-          if constexpr (D == 64) drain_row<ODT, D>(tacc + 64, nv2, out + off + kTileRows * job.os_s, valid2);
+          const bool wide = (((uintptr_t)job.out | (uintptr_t)((job.os_b | job.os_h | job.os_s) * (int64_t)sizeof(*out))) & 31u) == 0;
+          drain_row<ODT, D>(tacc, nv, out + off, valid, wide);
+          if constexpr (D == 64) drain_row<ODT, D>(tacc + 64, nv2, out + off + kTileRows * job.os_s, valid2, wide);
         };
         if (D == 128 || job.out_dtype == TQ_F32) drain(std::integral_constant<int, TQ_F32>{}, reinterpret_cast<float*>(job.out));
         else if (job.out_dtype == TQ_F16) drain(std::integral_constant<int, TQ_F16>{}, reinterpret_cast<uint16_t*>(job.out));
