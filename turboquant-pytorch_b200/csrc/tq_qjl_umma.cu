@@ -6,8 +6,8 @@
 // is ONE contraction of length 2D when the key side is written as the row
 // [k_mse_key | signs_key * ||r_key||] (both halves exact in fp16: k_mse and ||r|| are stored
 // as fp16, signs are +-1) and the query side as [Q_q | sqrt(pi/2)/D * S Q_q], split into
-// fp16 pieces hi + lo (lo reaches into fp16 subnormals, so both passes accumulate into one
-// fp32 TMEM accumulator and the products match an fp32 matmul to ~1e-7).
+// fp16 pieces hi + lo (lo reaches into fp16 subnormals) that are separate columns of one fp32 TMEM accumulator; their sum
+// matches an fp32 matmul to ~1e-7.
 //
 // A persistent, warp-specialised CTA per SM walks 128-key tiles of one (batch*head, block of
 // up to 64 queries) unit after the other:
@@ -15,8 +15,11 @@
 //                swizzle: already the operand layout) and of raw sign chunks (128 x 64 bytes);
 //                the unit's query image (all chunks, hi and lo) by bulk copy on unit change
 //   warps 2..9   expanders: signs -> fp16 +-||r|| written in the swizzled operand layout
-//   warp 1       issues tcgen05.mma kind::f16, M=128 N=64 K=16: 2 pieces x 4 k-steps per chunk
-//   warps 10..13 drain: TMEM -> 128-byte rows of scores[q][key0 .. key0+31]
+//   warp 1       issues tcgen05.mma kind::f16, M=128 N=128 K=16: columns 0..63 are the queries' high pieces, 64..127 their
+//                low pieces, 4 k-steps per chunk.  An MMA of N = 64 takes as long as one of N = 128 (66 and 65 clocks), so
+//                a pass per piece over the same keys cost twice the tensor time and read every key operand twice (70 us
+//                for 16 heads x 16384 keys of head_dim 256, 66 so)
+//   warps 10..13 drain: TMEM -> high + low -> 128-byte rows of scores[q][key0 .. key0+31]
 // Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, records a status
 // word and leaves through the normal exit.
 
@@ -47,7 +50,7 @@ template <int D>
 struct QCfg {
   static constexpr int kHalfChunks = D / 64;                     // chunks per operand half (k_mse | signs)
   static constexpr int kChunks = 2 * kHalfChunks;                // contraction length 2D in chunks of 64
-  static constexpr uint32_t kImageBytes = 2u * kChunks * kChunkB;   // hi pieces then lo pieces
+  static constexpr uint32_t kImageBytes = 2u * kChunks * kChunkB;   // per chunk the high pieces of 64 queries, then the low ones
   static constexpr uint32_t kOffImg = 0;
   static constexpr uint32_t kOffK = kOffImg + kImageBytes;
   static constexpr uint32_t kOffG = kOffK + kNSK * kChunkA;
@@ -62,7 +65,7 @@ struct QjlBatch {
   CUtensorMap kmse_map;      // fp16 (D, Sk, BH), box 64 x 128, 128-byte swizzle
   CUtensorMap sign_map;      // uint8 (D, Sk, BH), box 64 x 128, no swizzle
   const uint16_t* rnorm;     // fp16 bits (BH, Sk)
-  const uint8_t* images;     // [unit][hi | lo][chunk][64 rows x 128 bytes swizzled]
+  const uint8_t* images;     // [unit][chunk][hi | lo][64 rows x 128 bytes swizzled]
   float* scores;             // (BH, Sq, Sk)
   int32_t* status;
   int64_t Sq, Sk;
@@ -136,7 +139,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(smem_u32((const void*)tmem_slot), 256);
+  if (warp == 1) tmem_alloc(smem_u32((const void*)tmem_slot), 2 * kQ * kNT);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -195,9 +198,8 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
     bool ok = true;
     int img_uses = 0, cur_unit = -1;
     int kc = 0, gc = 0;
-    const uint32_t idesc = idesc_f16_n(kQ);
-    const uint64_t b_hi = smem_desc_sw128(img_smem);
-    const uint64_t b_lo = smem_desc_sw128(img_smem + kChunks * kChunkB);
+    const uint32_t idesc = idesc_f16_n(2 * kQ);
+    const uint64_t b_base = smem_desc_sw128(img_smem);
     for (int i = 0; i < n_local && ok; ++i) {
       const int t = t0 + i;
       const int unit = t / tpu;
@@ -210,7 +212,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
       ok = ok && mbar_wait(bar_tempty + 8 * b, (uint32_t)(((i / kNT) & 1) ^ 1), abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      const uint32_t d_tmem = tmem_base + (uint32_t)(b * kQ);
+      const uint32_t d_tmem = tmem_base + (uint32_t)(b * 2 * kQ);
       const bool last_of_unit = i + 1 >= n_local || (t + 1) / tpu != unit;
 #pragma unroll 1
       for (int c = 0; c < kChunks; ++c) {
@@ -233,14 +235,11 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
         if (!ok) break;
         tc_fence_after();
         const uint64_t a_base = smem_desc_sw128(a_addr);
-        const uint64_t b_off = (uint64_t)((uint32_t)c * kChunkB / 16);
+        const uint64_t b_off = (uint64_t)((uint32_t)c * 2u * kChunkB / 16);
         if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_f16(d_tmem, a_base + (uint64_t)(k * 2), b_hi + b_off + (uint64_t)(k * 2), idesc, (c | k) != 0 ? 1u : 0u);
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_f16(d_tmem, a_base + (uint64_t)(k * 2), b_lo + b_off + (uint64_t)(k * 2), idesc, 1u);
+            umma_f16(d_tmem, a_base + (uint64_t)(k * 2), b_base + b_off + (uint64_t)(k * 2), idesc, (c | k) != 0 ? 1u : 0u);
           umma_commit(empty_bar);                          // the operand stage is free once these MMAs are done
           if (c == kChunks - 1) {
             umma_commit(bar_tfull + 8 * b);
@@ -314,21 +313,20 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
       ok = __all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * b, (uint32_t)((i / kNT) & 1), abort_flag));   // warp-collective TMEM loads follow
       if (!ok) break;
       tc_fence_after();
-      const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * kQ);
+      const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * 2 * kQ);
       float* out = batch.scores + (bh * batch.Sq + q0) * batch.Sk + key;
       const bool key_ok = key < batch.Sk;
-      uint32_t ra[16], rb[16];
-      tmem_issue16(tacc, ra);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        uint32_t (&cur)[16] = (c & 1) ? rb : ra;
-        uint32_t (&nxt)[16] = (c & 1) ? ra : rb;
+        uint32_t cur[16], low[16];
+        tmem_issue16(tacc + c * 16, cur);
+        tmem_issue16(tacc + kQ + c * 16, low);
         tmem_wait16(cur);
-        if (c + 1 < 4) tmem_issue16(tacc + (c + 1) * 16, nxt);
+        tmem_wait16(low);
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
           const int q = c * 16 + e;
-          if (key_ok && q0 + q < batch.Sq) out[(int64_t)q * batch.Sk] = __uint_as_float(cur[e]);
+          if (key_ok && q0 + q < batch.Sq) out[(int64_t)q * batch.Sk] = __uint_as_float(cur[e]) + __uint_as_float(low[e]);
         }
       }
       tc_fence_before();
@@ -344,7 +342,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 256);
+    tmem_dealloc(tmem_base, 2 * kQ * kNT);
   }
 }
 

@@ -963,7 +963,7 @@ __global__ void __launch_bounds__(NT) k_qjl_scores(TqQjlScoreJob job, const floa
 }
 
 // Query operand of the tensor-core score kernel (tq_qjl_umma.cu), head_dim a multiple of 64: per unit (head, block of
-// 64 queries) the rows [Q | corr * Q S^T] as fp16 pieces hi + lo, laid out [piece][chunk of 64 columns][row][64], rows of
+// 64 queries) the rows [Q | corr * Q S^T] as fp16 pieces hi + lo, laid out [chunk of 64 columns][piece][row][64], rows of
 // 128 bytes with 16-byte chunk c at c ^ (row & 7); rows past Sq are zero.  A CTA takes 32 rows and 64 columns: the
 // projection (one sequential chain per output, as tq_project), then the query's own columns and the projected ones.
 // 1024 queries of head_dim 256 took 27 us as projection, upcast and image kernels (the projection read the whole matrix
@@ -987,8 +987,8 @@ __global__ void __launch_bounds__(NT) k_qjl_query_operand(const void* q, int D, 
   zero_acc<RI, 1>(acc);
   tile_gemm<RI, 1, B_KN>(As, lda, D, qjl_t + cb * 64, D, 64, Bs, acc);
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const size_t piece = (size_t)2 * chunks * 64 * 64;                       // elements of one piece
-  uint16_t* img = reinterpret_cast<uint16_t*>(images) + (size_t)unit * 2 * piece;
+  constexpr size_t piece = 64 * 64;                                        // elements of one piece of a chunk
+  uint16_t* img = reinterpret_cast<uint16_t*>(images) + (size_t)unit * 2 * chunks * 2 * piece;
 #pragma unroll
   for (int ri = 0; ri < RI; ++ri) {
     const int r = ty * RI + ri, n = half * ROWS + r;
@@ -1002,7 +1002,7 @@ __global__ void __launch_bounds__(NT) k_qjl_query_operand(const void* q, int D, 
         hi[c] = __half_as_ushort(h);
         lo[c] = __half_as_ushort(__float2half_rn(v - __half2float(h)));
       }
-      const size_t off = (size_t)(part * chunks + cb) * (64 * 64) + (size_t)n * 64 + (size_t)((((4 * tx) >> 3) ^ (n & 7)) * 8 + ((4 * tx) & 7));
+      const size_t off = (size_t)(part * chunks + cb) * 2 * piece + (size_t)n * 64 + (size_t)((((4 * tx) >> 3) ^ (n & 7)) * 8 + ((4 * tx) & 7));
       *reinterpret_cast<uint2*>(img + off) = make_uint2(hi[0] | ((uint32_t)hi[1] << 16), hi[2] | ((uint32_t)hi[3] << 16));
       *reinterpret_cast<uint2*>(img + piece + off) = make_uint2(lo[0] | ((uint32_t)lo[1] << 16), lo[2] | ((uint32_t)lo[3] << 16));
     }
