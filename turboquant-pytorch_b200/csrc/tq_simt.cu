@@ -199,29 +199,70 @@ __device__ __forceinline__ void load_codebook(const float* cb, float* cent_s, fl
   }
 }
 
+// quantize_scalar for U values side by side: a search is `bits` dependent look-ups, so several in step hide one another
+// (with 16-byte stores in k_dequantize: first-generation cache of 8192 keys and values 111 -> 106 us a pass, fp32 round trip of
+// 4096 vectors 26.7 -> 24.6 us).
+template <int U>
+__device__ __forceinline__ void quantize_many(const float (&y)[U], const float* thr, int bits, int (&q)[U]) {
+#pragma unroll
+  for (int u = 0; u < U; ++u) q[u] = 0;
+  for (int half = 1 << (bits - 1); half > 0; half >>= 1) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (y[u] > thr[q[u] + half - 1]) q[u] += half;
+  }
+}
+
+// Packed bytes of one row, NB bytes per lane and step.
+template <int IPB, int NB>
+__device__ __forceinline__ void emit_packed_row(const float* row, int D, int bits, const float* thr_s, uint8_t* o, int lane) {
+  const int G = (D + IPB - 1) / IPB;
+  for (int g0 = lane; g0 < G; g0 += 32 * NB) {
+    float y[IPB * NB];
+    int q[IPB * NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int i = 0; i < IPB; ++i) {
+        const int c = (g0 + 32 * b) * IPB + i;
+        y[b * IPB + i] = c < D ? row[c] : -INFINITY;          // past the end: index 0
+      }
+    quantize_many<IPB * NB>(y, thr_s, bits, q);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      unsigned byte = 0;
+#pragma unroll
+      for (int i = 0; i < IPB; ++i) byte |= (unsigned)q[b * IPB + i] << (bits * (IPB - 1 - i));
+      if (g0 + 32 * b < G) o[g0 + 32 * b] = (uint8_t)byte;
+    }
+  }
+}
+
 // Quantise the row Cs[r][0..D) and write it in the requested layout.
 __device__ __forceinline__ void emit_indices_row(const float* row, int D, int bits, int mode, const float* thr_s,
                                                  void* out, int64_t n, int lane) {
-  const int levels = 1 << bits;
   if (mode == TQ_IDX_PACKED) {
     const int ipb = 8 / bits;
-    const int G = (D + ipb - 1) / ipb;
-    uint8_t* o = reinterpret_cast<uint8_t*>(out) + n * (int64_t)G;
-    for (int g = lane; g < G; g += 32) {
-      unsigned byte = 0;
-      for (int i = 0; i < ipb; ++i) {
-        int c = g * ipb + i;
-        unsigned q = (c < D) ? (unsigned)quantize_scalar(row[c], thr_s, levels) : 0u;
-        byte |= q << (bits * (ipb - 1 - i));
-      }
-      o[g] = (uint8_t)byte;
+    uint8_t* o = reinterpret_cast<uint8_t*>(out) + n * (int64_t)((D + ipb - 1) / ipb);
+    if (ipb == 1) emit_packed_row<1, 4>(row, D, bits, thr_s, o, lane);
+    else if (ipb == 2) emit_packed_row<2, 2>(row, D, bits, thr_s, o, lane);
+    else if (ipb == 4) emit_packed_row<4, 1>(row, D, bits, thr_s, o, lane);
+    else emit_packed_row<8, 1>(row, D, bits, thr_s, o, lane);
+    return;
+  }
+  for (int c0 = lane; c0 < D; c0 += 128) {
+    float y[4];
+    int q[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) y[u] = c0 + 32 * u < D ? row[c0 + 32 * u] : 0.f;
+    quantize_many<4>(y, thr_s, bits, q);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int c = c0 + 32 * u;
+      if (c >= D) continue;
+      if (mode == TQ_IDX_U8) reinterpret_cast<uint8_t*>(out)[n * (int64_t)D + c] = (uint8_t)q[u];
+      else reinterpret_cast<int64_t*>(out)[n * (int64_t)D + c] = (int64_t)q[u];
     }
-  } else if (mode == TQ_IDX_U8) {
-    uint8_t* o = reinterpret_cast<uint8_t*>(out) + n * (int64_t)D;
-    for (int c = lane; c < D; c += 32) o[c] = (uint8_t)quantize_scalar(row[c], thr_s, levels);
-  } else {
-    int64_t* o = reinterpret_cast<int64_t*>(out) + n * (int64_t)D;
-    for (int c = lane; c < D; c += 32) o[c] = (int64_t)quantize_scalar(row[c], thr_s, levels);
   }
 }
 
@@ -342,15 +383,19 @@ __global__ void __launch_bounds__(NT) k_dequantize(TqDequantizeJob job) {
       float nv = (job.norms != nullptr) ? __half2float(__ushort_as_half(job.norms[n])) : 1.f;
       int64_t off = vec_offset(n, job.H, job.S, job.ostride_b, job.ostride_h, job.ostride_s);
 #pragma unroll
-      for (int j = 0; j < NJ; ++j)
+      for (int j = 0; j < NJ; ++j) {
+        const int col = tx * 4 + 64 * j;
+        float v[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          int col = tx * 4 + 64 * j + c;
-          if (col < D) {
-            float v = (job.norms != nullptr) ? acc[ri][4 * j + c] * nv : acc[ri][4 * j + c];
-            store_elem<ODT>(job.out, off + col, v);
-          }
+        for (int c = 0; c < 4; ++c) v[c] = (job.norms != nullptr) ? acc[ri][4 * j + c] * nv : acc[ri][4 * j + c];
+        if (ODT == TQ_F32 && col + 4 <= D && ((uintptr_t)(reinterpret_cast<float*>(job.out) + off + col) & 15u) == 0) {
+          *reinterpret_cast<float4*>(reinterpret_cast<float*>(job.out) + off + col) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (col + c < D) store_elem<ODT>(job.out, off + col + c, v[c]);
         }
+      }
     }
   }
 }
@@ -784,7 +829,6 @@ __global__ void __launch_bounds__(NT) k_qjl_compress(TqQjlCompressJob job) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int kpad = round_up(D, KC);
-  const int levels = 1 << job.bits;
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t row0 = tile * TM;
     __syncthreads();
@@ -809,17 +853,21 @@ __global__ void __launch_bounds__(NT) k_qjl_compress(TqQjlCompressJob job) {
     // quantise in place: As <- centroid of the nearest level
     for (int r = warp; r < TM; r += NT / 32) {
       int64_t n = row0 + r;
-      for (int c = lane; c < kpad; c += 32) {
-        float v = 0.f;
-        if (c < D) {
-          int q = quantize_scalar(As[r * lda + c], thr_s, levels);
-          v = cent_s[q];
-          if (job.idx_out != nullptr && n < n_total) {
-            if (job.idx_mode == TQ_IDX_I64) reinterpret_cast<int64_t*>(job.idx_out)[n * D + c] = q;
-            else if (job.idx_mode == TQ_IDX_U8) reinterpret_cast<uint8_t*>(job.idx_out)[n * D + c] = (uint8_t)q;
+      for (int c0 = lane; c0 < kpad; c0 += 128) {
+        float y[4];
+        int q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) y[u] = c0 + 32 * u < D ? As[r * lda + c0 + 32 * u] : 0.f;
+        quantize_many<4>(y, thr_s, job.bits, q);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = c0 + 32 * u;
+          if (c < D && job.idx_out != nullptr && n < n_total) {
+            if (job.idx_mode == TQ_IDX_I64) reinterpret_cast<int64_t*>(job.idx_out)[n * D + c] = q[u];
+            else if (job.idx_mode == TQ_IDX_U8) reinterpret_cast<uint8_t*>(job.idx_out)[n * D + c] = (uint8_t)q[u];
           }
+          if (c < kpad) As[r * lda + c] = c < D ? cent_s[q[u]] : 0.f;
         }
-        As[r * lda + c] = v;
       }
     }
     {
