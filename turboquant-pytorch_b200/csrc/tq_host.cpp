@@ -167,7 +167,9 @@ bool read_shape(PyObject* dict, int64_t (&v)[4]) {
 }
 
 // dequantise job of a packed dict into the tokens [0, s) of `out`; false when the dict is not in the plain form
-bool dequantize_job(PyObject* dict, const Codec& c, int dev, const int64_t (&shape)[4], const at::Tensor& out, TqDequantizeJob* j) {
+// (`keep` holds its tensors until the launch is out: the interpreter lock is given up for that)
+bool dequantize_job(PyObject* dict, const Codec& c, int dev, const int64_t (&shape)[4], const at::Tensor& out, TqDequantizeJob* j,
+                    at::Tensor (&keep)[2]) {
   TQ_NAME(k_idx, "idx_bytes"); TQ_NAME(k_norms, "vec_norms");
   PyObject *io = PyDict_GetItem(dict, k_idx), *no = PyDict_GetItem(dict, k_norms);
   if (io == nullptr || no == nullptr || !plain(io, dev) || !plain(no, dev)) return false;
@@ -176,6 +178,8 @@ bool dequantize_job(PyObject* dict, const Codec& c, int dev, const int64_t (&sha
   if (idx.scalar_type() != at::kByte || norms.scalar_type() != at::kHalf || !idx.is_contiguous() || !norms.is_contiguous() ||
       idx.numel() != n * row_bytes(shape[3], c.bits) || norms.numel() != n || shape[3] != c.dim)
     return false;
+  keep[0] = idx;
+  keep[1] = norms;
   *j = TqDequantizeJob{};
   j->idx = idx.data_ptr(); j->norms = (const uint16_t*)norms.data_ptr(); j->idx_mode = TQ_IDX_PACKED;
   j->D = (int32_t)shape[3]; j->bits = (int32_t)c.bits; j->out_dtype = dtype_of(out);
@@ -242,7 +246,7 @@ PyObject* decompress_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   PyObject* comps[2];
   Codec codec[2];
   int64_t inner[2][4], outer[2][4];
-  at::Tensor windows[2];
+  at::Tensor windows[2], keep[2][2];
   for (int i = 0; i < 2; ++i) {                       // look everything over before anything is allocated or launched
     PyObject* side = a[2 + i];
     if (!PyDict_CheckExact(side) || !read_codec(a[i], dev, &codec[i])) return none();
@@ -261,7 +265,7 @@ PyObject* decompress_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (windows[0].scalar_type() != windows[1].scalar_type()) return none();
   for (int i = 0; i < 2; ++i) {
     full[i] = make({outer[i][0], outer[i][1], outer[i][2], outer[i][3]}, windows[i].scalar_type(), dev);
-    if (!dequantize_job(comps[i], codec[i], dev, inner[i], full[i], &jobs[i])) return none();
+    if (!dequantize_job(comps[i], codec[i], dev, inner[i], full[i], &jobs[i], keep[i])) return none();
   }
   int n_copies = 0;
   for (int i = 0; i < 2; ++i) {
@@ -314,7 +318,8 @@ PyObject* decompress(PyObject*, PyObject* const* a, Py_ssize_t n) {
   c10::AutoGradMode no_grad(false);
   at::Tensor out = make({shape[0], shape[1], shape[2], shape[3]}, at::kFloat, dev);
   TqDequantizeJob job;
-  if (!dequantize_job(a[1], c, dev, shape, out, &job)) return none();
+  at::Tensor keep[2];
+  if (!dequantize_job(a[1], c, dev, shape, out, &job, keep)) return none();
   void* st = stream_of(dev);
   if (!call("tq_dequantize", [&] { return api.dequantize(&job, 1, st); })) return nullptr;
   return THPVariable_Wrap(out);
@@ -461,35 +466,52 @@ struct StepPlan {
 const char* const kPlanName = "turboquant.step_plan";
 void free_plan(PyObject* cap) { delete static_cast<StepPlan*>(PyCapsule_GetPointer(cap, kPlanName)); }
 
-bool int_list(PyObject* o, std::vector<int64_t>* v, size_t want) {
-  Ref seq(PySequence_Fast(o, "expected a sequence"));
-  if (!seq || (size_t)PySequence_Fast_GET_SIZE(seq.p) != want) { PyErr_Clear(); return false; }
-  v->resize(want);
-  for (size_t i = 0; i < want; ++i) (*v)[i] = (int64_t)PyLong_AsUnsignedLongLong(PySequence_Fast_GET_ITEM(seq.p, (Py_ssize_t)i));
-  return PyErr_Occurred() == nullptr;
-}
-
-// step_plan(q bytes, d bytes, c bytes, row bytes of each job, base addresses, (L, B, H, D, cap, window, tok_bytes, dtype, dev))
+// step_plan(layer states, window) -> capsule | None.  Fills in what does not change from step to step: the layers'
+// buffers (equal shape, strides of their own, capacity the least of all), codecs and constants.
 PyObject* step_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 6 || !PyBytes_Check(a[0]) || !PyBytes_Check(a[1]) || !PyBytes_Check(a[2])) return none();
-  std::vector<int64_t> v;
-  if (!int_list(a[5], &v, 9)) { PyErr_Clear(); return none(); }
-  const size_t jobs = (size_t)(2 * v[0]);
-  if ((size_t)PyBytes_GET_SIZE(a[0]) != jobs * sizeof(TqQuantizeJob) || (size_t)PyBytes_GET_SIZE(a[1]) != jobs * sizeof(TqDequantizeJob) ||
-      (size_t)PyBytes_GET_SIZE(a[2]) != jobs * sizeof(TqCopyJob))
-    return none();
+  TQ_NAME(n_k, "k"); TQ_NAME(n_v, "v"); TQ_NAME(n_codec, "codec"); TQ_NAME(n_kc, "key_compressor"); TQ_NAME(n_vc, "val_compressor");
+  if (n != 2 || !PyList_CheckExact(a[0]) || PyList_GET_SIZE(a[0]) < 1 || !PyLong_Check(a[1])) return none();
+  const int dev = c10::cuda::current_device();
   auto* p = new StepPlan;
   Ref cap(PyCapsule_New(p, kPlanName, free_plan));
   if (!cap) { delete p; return nullptr; }
-  const auto* q = reinterpret_cast<const TqQuantizeJob*>(PyBytes_AS_STRING(a[0]));
-  const auto* d = reinterpret_cast<const TqDequantizeJob*>(PyBytes_AS_STRING(a[1]));
-  const auto* c = reinterpret_cast<const TqCopyJob*>(PyBytes_AS_STRING(a[2]));
-  p->q.assign(q, q + jobs); p->d.assign(d, d + jobs); p->c.assign(c, c + jobs);
-  if (!int_list(a[3], &p->row, jobs) || !int_list(a[4], &p->base, jobs)) { PyErr_Clear(); return none(); }
-  p->size_a.resize(jobs); p->size_b.resize(jobs);
-  p->L = v[0]; p->B = v[1]; p->H = v[2]; p->D = v[3]; p->cap = v[4]; p->window = v[5]; p->tok_bytes = v[6];
-  p->dtype = (int)v[7]; p->dev = (int)v[8];
+  p->L = PyList_GET_SIZE(a[0]);
+  p->window = PyLong_AsLongLong(a[1]);
+  p->dev = dev;
+  const size_t jobs = (size_t)(2 * p->L);
+  p->q.assign(jobs, TqQuantizeJob{}); p->d.assign(jobs, TqDequantizeJob{}); p->c.assign(jobs, TqCopyJob{});
+  p->row.resize(jobs); p->base.resize(jobs); p->size_a.resize(jobs); p->size_b.resize(jobs);
+  for (size_t i = 0; i < jobs; ++i) {
+    PyObject* st = PyList_GET_ITEM(a[0], (Py_ssize_t)(i / 2));
+    Ref buf(PyObject_GetAttr(st, (i & 1) ? n_v : n_k)), codec(PyObject_GetAttr(st, n_codec));
+    Ref comp(codec ? PyObject_GetAttr(codec.p, (i & 1) ? n_vc : n_kc) : nullptr);
+    Codec c;
+    if (!buf || !comp) { PyErr_Clear(); return none(); }
+    if (!float_plain(buf.p, dev) || !read_codec(comp.p, dev, &c)) return none();
+    const at::Tensor& t = THPVariable_Unpack(buf.p);
+    if (t.dim() != 4 || t.stride(3) != 1 || t.size(3) != c.dim) return none();
+    if (i == 0) {
+      p->B = t.size(0); p->H = t.size(1); p->D = t.size(3); p->cap = t.size(2);
+      p->dtype = dtype_of(t);
+      p->tok_bytes = p->D * (int64_t)t.element_size();
+    }
+    if (t.size(0) != p->B || t.size(1) != p->H || t.size(3) != p->D || dtype_of(t) != p->dtype || t.stride(2) != p->D) return none();
+    if (t.size(2) < p->cap) p->cap = t.size(2);
+    p->row[i] = row_bytes(p->D, c.bits);
+    p->base[i] = (int64_t)(uintptr_t)t.data_ptr();
+    TqQuantizeJob& q = p->q[i];
+    q.x_dtype = p->dtype; q.D = (int32_t)p->D; q.bits = (int32_t)c.bits; q.normalize = 1;
+    q.B = p->B; q.H = p->H; q.stride_b = t.stride(0); q.stride_h = t.stride(1); q.stride_s = t.stride(2);
+    q.rotation_t = (const float*)c.pi_t; q.codebook = (const float*)c.cb; q.idx_mode = TQ_IDX_PACKED; q.rotation_image = c.img_q;
+    TqDequantizeJob& d = p->d[i];
+    d.idx_mode = TQ_IDX_PACKED; d.D = (int32_t)p->D; d.bits = (int32_t)c.bits; d.out_dtype = p->dtype;
+    d.B = p->B; d.H = p->H; d.ostride_b = t.stride(0); d.ostride_h = t.stride(1); d.ostride_s = t.stride(2);
+    d.rotation = (const float*)c.pi; d.codebook = (const float*)c.cb; d.rotation_image = c.img_d;
+    TqCopyJob& k = p->c[i];
+    k.elem_bytes = (int32_t)t.element_size(); k.D = (int32_t)p->D; k.B = p->B; k.H = p->H;
+    k.dstride_b = t.stride(0); k.dstride_h = t.stride(1); k.dstride_s = t.stride(2);
+  }
   return cap.release();
   END_HANDLE_TH_ERRORS
 }

@@ -77,6 +77,7 @@ class V3Cache(_Base):
         self.initial_capacity = initial_capacity
         self._layers: Dict[int, _Layer] = {}
         self._step_plan = None
+        self._native_plan = None
         self._step_log: List[tuple] = []               # native steps whose packed rows are not in the layers' lists yet
 
     # ------------------------------------------------------------------ layers and buffers
@@ -87,7 +88,7 @@ class V3Cache(_Base):
                                  residual_window=0, layer_idx=layer_idx, n_layers=self.n_layers,
                                  protected_layers=self.protected_layers, seed=42, device=device)
             st = self._layers[layer_idx] = _Layer(codec)
-            self._step_plan = None
+            self._step_plan = self._native_plan = None
         if _DynamicLayer is not None and hasattr(self, "layers"):
             while len(self.layers) <= layer_idx:       # keeps the base class's per-layer bookkeeping in step
                 self.layers.append(_DynamicLayer())
@@ -104,7 +105,7 @@ class V3Cache(_Base):
         new = torch.empty((B, H, new_cap, D), dtype=like.dtype, device=like.device)
         if buf is not None and used:
             new[:, :, :used].copy_(buf[:, :, :used])
-        self._step_plan = None
+        self._step_plan = self._native_plan = None
         return new
 
     def _leaving(self, st: _Layer, need: int) -> int:
@@ -171,12 +172,18 @@ class V3Cache(_Base):
                                  dstride_b=buf.stride(0), dstride_h=buf.stride(1), dstride_s=buf.stride(2))
         base = [(st.k.data_ptr(), st.v.data_ptr()) for st in sts]
         cap = min(min(st.k.shape[2], st.v.shape[2]) for st in sts)
-        # the same for the native form of step(), which keeps its own copy of the job arrays
-        native = N.host().step_plan(bytes(q), bytes(d), bytes(c), row_bytes, [x for pair in base for x in pair],
-                                    (L, B, H, D, cap, self.residual_window, D * eb, N.dtype_code(like), like.device.index))
         return {"L": L, "B": B, "H": H, "D": D, "eb": eb, "dtype": like.dtype, "device": like.device, "q": q, "d": d, "c": c,
-                "row_bytes": row_bytes, "base": base, "cap": cap, "tok_bytes": D * eb, "native": native, "states": sts,
-                "window": self.residual_window}
+                "row_bytes": row_bytes, "base": base, "cap": cap, "tok_bytes": D * eb}
+
+    def _make_native_plan(self, L: int):
+        """(plan, layers, states, window) for the native form of step(), or None while layers are missing."""
+        self._native_plan = None
+        states = [self._layers.get(l) for l in range(L)]
+        if L and all(st is not None and st.k is not None and st.k.is_cuda for st in states):
+            plan = N.host().step_plan(states, self.residual_window)
+            if plan is not None:
+                self._native_plan = (plan, L, states, self.residual_window)
+        return self._native_plan
 
     def step(self, key_states: Sequence[torch.Tensor], value_states: Sequence[torch.Tensor], return_views: bool = True):
         """One step for layers 0..L-1 at once: append key_states[l] / value_states[l] ((B, H, S_new, D) each) to
@@ -184,9 +191,11 @@ class V3Cache(_Base):
 
         Returns [(keys, values)] per layer as update() would (views of the persistent buffers), or None with
         return_views=False.  Falls back to per-layer update() calls while layers are being created or grown."""
-        p = self._step_plan
-        if p is not None and p["native"] is not None and p["L"] == len(key_states) and p["window"] == self.residual_window:
-            done = N.host().step(p["native"], p["states"], key_states, value_states, return_views, self._step_log)
+        p = self._native_plan
+        if p is None or p[1] != len(key_states) or p[3] != self.residual_window:
+            p = self._make_native_plan(len(key_states))
+        if p is not None:
+            done = N.host().step(p[0], p[2], key_states, value_states, return_views, self._step_log)
             if done is not None:
                 return done if return_views else None
         return self._step_general(key_states, value_states, return_views)
