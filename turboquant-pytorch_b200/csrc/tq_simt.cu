@@ -13,6 +13,7 @@
 
 #include "tq_common.cuh"
 #include "tq_internal.h"
+#include "tq_pdl.cuh"
 
 namespace tq {
 
@@ -595,6 +596,7 @@ __device__ __forceinline__ void project_rows(const void* x, int64_t n, int K, co
 
 template <int XDT, int RPB>
 __global__ void k_project_rows(const void* x, int64_t n, int K, const float* __restrict__ m, int N, float* out) {
+  pdl_trigger();
   project_rows<XDT, RPB>(x, n, K, m, N, out);
 }
 // the same rows by two matrices: blockIdx.y picks one
@@ -773,9 +775,9 @@ __global__ void __launch_bounds__(NT) k_score_packed_d128(TqScoreJob job, const 
 }
 
 // probs = exp(l - M) / Z with (M, Z) folded from the per-block partials.
-__global__ void __launch_bounds__(NT) k_softmax_finish(const float* __restrict__ logits, const float* __restrict__ stats,
-                                                      int nblk, int64_t Sk, float* probs) {
+__global__ void __launch_bounds__(NT) k_softmax_finish(const float* logits, const float* stats, int nblk, int64_t Sk, float* probs) {
   __shared__ float sh_m, sh_z;
+  pdl_wait();
   const int64_t row = blockIdx.x;
   if (threadIdx.x < 32) {
     float m = -INFINITY;
@@ -1326,7 +1328,8 @@ int simt_score_packed(const TqScoreJob& job, cudaStream_t st) {
   if (rc != TQ_OK || job.probs == nullptr) return rc;
   int chunks = (int)((job.Sk + 4095) / 4096);
   dim3 grid((unsigned)rows, (unsigned)chunks);
-  k_softmax_finish<<<grid, NT, 0, st>>>(job.logits, stats, nblk, job.Sk, job.probs);
+  if (use_mma) launch_after(k_softmax_finish, grid, dim3(NT), 0, st, job.logits, stats, nblk, job.Sk, job.probs);
+  else k_softmax_finish<<<grid, NT, 0, st>>>(job.logits, stats, nblk, job.Sk, job.probs);
   return check_launch();
 }
 
