@@ -15,6 +15,7 @@
 
 #include "tq_common.cuh"
 #include "tq_internal.h"
+#include "tq_pdl.cuh"
 
 namespace tq {
 
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 2 : 1) k_qjl_score_packed(
       sgn[threadIdx.x] = first | (second << 16);
     }
   }
+  pdl_wait();                                    // the projected queries come from the launch before
   // query operand: one 16-byte word group per (tile, k-step, lane)
   for (int e = threadIdx.x; e < kNT * 2 * KS * 32; e += kThreads) {
     const int ln = e & 31, ks = (e >> 5) % (2 * KS), nt = e / (64 * KS);
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(kThreads, NT <= 2 ? 2 : 1) k_qjl_score_packed(
     if (q < P.Sq) {
       const bool second = ks >= KS;
       const float* src = (second ? P.qproj : P.qrot) + (bh * P.Sq + q) * D + DQ * tt + 4 * (second ? ks - KS : ks);
-      const float4 f = __ldg(reinterpret_cast<const float4*>(src));
+      const float4 f = *reinterpret_cast<const float4*>(src);
       const float s = second ? P.coef : 1.0f;
       v[0] = f.x * s; v[1] = f.y * s; v[2] = f.z * s; v[3] = f.w * s;
     }
@@ -271,7 +273,7 @@ int launch_packed(const PackedScoreParams& P, int bits, unsigned grid, size_t sm
   auto go = [&](auto kern) -> int {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
-    kern<<<grid, kThreads, smem, st>>>(P);
+    launch_after(kern, dim3(grid), dim3(kThreads), smem, st, P);
     return check_launch();
   };
   switch (bits) {

@@ -30,6 +30,7 @@
 
 #include "tq_common.cuh"
 #include "tq_internal.h"
+#include "tq_pdl.cuh"
 
 namespace tq {
 
@@ -91,6 +92,7 @@ __device__ __forceinline__ uint32_t idesc_f16_n(uint32_t n) {
 
 template <int D>
 __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_constant__ QjlBatch batch) {
+  pdl_wait();                                    // before the TMEM allocation: see tq_v2_umma.cu
   using C = QCfg<D>;
   constexpr int kHalfChunks = C::kHalfChunks, kChunks = C::kChunks;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -390,7 +392,7 @@ int launch(const TqQjlScoreJob& job, uint8_t* images, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k_umma_qjl_scores<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)QCfg<D>::kSmemBytes);
   if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
-  k_umma_qjl_scores<D><<<grid, kThreadsQ, QCfg<D>::kSmemBytes, st>>>(batch);
+  launch_after(k_umma_qjl_scores<D>, dim3(grid), dim3(kThreadsQ), QCfg<D>::kSmemBytes, st, batch);
   return check_launch();
 }
 

@@ -602,6 +602,7 @@ __global__ void k_project_rows(const void* x, int64_t n, int K, const float* __r
 // the same rows by two matrices: blockIdx.y picks one
 template <int XDT>
 __global__ void k_project_rows_two(const void* x, int64_t n, int D, const float* m0, const float* m1, float* out0, float* out1) {
+  pdl_trigger();
   project_rows<XDT, 1>(x, n, D, blockIdx.y ? m1 : m0, D, blockIdx.y ? out1 : out0);
 }
 
@@ -1022,6 +1023,7 @@ template <int QDT>
 __global__ void __launch_bounds__(NT) k_qjl_query_operand(const void* q, int D, int64_t Sq, int n_qblocks,
                                                          const float* __restrict__ qjl_t, float corr, uint8_t* __restrict__ images) {
   constexpr int RI = 2, ROWS = 16 * RI;
+  pdl_trigger();
   extern __shared__ __align__(16) float smem[];
   const int lda = lda_for(D);
   float* As = smem;

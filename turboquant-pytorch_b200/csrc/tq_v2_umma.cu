@@ -27,6 +27,7 @@
 
 #include "tq_common.cuh"
 #include "tq_internal.h"
+#include "tq_pdl.cuh"
 
 namespace tq {
 
@@ -103,6 +104,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 template <int D>
 __global__ void k_v2_operand_image(const float* __restrict__ rotation, const float* __restrict__ qjl_t, int64_t M,
                                   uint8_t* __restrict__ images) {
+  pdl_trigger();
   constexpr int KC = VCfg<D>::KC, NBLK = VCfg<D>::NBLK;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= D * D) return;
@@ -176,6 +178,10 @@ __device__ __forceinline__ void tmem_ld_quads(uint32_t taddr, uint32_t (&r)[32])
 
 template <int D, int STAGE>
 __global__ void __launch_bounds__(VCfg<D>::kThreads + (STAGE == 2 ? kExpandThreads : 0), 1) k_umma_v2_stage(const __grid_constant__ V2Stage p) {
+  // The wait comes before the TMEM allocation: a dependent that held TMEM while its predecessor still had to allocate some
+  // on the same SM would wait for good.
+  pdl_trigger();
+  pdl_wait();
   using C = VCfg<D>;
   constexpr int KC = C::KC, NBLK = C::NBLK;
   constexpr int PA = STAGE == 1 ? 1 : 2;       // pieces of A
@@ -681,7 +687,7 @@ int launch_stage(const V2Stage& p, int grid, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k_umma_v2_stage<D, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)VCfg<D>::kSmemBytes);
   if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
-  k_umma_v2_stage<D, STAGE><<<grid, VCfg<D>::threads(STAGE), VCfg<D>::kSmemBytes, st>>>(p);
+  launch_after(k_umma_v2_stage<D, STAGE>, dim3(grid), dim3(VCfg<D>::threads(STAGE)), VCfg<D>::kSmemBytes, st, p);
   return check_launch();
 }
 
