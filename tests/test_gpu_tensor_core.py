@@ -256,3 +256,24 @@ def test_head_dim_64_keeps_infinite_and_nan_norms():
             assert torch.equal(c["idx_bytes"][0, h, s], ref["idx_bytes"][0, h, s])
             a, b = c["vec_norms"][0, h, s], ref["vec_norms"][0, h, s]
             assert bool(a.isnan()) == bool(b.isnan()) and (bool(a.isnan()) or bool(a == b))
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+def test_one_long_slab(dim):
+    """(1, 1, S, D): the strides of the size-1 dimensions in the tensor map stay below 2^40 bytes."""
+    comp = tq.MSECompressor(dim, 2, seed=1, device=DEV)
+    x = torch.randn(1, 1, 150001, dim, device=DEV).half()
+    c = comp.compress(x)
+    tail = comp.compress(x[:, :, 150001 - 300:])
+    assert torch.equal(c["idx_bytes"][:, :, -300:], tail["idx_bytes"]) and torch.equal(c["vec_norms"][:, :, -300:], tail["vec_norms"])
+    out = torch.empty_like(x)
+    job, _keep = comp.decompress_job(c, out)
+    _ops.run_dequantize([job], DEV)
+    assert torch.equal(out[:, :, -300:], _rebuild(comp, tail, x.dtype))
+
+
+def _rebuild(comp, packed, dtype):
+    out = torch.empty(packed["shape"], dtype=dtype, device=DEV)
+    job, _keep = comp.decompress_job(packed, out)
+    _ops.run_dequantize([job], DEV)
+    return out

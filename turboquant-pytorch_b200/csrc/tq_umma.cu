@@ -1521,10 +1521,10 @@ int umma_quantize(const TqQuantizeJob* jobs, int n_jobs, cudaStream_t st) {
       const int64_t tps = (j.S + tile_vecs_of(D) - 1) / tile_vecs_of(D);
       job_tiles[i] = tps * j.B * j.H;
       job_weight[i] = quantize_tile_weight(j.bits, j.x_dtype == TQ_BF16);
-      // size-1 dimensions get a harmless stride; TMA wants multiples of 16 bytes
+      // size-1 dimensions get a harmless stride; TMA wants multiples of 16 bytes below 2^40
       const int64_t ss = j.S > 1 ? j.stride_s : D;
       const int64_t sh = j.H > 1 ? j.stride_h : ss * j.S;
-      const int64_t sb = j.B > 1 ? j.stride_b : (sh > ss ? sh : ss) * (j.H > 1 ? j.H : j.S);
+      const int64_t sb = j.B > 1 ? j.stride_b : (sh > ss ? sh : ss) * j.H;
       cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)j.S, (cuuint64_t)j.H, (cuuint64_t)j.B};
       cuuint64_t strides[3] = {(cuuint64_t)ss * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
       cuuint32_t box[4] = {64, (cuuint32_t)kTileRows, 1, 1};
@@ -1642,7 +1642,7 @@ int umma_dequantize(const TqDequantizeJob* jobs, int n_jobs, cudaStream_t st) {
       if (j.out_dtype != TQ_F32 && D == 128) {
         const int64_t ss = j.S > 1 ? j.ostride_s : D;
         const int64_t sh = j.H > 1 ? j.ostride_h : ss * j.S;
-        const int64_t sb = j.B > 1 ? j.ostride_b : (sh > ss ? sh : ss) * (j.H > 1 ? j.H : j.S);
+        const int64_t sb = j.B > 1 ? j.ostride_b : (sh > ss ? sh : ss) * j.H;
         cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)j.S, (cuuint64_t)j.H, (cuuint64_t)j.B};
         cuuint64_t strides[3] = {(cuuint64_t)ss * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
         cuuint32_t box[4] = {64, (cuuint32_t)kTileRows, 1, 1};
