@@ -230,7 +230,7 @@ __device__ __forceinline__ void score_block(const uint32_t (&w0)[Packed<BITS>::C
 template <int BITS, int ROWS>
 __global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const float* qrot, float* stats, int nblk,
                                                         int keys_per_block) {
-  pdl_trigger();
+  if (stats != nullptr) pdl_trigger();           // the softmax pass follows
   constexpr int G = Packed<BITS>::G;
   constexpr int CW = Packed<BITS>::CW;
   __shared__ __align__(1024) uint32_t lut[256];
@@ -887,7 +887,7 @@ int decode_attention(const TqDecodeAttnJob& job, cudaStream_t st) {
   float* part = reinterpret_cast<float*>(reinterpret_cast<char*>(job.workspace) + qbytes);
   int rc = TQ_OK;
   if (job.Sk > 0) {
-    rc = simt_project(job.q, job.q_dtype, rows, kDimA, job.k_rotation_t, kDimA, qrot, st);
+    rc = simt_project(job.q, job.q_dtype, rows, kDimA, job.k_rotation_t, kDimA, qrot, st, true);
     if (rc != TQ_OK) return rc;
     DecodeParams P;
     P.qrot = qrot;

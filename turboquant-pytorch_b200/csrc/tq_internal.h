@@ -19,7 +19,9 @@ int simt_quantize_rotated(const float* y, int64_t n, int D, int bits, const floa
                           cudaStream_t st);
 int simt_quantize(const TqQuantizeJob& job, cudaStream_t st);
 int simt_dequantize(const TqDequantizeJob& job, cudaStream_t st);
-int simt_project(const void* x, int x_dtype, int64_t n, int K, const float* m, int N, float* out, cudaStream_t st);
+// `followed`: the caller launches the next kernel with launch_after()
+int simt_project(const void* x, int x_dtype, int64_t n, int K, const float* m, int N, float* out, cudaStream_t st,
+                 bool followed = false);
 size_t simt_score_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int D);
 int simt_score_packed(const TqScoreJob& job, cudaStream_t st);
 int simt_qjl_compress(const TqQjlCompressJob& job, cudaStream_t st);

@@ -2,7 +2,8 @@
 // while its predecessor still runs and waits (pdl_wait) before it touches what the predecessor wrote; what an earlier
 // kernel of the stream wrote is there already, because the first kernel of the chain is an ordinary launch.  The
 // predecessor lets it start with pdl_trigger at its own beginning: by then all its CTAs are running, so the dependent
-// takes no place from it.  Packed scores of 131072 keys x 8 heads with softmax 64 -> 59.5 us, decode attention of 32640 tokens
+// takes no place from it.  Only a kernel that a launch_after() of the same call follows may trigger: the last kernel of a call
+// would let another library's dependent kernel start beside it.  Packed scores of 131072 keys x 8 heads with softmax 64 -> 59.5 us, decode attention of 32640 tokens
 // 41 -> 35 us, three launches each; MSE + QJL: compress and
 // scores of 8 x 4096 packed keys 64 -> 58 us, scores of 16 x 16384 keys 84 -> 81 us.
 #pragma once

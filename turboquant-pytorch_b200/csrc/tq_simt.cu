@@ -594,9 +594,10 @@ __device__ __forceinline__ void project_rows(const void* x, int64_t n, int K, co
   }
 }
 
+// `followed`: a kernel launched with launch_after() comes next in the call (see tq_pdl.cuh)
 template <int XDT, int RPB>
-__global__ void k_project_rows(const void* x, int64_t n, int K, const float* __restrict__ m, int N, float* out) {
-  pdl_trigger();
+__global__ void k_project_rows(const void* x, int64_t n, int K, const float* __restrict__ m, int N, float* out, bool followed) {
+  if (followed) pdl_trigger();
   project_rows<XDT, RPB>(x, n, K, m, N, out);
 }
 // the same rows by two matrices: blockIdx.y picks one
@@ -1250,14 +1251,14 @@ int simt_dequantize(const TqDequantizeJob& job, cudaStream_t st) {
   return rc != TQ_OK ? rc : check_launch();
 }
 
-int simt_project(const void* x, int x_dtype, int64_t n, int K, const float* m, int N, float* out, cudaStream_t st) {
+int simt_project(const void* x, int x_dtype, int64_t n, int K, const float* m, int N, float* out, cudaStream_t st, bool followed) {
   if (n == 0) return TQ_OK;
   if (n <= 8192) {         // few rows: a 64-row tile kernel would run on a handful of SMs
     const int threads = N <= 128 ? 128 : 256;
     if (n <= 512) {
-      TQ_DISPATCH_DT(x_dtype, (k_project_rows<DT_, 1><<<(unsigned)n, threads, 0, st>>>(x, n, K, m, N, out)));
+      TQ_DISPATCH_DT(x_dtype, (k_project_rows<DT_, 1><<<(unsigned)n, threads, 0, st>>>(x, n, K, m, N, out, followed)));
     } else {
-      TQ_DISPATCH_DT(x_dtype, (k_project_rows<DT_, 4><<<(unsigned)((n + 3) / 4), threads, 0, st>>>(x, n, K, m, N, out)));
+      TQ_DISPATCH_DT(x_dtype, (k_project_rows<DT_, 4><<<(unsigned)((n + 3) / 4), threads, 0, st>>>(x, n, K, m, N, out, followed)));
     }
     return check_launch();
   }
@@ -1273,7 +1274,8 @@ int simt_project(const void* x, int x_dtype, int64_t n, int K, const float* m, i
   return rc != TQ_OK ? rc : check_launch();
 }
 
-// Two projections of the same rows (head_dim square matrices) in one launch, or in two where the rows are many.
+// Two projections of the same rows (head_dim square matrices) in one launch, or in two where the rows are many; a kernel
+// launched with launch_after() follows.
 int simt_project_two(const void* x, int x_dtype, int64_t n, int D, const float* m0, const float* m1, float* out0, float* out1,
                      cudaStream_t st) {
   if (n == 0) return TQ_OK;
@@ -1283,7 +1285,7 @@ int simt_project_two(const void* x, int x_dtype, int64_t n, int D, const float* 
     return check_launch();
   }
   const int rc = simt_project(x, x_dtype, n, D, m0, D, out0, st);
-  return rc != TQ_OK ? rc : simt_project(x, x_dtype, n, D, m1, D, out1, st);
+  return rc != TQ_OK ? rc : simt_project(x, x_dtype, n, D, m1, D, out1, st, true);
 }
 
 size_t simt_score_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int D) {
@@ -1305,7 +1307,7 @@ int simt_score_packed(const TqScoreJob& job, cudaStream_t st) {
   float* qrot = reinterpret_cast<float*>(job.workspace);
   size_t qbytes = ((size_t)rows * job.D * sizeof(float) + 255) / 256 * 256;
   float* stats = reinterpret_cast<float*>(reinterpret_cast<char*>(job.workspace) + qbytes);
-  int rc = simt_project(job.q, job.q_dtype, rows, job.D, job.rotation_t, job.D, qrot, st);
+  int rc = simt_project(job.q, job.q_dtype, rows, job.D, job.rotation_t, job.D, qrot, st, use_mma);
   if (rc != TQ_OK) return rc;
   const int64_t blocks = job.B * job.Hkv * nblk;
   float* st_ptr = job.probs != nullptr ? stats : nullptr;

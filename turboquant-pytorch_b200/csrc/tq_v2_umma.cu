@@ -179,8 +179,9 @@ __device__ __forceinline__ void tmem_ld_quads(uint32_t taddr, uint32_t (&r)[32])
 template <int D, int STAGE>
 __global__ void __launch_bounds__(VCfg<D>::kThreads + (STAGE == 2 ? kExpandThreads : 0), 1) k_umma_v2_stage(const __grid_constant__ V2Stage p) {
   // The wait comes before the TMEM allocation: a dependent that held TMEM while its predecessor still had to allocate some
-  // on the same SM would wait for good.
-  pdl_trigger();
+  // on the same SM would wait for good.  For the same reason the last stage does not let a dependent start: what follows it
+  // is not this library's, and may allocate TMEM before it waits.
+  if constexpr (STAGE != 3) pdl_trigger();
   pdl_wait();
   using C = VCfg<D>;
   constexpr int KC = C::KC, NBLK = C::NBLK;
