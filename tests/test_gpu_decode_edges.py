@@ -61,6 +61,21 @@ def test_decode_attention_blocks_and_windows(window, packed, bits, dtype, monkey
         codec.decode_attention(q, ck, cv)
 
 
+def test_a_refused_window_does_not_fail_the_next_call():
+    """A window whose logits do not fit shared memory is refused before the launch; that error is this call's alone."""
+    codec = tq.TurboQuantV3(128, key_bits=4, value_bits=2, residual_window=60000, layer_idx=9, n_layers=32, device=DEV)
+    mse = codec.key_compressor
+    small = O.synthetic_kv((1, 1, 300, 128), torch.float16, seed=1).to(DEV)
+    want = mse.compress(small)["idx_bytes"]
+    x = torch.zeros(1, 1, 60016, 128, dtype=torch.float16, device=DEV)
+    ck, cv = codec.compress_kv(x, x)
+    q = torch.ones(1, 1, 1, 128, dtype=torch.float16, device=DEV)
+    with pytest.raises(RuntimeError):
+        codec.decode_attention(q, ck, cv)
+    assert torch.equal(mse.compress(small)["idx_bytes"], want)
+    assert float((q + 1).sum()) == 256                                     # nor torch's own next launch
+
+
 def test_back_to_back_calls_and_capture():
     """Scores and attention launch their kernels as a programmatic chain: calls in a row on one stream share scratch from the
     caching allocator, and a captured call replays the same."""

@@ -885,6 +885,32 @@ int decode_attention(const TqDecodeAttnJob& job, cudaStream_t st) {
   float* qrot = reinterpret_cast<float*>(job.workspace);
   const size_t qbytes = ((size_t)rows * kDimA * sizeof(float) + 255) / 256 * 256;
   float* part = reinterpret_cast<float*>(reinterpret_cast<char*>(job.workspace) + qbytes);
+  FinishParams F;
+  F.q = job.q; F.q_dtype = job.q_dtype;
+  F.part = part; F.nblk = nblk;
+  F.v_rotation = job.v_rotation;
+  F.k_window = job.k_window; F.v_window = job.v_window; F.window_dtype = job.window_dtype;
+  F.W = job.k_window != nullptr ? job.W : 0;
+  F.ws_b = job.wstride_b; F.ws_h = job.wstride_h; F.ws_s = job.wstride_s;
+  F.B = job.B; F.Hq = job.Hq; F.Sq = job.Sq; F.Hkv = job.Hkv; F.Sk = job.Sk;
+  F.scale = job.scale;
+  F.out = job.out;
+  const size_t smem = (size_t)(F.W > 0 ? F.W : 1) * sizeof(float);
+  const int wdt = F.W > 0 ? job.window_dtype : TQ_F16;
+  // 16-byte loads where every row of the windows and of Pi_v starts on such a boundary
+  const int64_t per16 = wdt == TQ_F32 ? 4 : 8;
+  const bool vec = (((uintptr_t)F.k_window | (uintptr_t)F.v_window | (uintptr_t)F.v_rotation) & 15u) == 0 &&
+                   (F.ws_b % per16 == 0 && F.ws_h % per16 == 0 && F.ws_s % per16 == 0);
+  void (*finish)(FinishParams) = nullptr;
+#define TQ_FIN(QD, WD) finish = vec ? k_decode_finish<QD, WD, true> : k_decode_finish<QD, WD, false>
+  if (job.q_dtype == TQ_F32) { if (wdt == TQ_F16) TQ_FIN(TQ_F32, TQ_F16); else if (wdt == TQ_BF16) TQ_FIN(TQ_F32, TQ_BF16); else TQ_FIN(TQ_F32, TQ_F32); }
+  else if (job.q_dtype == TQ_F16) { if (wdt == TQ_F16) TQ_FIN(TQ_F16, TQ_F16); else if (wdt == TQ_BF16) TQ_FIN(TQ_F16, TQ_BF16); else TQ_FIN(TQ_F16, TQ_F32); }
+  else { if (wdt == TQ_F16) TQ_FIN(TQ_BF16, TQ_F16); else if (wdt == TQ_BF16) TQ_FIN(TQ_BF16, TQ_BF16); else TQ_FIN(TQ_BF16, TQ_F32); }
+#undef TQ_FIN
+  if (smem > 36 * 1024) {                          // with its 10 KB of static shared memory past the default limit
+    const cudaError_t e = cudaFuncSetAttribute(finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return refused(e);       // before the first launch: the attention kernel counts on this one
+  }
   int rc = TQ_OK;
   if (job.Sk > 0) {
     rc = simt_project(job.q, job.q_dtype, rows, kDimA, job.k_rotation_t, kDimA, qrot, st, true);
@@ -910,38 +936,8 @@ int decode_attention(const TqDecodeAttnJob& job, cudaStream_t st) {
     }
     if (rc != TQ_OK) return rc;
   }
-  FinishParams F;
-  F.q = job.q; F.q_dtype = job.q_dtype;
-  F.part = part; F.nblk = nblk;
-  F.v_rotation = job.v_rotation;
-  F.k_window = job.k_window; F.v_window = job.v_window; F.window_dtype = job.window_dtype;
-  F.W = job.k_window != nullptr ? job.W : 0;
-  F.ws_b = job.wstride_b; F.ws_h = job.wstride_h; F.ws_s = job.wstride_s;
-  F.B = job.B; F.Hq = job.Hq; F.Sq = job.Sq; F.Hkv = job.Hkv; F.Sk = job.Sk;
-  F.scale = job.scale;
-  F.out = job.out;
-  const size_t smem = (size_t)(F.W > 0 ? F.W : 1) * sizeof(float);
-  const int wdt = F.W > 0 ? job.window_dtype : TQ_F16;
-  // 16-byte loads where every row of the windows and of Pi_v starts on such a boundary
-  const int64_t per16 = wdt == TQ_F32 ? 4 : 8;
-  const bool vec = (((uintptr_t)F.k_window | (uintptr_t)F.v_window | (uintptr_t)F.v_rotation) & 15u) == 0 &&
-                   (F.ws_b % per16 == 0 && F.ws_h % per16 == 0 && F.ws_s % per16 == 0);
-  cudaError_t attr = cudaSuccess;
-  auto launch = [&](auto vec_kernel, auto any_kernel) {
-    auto kern = vec ? vec_kernel : any_kernel;
-    if (smem > 36 * 1024) {                        // with its 10 KB of static shared memory past the default limit
-      attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (attr != cudaSuccess) return;
-    }
-    if (job.Sk > 0) launch_after(kern, dim3((unsigned)rows), dim3(kFinThreads), smem, st, F);
-    else kern<<<(unsigned)rows, kFinThreads, smem, st>>>(F);
-  };
-#define TQ_FIN(QD, WD) launch(k_decode_finish<QD, WD, true>, k_decode_finish<QD, WD, false>)
-  if (job.q_dtype == TQ_F32) { if (wdt == TQ_F16) TQ_FIN(TQ_F32, TQ_F16); else if (wdt == TQ_BF16) TQ_FIN(TQ_F32, TQ_BF16); else TQ_FIN(TQ_F32, TQ_F32); }
-  else if (job.q_dtype == TQ_F16) { if (wdt == TQ_F16) TQ_FIN(TQ_F16, TQ_F16); else if (wdt == TQ_BF16) TQ_FIN(TQ_F16, TQ_BF16); else TQ_FIN(TQ_F16, TQ_F32); }
-  else { if (wdt == TQ_F16) TQ_FIN(TQ_BF16, TQ_F16); else if (wdt == TQ_BF16) TQ_FIN(TQ_BF16, TQ_BF16); else TQ_FIN(TQ_BF16, TQ_F32); }
-#undef TQ_FIN
-  if (attr != cudaSuccess) { note_cuda_error((int)attr); return TQ_ELAUNCH; }
+  if (job.Sk > 0) launch_after(finish, dim3((unsigned)rows), dim3(kFinThreads), smem, st, F);
+  else finish<<<(unsigned)rows, kFinThreads, smem, st>>>(F);
   return check_launch();
 }
 

@@ -10,6 +10,7 @@ namespace tq {
 
 int last_cuda_error();
 void note_cuda_error(int e);
+int refused(cudaError_t e);   // a runtime call before a launch failed: notes the error and clears it; TQ_ELAUNCH
 long long launch_count();
 int check_launch();   // cudaGetLastError -> TQ_OK / TQ_ELAUNCH, counts successful launches
 bool force_simt();    // TQ_FORCE_SIMT=1 in the environment: route everything to the FP32 kernels (second opinion in tests)

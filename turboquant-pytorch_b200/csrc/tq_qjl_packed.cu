@@ -272,7 +272,7 @@ template <int D, int NT>
 int launch_packed(const PackedScoreParams& P, int bits, unsigned grid, size_t smem, cudaStream_t st) {
   auto go = [&](auto kern) -> int {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
+    if (e != cudaSuccess) return refused(e);
     launch_after(kern, dim3(grid), dim3(kThreads), smem, st, P);
     return check_launch();
   };

@@ -391,7 +391,7 @@ int launch(const TqQjlScoreJob& job, uint8_t* images, cudaStream_t st) {
   const int grid = (int)(total < sms ? total : sms);
   cudaError_t e = cudaFuncSetAttribute(k_umma_qjl_scores<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)QCfg<D>::kSmemBytes);
-  if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
+  if (e != cudaSuccess) return refused(e);
   launch_after(k_umma_qjl_scores<D>, dim3(grid), dim3(kThreadsQ), QCfg<D>::kSmemBytes, st, batch);
   return check_launch();
 }

@@ -31,13 +31,13 @@ void* g_scratch_ptr[kMaxDevices] = {};   // device address of g_score_scratch, p
 int scratch_for_current_device(void** out) {
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) { tq::note_cuda_error((int)e); return TQ_ELAUNCH; }
+  if (e != cudaSuccess) return tq::refused(e);
   if (dev < 0 || dev >= kMaxDevices) return TQ_EDEVICE;    // device ordinals beyond the table below
   std::lock_guard<std::mutex> lock(g_mu);
   if (g_scratch_ptr[dev] == nullptr) {
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_score_scratch);
-    if (e != cudaSuccess || p == nullptr) { tq::note_cuda_error((int)e); return TQ_ELAUNCH; }
+    if (e != cudaSuccess || p == nullptr) return tq::refused(e);
     g_scratch_ptr[dev] = p;
   }
   *out = g_scratch_ptr[dev];

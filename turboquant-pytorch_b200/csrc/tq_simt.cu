@@ -1157,6 +1157,11 @@ static std::atomic<long long> g_launches{0};
 int last_cuda_error() { return g_last_cuda_error; }
 long long launch_count() { return g_launches.load(); }
 void note_cuda_error(int e) { g_last_cuda_error = e; }
+int refused(cudaError_t e) {
+  g_last_cuda_error = (int)e;
+  cudaGetLastError();                            // it is this call's error: the next launch must not find it
+  return TQ_ELAUNCH;
+}
 
 int check_launch() {
   cudaError_t e = cudaGetLastError();
@@ -1181,7 +1186,7 @@ template <typename K>
 static int set_smem(K kernel, size_t bytes) {
   if (bytes > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) { g_last_cuda_error = (int)e; return TQ_ELAUNCH; }
+    if (e != cudaSuccess) return refused(e);
   }
   return TQ_OK;
 }

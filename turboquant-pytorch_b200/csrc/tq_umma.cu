@@ -1467,7 +1467,7 @@ template <typename P, typename Batch, typename K>
 static int launch_prefix(K kern, const Batch& batch, int grid, int threads, uint32_t smem, bool set_attr, cudaStream_t st) {
   if (set_attr) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
+    if (e != cudaSuccess) return refused(e);
   }
   static_assert(sizeof(P) <= sizeof(Batch) && offsetof(P, jobs) == offsetof(Batch, jobs), "a prefix");
   kern<<<grid, threads, smem, st>>>(reinterpret_cast<const P&>(batch));

@@ -687,7 +687,7 @@ template <int D, int STAGE>
 int launch_stage(const V2Stage& p, int grid, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k_umma_v2_stage<D, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)VCfg<D>::kSmemBytes);
-  if (e != cudaSuccess) { note_cuda_error((int)e); return TQ_ELAUNCH; }
+  if (e != cudaSuccess) return refused(e);
   launch_after(k_umma_v2_stage<D, STAGE>, dim3(grid), dim3(VCfg<D>::threads(STAGE)), VCfg<D>::kSmemBytes, st, p);
   return check_launch();
 }
