@@ -1,5 +1,7 @@
 """Which calls the native host path stands in for, checked on the CPU with a stand-in for the extension."""
 
+import os
+import sys
 import types
 
 import pytest
@@ -85,3 +87,42 @@ def test_a_layer_with_such_a_codec_asks_it(host, side):
     assert sorted(r["compressed"] for r in results) == ["mine", "replaced on the object"]
     codec.decompress_kv(SIDE, SIDE)
     assert host == []
+
+
+@pytest.fixture
+def unloaded(monkeypatch):
+    monkeypatch.setattr(N, "_host", None)              # what host() leaves there goes with the test
+
+
+@pytest.mark.parametrize("reason", ["does not load", "of another torch"])
+def test_calls_take_the_general_path_without_the_extension(unloaded, monkeypatch, tmp_path, reason):
+    if reason == "does not load":
+        monkeypatch.setitem(sys.modules, "turboquant._tq_host", None)
+        monkeypatch.delattr(tq, "_tq_host", raising=False)
+    else:
+        (tmp_path / "_tq_host.built_for").write_text("torch 1.0 other\n")
+        monkeypatch.setattr(N, "_HERE", str(tmp_path))
+    with pytest.warns(RuntimeWarning, match="is not used"):
+        host = N.host()
+    assert host.compress(None, None) is None and host.step_plan([], 0) is None
+    assert N.host() is host                                                  # said once
+
+
+def test_the_extension_that_is_here_loads(unloaded):
+    assert not isinstance(N.host(), N._GeneralPath)
+
+
+def test_a_build_for_another_torch_is_stale(monkeypatch, tmp_path):
+    sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(tq.__file__))))
+    import build
+    out, stamp = tmp_path / "_tq_host.so", tmp_path / "_tq_host.built_for"
+    built = []
+    monkeypatch.setattr(build, "HOST_OUT", str(out))
+    monkeypatch.setattr(build, "HOST_STAMP", str(stamp))
+    monkeypatch.setattr(build.subprocess, "check_call", lambda cmd: (built.append(cmd), out.write_bytes(b"")))
+    build.build_host()
+    build.build_host()
+    assert len(built) == 1 and stamp.read_text() == build.host_built_for()
+    stamp.write_text("torch 1.0 other\n")
+    build.build_host()
+    assert len(built) == 2 and stamp.read_text() == build.host_built_for()

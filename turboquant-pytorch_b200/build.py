@@ -23,6 +23,7 @@ SOURCES = ["tq_api.cu", "tq_simt.cu", "tq_few.cu", "tq_umma.cu", "tq_qjl_umma.cu
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 HOST_SRC = os.path.join(CSRC, "tq_host.cpp")
 HOST_OUT = os.path.join(HERE, "turboquant", "_tq_host.so")
+HOST_STAMP = os.path.join(HERE, "turboquant", "_tq_host.built_for")
 
 
 def nvcc_path() -> str:
@@ -44,11 +45,22 @@ def stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def host_built_for() -> str:
+    """What the host extension has to be built for again: it is linked against torch and includes its headers."""
+    import sysconfig
+
+    import torch
+    return f"torch {torch.__version__} {sysconfig.get_config_var('SOABI')}\n"
+
+
 def build_host(force: bool = False) -> str:
-    """Compile the Python extension that fills in and submits the jobs (no kernels in it)."""
+    """Compile the Python extension that fills in and submits the jobs (no kernels in it).  What it was built for is
+    written beside it: a module of another torch is rebuilt here and not loaded by the package."""
     deps = [HOST_SRC, os.path.join(HERE, "..", "include", "turboquant_b200.h")]
+    want = host_built_for()
     if not force and os.path.exists(HOST_OUT) and all(os.path.getmtime(d) <= os.path.getmtime(HOST_OUT) for d in deps):
-        return HOST_OUT
+        if os.path.exists(HOST_STAMP) and open(HOST_STAMP).read() == want:
+            return HOST_OUT
     import sysconfig
 
     import torch
@@ -60,7 +72,11 @@ def build_host(force: bool = False) -> str:
            "-I" + cuda, "-o", HOST_OUT, HOST_SRC, "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
            "-ltorch_python"]
     print(" ".join(cmd), flush=True)
+    if os.path.exists(HOST_STAMP):
+        os.remove(HOST_STAMP)
     subprocess.check_call(cmd)
+    with open(HOST_STAMP, "w") as f:
+        f.write(want)
     return HOST_OUT
 
 

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sysconfig
 
 import torch
 
@@ -159,19 +160,46 @@ def lib():
 _host = None
 
 
+class _GeneralPath:
+    """Stands in for the host extension where that cannot be loaded: every function declines, so that each call takes the
+    general Python path to the same kernels."""
+
+    def __getattr__(self, _name):
+        return lambda *args: None
+
+
+def _load_host():
+    """The extension, or the reason why it is not used."""
+    stamp = os.path.join(_HERE, "_tq_host.built_for")                  # written by build.py
+    if os.path.exists(stamp):
+        with open(stamp) as f:
+            built_for = f.read().strip()
+        here = f"torch {torch.__version__} {sysconfig.get_config_var('SOABI')}"
+        if built_for != here:
+            return None, f"it was built for {built_for}, this is {here}"
+    try:
+        from . import _tq_host
+        return _tq_host, None
+    except ImportError as e:
+        return None, str(e)
+
+
 def host():
-    """The extension that does the per-call host work for plain CUDA tensors (csrc/tq_host.cpp), bound to lib()."""
+    """The extension that does the per-call host work for plain CUDA tensors (csrc/tq_host.cpp), bound to lib().  Without
+    it calls take several times the host time and give the same results, so that is a warning and no error."""
     global _host
     if _host is None:
         L = lib()
-        try:
-            from . import _tq_host as H
-        except ImportError as e:
-            raise RuntimeError(f"{os.path.join(_HERE, '_tq_host.so')} is missing or does not load ({e}): build it with "
-                               "`python turboquant-pytorch_b200/build.py`.") from e
-        H.bind(*(C.cast(getattr(L, n), C.c_void_p).value for n in
-                 ("tq_quantize", "tq_dequantize", "tq_copy_rows", "tq_qjl_compress", "tq_qjl_compress_workspace_bytes",
-                  "tq_prod_inner_product")), check)
+        H, why = _load_host()
+        if H is None:
+            import warnings
+            warnings.warn(f"{os.path.join(_HERE, '_tq_host.so')} is not used ({why}): calls take the slower general host path; "
+                          "build it with `python turboquant-pytorch_b200/build.py`", RuntimeWarning, stacklevel=3)
+            H = _GeneralPath()
+        else:
+            H.bind(*(C.cast(getattr(L, n), C.c_void_p).value for n in
+                     ("tq_quantize", "tq_dequantize", "tq_copy_rows", "tq_qjl_compress", "tq_qjl_compress_workspace_bytes",
+                      "tq_prod_inner_product")), check)
         _host = H
     return _host
 
