@@ -10,6 +10,7 @@ import torch
 import turboquant as tq
 from turboquant import _native as N
 from turboquant import _ops
+from turboquant import cache
 
 pytestmark = pytest.mark.filterwarnings("ignore::RuntimeWarning")
 
@@ -126,3 +127,34 @@ def test_a_build_for_another_torch_is_stale(monkeypatch, tmp_path):
     stamp.write_text("torch 1.0 other\n")
     build.build_host()
     assert len(built) == 2 and stamp.read_text() == build.host_built_for()
+
+
+def test_a_cache_that_the_native_step_refuses_is_not_looked_over_again(monkeypatch):
+    tried = []
+    monkeypatch.setattr(N, "host", lambda: types.SimpleNamespace(step_plan=lambda states, window: tried.append(window)))
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: device)
+    device = 0
+    c = cache.V3Cache(n_layers=2)
+    monkeypatch.setattr(c, "_step_general", lambda keys, values, views: "general")
+    for l in range(2):
+        c._layers[l] = types.SimpleNamespace(k=_OnCuda(1, 2, 16, 16))
+    tokens = [None, None]
+    assert [c.step(tokens, tokens) for _ in range(3)] == ["general"] * 3 and len(tried) == 1
+    device = 1                                                               # another device may hold what this one does not
+    c.step(tokens, tokens)
+    c.step(tokens, tokens)
+    assert len(tried) == 2
+    c._native_plan = None                                                    # a layer was made or grown
+    c.step(tokens, tokens)
+    c.residual_window += 1
+    c.step(tokens, tokens)
+    assert len(tried) == 4
+
+
+def test_a_step_before_the_layers_exist_makes_its_plan_afterwards(monkeypatch):
+    """Layers that update() creates drop the answer that there is no plan."""
+    c = cache.V3Cache(n_layers=2, residual_window=128)
+    token = [torch.zeros(1, 2, 1, 16) for _ in range(2)]
+    c.step(token, token)
+    assert c._native_plan is None
+    assert c.get_seq_length(1) == 1

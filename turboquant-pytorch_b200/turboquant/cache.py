@@ -176,13 +176,14 @@ class V3Cache(_Base):
                 "row_bytes": row_bytes, "base": base, "cap": cap, "tok_bytes": D * eb}
 
     def _make_native_plan(self, L: int):
-        """(plan, layers, states, window) for the native form of step(), or None while layers are missing."""
-        self._native_plan = None
+        """(plan, layers, states, window, device) for the native form of step().  `plan` is None for a cache that this form
+        does not take; that answer stands until a layer is made or grown, or the current device changes."""
         states = [self._layers.get(l) for l in range(L)]
+        plan = dev = None
         if L and all(st is not None and st.k is not None and st.k.is_cuda for st in states):
+            dev = torch.cuda.current_device()
             plan = N.host().step_plan(states, self.residual_window)
-            if plan is not None:
-                self._native_plan = (plan, L, states, self.residual_window)
+        self._native_plan = (plan, L, states, self.residual_window, dev)
         return self._native_plan
 
     def step(self, key_states: Sequence[torch.Tensor], value_states: Sequence[torch.Tensor], return_views: bool = True):
@@ -192,9 +193,10 @@ class V3Cache(_Base):
         Returns [(keys, values)] per layer as update() would (views of the persistent buffers), or None with
         return_views=False.  Falls back to per-layer update() calls while layers are being created or grown."""
         p = self._native_plan
-        if p is None or p[1] != len(key_states) or p[3] != self.residual_window:
+        if p is None or p[1] != len(key_states) or p[3] != self.residual_window or \
+                (p[0] is None and p[4] is not None and p[4] != torch.cuda.current_device()):
             p = self._make_native_plan(len(key_states))
-        if p is not None:
+        if p[0] is not None:
             done = N.host().step(p[0], p[2], key_states, value_states, return_views, self._step_log)
             if done is not None:
                 return done if return_views else None
