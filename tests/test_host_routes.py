@@ -1,6 +1,7 @@
 """Which calls the native host path stands in for, checked on the CPU with a stand-in for the extension."""
 
 import os
+import struct
 import sys
 import types
 
@@ -158,3 +159,26 @@ def test_a_step_before_the_layers_exist_makes_its_plan_afterwards(monkeypatch):
     c.step(token, token)
     assert c._native_plan is None
     assert c.get_seq_length(1) == 1
+
+
+def _record(*layers):
+    """The record of one native step: (first token, tokens, four offsets) of every layer."""
+    firsts, counts, offsets = zip(*layers)
+    return struct.pack(f"{6 * len(layers)}q", *firsts, *counts, *(o for four in offsets for o in four))
+
+
+def test_native_steps_are_read_where_they_are_recorded():
+    """Nothing is left for a later call: the entries of a layer come from its own list and from the steps' records, in token
+    order, and asking for them changes neither."""
+    c = cache.V3Cache(n_layers=3)
+    for l in range(3):
+        c._layers[l] = types.SimpleNamespace(packed=[])
+    c._layers[0].packed.append((0, 5, "update"))
+    c._step_log.append(("first", _record((5, 1, (0, 16, 32, 48)), (0, 2, (64, 80, 96, 112)))))
+    c._layers[0].packed.append((6, 2, "update again"))
+    c._step_log.append(("second", _record((8, 0, (0, 0, 0, 0)), (2, 1, (0, 16, 32, 48)), (0, 1, (64, 80, 96, 112)))))
+    for _ in range(2):
+        assert c._entries(0) == [(0, 5, "update"), (5, 1, "first", (0, 16, 32, 48)), (6, 2, "update again")]
+        assert c._entries(1) == [(0, 2, "first", (64, 80, 96, 112)), (2, 1, "second", (0, 16, 32, 48))]
+        assert c._entries(2) == [(0, 1, "second", (64, 80, 96, 112))]
+    assert len(c._step_log) == 2 and len(c._layers[0].packed) == 2 and not hasattr(c, "_file_steps")

@@ -78,7 +78,8 @@ class V3Cache(_Base):
         self._layers: Dict[int, _Layer] = {}
         self._step_plan = None
         self._native_plan = None
-        self._step_log: List[tuple] = []               # native steps whose packed rows are not in the layers' lists yet
+        # packed rows of the native steps, one entry (store, int64 record) per step for all layers: see _entries()
+        self._step_log: List[tuple] = []
 
     # ------------------------------------------------------------------ layers and buffers
     def _layer(self, layer_idx: int, head_dim: int, device) -> _Layer:
@@ -129,7 +130,6 @@ class V3Cache(_Base):
         st.total = need
         n_c = self._leaving(st, need)
         if n_c > 0:
-            self._file_steps()
             lo, hi = st.compressed, st.compressed + n_c
             view_k, view_v = st.k[:, :, lo:hi], st.v[:, :, lo:hi]
             kc, vc = st.codec.key_compressor, st.codec.val_compressor
@@ -205,7 +205,6 @@ class V3Cache(_Base):
     @torch.no_grad()
     def _step_general(self, key_states, value_states, return_views):
         """step() in Python: the first call, calls that create or grow layers, and inputs the native form does not take."""
-        self._file_steps()
         L = len(key_states)
         k0 = key_states[0]
         B, H, S_new, D = k0.shape
@@ -285,17 +284,19 @@ class V3Cache(_Base):
         return f"{comp} compressed, {total - comp} fp16, {total} total"
 
     # ------------------------------------------------------------------ beyond the reference
-    def _file_steps(self):
-        """Moves what the native steps recorded into the layers' lists of packed rows."""
-        if not self._step_log:
-            return
-        for store, blob in self._step_log:
-            r = struct.unpack(f"{len(blob) // 8}q", blob)
-            L = len(r) // 6
-            for l in range(L):
-                if r[L + l]:
-                    self._layers[l].packed.append((r[l], r[L + l], store, r[2 * L + 4 * l:2 * L + 4 * l + 4]))
-        self._step_log.clear()
+    def _entries(self, layer_idx: int) -> List[tuple]:
+        """The compressed-store entries of a layer in token order: its own list (update() and the general step) and its
+        part of every native step's record, which holds the first tokens, the counts and four offsets of each layer."""
+        found = list(self._layers[layer_idx].packed)
+        for store, record in self._step_log:
+            L = len(record) // 48
+            if layer_idx < L:
+                first, = struct.unpack_from("q", record, 8 * layer_idx)
+                n, = struct.unpack_from("q", record, 8 * (L + layer_idx))
+                if n:
+                    found.append((first, n, store, struct.unpack_from("4q", record, 8 * (2 * L + 4 * layer_idx))))
+        found.sort(key=lambda entry: entry[0])
+        return found
 
     def _chunk_tensors(self, st: _Layer, entry):
         """(first token, n, k idx, k norms, v idx, v norms) of one compressed-store entry, as (B, H, n, ...) tensors."""
@@ -314,11 +315,10 @@ class V3Cache(_Base):
 
     def packed_chunks(self, layer_idx: int):
         """The compressed store of a layer: lists of MSECompressor dicts for keys and values, in token order."""
-        self._file_steps()
         st = self._layers[layer_idx]
         B, H, _, D = st.k.shape
         cks, cvs = [], []
-        for entry in st.packed:
+        for entry in self._entries(layer_idx):
             _lo, n, k_idx, k_nrm, v_idx, v_nrm = self._chunk_tensors(st, entry)
             cks.append({"idx_bytes": k_idx, "vec_norms": k_nrm, "shape": (B, H, n, D), "idx_pad": 0})
             cvs.append({"idx_bytes": v_idx, "vec_norms": v_nrm, "shape": (B, H, n, D), "idx_pad": 0})
