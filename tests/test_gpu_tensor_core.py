@@ -258,6 +258,34 @@ def test_head_dim_64_keeps_infinite_and_nan_norms():
             assert bool(a.isnan()) == bool(b.isnan()) and (bool(a.isnan()) or bool(a == b))
 
 
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dim", [64])
+def test_rows_with_infinities_leave_the_others_alone(dim, dtype, bits):
+    """A row with an infinity or a NaN takes its norm from the vector itself, out of the sweep's line.  The other rows of its
+    warp, whose accumulator loads are under way meanwhile, come out as without it."""
+    x = O.synthetic_kv((1, 2, 600, dim), dtype, seed=bits).to(DEV)
+    comp = tq.MSECompressor(dim, bits, seed=42, device=DEV)
+    plain = comp.compress(x)
+    odd = {(0, 5): "inf", (0, 6): "-inf", (0, 40): "nan", (0, 130): "inf", (1, 0): "nan", (1, 31): "inf", (1, 599): "-inf"}
+    y = x.clone()
+    for i, ((h, s), value) in enumerate(odd.items()):
+        y[0, h, s, (7 * i) % dim] = float(value)
+    y[0, 1, 300:364, 3] = float("inf")                                      # whole warps
+    got = comp.compress(y)
+    assert N.lib().tq_last_device_status() == 0
+    touched = torch.zeros(2, 600, dtype=torch.bool, device=DEV)
+    touched[1, 300:364] = True
+    for (h, s), value in odd.items():
+        touched[h, s] = True
+        norm = got["vec_norms"][0, h, s]
+        assert bool(norm.isnan()) if value == "nan" else float(norm) == float("inf")
+    assert bool((got["vec_norms"][0, 1, 300:364] == float("inf")).all())
+    assert bool((got["idx_bytes"][0][touched] == 0).all())
+    for key in ("idx_bytes", "vec_norms"):
+        assert torch.equal(got[key][0][~touched], plain[key][0][~touched])
+
+
 @pytest.mark.parametrize("dim", [64, 128])
 def test_one_long_slab(dim):
     """(1, 1, S, D): the strides of the size-1 dimensions in the tensor map stay below 2^40 bytes."""

@@ -736,10 +736,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
           else ssq = ssq_row_fast<D>(tacc, ra, rb);
           float norm = __fsqrt_rn(ssq);
           if constexpr (D == 64) {
-            if (!(ssq == ssq) && valid) {
-              const UmmaQuantJob& full = batch.jobs[job.j];
-              const int bb = slab / job.H, hh = slab - bb * job.H;
-              norm = x_norm<BF16, D>(full.x + bb * full.xs_b + hh * full.xs_h + s_row * full.xs_s);
+            // The sweep left a load in flight into `ra`: it lands before the call out of line, which may move or reuse those
+            // registers, and the warp is whole again before the next collective load.
+            if (__any_sync(0xffffffffu, !(ssq == ssq))) {
+              tmem_wait16(ra);
+              if (!(ssq == ssq) && valid) {
+                const UmmaQuantJob& full = batch.jobs[job.j];
+                const int bb = slab / job.H, hh = slab - bb * job.H;
+                norm = x_norm<BF16, D>(full.x + bb * full.xs_b + hh * full.xs_h + s_row * full.xs_s);
+              }
+              __syncwarp();
             }
           }
           const float inv = __fdiv_rn(1.0f, norm + 1e-8f);
