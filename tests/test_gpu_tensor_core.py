@@ -260,7 +260,7 @@ def test_head_dim_64_keeps_infinite_and_nan_norms():
 
 @pytest.mark.parametrize("bits", [1, 2, 3, 4, 5, 6, 7, 8])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("dim", [64])
+@pytest.mark.parametrize("dim", [64, 128])
 def test_rows_with_infinities_leave_the_others_alone(dim, dtype, bits):
     """A row with an infinity or a NaN takes its norm from the vector itself, out of the sweep's line.  The other rows of its
     warp, whose accumulator loads are under way meanwhile, come out as without it."""
@@ -284,6 +284,21 @@ def test_rows_with_infinities_leave_the_others_alone(dim, dtype, bits):
     assert bool((got["idx_bytes"][0][touched] == 0).all())
     for key in ("idx_bytes", "vec_norms"):
         assert torch.equal(got[key][0][~touched], plain[key][0][~touched])
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_an_infinite_vector_has_one_norm_in_calls_of_any_size(dim, dtype):
+    comp = tq.MSECompressor(dim, 4, seed=42, device=DEV)
+    x = O.synthetic_kv((1, 1, 300, dim), dtype, seed=3).to(DEV)
+    x[0, 0, 77, 9], x[0, 0, 78, 9] = float("inf"), float("nan")
+    long, ref = comp.compress(x), _simt(lambda: comp.compress(x))
+    for s in (77, 78):
+        token = comp.compress(x[:, :, s:s + 1])
+        for c in (token["vec_norms"][0, 0, 0], long["vec_norms"][0, 0, s], ref["vec_norms"][0, 0, s]):
+            assert bool(c.isnan()) if s == 78 else float(c) == float("inf")
+        assert torch.equal(token["idx_bytes"][0, 0, 0], long["idx_bytes"][0, 0, s])
+        assert torch.equal(token["idx_bytes"][0, 0, 0], ref["idx_bytes"][0, 0, s])
 
 
 @pytest.mark.parametrize("dim", [64, 128])

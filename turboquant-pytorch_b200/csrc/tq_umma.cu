@@ -224,18 +224,6 @@ __device__ __noinline__ void quant_row_search(int bits, uint32_t tacc, float inv
   }
 }
 
-// Norm of a vector from its own coordinates.  The rotated row of a vector with an infinity is NaN throughout (the
-// pieces of Pi meet it with both signs) while its norm is infinite; such rows come here.  Out of line: cold.
-template <bool BF16, int D>
-__device__ __noinline__ float x_norm(const uint16_t* x) {
-  float ssq = 0.f;
-  for (int k = 0; k < D; ++k) {
-    const float v = BF16 ? __uint_as_float((uint32_t)__ldg(x + k) << 16) : __half2float(__ushort_as_half(__ldg(x + k)));
-    ssq = fmaf(v, v, ssq);
-  }
-  return __fsqrt_rn(ssq);
-}
-
 // Search shortcut (see the codebook block): one cubic, one lane look-up of the candidate
 // threshold, one compare.  Arithmetic is kept on the FMA pipe: the index is built as a
 // float next to 2^23 and shifted into the packed word by an integer multiply-add; the
@@ -472,6 +460,26 @@ __device__ __forceinline__ void quant_row_cells(uint32_t tacc, uint32_t (&a)[16]
     quant_chunk_cells(b, sc, cells_lane, thr_lane, wb);
     if (valid) store_index_pair(idx_row + c * 16, wa, wb, wide);
   }
+}
+
+// Norm of vector `row` of a job's tile `lt` from its own coordinates, for the lanes that `mine` names.  The rotated row of a
+// vector with an infinity is NaN (the pieces of Pi meet it with both signs) while its norm is infinite, as the FP32 kernels
+// have it; such rows come here.  Out of line and after the sweeps: cold, and no accumulator load is under way.
+template <bool BF16, int D>
+__device__ __noinline__ void norm_from_vector(const UmmaQuantJob& job, int lt, int row, bool mine) {
+  const int slab = lt / job.tiles_per_slab;
+  const int64_t s_row = (int64_t)(lt - slab * job.tiles_per_slab) * kTileVecs<D> + row;
+  if (mine && s_row < job.S) {
+    const int bb = slab / job.H, hh = slab - bb * job.H;
+    const uint16_t* x = job.x + bb * job.xs_b + hh * job.xs_h + s_row * job.xs_s;
+    float ssq = 0.f;
+    for (int k = 0; k < D; ++k) {
+      const float v = BF16 ? __uint_as_float((uint32_t)__ldg(x + k) << 16) : __half2float(__ushort_as_half(__ldg(x + k)));
+      ssq = fmaf(v, v, ssq);
+    }
+    job.norms_out[(int64_t)slab * job.S + s_row] = __half_as_ushort(__float2half_rn(__fsqrt_rn(ssq)));
+  }
+  __syncwarp();
 }
 
 // Rest of a role's walk after one of its waits ran out: only the two named barriers of every job
@@ -734,20 +742,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
           float ssq;
           if (TQ_ABL(batch, 512)) { ssq = 1.0f; tmem_issue16(tacc, ra); }
           else ssq = ssq_row_fast<D>(tacc, ra, rb);
-          float norm = __fsqrt_rn(ssq);
-          if constexpr (D == 64) {
-            // The sweep left a load in flight into `ra`: it lands before the call out of line, which may move or reuse those
-            // registers, and the warp is whole again before the next collective load.
-            if (__any_sync(0xffffffffu, !(ssq == ssq))) {
-              tmem_wait16(ra);
-              if (!(ssq == ssq) && valid) {
-                const UmmaQuantJob& full = batch.jobs[job.j];
-                const int bb = slab / job.H, hh = slab - bb * job.H;
-                norm = x_norm<BF16, D>(full.x + bb * full.xs_b + hh * full.xs_h + s_row * full.xs_s);
-              }
-              __syncwarp();
-            }
-          }
+          const float norm = __fsqrt_rn(ssq);
           const float inv = __fdiv_rn(1.0f, norm + 1e-8f);
           if (valid) job.norms_out[n] = __half_as_ushort(__float2half_rn(norm));
           sc.s_inv = sc.s * inv;
@@ -783,6 +778,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
             // wide launches have no plain threshold table in shared memory: the search reads the codebook block
             quant_row_search<D>(job.bits, tacc, inv, WIDE ? job.codebook + kThresholdOff : thr, idx_row, valid);
           }
+          // the norm is NaN, and with it the scale: the indices are 0 by now, the norm comes from the vector itself
+          if (__any_sync(0xffffffffu, sc.s_inv != sc.s_inv))
+            norm_from_vector<BF16, D>(batch.jobs[job.j], lt, h * kTileRows + row, sc.s_inv != sc.s_inv);
         }
       }
       tc_fence_before();
