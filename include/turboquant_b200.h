@@ -375,7 +375,7 @@ int tq_qjl_scores(const TqQjlScoreJob* job, void* stream);
 
 /* Row-paired estimator <y_n, x_mse_n> + ||r_n|| sqrt(pi/2)/M <S y_n, signs_n>.
  * y (ny, D) fp32 with ny == n or ny == 1; idx int64 (n, D); signs fp32 (n, M);
- * rnorm fp32 (n); workspace >= (n + ny) * 256 * 4 bytes.
+ * rnorm fp32 (n); workspace >= (n + ny) * 256 * 4 bytes, 2 * 256 * 4 for one query (ny = 1).
  * Replaces: TurboQuantProd.inner_product turboquant/turboquant.py:165-192.     */
 int tq_prod_inner_product(const float* y, int64_t ny, const int64_t* idx, const float* signs, const float* rnorm,
                           int64_t n, int D, int M, const float* rotation, const float* codebook,

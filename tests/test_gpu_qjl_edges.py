@@ -47,3 +47,45 @@ def test_qjl_scores_query_blocks(d, dtype, sq):
     want = qd @ c["k_mse"].double().transpose(-1, -2) + (qd @ comp.S.double().T) @ c["qjl_signs"].double().transpose(-1, -2) * corr
     assert float((got.double() - want).norm() / want.norm()) <= 1e-5
     assert N.lib().tq_last_device_status() == 0
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("sq", [1, 64, 100])
+def test_scores_use_no_more_scratch_than_they_ask_for(d, sq, monkeypatch):
+    """The operand images and the FP32 kernels' projections share one buffer; a guard behind it stays as it was."""
+    comp = tq.TurboQuantCompressorV2(d, 3, seed=9, device=DEV)
+    c = comp.compress(O.synthetic_kv((1, 3, 200, d), torch.float16, seed=sq).to(DEV))
+    q = torch.randn(1, 3, sq, d, generator=_gen(sq), device=DEV)
+    want = comp.asymmetric_attention_scores(q, c)
+    wanted = N.lib().tq_qjl_scores_workspace_bytes(3, sq, d)
+    units = 3 * -(-sq // 64)
+    images = units * 8 * 64 * d + 1024 if d >= 128 else 0                   # four bytes (two pieces) of 2 D columns of 64 rows
+    assert wanted == max(2 * 3 * sq * d * 4, images)
+    made = []
+    real = torch.empty
+
+    def guarded(*size, **kw):
+        if size == (max(wanted, 256),) and kw.get("dtype") is torch.uint8:
+            made.append(torch.full((size[0] + 4096,), 0xA5, dtype=torch.uint8, device=DEV))
+            return made[-1][:size[0]]
+        return real(*size, **kw)
+    monkeypatch.setattr(torch, "empty", guarded)
+    got = comp.asymmetric_attention_scores(q, c)
+    monkeypatch.undo()
+    assert torch.equal(got, want) and len(made) == 1 and bool((made[0][-4096:] == 0xA5).all())
+
+
+def test_one_query_needs_scratch_for_one_query():
+    prod = tq.TurboQuantProd(128, 3, device=DEV)
+    x = torch.randn(500, 128, generator=_gen(1), device=DEV)
+    c = prod.quantize(x)
+    L, y = N.lib(), torch.randn(1, 128, generator=_gen(2), device=DEV)
+    want = prod.inner_product(y, c)
+    out, ws = torch.empty(500, device=DEV), torch.full((2048 + 4096,), 0xA5, dtype=torch.uint8, device=DEV)
+
+    def call(ny, n_bytes):
+        return L.tq_prod_inner_product(y.data_ptr(), ny, c["mse_indices"].data_ptr(), c["qjl_signs"].data_ptr(), c["residual_norm"].data_ptr(),
+                                       500, 128, c["qjl_signs"].shape[1], prod.mse.Pi.data_ptr(), prod.mse._cb.data_ptr(),
+                                       prod._s_t.data_ptr(), out.data_ptr(), ws.data_ptr(), n_bytes, N.stream_ptr(DEV))
+    assert call(1, 2048) == 0 and torch.equal(out, want) and bool((ws[2048:] == 0xA5).all())
+    assert call(1, 2044) == -8 and call(500, 500 * 2048 - 4) == -8

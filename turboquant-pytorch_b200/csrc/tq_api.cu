@@ -509,7 +509,9 @@ int tq_qjl_scores_packed(const TqQjlPackedScoreJob* job, void* stream) {
 
 size_t tq_qjl_scores_workspace_bytes(int64_t BH, int64_t Sq, int D) {
   if (BH < 0 || Sq < 0 || D < 1) return 0;
-  return tq::simt_qjl_scores_workspace(BH, Sq, D) + tq::umma_qjl_scores_image_bytes(BH, Sq, D);
+  // the FP32 kernels' projected queries or the tensor-core kernel's operand images: a call uses one of them
+  const size_t simt_ws = tq::simt_qjl_scores_workspace(BH, Sq, D), img = tq::umma_qjl_scores_image_bytes(BH, Sq, D);
+  return simt_ws > img ? simt_ws : img;
 }
 
 int tq_qjl_scores(const TqQjlScoreJob* job, void* stream) {
@@ -522,13 +524,11 @@ int tq_qjl_scores(const TqQjlScoreJob* job, void* stream) {
       job->qjl_t == nullptr || job->scores == nullptr || job->workspace == nullptr)
     return TQ_ENULL;
   if (((uintptr_t)job->workspace & 15u) != 0) return TQ_EALIGN;
-  const size_t simt_ws = tq::simt_qjl_scores_workspace(job->BH, job->Sq, job->D);
-  if (job->workspace_bytes < simt_ws) return TQ_EWORKSPACE;
   if (tq::umma_qjl_scores_eligible(*job)) {
-    const size_t img = tq::umma_qjl_scores_image_bytes(job->BH, job->Sq, job->D);
-    if (job->workspace_bytes < simt_ws + img) return TQ_EWORKSPACE;
-    return tq::umma_qjl_scores(*job, reinterpret_cast<char*>(job->workspace) + simt_ws, (cudaStream_t)stream);
+    if (job->workspace_bytes < tq::umma_qjl_scores_image_bytes(job->BH, job->Sq, job->D)) return TQ_EWORKSPACE;
+    return tq::umma_qjl_scores(*job, job->workspace, (cudaStream_t)stream);
   }
+  if (job->workspace_bytes < tq::simt_qjl_scores_workspace(job->BH, job->Sq, job->D)) return TQ_EWORKSPACE;
   return tq::simt_qjl_scores(*job, (cudaStream_t)stream);
 }
 
@@ -542,7 +542,7 @@ int tq_prod_inner_product(const float* y, int64_t ny, const int64_t* idx, const 
       codebook == nullptr || qjl_t == nullptr || out == nullptr || workspace == nullptr)
     return TQ_ENULL;
   if (((uintptr_t)workspace & 15u) != 0) return TQ_EALIGN;
-  if (workspace_bytes < (size_t)(n + ny) * 256 * sizeof(float)) return TQ_EWORKSPACE;
+  if (workspace_bytes < (size_t)(ny == 1 ? 2 : n + ny) * 256 * sizeof(float)) return TQ_EWORKSPACE;
   return tq::simt_prod_inner_product(y, ny, idx, signs, rnorm, n, D, M, rotation, codebook, qjl_t, out, workspace,
                                      (cudaStream_t)stream);
 }

@@ -384,7 +384,7 @@ PyObject* prod_inner(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (rows < 1 || y.size(1) != d || (y.size(0) != rows && y.size(0) != 1) || signs.size(0) != rows || rn.size(0) != rows) return none();
   c10::AutoGradMode no_grad(false);
   at::Tensor out = make({rows}, at::kFloat, dev);
-  at::Tensor ws = make({(rows + y.size(0)) * 256 * 4}, at::kByte, dev);
+  at::Tensor ws = make({(y.size(0) == 1 ? 2 : rows + y.size(0)) * 256 * 4}, at::kByte, dev);
   void* st = stream_of(dev);
   const float *pi = (const float*)THPVariable_Unpack(a[4]).data_ptr(), *cb = (const float*)THPVariable_Unpack(a[5]).data_ptr(),
               *qt = (const float*)THPVariable_Unpack(a[6]).data_ptr();

@@ -1432,10 +1432,8 @@ int simt_prod_inner_product(const float* y, int64_t ny, const int64_t* idx, cons
                             float* out, void* workspace, cudaStream_t st) {
   if (n == 0) return TQ_OK;
   const float corr = (float)(1.2533141373155001 / (double)M);
-  float* xhat = reinterpret_cast<float*>(workspace);
-  float* sy = xhat + n * 256;
   if (ny == 1) {
-    float* yr = xhat;
+    float *yr = reinterpret_cast<float*>(workspace), *sy = yr + 256;
     k_query_rotate<<<(unsigned)((D + 7) / 8 + (M + 31) / 32), NT, 0, st>>>(y, D, M, rotation, qjl_t, yr, sy);
     int rc = check_launch();
     if (rc != TQ_OK) return rc;
@@ -1443,6 +1441,8 @@ int simt_prod_inner_product(const float* y, int64_t ny, const int64_t* idx, cons
     k_prod_inner_one<<<grid, NT, 0, st>>>(idx, signs, rnorm, n, D, M, codebook, yr, sy, corr, out);
     return check_launch();
   }
+  float* xhat = reinterpret_cast<float*>(workspace);
+  float* sy = xhat + n * 256;
   TqDequantizeJob dj{};
   dj.idx = idx; dj.norms = nullptr; dj.idx_mode = TQ_IDX_I64; dj.D = D; dj.bits = 8; dj.out_dtype = TQ_F32;
   dj.B = 1; dj.H = 1; dj.S = n; dj.out = xhat; dj.ostride_b = 0; dj.ostride_h = 0; dj.ostride_s = D;

@@ -402,7 +402,7 @@ def prod_inner_product(y: torch.Tensor, idx: torch.Tensor, signs: torch.Tensor, 
     M = signs.shape[1]
     y = y.float().contiguous()
     out = torch.empty((n,), dtype=torch.float32, device=idx.device)
-    ws = torch.empty(max((n + y.shape[0]) * 256 * 4, 256), dtype=torch.uint8, device=idx.device)
+    ws = torch.empty((2 if y.shape[0] == 1 else n + y.shape[0]) * 256 * 4, dtype=torch.uint8, device=idx.device)
     with torch.cuda.device(idx.device):
         N.check(N.lib().tq_prod_inner_product(
             y.data_ptr(), y.shape[0], idx.contiguous().data_ptr(), signs.contiguous().data_ptr(),
