@@ -95,8 +95,8 @@ int tq_packed_row_bytes(int D, int bits);
 int tq_build_codebook(const float* centroids, int bits, float* block);
 
 /* Tensor-core operand image of a (D, D) row-major fp32 matrix m [dev]: two fp16 pieces
- * (m = hi + lo) and three bf16 pieces, K-major, 128-byte swizzled, tq_rotation_image_bytes(D) bytes
- * (0 when D has no tensor-core path; D = 64 and 128 have one).  Built once per compressor.
+ * (m = hi + lo; at D = 64 of 2^8 m, whose entries have to stay below 2^8) and three bf16 pieces,
+ * K-major, 128-byte swizzled, tq_rotation_image_bytes(D) bytes (0 when D has no tensor-core path; D = 64 and 128 have one).  Built once per compressor.
  * For TqQuantizeJob pass m = Pi; for TqDequantizeJob pass m = Pi^T.
  * Replaces nothing in the reference (a constant of this implementation).       */
 size_t tq_rotation_image_bytes(int D);

@@ -238,7 +238,9 @@ def test_head_dim_64_round_trip(rows, dtype, bits):
     got, ref = out[:, :, 1:rows + 1].float(), want.to(dtype).float()
     step = 2.0 ** (-10 if dtype == torch.float16 else -7)
     assert bool(((got - ref).abs() <= step * ref.abs() + 2.0 ** -18 * float(want.abs().max())).all())
-    assert float((got != ref).float().mean()) <= 0.01 if dtype == torch.bfloat16 else True
+    # which is rare: two results 2e-8 apart straddle an edge of fp16 in about 2e-3 of the values (1.2e-4 for each of the binades
+    # below the largest value, whose steps halve with it), of bf16 in an eighth of that
+    assert float((got != ref).float().mean()) <= 0.01
     assert bool((out[:, :, 0] == -7).all()) and bool((out[:, :, rows + 1:] == -7).all())
 
 
@@ -286,6 +288,32 @@ def test_rows_with_infinities_leave_the_others_alone(dim, dtype, bits):
         assert torch.equal(got[key][0][~touched], plain[key][0][~touched])
 
 
+@pytest.mark.parametrize("bits", [2, 3, 4, 6, 8])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_head_dim_64_is_no_further_from_64_bits_than_the_fp32_kernels(dtype, bits):
+    """Norms are the FP32 kernels' bit for bit.  Rebuilt values are nearer to 64 bits than theirs, by their root mean square over
+    four million values; indices off by rounding are as rare, up to the scatter of such small counts."""
+    comp = tq.MSECompressor(64, bits, seed=42, device=DEV)
+    x = O.synthetic_kv((2, 8, 3851, 64), dtype, seed=bits).to(DEV)
+    got, ref = comp.compress(x), _simt(lambda: comp.compress(x))
+    assert torch.equal(got["vec_norms"], ref["vec_norms"])
+    cent = comp.centroids.double()
+    unit = x.double() / (x.double().norm(dim=-1, keepdim=True) + 1e-8)
+    want = torch.searchsorted((cent[1:] + cent[:-1]) / 2, unit @ comp.Pi.double().T)
+    per = 8 // bits
+
+    def indices(c):
+        return torch.stack([(c["idx_bytes"].long() >> (bits * (per - 1 - i))) & ((1 << bits) - 1) for i in range(per)], -1).flatten(-2)
+
+    flips, ref_flips = (int((indices(c) != want).sum()) for c in (got, ref))
+    assert flips <= ref_flips + 3 * max(1.0, ref_flips) ** 0.5 + 3, (flips, ref_flips)
+    exact = cent[indices(ref)] @ comp.Pi.double()
+    scale = ref["vec_norms"].double().unsqueeze(-1)
+    error, ref_error = (float((back.double() / scale - exact).square().mean().sqrt())
+                        for back in (comp.decompress(ref), _simt(lambda: comp.decompress(ref))))
+    assert error <= ref_error, (error, ref_error)
+
+
 @pytest.mark.parametrize("dim", [64, 128])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_an_infinite_vector_has_one_norm_in_calls_of_any_size(dim, dtype):
@@ -320,3 +348,25 @@ def _rebuild(comp, packed, dtype):
     job, _keep = comp.decompress_job(packed, out)
     _ops.run_dequantize([job], DEV)
     return out
+
+
+@pytest.mark.parametrize("dim,dtype", [(64, torch.float16), (64, torch.bfloat16), (64, torch.float32), (128, torch.float32)])
+@pytest.mark.parametrize("bits", [4, 8])
+def test_rebuilt_rows_off_a_32_byte_boundary(dim, dtype, bits):
+    """Outputs that start on an odd multiple of 16 bytes leave as 16-byte stores and are the same values."""
+    comp = tq.MSECompressor(dim, bits, seed=80, device=DEV)
+    x = O.synthetic_kv((1, 2, 300, dim), torch.float16, seed=bits).to(DEV)
+    c = comp.compress(x)
+    n = x.numel()
+    step = 16 // torch.empty(0, dtype=dtype).element_size()
+    results = []
+    for off in (0, step):
+        raw = torch.full((n + 4 * step,), -7.0, dtype=dtype, device=DEV)
+        start = 2 * step + off
+        out = raw[start:start + n].view(1, 2, 300, dim)
+        assert out.data_ptr() % 32 == (16 if off else 0)
+        job, _keep = comp.decompress_job(c, out)
+        _ops.run_dequantize([job], DEV)
+        assert bool((raw[:start] == -7).all()) and bool((raw[start + n:] == -7).all())
+        results.append(out)
+    assert torch.equal(*results) and N.lib().tq_last_device_status() == 0

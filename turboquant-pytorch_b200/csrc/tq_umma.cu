@@ -46,10 +46,26 @@ constexpr uint32_t kHalfBytes = kTileBytes / 2;        // one 64-column box
 // operand) or 256 vectors of head_dim 64 (the boxes are two operands of 128 vectors; each has its own 64 columns of
 // the tile's accumulator).  Ring, accumulator and staging sizes are then the same for both.
 // Head_dim 64 ran on the FP32 kernels before, which are bound by their fused multiply-adds: 124 us to quantise and 80 us to
-// rebuild one (2, 8, 4875, 64) bf16 tensor; compress_kv + decompress_kv of such a layer (K4/V3) went from 376 to 108 us,
-// most of which is the host's.
+// rebuild one (2, 8, 4875, 64) bf16 tensor; compress_kv + decompress_kv of such a layer (K4/V3) take 38 us here, 290 on the FP32
+// kernels with the same host path.
 template <int D> constexpr int kTileVecs = (int)(kTileBytes / 2) / D;
 template <int D> constexpr uint32_t kImagePiece = (uint32_t)(D * D * 2);                 // one piece of a rotation image
+// Head_dim 64 ran in fp32 chains before and may be no further from 64 bits than those.  Its fp16 pieces, of the rotation and
+// of the centroids, are those of 2^8 times the value: unscaled, the low piece of a typical entry is an fp16 subnormal and
+// right to 2^-25 only.  The low piece is rounded away from zero, because the tensor core truncates its sums towards it, and
+// the passes go from the lowest product to the highest, so that only the last k-steps truncate at full magnitude.
+// Over 10^8 coordinates a width: rebuilt values are 1.1e-8 to 1.5e-8 (root mean square, unit vectors) from 64 bits, 1.8e-8 in
+// the FP32 kernels and 4.2e-8 to 5.9e-8 with unscaled pieces, three passes and hi.hi first; 4-bit indices off by rounding 19
+// (fp16) and 13 (bf16), 28 and 32 in the FP32 kernels, 54 and 31 before.
+// (Head_dim 128 has no fp32 chain to keep up with and is as it was.)
+template <int D> constexpr float kPieceScale = D == 64 ? 256.f : 1.f;
+template <int D>
+__device__ __forceinline__ void fp16_pieces(float v, __half& hi, __half& lo) {
+  v *= kPieceScale<D>;                                   // a power of two: exact, and taken out again exactly
+  hi = __float2half_rn(v);
+  const float rest = v - __half2float(hi);
+  lo = D != 64 ? __float2half_rn(rest) : v < 0.f ? __float2half_rd(rest) : __float2half_ru(rest);
+}
 constexpr int tile_vecs_of(int D) { return (int)(kTileBytes / 2) / D; }
 constexpr int kMaxJobs = 96;
 constexpr int kFewJobs = 8;
@@ -462,24 +478,65 @@ __device__ __forceinline__ void quant_row_cells(uint32_t tacc, uint32_t (&a)[16]
   }
 }
 
-// Norm of vector `row` of a job's tile `lt` from its own coordinates, for the lanes that `mine` names.  The rotated row of a
-// vector with an infinity is NaN (the pieces of Pi meet it with both signs) while its norm is infinite, as the FP32 kernels
-// have it; such rows come here.  Out of line and after the sweeps: cold, and no accumulator load is under way.
-template <bool BF16, int D>
-__device__ __noinline__ void norm_from_vector(const UmmaQuantJob& job, int lt, int row, bool mine) {
-  const int slab = lt / job.tiles_per_slab;
-  const int64_t s_row = (int64_t)(lt - slab * job.tiles_per_slab) * kTileVecs<D> + row;
-  if (mine && s_row < job.S) {
-    const int bb = slab / job.H, hh = slab - bb * job.H;
+// Norms that came out NaN, once more from the vectors' own coordinates: of vector `row` in every fourth of the CTA's tiles from
+// `first` on, up to tile `end`.  The rotated row of a vector with an infinity is NaN (the pieces of Pi meet it with both signs)
+// while its norm is infinite, as the FP32 kernels have it.  Out of line and after the last tile: a look at every tile's
+// norms in the loop, with the call behind it, cost 2 % of a launch.
+template <bool BF16, int D, int J>
+__device__ __noinline__ void norms_from_vectors(const UmmaQuantBatchOf<J>& batch, int t0, int first, int end, int row) {
+  QuantJobView v;
+  for (int i = first; i < end; i += 4) {
+    view_advance<D>(batch, t0 + i, v);
+    const UmmaQuantJob& job = batch.jobs[v.j];
+    const int lt = t0 + i - v.begin;
+    const int slab = lt / v.tps;
+    const int64_t s_row = (int64_t)(lt - slab * v.tps) * kTileVecs<D> + row;
+    if (s_row >= v.S) continue;
+    uint16_t* out = v.norms_out + (int64_t)slab * v.S + s_row;              // written by this thread
+    if ((*out & 0x7FFFu) <= 0x7C00u) continue;
+    const int bb = slab / v.H, hh = slab - bb * v.H;
     const uint16_t* x = job.x + bb * job.xs_b + hh * job.xs_h + s_row * job.xs_s;
     float ssq = 0.f;
     for (int k = 0; k < D; ++k) {
-      const float v = BF16 ? __uint_as_float((uint32_t)__ldg(x + k) << 16) : __half2float(__ushort_as_half(__ldg(x + k)));
-      ssq = fmaf(v, v, ssq);
+      const float c = BF16 ? __uint_as_float((uint32_t)__ldg(x + k) << 16) : __half2float(__ushort_as_half(__ldg(x + k)));
+      ssq = fmaf(c, c, ssq);
     }
-    job.norms_out[(int64_t)slab * job.S + s_row] = __half_as_ushort(__float2half_rn(__fsqrt_rn(ssq)));
+    *out = __half_as_ushort(__float2half_rn(__fsqrt_rn(ssq)));
   }
-  __syncwarp();
+}
+
+// Norm of a head_dim 64 vector from its operand row in shared memory (chunk c of eight values at c ^ (row & 7)), with the
+// additions in the order of the FP32 kernels' warp sum: lane l of theirs holds values l and l + 32.
+template <bool BF16>
+__device__ __forceinline__ float norm_of_row64(uint32_t row_addr, int row) {
+  auto squares = [&](int c, float (&p)[8]) {              // values of chunks c and c + 4: fma(v1, v1, v0 * v0)
+    const uint4 a = ld_shared_v4(row_addr + (uint32_t)((c ^ (row & 7)) << 4));
+    const uint4 b = ld_shared_v4(row_addr + (uint32_t)(((c + 4) ^ (row & 7)) << 4));
+    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      auto value = [&](uint32_t w) {
+        if constexpr (BF16) return __uint_as_float((e & 1) ? (w & 0xFFFF0000u) : (w << 16));
+        else return __half2float(__ushort_as_half((uint16_t)((e & 1) ? (w >> 16) : (w & 0xFFFFu))));
+      };
+      const float v0 = value(aw[e >> 1]), v1 = value(bw[e >> 1]);
+      p[e] = fmaf(v1, v1, fmaf(v0, v0, 0.f));
+    }
+  };
+  float sum[8];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    float p[8], q[8];
+    squares(c, p);
+    squares(c + 2, q);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sum[e] = c == 0 ? p[e] + q[e] : sum[e] + (p[e] + q[e]);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < o; ++e) sum[e] += sum[e + o];
+  return __fsqrt_rn(sum[0]);
 }
 
 // Rest of a role's walk after one of its waits ran out: only the two named barriers of every job
@@ -515,7 +572,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
   const uint32_t bar0 = base + kOffBar;
   // barrier slots (8 bytes each)
   const uint32_t bar_full = bar0;                  // [kStages]
-  const uint32_t bar_empty = bar0 + 8 * kStages;   // [kStages]
+  const uint32_t bar_xread = bar0 + 8 * kStages;   // [kStages] head_dim 64: the epilogue has read the stage's vectors
   const uint32_t bar_tfull = bar0 + 16 * kStages;  // [kAccBufs]
   const uint32_t bar_tempty = bar_tfull + 8 * kAccBufs;
   const uint32_t bar_pifull = bar_tempty + 8 * kAccBufs;
@@ -529,7 +586,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
   const int n_local = t1 - t0;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kStages; ++i) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
+    for (int i = 0; i < kStages; ++i) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_xread + 8 * i, 4); }
     for (int i = 0; i < kAccBufs; ++i) { mbar_init(bar_tfull + 8 * i, 1); mbar_init(bar_tempty + 8 * i, 4); }
     mbar_init(bar_pifull, 1);
     mbar_init(bar_pifree, 1);
@@ -564,6 +621,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
         if (i >= kStages) {     // the stage is free once the MMAs of tile i - kStages are done (one commit serves both rings)
           const int d = i - kStages;
           ok = mbar_wait(bar_tfull + 8 * (d % kAccBufs), (uint32_t)((d / kAccBufs) & 1), abort_flag);
+          if constexpr (D == 64) ok = ok && mbar_wait(bar_xread + 8 * s, (uint32_t)((d / kStages) & 1), abort_flag);
           if (!ok) break;
         }
         const int lt = t - job.begin;
@@ -628,14 +686,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
 #pragma unroll
             for (int h = 0; h < 128 / D; ++h) {        // head_dim 64: the two operands of a tile, 64 columns each
 #pragma unroll
-              for (int piece = 0; piece < kPieces; ++piece) {
+              for (int pass = 0; pass < kPieces; ++pass) {
+                // head_dim 64: the lowest piece first (see fp16_pieces)
+                const int piece = D == 64 ? kPieces - 1 - pass : pass;
 #pragma unroll
                 for (int k = 0; k < D / 16; ++k) {
                   constexpr uint32_t kUnit = 16;
                   const uint64_t koff = (uint64_t)(((k >> 2) * kHalfBytes + (k & 3) * 32) / kUnit);
                   const uint64_t hoff = (uint64_t)(h * kHalfBytes / kUnit);
                   const uint64_t poff = (uint64_t)((piece * C::kPieceBytes) / kUnit);
-                  umma_f16(d_tmem + h * 64, a_base + hoff + koff, b_base + poff + koff, idesc, (piece | k) != 0 ? 1u : 0u);
+                  umma_f16(d_tmem + h * 64, a_base + hoff + koff, b_base + poff + koff, idesc, (pass | k) != 0 ? 1u : 0u);
                 }
               }
             }
@@ -665,6 +725,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
     int mode = 0;                               // 0 search, 1 cubic shortcut, 2 cell table
     bool ok = true;
     bool fast = false, fast_lds = false, linear = false;
+    float odd_norms = 0.f;
     Shortcut sc = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     QuantJobView job;
     // Wide launches keep ONE set of tables per CTA.  Every epilogue warp walks the CTA's jobs in order,
@@ -728,6 +789,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
       ok = __all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * wg, (uint32_t)((i / kAccBufs) & 1), abort_flag));
       if (!ok) break;
       tc_fence_after();
+      // head_dim 64: norms from the vectors, as in the FP32 kernels; the stage cannot be filled again before these reads
+      float norm64[128 / D] = {};
+      if constexpr (D == 64) {
+        const int s = i % kStages;
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * s, (uint32_t)((i / kStages) & 1), abort_flag));
+        if (!ok) break;
+        const uint32_t rows = a_smem + s * kTileBytes + (uint32_t)row * 128u;
+        norm64[0] = norm_of_row64<BF16>(rows, row);
+        norm64[1] = norm_of_row64<BF16>(rows + kHalfBytes, row);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_xread + 8 * s);
+      }
       const int lt = t - job.begin;
       const int slab = lt / job.tps;
 #pragma unroll 1
@@ -739,11 +812,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
         uint8_t* idx_row = job.idx_out + n * (int64_t)job.g;
         if (!TQ_ABL(batch, 2)) {
           uint32_t ra[16], rb[16];
-          float ssq;
-          if (TQ_ABL(batch, 512)) { ssq = 1.0f; tmem_issue16(tacc, ra); }
-          else ssq = ssq_row_fast<D>(tacc, ra, rb);
-          const float norm = __fsqrt_rn(ssq);
-          const float inv = __fdiv_rn(1.0f, norm + 1e-8f);
+          constexpr float kUnscale = BF16 ? 1.f : 1.f / kPieceScale<D>;       // a power of two: exact
+          float norm;
+          if constexpr (D == 64) {
+            norm = h ? norm64[128 / D - 1] : norm64[0];
+            tmem_issue16(tacc, ra);
+          } else {
+            float ssq;
+            if (TQ_ABL(batch, 512)) { ssq = 1.0f; tmem_issue16(tacc, ra); }
+            else ssq = ssq_row_fast<D>(tacc, ra, rb);
+            norm = __fsqrt_rn(ssq);
+            odd_norms = fmaf(ssq, 0.f, odd_norms);       // NaN from the first NaN (or infinite) sum on
+          }
+          const float inv = __fdiv_rn(1.0f, norm + 1e-8f) * kUnscale;
           if (valid) job.norms_out[n] = __half_as_ushort(__float2half_rn(norm));
           sc.s_inv = sc.s * inv;
           sc.h_inv = 1099511627776.0f * inv;            // 2^40: exact scaling
@@ -774,13 +855,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
               default: quant_row_fast<D, 5>(tacc, ra, rb, sc, idx_row, valid); break;
             }
           } else {
-            tmem_wait16(ra);                       // the norm sweep left a load in flight
+            tmem_wait16(ra);                       // step 0 of the sweep is in flight
             // wide launches have no plain threshold table in shared memory: the search reads the codebook block
             quant_row_search<D>(job.bits, tacc, inv, WIDE ? job.codebook + kThresholdOff : thr, idx_row, valid);
           }
-          // the norm is NaN, and with it the scale: the indices are 0 by now, the norm comes from the vector itself
-          if (__any_sync(0xffffffffu, sc.s_inv != sc.s_inv))
-            norm_from_vector<BF16, D>(batch.jobs[job.j], lt, h * kTileRows + row, sc.s_inv != sc.s_inv);
         }
       }
       tc_fence_before();
@@ -796,6 +874,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
     } else {
       if (!ok) walk_job_barriers<D>(batch, job.j, t0, i, 4, n_local, wg + 1, 128);
     }
+    if constexpr (D == 128)
+      if (odd_norms != odd_norms) norms_from_vectors<BF16, D>(batch, t0, wg, i < n_local ? i : n_local, row);
   }
   tc_fence_before();
   __syncthreads();
@@ -1122,7 +1202,8 @@ __global__ void __launch_bounds__(DCfg<ROWS, NARROW, D>::kThreadsD, 1) k_umma_de
         const uint32_t d_tmem = tmem_base + (uint32_t)(b * 128);
         const uint64_t a_base = smem_desc_sw128(a_smem + a * C::kPiecesA * kTileBytes);
         const uint64_t b_base = smem_desc_sw128(pi_smem);
-        constexpr int kPasses = ROWS ? 3 : 1;      // hi.hi [, lo.hi, hi.lo]
+        // hi.hi [, lo.hi, hi.lo]; head_dim 64: all four, lo.lo first and hi.hi last (see fp16_pieces)
+        constexpr int kPasses = D == 64 ? 4 : ROWS ? 3 : 1;
         if (!TQ_ABL(batch, 4)) {
 #pragma unroll
           for (int h = 0; h < 128 / D; ++h) {          // head_dim 64: the two operands of a tile, 64 columns each
@@ -1133,8 +1214,8 @@ __global__ void __launch_bounds__(DCfg<ROWS, NARROW, D>::kThreadsD, 1) k_umma_de
                 // descriptor = per-tile base + compile-time offset in 16-byte units
                 const uint64_t koff = (uint64_t)(((k >> 2) * kHalfBytes + (k & 3) * 32) / 16);
                 const uint64_t hoff = (uint64_t)(h * kHalfBytes / 16);
-                const uint64_t pa = (uint64_t)(((pass == 1) ? kTileBytes : 0u) / 16);
-                const uint64_t pb = (uint64_t)(((pass == 2) ? C::kPieceBytes : 0u) / 16);
+                const uint64_t pa = (uint64_t)(((D == 64 ? pass < 2 : pass == 1) ? kTileBytes : 0u) / 16);
+                const uint64_t pb = (uint64_t)(((D == 64 ? (pass & 1) == 0 && pass < 3 : pass == 2) ? C::kPieceBytes : 0u) / 16);
                 umma_f16(d_tmem + h * 64, a_base + hoff + pa + koff, b_base + pb + koff, idesc, (pass | k) != 0 ? 1u : 0u);
               }
             }
@@ -1164,9 +1245,8 @@ __global__ void __launch_bounds__(DCfg<ROWS, NARROW, D>::kThreadsD, 1) k_umma_de
       const int t = t0 + i;
       if (view_advance<D>(batch, t, job)) {
         asm volatile("bar.sync 1, 256;" ::: "memory");       // everyone is past the previous tile's look-ups
-        const float c = __ldg(job.codebook + kCentroidOff + et);
-        const __half h = __float2half_rn(c);
-        const __half l = __float2half_rn(c - __half2float(h));
+        __half h, l;
+        fp16_pieces<D>(__ldg(job.codebook + kCentroidOff + et), h, l);
         lut[et] = (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
         if constexpr (C::kWide16) {
           if (job.bits >= 5) {                  // entry `et` (fp16 bits in both halves): 32 copies, or 16 for 8-bit codes
@@ -1270,12 +1350,13 @@ __global__ void __launch_bounds__(DCfg<ROWS, NARROW, D>::kThreadsD, 1) k_umma_de
       tc_fence_after();
       const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * 128);
       if constexpr (ROWS) {
+        constexpr float kUnscale = 1.f / (kPieceScale<D> * kPieceScale<D>);       // a power of two: exact
         const int64_t off = (int64_t)bb * job.os_b + (int64_t)hh * job.os_h + s_row * job.os_s;
         auto drain = [&](auto odt, auto* out) {
           constexpr int ODT = decltype(odt)::value;
           const bool wide = (((uintptr_t)job.out | (uintptr_t)((job.os_b | job.os_h | job.os_s) * (int64_t)sizeof(*out))) & 31u) == 0;
-          drain_row<ODT, D>(tacc, nv, out + off, valid, wide);
-          if constexpr (D == 64) drain_row<ODT, D>(tacc + 64, nv2, out + off + kTileRows * job.os_s, valid2, wide);
+          drain_row<ODT, D>(tacc, nv * kUnscale, out + off, valid, wide);
+          if constexpr (D == 64) drain_row<ODT, D>(tacc + 64, nv2 * kUnscale, out + off + kTileRows * job.os_s, valid2, wide);
         };
         if (D == 128 || job.out_dtype == TQ_F32) drain(std::integral_constant<int, TQ_F32>{}, reinterpret_cast<float*>(job.out));
         else if (job.out_dtype == TQ_F16) drain(std::integral_constant<int, TQ_F16>{}, reinterpret_cast<uint16_t*>(job.out));
@@ -1328,14 +1409,15 @@ __global__ void __launch_bounds__(DCfg<ROWS, NARROW, D>::kThreadsD, 1) k_umma_de
 
 // ---------------------------------------------------------------- rotation image
 // image[piece][khalf][row n][64 cols], rows of 128 bytes, 16-byte chunk c stored at c ^ (n & 7).
-// Pieces 0-1: fp16 hi / lo (m = hi + lo, lo in fp16 subnormals).  Pieces 2-4: bf16 p0 + p1 + p2.
-__global__ void k_rotation_image(const float* __restrict__ m, int D, uint16_t* __restrict__ image) {
+// Pieces 0-1: fp16 hi / lo (see fp16_pieces; at head_dim 128 lo is an fp16 subnormal).  Pieces 2-4: bf16 p0 + p1 + p2 = m.
+template <int D>
+__global__ void k_rotation_image(const float* __restrict__ m, uint16_t* __restrict__ image) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;     // over D x D
   if (idx >= D * D) return;
   const int n = idx / D, k = idx % D;
   const float v = m[idx];
-  const __half hi = __float2half_rn(v);
-  const __half lo = __float2half_rn(v - __half2float(hi));
+  __half hi, lo;
+  fp16_pieces<D>(v, hi, lo);
   const __nv_bfloat16 p0 = __float2bfloat16_rn(v);
   const float r1 = v - __bfloat162float(p0);
   const __nv_bfloat16 p1 = __float2bfloat16_rn(r1);
@@ -1432,7 +1514,8 @@ size_t umma_rotation_image_bytes(int D) { return tc_dim(D) ? (size_t)5 * D * D *
 
 int umma_prepare_rotation_image(const float* m, int D, void* image, cudaStream_t st) {
   if (!tc_dim(D)) return TQ_EDIM;
-  k_rotation_image<<<(D * D + 255) / 256, 256, 0, st>>>(m, D, reinterpret_cast<uint16_t*>(image));
+  if (D == 64) k_rotation_image<64><<<(64 * 64 + 255) / 256, 256, 0, st>>>(m, reinterpret_cast<uint16_t*>(image));
+  else k_rotation_image<128><<<(128 * 128 + 255) / 256, 256, 0, st>>>(m, reinterpret_cast<uint16_t*>(image));
   return check_launch();
 }
 
