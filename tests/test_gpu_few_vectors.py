@@ -89,3 +89,45 @@ def test_many_jobs_of_few_vectors(jobs):
 
     for a, b in zip(run(), _simt(run)):
         assert all(torch.equal(s, t) for s, t in zip(a, b))
+
+
+def _round_trip(comp, x, room):
+    """One call over all of x and back into 16-bit rows; `room` more elements per row keep the rows off 16-byte boundaries."""
+    packed = [comp.compress_job(t) for t in x]
+    _ops.run_quantize([p[0] for p in packed], DEV)
+    outs, back = [], []
+    for t, p, r in zip(x, packed, room):
+        outs.append(torch.empty(*t.shape[:3], t.shape[3] + r, dtype=t.dtype, device=DEV)[..., r // 2:r // 2 + t.shape[3]])
+        back.append(comp.decompress_job(p[1], outs[-1]))
+    _ops.run_dequantize([b[0] for b in back], DEV)
+    return [(p[1]["idx_bytes"], p[1]["vec_norms"], o) for p, o in zip(packed, outs)]
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("slabs", [(3000,), (1500, 1500), (2999, 1), (1, 2999)])
+@pytest.mark.parametrize("odd", [None, "first", "last"])
+def test_the_limit_counts_vectors_and_not_jobs(dim, slabs, odd):
+    """3000 tokens of a slab each run here as one job or as two, alone or before or behind 900 vectors that only the FP32
+    kernels take.  The tensor-core kernels' 16-bit reconstruction would not be the FP32 kernels'."""
+    comp = tq.MSECompressor(dim, 4, seed=4, device=DEV)
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    x = [torch.randn(1, n, 1, dim, generator=gen, device=DEV).half() for n in slabs]
+    room = [0] * len(x)
+    if odd is not None:
+        at = 0 if odd == "first" else len(x)
+        x.insert(at, torch.randn(1, 60, 15, dim + 6, generator=gen, device=DEV).half()[..., 3:dim + 3])
+        room.insert(at, 6)
+    for a, b in zip(_round_trip(comp, x, room), _simt(lambda: _round_trip(comp, x, room))):
+        assert all(torch.equal(s, t) for s, t in zip(a, b))
+
+
+@pytest.mark.parametrize("jobs", [1, 2, 8])
+def test_fuller_tiles_stay_on_the_tensor_cores(jobs):
+    """Slabs of 16 tokens, 4096 vectors in all at head_dim 128: the same values as in a long call of the same tokens."""
+    comp = tq.MSECompressor(128, 4, seed=4, device=DEV)
+    long = torch.randn(1, 256, 160, 128, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV).half()
+    (idx, norms, back), = _round_trip(comp, [long], [0])
+    x = [t.contiguous() for t in long[:, :, :16].chunk(jobs, dim=1)]
+    got = _round_trip(comp, x, [0] * jobs)
+    assert torch.equal(torch.cat([g[0] for g in got], 1), idx[:, :, :16]) and torch.equal(torch.cat([g[1] for g in got], 1), norms[:, :, :16])
+    assert torch.equal(torch.cat([g[2] for g in got], 1), back[:, :, :16])

@@ -233,9 +233,19 @@ bool mostly_padding(int64_t slabs, int64_t S, int D) {
   return 8 * S <= rows * ((S + rows - 1) / rows) && slabs > 0;
 }
 
-// Most vectors of one call that come here from the tensor-core kernels: 592 CTAs of 16 vectors and 64 columns are one
-// wave of four per SM.
+// Most vectors of one call that come here from the tensor-core kernels: 512 CTAs of 16 vectors and 64 columns at head_dim
+// 128, 256 at 64, all resident at four per SM (592).
 constexpr int64_t kFewVectors = 4096;
+// Whether `n` vectors of `jobs` jobs, which take `tiles` tiles on the tensor cores, run faster here.  Time per call with new buffers,
+// host included (bf16, 4 bits, quantise), head_dim 128: 9 us here up to about 1200 vectors, a CTA per SM, then 5 + 2.7 n / 1000;
+// over there 5 + 8 tiles / 1000, at least 9.7 + 0.2 jobs (a tensor map and a rotation image each).  One job of 2000 slabs of 2
+// tokens 17 here against 25 us there, 512 of 4 12.4 each, 256 of 8 12.4 against 10.2, 128 of 16 12.4 against 9.9; 8 jobs of 32
+// slabs of 8 12.4 against 10.7, of 16 17.6 against 11.0; 64 jobs of 8 slabs of 1 14 against 21, of 8 18.7 against 21.  At head_dim 64
+// this kernel reads half as much matrix and is the faster one throughout (4000 vectors in slabs of 8: 8.9 against 12.5; in slabs
+// of 16 9 against 10).
+bool few_faster(int D, int64_t n, int64_t tiles, int jobs) {
+  return n <= kFewVectors && (D == 64 || n <= 3 * tiles || n <= 1216 + 64 * jobs);
+}
 // The same for calls that would run on the FP32 kernels, whose tiles of 32 vectors reuse the matrix more.  Quantise into
 // int64 indices, here against there: head_dim 128, 1024 vectors 8.2 against 16.4 us, 2048 10.3 against 16.4, 4096 16.4 each (rebuilt
 // 16.4 against 14.4), 8192 24.6 against 20.5; head_dim 64, 4096 vectors 8.3 against 8.8, 8192 10.4 against 11.0.
@@ -255,24 +265,38 @@ int launch_few(const Batch& b, int blocks, K0 small, K1 large, cudaStream_t st) 
 }  // namespace
 
 // ---------------------------------------------------------------- dispatch
-// True when a whole call runs here: jobs of one dtype and head_dim, at most kFewVectors vectors in all where a job could
-// run on the tensor cores (and is mostly padding in their tiles), few_fp32() where none could.  A call with other jobs among
-// them stays in one launch over there.
-bool few_quantize_eligible(const TqQuantizeJob* jobs, int n_jobs) {
+// True when a whole call runs here: jobs of one dtype and head_dim whose matrices start on 16 bytes.  Where any job could run
+// on the tensor cores: each such job is mostly padding in their tiles and the call is faster here (a job that would take a
+// launch of the FP32 kernels of its own counts a tile for each vector); where none could: at most few_fp32() vectors.  A call
+// with other jobs among them stays in one launch over there.  The order of the jobs does not matter.
+template <typename Job, typename Dtype, typename Matrix, typename Tensor>
+static bool few_eligible(const Job* jobs, int n_jobs, Dtype dtype, Matrix matrix, Tensor on_tensor_cores) {
   if (force_simt()) return false;
-  int64_t vectors = 0, most = n_jobs > 0 ? few_fp32(jobs[0].D) : 0;
+  int64_t vectors = 0, tiles = 0;
+  bool tensor = false;
   for (int k = 0; k < n_jobs; ++k) {
-    const TqQuantizeJob& j = jobs[k];
-    if ((j.D != 64 && j.D != 128) || j.x_dtype != jobs[0].x_dtype || j.D != jobs[0].D || ((uintptr_t)j.rotation_t & 15u)) return false;
+    const Job& j = jobs[k];
+    if ((j.D != 64 && j.D != 128) || dtype(j) != dtype(jobs[0]) || j.D != jobs[0].D || ((uintptr_t)matrix(j) & 15u)) return false;
     if (j.B <= 0 || j.H <= 0 || j.S <= 0 || j.H > 65535 || j.S > 65535) return false;
-    vectors += j.B * j.H * j.S;
-    if (vectors > most) return false;
-    if (umma_quantize_eligible(j)) {
-      if (!mostly_padding(j.B * j.H, j.S, j.D) || vectors > kFewVectors) return false;
-      most = kFewVectors;
+    const int64_t n = j.B * j.H * j.S;
+    vectors += n;
+    if (vectors > kFewVectors && vectors > few_fp32(j.D)) return false;
+    if (on_tensor_cores(j)) {
+      if (!mostly_padding(j.B * j.H, j.S, j.D)) return false;
+      tensor = true;
+      const int64_t rows = 16384 / j.D;
+      tiles += j.B * j.H * ((j.S + rows - 1) / rows);
+    } else {
+      tiles += n;
     }
   }
-  return true;
+  if (n_jobs == 0) return false;
+  return tensor ? few_faster(jobs[0].D, vectors, tiles, n_jobs) : vectors <= few_fp32(jobs[0].D);
+}
+
+bool few_quantize_eligible(const TqQuantizeJob* jobs, int n_jobs) {
+  return few_eligible(jobs, n_jobs, [](const TqQuantizeJob& j) { return j.x_dtype; },
+                      [](const TqQuantizeJob& j) { return j.rotation_t; }, umma_quantize_eligible);
 }
 
 int few_quantize(const TqQuantizeJob* jobs, int n_jobs, cudaStream_t st) {
@@ -301,20 +325,8 @@ int few_quantize(const TqQuantizeJob* jobs, int n_jobs, cudaStream_t st) {
 }
 
 bool few_dequantize_eligible(const TqDequantizeJob* jobs, int n_jobs) {
-  if (force_simt()) return false;
-  int64_t vectors = 0, most = n_jobs > 0 ? few_fp32(jobs[0].D) : 0;
-  for (int k = 0; k < n_jobs; ++k) {
-    const TqDequantizeJob& j = jobs[k];
-    if ((j.D != 64 && j.D != 128) || j.out_dtype != jobs[0].out_dtype || j.D != jobs[0].D || ((uintptr_t)j.rotation & 15u)) return false;
-    if (j.B <= 0 || j.H <= 0 || j.S <= 0 || j.H > 65535 || j.S > 65535) return false;
-    vectors += j.B * j.H * j.S;
-    if (vectors > most) return false;
-    if (umma_dequantize_eligible(j)) {
-      if (!mostly_padding(j.B * j.H, j.S, j.D) || vectors > kFewVectors) return false;
-      most = kFewVectors;
-    }
-  }
-  return true;
+  return few_eligible(jobs, n_jobs, [](const TqDequantizeJob& j) { return j.out_dtype; },
+                      [](const TqDequantizeJob& j) { return j.rotation; }, umma_dequantize_eligible);
 }
 
 int few_dequantize(const TqDequantizeJob* jobs, int n_jobs, cudaStream_t st) {
