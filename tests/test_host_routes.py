@@ -10,7 +10,6 @@ import torch
 
 import turboquant as tq
 from turboquant import _native as N
-from turboquant import _ops
 from turboquant import cache
 
 pytestmark = pytest.mark.filterwarnings("ignore::RuntimeWarning")
@@ -25,70 +24,6 @@ class _OnCuda:
 
     def __getitem__(self, _index):
         return self
-
-
-@pytest.fixture
-def host(monkeypatch):
-    calls = []
-
-    def record(name):
-        return lambda *args: calls.append(name) or name
-    fake = types.SimpleNamespace(**{n: record(n) for n in ("compress", "decompress", "compress_kv", "decompress_kv")})
-    monkeypatch.setattr(N, "host", lambda: fake)
-    monkeypatch.setattr(_ops, "run_quantize", lambda jobs, device: None)
-    monkeypatch.setattr(_ops, "run_dequantize", lambda jobs, device: None)
-    real_empty = torch.empty
-    monkeypatch.setattr(torch, "empty", lambda *a, **kw: real_empty(*a, **dict(kw, device="cpu")))
-    return calls
-
-
-class _OwnJobs(tq.MSECompressor):
-    def compress_job(self, states):
-        return None, "mine", None
-
-    def decompress_job(self, compressed, out):
-        out.fill_(7)
-        return None, None
-
-
-class _OwnLayerJobs(tq.TurboQuantV3):
-    def compress_jobs(self, keys, values):
-        return [], ("mine", "mine"), ()
-
-    def decompress_jobs(self, compressed_k, compressed_v):
-        return [], (types.SimpleNamespace(device="cpu"),), ()
-
-
-X = _OnCuda(1, 2, 10, 16)
-PACKED = {"idx_bytes": _OnCuda(1, 2, 10, 8), "vec_norms": _OnCuda(1, 2, 10), "shape": (1, 2, 10, 16)}
-SIDE = {"compressed": PACKED, "fp16": _OnCuda(1, 2, 0, 16), "shape": (1, 2, 10, 16), "split_at": 10}
-
-
-def test_plain_codecs_go_to_the_native_path(host):
-    codec = tq.TurboQuantV3(16, residual_window=0)
-    assert codec.key_compressor.compress(X) == "compress" and codec.key_compressor.decompress(PACKED) == "decompress"
-    assert codec.compress_kv(X, X) == "compress_kv" and codec.decompress_kv(SIDE, SIDE) == "decompress_kv"
-
-
-def test_a_subclass_that_overrides_its_jobs_is_asked(host):
-    comp = _OwnJobs(16, 4, seed=1)
-    assert comp.compress(X) == "mine" and bool((comp.decompress(PACKED) == 7).all())
-    codec = _OwnLayerJobs(16, residual_window=0)
-    assert codec.compress_kv(X, X) == ("mine", "mine") and codec.decompress_kv(SIDE, SIDE)[0].device == "cpu"
-    assert host == []
-
-
-@pytest.mark.parametrize("side", ["key_compressor", "val_compressor"])
-def test_a_layer_with_such_a_codec_asks_it(host, side):
-    codec = tq.TurboQuantV3(16, residual_window=0)
-    setattr(codec, side, _OwnJobs(16, 4, seed=1))
-    other = codec.val_compressor if side == "key_compressor" else codec.key_compressor
-    other.compress_job = lambda states: (None, "replaced on the object", None)
-    other.decompress_job = lambda compressed, out: (None, None)
-    results = codec.compress_kv(X, X)
-    assert sorted(r["compressed"] for r in results) == ["mine", "replaced on the object"]
-    codec.decompress_kv(SIDE, SIDE)
-    assert host == []
 
 
 @pytest.fixture

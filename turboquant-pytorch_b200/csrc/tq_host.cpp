@@ -30,6 +30,8 @@ struct Api {
   decltype(&tq_qjl_compress_workspace_bytes) qjl_compress_ws = nullptr;
   decltype(&tq_prod_inner_product) prod_inner = nullptr;
   PyObject* check = nullptr;               // Python: check(rc, what) raises for rc != 0
+  // the classes' own job methods, as functions: MSECompressor.compress_job, decompress_job, TurboQuantV3.compress_jobs, decompress_jobs
+  PyObject* jobs = nullptr;
 } api;
 
 // ---------------------------------------------------------------- small helpers
@@ -95,6 +97,15 @@ bool read_codec(PyObject* o, int dev, Codec* c) {
   return attr_int(o, n_bits, &c->bits) && c->bits >= 1 && c->bits <= 8 && attr_int(o, n_dim, &c->dim) && c->dim >= 1 && c->dim <= 256 &&
          attr_ptr(o, n_pi, dev, &c->pi) == 1 && attr_ptr(o, n_pit, dev, &c->pi_t) == 1 && attr_ptr(o, n_cb, dev, &c->cb) == 1 &&
          attr_ptr(o, n_iq, dev, &c->img_q) >= 0 && attr_ptr(o, n_id, dev, &c->img_d) >= 0;
+}
+// `method` is number `i` of the classes' own job methods, bound.  What this file does stands in for them; a method that a
+// subclass, an object or a patch has put in their place is asked instead.
+bool own_method(PyObject* method, int i) { return PyMethod_Check(method) && PyMethod_GET_FUNCTION(method) == PyTuple_GET_ITEM(api.jobs, i); }
+bool own_codec(PyObject* codec, bool compress) {
+  TQ_NAME(n_c, "compress_job"); TQ_NAME(n_d, "decompress_job");
+  Ref m(PyObject_GetAttr(codec, compress ? n_c : n_d));
+  if (!m) { PyErr_Clear(); return false; }
+  return own_method(m.p, compress ? 0 : 1);
 }
 int64_t row_bytes(int64_t dim, int64_t bits) { const int64_t ipb = 8 / bits; return (dim + ipb - 1) / ipb; }
 
@@ -191,11 +202,13 @@ bool dequantize_job(PyObject* dict, const Codec& c, int dev, const int64_t (&sha
 }
 
 // ---------------------------------------------------------------- one layer's K and V
-// compress_kv(key_codec, value_codec, keys, values, window) -> (dict, dict) | None
+// compress_kv(key_codec, value_codec, keys, values, window, the layer's compress_jobs) -> (dict, dict) | None
 PyObject* compress_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const int dev = c10::cuda::current_device();
-  if (n != 5 || !float_plain(a[2], dev) || !float_plain(a[3], dev) || !PyLong_Check(a[4])) return none();
+  if (n != 6 || !float_plain(a[2], dev) || !float_plain(a[3], dev) || !PyLong_Check(a[4]) || !own_method(a[5], 2) || !own_codec(a[0], true) ||
+      !own_codec(a[1], true))
+    return none();
   const at::Tensor &k = THPVariable_Unpack(a[2]), &v = THPVariable_Unpack(a[3]);
   const int64_t window = PyLong_AsLongLong(a[4]);
   Codec ck, cv;
@@ -233,12 +246,12 @@ bool copy_fits(const at::Tensor& t, int64_t eb) {
   return t.stride(3) == 1 && t.size(3) * eb % 16 == 0;
 }
 
-// decompress_kv(key_codec, value_codec, compressed_k, compressed_v) -> (keys, values) | None
+// decompress_kv(key_codec, value_codec, compressed_k, compressed_v, the layer's decompress_jobs) -> (keys, values) | None
 PyObject* decompress_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TQ_NAME(k_comp, "compressed"); TQ_NAME(k_fp16, "fp16"); TQ_NAME(k_split, "split_at");
   const int dev = c10::cuda::current_device();
-  if (n != 4) return none();
+  if (n != 5 || !own_method(a[4], 3) || !own_codec(a[0], false) || !own_codec(a[1], false)) return none();
   c10::AutoGradMode no_grad(false);
   TqDequantizeJob jobs[2];
   TqCopyJob copies[2];
@@ -294,7 +307,7 @@ PyObject* compress(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const int dev = c10::cuda::current_device();
   Codec c;
-  if (n != 2 || !float_plain(a[1], dev) || !read_codec(a[0], dev, &c)) return none();
+  if (n != 2 || !float_plain(a[1], dev) || !own_codec(a[0], true) || !read_codec(a[0], dev, &c)) return none();
   const at::Tensor& x = THPVariable_Unpack(a[1]);
   if (!quantisable(x, c)) return none();
   c10::AutoGradMode no_grad(false);
@@ -312,7 +325,7 @@ PyObject* decompress(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int dev = c10::cuda::current_device();
   Codec c;
   int64_t shape[4];
-  if (n != 2 || !PyDict_CheckExact(a[1]) || !read_codec(a[0], dev, &c) || !read_shape(a[1], shape)) return none();
+  if (n != 2 || !PyDict_CheckExact(a[1]) || !own_codec(a[0], false) || !read_codec(a[0], dev, &c) || !read_shape(a[1], shape)) return none();
   for (int64_t s : shape)
     if (s < 0) return none();
   c10::AutoGradMode no_grad(false);
@@ -623,10 +636,13 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(addresses of the six C functions in the order of Api, check)
+// bind(addresses of the six C functions in the order of Api, check, the four job methods)
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   void* p[6];
-  if (n != 7) { PyErr_SetString(PyExc_TypeError, "bind takes six addresses and a function"); return nullptr; }
+  if (n != 8 || !PyTuple_Check(a[7]) || PyTuple_GET_SIZE(a[7]) != 4) {
+    PyErr_SetString(PyExc_TypeError, "bind takes six addresses, a function and a tuple of four");
+    return nullptr;
+  }
   for (int i = 0; i < 6; ++i) {
     p[i] = PyLong_AsVoidPtr(a[i]);
     if (p[i] == nullptr) { if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address"); return nullptr; }
@@ -637,6 +653,9 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Py_INCREF(a[6]);
   Py_XDECREF(api.check);
   api.check = a[6];
+  Py_INCREF(a[7]);
+  Py_XDECREF(api.jobs);
+  api.jobs = a[7];
   Py_RETURN_NONE;
 }
 

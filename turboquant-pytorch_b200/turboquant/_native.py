@@ -158,6 +158,8 @@ def lib():
 
 
 _host = None
+# the codecs' own job methods, which the host extension stands in for (compressors_v3.py sets them)
+JOB_METHODS: tuple = ()
 
 
 class _GeneralPath:
@@ -199,7 +201,7 @@ def host():
         else:
             H.bind(*(C.cast(getattr(L, n), C.c_void_p).value for n in
                      ("tq_quantize", "tq_dequantize", "tq_copy_rows", "tq_qjl_compress", "tq_qjl_compress_workspace_bytes",
-                      "tq_prod_inner_product")), check)
+                      "tq_prod_inner_product")), check, JOB_METHODS)
         _host = H
     return _host
 

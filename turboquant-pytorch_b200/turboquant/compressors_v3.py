@@ -20,12 +20,6 @@ from .lloyd_max import LloydMaxCodebook
 from .turboquant import generate_rotation_matrix
 
 
-def _own(method, function) -> bool:
-    """True when `method` is this module's own `function`, bound.  The native host path fills in the jobs itself, so it
-    stands in only for codecs whose job methods nobody has replaced, in a subclass or on the object."""
-    return getattr(method, "__func__", None) is function
-
-
 class MSECompressor:
     """L2-normalise, rotate, Lloyd-Max quantise, bit-pack; keeps fp16 norms."""
 
@@ -64,7 +58,7 @@ class MSECompressor:
 
     def compress(self, states: torch.Tensor) -> dict:
         """(B, H, S, D) -> {"idx_bytes" uint8 (B,H,S,G), "vec_norms" fp16 (B,H,S), "shape", "idx_pad"}."""
-        if states.is_cuda and _own(self.compress_job, MSECompressor.compress_job):
+        if states.is_cuda:
             result = N.host().compress(self, states)
             if result is not None:
                 return result
@@ -78,7 +72,7 @@ class MSECompressor:
 
     def decompress(self, compressed: dict) -> torch.Tensor:
         """Back to an fp32 (B, H, S, D) tensor."""
-        if compressed["idx_bytes"].is_cuda and _own(self.decompress_job, MSECompressor.decompress_job):
+        if compressed["idx_bytes"].is_cuda:
             out = N.host().decompress(self, compressed)
             if out is not None:
                 return out
@@ -146,10 +140,9 @@ class TurboQuantV3:
         return [jk, jv], (ck, cv), (keep_k, keep_v)
 
     def compress_kv(self, keys: torch.Tensor, values: torch.Tensor):
-        if keys.is_cuda and _own(self.compress_jobs, TurboQuantV3.compress_jobs) and \
-                _own(self.key_compressor.compress_job, MSECompressor.compress_job) and \
-                _own(self.val_compressor.compress_job, MSECompressor.compress_job):
-            result = N.host().compress_kv(self.key_compressor, self.val_compressor, keys, values, self.residual_window)
+        if keys.is_cuda:
+            result = N.host().compress_kv(self.key_compressor, self.val_compressor, keys, values, self.residual_window,
+                                          self.compress_jobs)
             if result is not None:
                 return result
         return self._compress_kv_general(keys, values)
@@ -180,10 +173,9 @@ class TurboQuantV3:
     def decompress_kv(self, compressed_k: dict, compressed_v: dict):
         if compressed_k["compressed"] is None:
             return compressed_k["fp16"], compressed_v["fp16"]
-        if compressed_k["fp16"].is_cuda and _own(self.decompress_jobs, TurboQuantV3.decompress_jobs) and \
-                _own(self.key_compressor.decompress_job, MSECompressor.decompress_job) and \
-                _own(self.val_compressor.decompress_job, MSECompressor.decompress_job):
-            result = N.host().decompress_kv(self.key_compressor, self.val_compressor, compressed_k, compressed_v)
+        if compressed_k["fp16"].is_cuda:
+            result = N.host().decompress_kv(self.key_compressor, self.val_compressor, compressed_k, compressed_v,
+                                            self.decompress_jobs)
             if result is not None:
                 return result
         return self._decompress_kv_general(compressed_k, compressed_v)
@@ -225,3 +217,7 @@ class TurboQuantV3:
                 "compression_ratio": dense / total if total > 0 else 0,
                 "compressed_tokens": packed_tokens, "fp16_tokens": window,
                 "key_bits": self.key_bits, "value_bits": self.value_bits}
+
+
+N.JOB_METHODS = (MSECompressor.compress_job, MSECompressor.decompress_job, TurboQuantV3.compress_jobs,
+                 TurboQuantV3.decompress_jobs)
