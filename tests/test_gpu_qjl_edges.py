@@ -1,5 +1,6 @@
 """MSE + QJL kernels: buffers that start off a 32-byte boundary, and query counts around the operand's blocks."""
 
+import ctypes as C
 import math
 
 import pytest
@@ -89,3 +90,79 @@ def test_one_query_needs_scratch_for_one_query():
                                        prod._s_t.data_ptr(), out.data_ptr(), ws.data_ptr(), n_bytes, N.stream_ptr(DEV))
     assert call(1, 2048) == 0 and torch.equal(out, want) and bool((ws[2048:] == 0xA5).all())
     assert call(1, 2044) == -8 and call(500, 500 * 2048 - 4) == -8
+
+
+def _guarded(n_bytes, off):
+    """n_bytes on the device that start `off` bytes past a 32-byte boundary, and the buffer around them."""
+    raw = torch.full((n_bytes + 128,), 0xA5, dtype=torch.uint8, device=DEV)
+    start = 32 + (-raw.data_ptr()) % 32 + off
+    return raw, start, raw[start:start + n_bytes]
+
+
+@pytest.mark.parametrize("d", [128, 256])
+@pytest.mark.parametrize("rows", [1, 127, 300])
+def test_qjl_outputs_off_a_32_byte_boundary(d, rows):
+    """k_mse and the signs may start on an odd multiple of 16 bytes: rows then leave as two 16-byte stores."""
+    comp = tq.TurboQuantCompressorV2(d, 3, seed=9, device=DEV)
+    x = O.synthetic_kv((1, 1, rows, d), torch.float16, seed=rows).to(DEV)
+    L = N.lib()
+    n_ws = L.tq_qjl_compress_workspace_bytes(rows, d)
+    results = []
+    for off in (0, 16):
+        ws = torch.empty(n_ws, dtype=torch.uint8, device=DEV)
+        raw_k, at_k, k = _guarded(rows * d * 2, off)
+        raw_s, at_s, s = _guarded(rows * d, off)
+        rnorm = torch.empty(rows, dtype=torch.float16, device=DEV)
+        assert k.data_ptr() % 32 == off and s.data_ptr() % 32 == off
+        job = N.QjlCompressJob(x=x.data_ptr(), x_dtype=N.F16, D=d, bits=comp.mse_bits, normalize=1, B=1, H=1, S=rows,
+                               stride_b=rows * d, stride_h=rows * d, stride_s=d, rotation_t=comp.PiT.data_ptr(),
+                               rotation=comp.Pi.data_ptr(), codebook=comp._cb.data_ptr(), qjl_t=comp._s_t.data_ptr(), M=d,
+                               signs_dtype=0, rnorm_dtype=N.F16, idx_mode=N.IDX_U8, k_mse_out=k.data_ptr(), idx_out=None,
+                               signs_out=s.data_ptr(), rnorm_out=rnorm.data_ptr(), workspace=ws.data_ptr(), workspace_bytes=n_ws,
+                               vec_norms_out=None)
+        N.check(L.tq_qjl_compress(C.byref(job), N.stream_ptr(DEV)), "tq_qjl_compress")
+        for raw, at, out in ((raw_k, at_k, k), (raw_s, at_s, s)):
+            assert bool((raw[:at] == 0xA5).all()) and bool((raw[at + out.numel():] == 0xA5).all())
+        results.append((k.clone(), s.clone(), rnorm))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    want = comp.compress(x)
+    assert torch.equal(results[0][0].view(torch.float16).view(1, 1, rows, d), want["k_mse"])
+    assert torch.equal(results[0][1].view(torch.int8).view(1, 1, rows, d), want["qjl_signs"])
+
+
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("sq", [4, 40])
+def test_back_to_back_mse_qjl_calls_and_capture(packed, sq):
+    """Compress and scores launch their kernels as programmatic chains: calls in a row on one stream share scratch from the
+    caching allocator, and a captured call replays the same."""
+    comp = tq.TurboQuantCompressorV2(128, 3, seed=9, device=DEV)
+    keys = [O.synthetic_kv((1, 2, 500, 128), torch.float16, seed=s).to(DEV) for s in range(20)]
+    q = torch.randn(1, 2, sq, 128, generator=_gen(1), device=DEV).half()
+
+    def both(x):
+        c = comp.compress(x, packed=packed)
+        return [v for v in c.values() if torch.is_tensor(v)] + [comp.asymmetric_attention_scores(q, c)]
+
+    alone = []
+    for x in keys:
+        alone.append([t.clone() for t in both(x)])
+        torch.cuda.synchronize()
+    row = [both(x) for x in keys]
+    torch.cuda.synchronize()
+    for a, b in zip(alone, row):
+        assert all(torch.equal(s, t) for s, t in zip(a, b))
+    static = keys[0].clone()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        both(static)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = both(static)
+    for x, a in zip(keys[:5], alone):
+        static.copy_(x)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(s, t) for s, t in zip(a, out))
+    assert N.lib().tq_last_device_status() == 0

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads + (STAGE == 2 ? kExpandThrea
   float* thr_s = reinterpret_cast<float*>(gbase + C::kOffTab);
   uint32_t* lut_s = reinterpret_cast<uint32_t*>(gbase + C::kOffTab + 1024);
   uint8_t* cells_s = gbase + C::kOffTab + 2048;                        // 1028 bytes
-  float* part_s = reinterpret_cast<float*>(gbase + C::kOffTab + 4096); // [slot 2][row 128] partial sums of the upper block
+  float* part_s = reinterpret_cast<float*>(gbase + C::kOffTab + 4096); // [slot 2][block 2][row 128] partial sums of the residual norms
   const uint32_t bar0 = base + C::kOffBar;
   const uint32_t bar_afull = bar0;                          // [kASlots] TMA -> MMA (all pieces of a k-chunk)
   const uint32_t bar_aempty = bar_afull + 8 * 4;            // [kASlots] MMA commit -> producer
