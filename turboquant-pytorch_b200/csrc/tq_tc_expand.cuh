@@ -1,4 +1,5 @@
-// Packed indices -> fp16 centroid pieces in the swizzled K-major operand layout (head_dim 128).
+// Packed indices -> fp16 centroid pieces in the swizzled K-major operand layout (head_dim 128; at head_dim 64 a "half row" is
+// a whole row and the two halves are the vectors r and r + 128 of a tile).
 // Included inside namespace tq { namespace { ... } } after tq_tc_ptx.cuh; expects
 // kDim = 128, kTileBytes = 32768 and kHalfBytes = 16384 to be defined by the including file.
 #pragma once
@@ -17,6 +18,8 @@
 // packed tile and write eight different 16-byte positions of the swizzled operand rows, so the packed
 // loads and the operand stores both run without bank conflicts.  (With lanes = consecutive rows of
 // one half, the 128-byte rows of one-byte codes put all eight lanes on the same four banks.)
+// At head_dim 64 the rows are half as far apart and the halves of a row 128 rows: the stores and the loads of 3- and 4-bit
+// codes are free of conflicts there too, the loads of 2-bit and of one-byte codes meet two by two.
 template <int BITS>
 __device__ __forceinline__ uint32_t expand_order(int row, int half) {
   constexpr int HB = kDim / (8 / BITS) / 2;     // packed bytes per half row
