@@ -478,14 +478,17 @@ __device__ __forceinline__ void quant_row_cells(uint32_t tacc, uint32_t (&a)[16]
   }
 }
 
-// Norms that came out NaN, once more from the vectors' own coordinates: of vector `row` in every fourth of the CTA's tiles from
-// `first` on, up to tile `end`.  The rotated row of a vector with an infinity is NaN (the pieces of Pi meet it with both signs)
-// while its norm is infinite, as the FP32 kernels have it.  Out of line and after the last tile: a look at every tile's
-// norms in the loop, with the call behind it, cost 2 % of a launch.
+// Norms that came out NaN, once more from the vectors' own coordinates, by the threads that wrote them.  The rotated row of a
+// vector with an infinity is NaN (the pieces of Pi meet it with both signs) while its norm is infinite, as the FP32 kernels
+// have it.  Out of line, after everything else, and with nothing but the batch for an argument: what the epilogue keeps alive for
+// such a call shows in its loop (K6/V4 and 8-bit layers of 32768 tokens: quantise 1609 us with the call behind the loop and its
+// position passed on, 1584 without any, 1580 so).
 template <bool BF16, int D, int J>
-__device__ __noinline__ void norms_from_vectors(const UmmaQuantBatchOf<J>& batch, int t0, int first, int end, int row) {
+__device__ __noinline__ void norms_from_vectors(const UmmaQuantBatchOf<J>& batch) {
   QuantJobView v;
-  for (int i = first; i < end; i += 4) {
+  const int t0 = batch.cta_begin[blockIdx.x], end = batch.cta_begin[blockIdx.x + 1] - t0;
+  const int warp = threadIdx.x >> 5, row = (warp & 3) * 32 + (threadIdx.x & 31);     // as in the epilogue
+  for (int i = (warp - 2) >> 2; i < end; i += 4) {
     view_advance<D>(batch, t0 + i, v);
     const UmmaQuantJob& job = batch.jobs[v.j];
     const int lt = t0 + i - v.begin;
@@ -579,6 +582,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
   const uint32_t bar_pifree = bar_pifull + 8;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + kOffBar + 200);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + kOffBar + 208);
+  volatile int* odd_norms = reinterpret_cast<volatile int*>(gbase + kOffBar + 212);      // a norm came out NaN
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t0 = batch.cta_begin[blockIdx.x];
@@ -590,6 +594,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
     for (int i = 0; i < kAccBufs; ++i) { mbar_init(bar_tfull + 8 * i, 1); mbar_init(bar_tempty + 8 * i, 4); }
     mbar_init(bar_pifull, 1);
     mbar_init(bar_pifree, 1);
+    *odd_norms = 0;
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -725,7 +730,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
     int mode = 0;                               // 0 search, 1 cubic shortcut, 2 cell table
     bool ok = true;
     bool fast = false, fast_lds = false, linear = false;
-    float odd_norms = 0.f;
     Shortcut sc = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     QuantJobView job;
     // Wide launches keep ONE set of tables per CTA.  Every epilogue warp walks the CTA's jobs in order,
@@ -822,7 +826,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
             if (TQ_ABL(batch, 512)) { ssq = 1.0f; tmem_issue16(tacc, ra); }
             else ssq = ssq_row_fast<D>(tacc, ra, rb);
             norm = __fsqrt_rn(ssq);
-            odd_norms = fmaf(ssq, 0.f, odd_norms);       // NaN from the first NaN (or infinite) sum on
+            if (norm != norm) *odd_norms = 1;
           }
           const float inv = __fdiv_rn(1.0f, norm + 1e-8f) * kUnscale;
           if (valid) job.norms_out[n] = __half_as_ushort(__float2half_rn(norm));
@@ -874,8 +878,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
     } else {
       if (!ok) walk_job_barriers<D>(batch, job.j, t0, i, 4, n_local, wg + 1, 128);
     }
-    if constexpr (D == 128)
-      if (odd_norms != odd_norms) norms_from_vectors<BF16, D>(batch, t0, wg, i < n_local ? i : n_local, row);
   }
   tc_fence_before();
   __syncthreads();
@@ -883,6 +885,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_quantize(const __grid_cons
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  if constexpr (D == 128)
+    if (warp >= 2 && *odd_norms) norms_from_vectors<BF16, D>(batch);
 }
 
 // ---------------------------------------------------------------- dequantize
