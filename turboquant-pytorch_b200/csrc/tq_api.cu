@@ -405,7 +405,7 @@ int tq_project(const void* x, int x_dtype, int64_t n, int K, const float* m, int
 
 size_t tq_score_workspace_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int D) {
   if (B < 0 || Hq < 0 || Sq < 0 || Sk < 0 || D < 1) return 0;
-  return tq::simt_score_workspace(B, Hq, Sq, Sk, D);
+  return tq::score_workspace_wanted(B, Hq, Sq, Sk, D);
 }
 
 int tq_score_packed(const TqScoreJob* job, void* stream) {

@@ -4,21 +4,21 @@
 // coordinates.  The FP32 kernel (tq_simt.cu) spends ~1 400 instructions per key on it; here the
 // multiply-adds run as mma.sync.m16n8k16 (fp16 inputs, fp32 accumulate) and only the centroid look-ups
 // stay on the CUDA cores:
-//   * M = 16 rows = 16 keys, K = 16 coordinates per instruction (8 k-steps per key), N = 8 columns = up to
-//     4 query rows (the query heads that share the KV head x query tokens) as fp16 pieces: columns 0..3
-//     hold q_hi, columns 4..7 q_lo;
+//   * M = 16 rows = 8 keys x the fp16 pieces hi and lo of their centroids (key gid's pieces are rows gid and gid + 8, which
+//     the same lanes hold), K = 16 coordinates per instruction (8 k-steps per key), N = 8 columns = up to 4 query rows (the
+//     query heads that share the KV head x query tokens) as fp16 pieces: columns 0..3 hold q_hi, columns 4..7 q_lo;
 //   * the key operand is assembled IN REGISTERS: thread (gid = lane / 4, t = lane % 4) reads quarter t of
-//     the packed rows of keys gid and gid + 8 (one 4..32-byte load each) and looks up the centroids each
-//     k-step needs in a shared table of (hi | lo << 16) fp16 pieces.  A dot product does not care in which
+//     the packed rows of its keys (one 4..32-byte load each) and looks up the centroids each
+//     k-step needs in a shared table.  A dot product does not care in which
 //     order its terms are visited, so the coordinates are assigned to k-steps in the order that makes a
 //     thread's operand elements come from its own contiguous bytes: k-step ks, thread t covers coordinates
 //     32 t + 4 ks + 0..3 (the query operand uses the same order);
-//   * a table entry (hi | lo << 16) IS an operand register: a register holds two neighbouring k, and these two are
-//     the pieces of ONE coordinate, with the query value of that coordinate in both of the other operand's places.
-//     Packing the high pieces of two coordinates into one register and the low pieces into another took a byte
-//     permute per coordinate and gave the same number of MMAs;
-//   * column g collects (c_hi + c_lo).q_hi, column g + 4 collects (c_hi + c_lo).q_lo; their sum is the fp32-accurate
-//     logit (all four cross terms), one shuffle away.
+//   * a look-up of one packed byte returns the high pieces of two neighbouring coordinates in one word and their low pieces in the
+//     next: two operand registers in a row (rows gid and gid + 8), as the instruction wants them.  With the pieces of ONE
+//     coordinate as the neighbouring k of a register, and 16 keys as the rows, the registers of an operand came from two
+//     look-ups each and took a move per coordinate (80 of the 311 instructions per 16 keys);
+//   * rows gid and gid + 8 of column g add up to (c_hi + c_lo).q_hi, of column g + 4 to (c_hi + c_lo).q_lo; their sum is the
+//     fp32-accurate logit (all four cross terms), one shuffle away.
 // The softmax partials per block of keys and the finishing pass are those of the FP32 path.
 
 #include <atomic>
@@ -85,53 +85,98 @@ __device__ __forceinline__ void load_quarter(const uint8_t* row, int t, uint32_t
   }
 }
 
-__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
-  uint32_t v;
-  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-
-// Shared-memory addresses of the table entries of one packed word's coordinates.  The table is 1024-byte
-// aligned; for codes of up to 6 bits an entry's offset (index * 4) fits one byte, so the fields of a word are
-// moved to byte position with one shift and mask per field position (shared by the word's four bytes) and
-// each address is then ONE byte permute that drops the offset byte into the table's base address.
+// Table of a packed BYTE: row v (128 bytes) holds what a byte of value v stands for, once per lane that reads in the same
+// shared-memory wavefront: 32 copies of one coordinate (5 to 8 bits), 16 of two (3 and 4 bits), 8 of four (2 bits), 4 of
+// eight (1 bit).  A look-up is then one load of 4, 8 or 16 bytes that never meets another lane's in a bank, and its address a
+// shift, a mask and the lane's own offset.  With one 4-byte entry per coordinate, stored once, a coordinate cost a byte permute
+// and a load of its own, and 64 or more entries collided in the banks (131072 keys x 8 heads, four query rows, with projection
+// and softmax: 4 bits 59 -> 49 us, 8 bits 86 -> 56 us).
+// PAIRS: the words of a row are {hi0 | hi1 << 16, lo0 | lo1 << 16} for every two coordinates; otherwise, and for codes of one
+// coordinate a byte, hi | lo << 16 for each.
 template <int BITS>
-struct WordAddr {
+struct ByteTable {
   static constexpr int IPB = Packed<BITS>::IPB;
-  static constexpr bool kFast = BITS <= 6;
-  uint32_t f[IPB];                              // field position p of every byte, as offset bytes (fast path)
-  uint32_t x, base;
-  __device__ __forceinline__ WordAddr(uint32_t word, uint32_t lut_base) : x(word), base(lut_base) {
-    if constexpr (kFast) {
-      constexpr uint32_t M = (((1u << BITS) - 1u) << 2) * 0x01010101u;
-#pragma unroll
-      for (int p = 0; p < IPB; ++p) {
-        const int sh = BITS * (IPB - 1 - p);    // field p sits sh bits up in its byte (first index in the high bits)
-        f[p] = sh >= 2 ? ((word >> (sh - 2)) & M) : ((word << (2 - sh)) & M);
-      }
-    }
-  }
-  // address of the entry of coordinate c (0 .. 4 * IPB - 1) of this word
-  __device__ __forceinline__ uint32_t operator()(int c) const {
-    const int byte = c / IPB, p = c % IPB;
-    if constexpr (kFast) {
-      return __byte_perm(f[p], base, 0x7650u | (uint32_t)byte);
-    } else {
-      constexpr uint32_t MASK = ((1u << BITS) - 1u) << 2;
-      const int sh = 8 * byte;
-      return base + (sh >= 2 ? ((x >> (sh - 2)) & MASK) : ((x << (2 - sh)) & MASK));
-    }
-  }
+  static constexpr int kEntries = 1 << (BITS * IPB);       // 3 bits: 64, the fields that a byte can hold
+  static constexpr uint32_t kEntryBytes = 4 * IPB;
+  static constexpr uint32_t kLanes = 128 / kEntryBytes;    // copies
+  static constexpr uint32_t kBytes = 128 * kEntries;
+  static constexpr uint32_t kMask = (uint32_t)(kEntries - 1) << 7;
+  __device__ __forceinline__ static uint32_t lane_offset(int lane) { return ((uint32_t)lane % kLanes) * kEntryBytes; }
 };
 
-// table entries (hi | lo << 16) of the thread's local coordinates 4 ks .. 4 ks + 3
-template <int BITS>
-__device__ __forceinline__ void key_entries(const uint32_t (&w)[Packed<BITS>::CW], int ks, uint32_t lut_base, uint32_t (&e)[4]) {
-  constexpr int CPW = 4 * Packed<BITS>::IPB;    // coordinates per word: 4 (wide codes) .. 32 (1 bit)
-  const int u0 = 4 * ks;
-  const WordAddr<BITS> wa(w[u0 / CPW], lut_base);
+// all threads of the CTA, kThreads >= kEntries; the caller synchronises
+template <int BITS, bool PAIRS>
+__device__ __forceinline__ void build_table(uint8_t* table, const float* codebook) {
+  using T = ByteTable<BITS>;
+  const int v = threadIdx.x;
+  if (v >= T::kEntries) return;
+  uint32_t e[T::IPB];
 #pragma unroll
-  for (int p = 0; p < 4; ++p) e[p] = lds_u32(wa((u0 + p) % CPW));
+  for (int p = 0; p < T::IPB; ++p) {                       // field p, the first index in the high bits
+    const float c = __ldg(codebook + kCentroidOff + ((v >> (BITS * (T::IPB - 1 - p))) & ((1 << BITS) - 1)));
+    const __half h = __float2half_rn(c);
+    e[p] = (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(__float2half_rn(c - __half2float(h))) << 16);
+  }
+  if constexpr (PAIRS && T::IPB > 1) {
+#pragma unroll
+    for (int p = 0; p < T::IPB; p += 2) {
+      const uint32_t hi = __byte_perm(e[p], e[p + 1], 0x5410), lo = __byte_perm(e[p], e[p + 1], 0x7632);
+      e[p] = hi; e[p + 1] = lo;
+    }
+  }
+  uint4* row = reinterpret_cast<uint4*>(table + 128 * v);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {                            // rotated: the stores of a warp spread over the banks
+    const int j = (k + v) & 7;
+    if constexpr (T::IPB == 8) row[j] = (j & 1) ? make_uint4(e[4], e[5], e[6], e[7]) : make_uint4(e[0], e[1], e[2], e[3]);
+    else row[j] = make_uint4(e[0], e[1 % T::IPB], e[2 % T::IPB], e[3 % T::IPB]);
+  }
+}
+
+// table words of the thread's local coordinates 4 ks .. 4 ks + 3, whose packed bytes are consecutive in w; `lane_off` from
+// ByteTable::lane_offset
+template <int BITS, int W>
+__device__ __forceinline__ void entries4(const uint32_t (&w)[W], int ks, const uint8_t* table, uint32_t lane_off, uint32_t (&e)[4]) {
+  using T = ByteTable<BITS>;
+  auto row = [&](int byte) -> const uint8_t* {
+    const int sh = 8 * (byte & 3) - 7;
+    const uint32_t x = w[byte >> 2];
+    return table + (((sh < 0 ? x << 7 : x >> (sh < 0 ? 0 : sh)) & T::kMask) | lane_off);
+  };
+  if constexpr (T::IPB == 1) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p) e[p] = *reinterpret_cast<const uint32_t*>(row(4 * ks + p));
+  } else if constexpr (T::IPB == 2) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const uint2 v = *reinterpret_cast<const uint2*>(row(2 * ks + p));
+      e[2 * p] = v.x; e[2 * p + 1] = v.y;
+    }
+  } else {
+    const uint4 v = *reinterpret_cast<const uint4*>(row(T::IPB == 4 ? ks : ks >> 1) + (T::IPB == 8 ? 16 * (ks & 1) : 0));
+    e[0] = v.x; e[1] = v.y; e[2] = v.z; e[3] = v.w;
+  }
+}
+
+// operand of one key, k-step ks, from a table of PAIRS: high pieces of coordinates 4 ks, 4 ks + 1 (row gid), their low pieces
+// (row gid + 8), and the same of 4 ks + 2, 4 ks + 3
+template <int BITS, int W>
+__device__ __forceinline__ void key_operand(const uint32_t (&w)[W], int ks, const uint8_t* table, uint32_t lane_off, uint32_t (&a)[4]) {
+  entries4<BITS>(w, ks, table, lane_off, a);
+  if constexpr (ByteTable<BITS>::IPB == 1) {
+#pragma unroll
+    for (int p = 0; p < 4; p += 2) {
+      const uint32_t hi = __byte_perm(a[p], a[p + 1], 0x5410), lo = __byte_perm(a[p], a[p + 1], 0x7632);
+      a[p] = hi; a[p + 1] = lo;
+    }
+  }
+}
+
+// exp for arguments <= 0: below 2^-126 the result is zero
+__device__ __forceinline__ float exp_neg(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+  return y;
 }
 
 // (max, sum of exp) running pair
@@ -141,29 +186,41 @@ __device__ __forceinline__ void stat_merge(float& m, float& s, float m2, float s
   m = nm;
 }
 
-// Query operand of one pass: column n = lane / 4 of the 8-column operand is row r0 + (n & 3) of the rotated
-// queries, as its high piece (n < 4) or low piece (n >= 4); thread t holds coordinates 32 t + 4 ks + 0..3, each value in
-// both halves of its register.
-__device__ __forceinline__ void query_fragments(const float* qrot, int64_t row, bool row_ok, int lane,
-                                                uint32_t (&bq)[8][4]) {
+// Codes of one coordinate a byte (5 to 8 bits) with four query rows: the words of a byte table already are operand registers if
+// the two neighbouring k of a register are the pieces of ONE coordinate, the rows are 16 keys and the query value stands in
+// both places of the other operand.  Pairing the high and the low pieces of two look-ups takes a byte permute per coordinate
+// more: 131072 8-bit keys x 8 heads 56 us against 66.  With eight query rows the permutes serve twice the products and the
+// widened query values would not fit the registers (65536 6-bit keys x 8 heads, 16 query rows: 90 against 81).
+template <int BITS> constexpr bool kCoordWords = BITS >= 5;
+
+// Query operand of one pass of four rows: column n = lane / 4 of the 8-column operand is row r0 + (n & 3) of the rotated
+// queries, as its high piece (n < 4) or low piece (n >= 4); thread t holds coordinates 32 t + 4 ks + 0..3, two a register
+// (N = 2 registers a k-step) or each in both halves of its own (N = 4).
+template <int N>
+__device__ __forceinline__ void query_fragments(const float* qrot, int64_t row, bool row_ok, int lane, uint32_t (&bq)[8][N]) {
   const int t = lane & 3;
   const bool low = (lane >> 2) >= 4;
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row_ok) v = *reinterpret_cast<const float4*>(qrot + row * kDimA + 32 * t + 4 * ks);
-    const float f[4] = {v.x, v.y, v.z, v.w};
+    uint32_t hi[2], lo[2];
+    split2(v.x, v.y, hi[0], lo[0]);
+    split2(v.z, v.w, hi[1], lo[1]);
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      const __half h = __float2half_rn(f[p]);
-      const __half piece = low ? __float2half_rn(f[p] - __half2float(h)) : h;
-      bq[ks][p] = (uint32_t)__half_as_ushort(piece) * 0x00010001u;
+    for (int p = 0; p < 2; ++p) {
+      const uint32_t two = low ? lo[p] : hi[p];
+      if constexpr (N == 2) {
+        bq[ks][p] = two;
+      } else {
+        bq[ks][2 * p] = __byte_perm(two, 0u, 0x1010);
+        bq[ks][2 * p + 1] = __byte_perm(two, 0u, 0x3232);
+      }
     }
   }
 }
 
-// The same for eight query rows per pass: column n is row r0 + n, high pieces in bh, low pieces in bl; a register holds
-// two coordinates and is widened at its use (both values in both halves would be 64 registers).
+// The same for eight query rows per pass: column n is row r0 + n, high pieces in bh, low pieces in bl.
 __device__ __forceinline__ void query_fragments8(const float* qrot, int64_t row, bool row_ok, int lane,
                                                  uint32_t (&bh)[8][2], uint32_t (&bl)[8][2]) {
   const int t = lane & 3;
@@ -175,55 +232,72 @@ __device__ __forceinline__ void query_fragments8(const float* qrot, int64_t row,
     split2(v.z, v.w, bh[ks][1], bl[ks][1]);
   }
 }
+// 16 keys x 8 query rows: c[0..1] = key gid, c[2..3] = key gid + 8, rows 2t, 2t + 1
 template <int BITS>
 __device__ __forceinline__ void score_block8(const uint32_t (&w0)[Packed<BITS>::CW], const uint32_t (&w1)[Packed<BITS>::CW],
-                                             const uint32_t (&bh)[8][2], const uint32_t (&bl)[8][2], uint32_t lut_base, float (&c)[4]) {
-  float d[4] = {0.f, 0.f, 0.f, 0.f};
-  c[0] = c[1] = c[2] = c[3] = 0.f;
+                                             const uint32_t (&bh)[8][2], const uint32_t (&bl)[8][2], const uint8_t* table,
+                                             uint32_t lane_off, float (&c)[4]) {
+  // the high and the low query pieces in accumulators of their own: the tensor core truncates its sums at their size
+  float x[2][4] = {}, y[2][4] = {};
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) {
     uint32_t e[4], f[4];
-    key_entries<BITS>(w0, ks, lut_base, e);
-    key_entries<BITS>(w1, ks, lut_base, f);
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      mma_16816(c, e[2 * p], f[2 * p], e[2 * p + 1], f[2 * p + 1], __byte_perm(bh[ks][p], 0u, 0x1010), __byte_perm(bh[ks][p], 0u, 0x3232));
-      mma_16816(d, e[2 * p], f[2 * p], e[2 * p + 1], f[2 * p + 1], __byte_perm(bl[ks][p], 0u, 0x1010), __byte_perm(bl[ks][p], 0u, 0x3232));
-    }
+    key_operand<BITS>(w0, ks, table, lane_off, e);
+    key_operand<BITS>(w1, ks, table, lane_off, f);
+    mma_16816(x[0], e[0], e[1], e[2], e[3], bh[ks][0], bh[ks][1]);
+    mma_16816(y[0], f[0], f[1], f[2], f[3], bh[ks][0], bh[ks][1]);
+    mma_16816(x[1], e[0], e[1], e[2], e[3], bl[ks][0], bl[ks][1]);
+    mma_16816(y[1], f[0], f[1], f[2], f[3], bl[ks][0], bl[ks][1]);
   }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) c[j] += d[j];
+  for (int j = 0; j < 2; ++j) {
+    c[j] = x[0][j] + ((x[0][j + 2] + x[1][j]) + x[1][j + 2]);
+    c[j + 2] = y[0][j] + ((y[0][j + 2] + y[1][j]) + y[1][j + 2]);
+  }
 }
 
-// 16 keys x 4 query rows: c[0..1] = key gid, c[2..3] = key gid + 8, columns (2t, 2t + 1) of [q_hi | q_lo].
-// Two accumulators, so that neighbouring MMAs do not wait for one another.
-template <int BITS>
+// 16 keys x 4 query rows, before the low query pieces (columns g + 4, two lanes away) are added: c[0..1] = key gid,
+// c[2..3] = key gid + 8, columns 2t, 2t + 1.  Neighbouring MMAs go to different accumulators and do not wait for one another.
+template <int BITS, int N>
 __device__ __forceinline__ void score_block(const uint32_t (&w0)[Packed<BITS>::CW], const uint32_t (&w1)[Packed<BITS>::CW],
-                                            const uint32_t (&bq)[8][4], uint32_t lut_base, float (&c)[4]) {
-  float d[4] = {0.f, 0.f, 0.f, 0.f};
-  c[0] = c[1] = c[2] = c[3] = 0.f;
+                                            const uint32_t (&bq)[8][N], const uint8_t* table, uint32_t lane_off, float (&c)[4]) {
+  if constexpr (N == 2) {
+    // per key one accumulator for each half of the coordinates
+    float x[2][4] = {}, y[2][4] = {};
 #pragma unroll
-  for (int ks = 0; ks < 8; ++ks) {
-    uint32_t e[4], f[4];
-    key_entries<BITS>(w0, ks, lut_base, e);
-    key_entries<BITS>(w1, ks, lut_base, f);
-    mma_16816(c, e[0], f[0], e[1], f[1], bq[ks][0], bq[ks][1]);
-    mma_16816(d, e[2], f[2], e[3], f[3], bq[ks][2], bq[ks][3]);
-  }
-  // column g + 4 (low query piece) lives two lanes away: afterwards lanes t and t ^ 2 both hold the full sums
+    for (int ks = 0; ks < 8; ++ks) {
+      uint32_t e[4], f[4];
+      key_operand<BITS>(w0, ks, table, lane_off, e);
+      key_operand<BITS>(w1, ks, table, lane_off, f);
+      mma_16816(x[ks & 1], e[0], e[1], e[2], e[3], bq[ks][0], bq[ks][1]);
+      mma_16816(y[ks & 1], f[0], f[1], f[2], f[3], bq[ks][0], bq[ks][1]);
+    }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    c[j] += d[j];
-    c[j] += __shfl_xor_sync(0xffffffffu, c[j], 2);
+    for (int j = 0; j < 2; ++j) {
+      c[j] = (x[0][j] + x[1][j]) + (x[0][j + 2] + x[1][j + 2]);
+      c[j + 2] = (y[0][j] + y[1][j]) + (y[0][j + 2] + y[1][j + 2]);
+    }
+  } else {
+    float x[4] = {}, y[4] = {};
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      uint32_t e[4], f[4];
+      entries4<BITS>(w0, ks, table, lane_off, e);
+      entries4<BITS>(w1, ks, table, lane_off, f);
+      mma_16816(x, e[0], f[0], e[1], f[1], bq[ks][0], bq[ks][1]);
+      mma_16816(y, e[2], f[2], e[3], f[3], bq[ks][2], bq[ks][3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[j] = x[j] + y[j];
   }
 }
 
 // grid: B * Hkv * nblk CTAs, each over keys_per_block keys of one KV head; stats as in the FP32 path:
 // stats[(row * nblk + blk) * 2 + {0, 1}] = (max, sum of exp(l - max)) of the block's keys.
-// Two CTAs per SM: three (80 registers) spill, 70 us against 65 for the call below.
-// 8 KV heads x 131072 4-bit keys, 32 query heads: the call, with projection and softmax, 75 us with packed pieces, one
-// accumulator and a rescaled sum for every logit, 65 us as it is.
-// 8 KV heads x 65536 4-bit keys with 8 query rows per KV head: 65 -> 43 us for the call, with 16 rows 117 -> 78 us.
+// Two CTAs per SM: three (80 registers) 49 us against 45 for the call below.
+// 8 KV heads x 131072 4-bit keys, 32 query heads: the call, with projection and softmax, 59 us with a table entry per
+// coordinate and three waves of blocks, 45 us as it is (kernel 48 -> 36 under ncu: 386 -> 245 instructions per 16 keys, issued
+// 0.55 of the time).  8 KV heads x 65536 keys with 8 query rows per KV head: 42 -> 35 us.
 //
 // ROWS: query rows per pass over the keys.  With eight a lane finishes keys gid and gid + 8 for rows 2t, 2t + 1 and the
 // look-ups of a key serve twice the rows; four rows put their low pieces into the other four columns instead.
@@ -233,16 +307,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const
   if (stats != nullptr) pdl_trigger();           // the softmax pass follows
   constexpr int G = Packed<BITS>::G;
   constexpr int CW = Packed<BITS>::CW;
-  __shared__ __align__(1024) uint32_t lut[256];
+  __shared__ __align__(128) uint8_t table[ByteTable<BITS>::kBytes];
   constexpr bool kEight = ROWS == 8;
   __shared__ float red_m[kWarps][ROWS], red_s[kWarps][ROWS];
-  {
-    const float c = __ldg(job.codebook + kCentroidOff + threadIdx.x);
-    const __half h = __float2half_rn(c);
-    const __half l = __float2half_rn(c - __half2float(h));
-    lut[threadIdx.x] = (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
-  }
-  const uint32_t lut_base = (uint32_t)__cvta_generic_to_shared(lut);
+  build_table<BITS, true>(table, job.codebook);
   const int blk = blockIdx.x % nblk;
   const int64_t bh = blockIdx.x / nblk;
   const int64_t b = bh / job.Hkv, hkv = bh % job.Hkv;
@@ -252,6 +320,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const
   const int n_keys = (int)min((int64_t)keys_per_block, job.Sk - s_begin);      // of this CTA; keys below count from s_begin
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, t = lane & 3;
+  const uint32_t lane_off = ByteTable<BITS>::lane_offset(lane);
   const int my = gid + (!kEight && t >= 2 ? 8 : 0);     // the (first) key of a block whose logits this lane finishes
   const uint8_t* keys = job.idx_bytes + (bh * job.Sk + s_begin) * G + t * Packed<BITS>::CB;
   const uint16_t* norms = job.norms + bh * job.Sk + s_begin;
@@ -262,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const
   };
   pdl_wait();                                    // the rotated queries come from the launch before
   for (int r0 = 0; r0 < R; r0 += ROWS) {
-    uint32_t bq[kEight ? 1 : 8][4], bh[kEight ? 8 : 1][2], bl[kEight ? 8 : 1][2];
+    uint32_t bq[8][kCoordWords<BITS> ? 4 : 2], bh[8][2], bl[8][2];        // four or eight rows: the others stay unused
     if constexpr (kEight) {
       const int r = r0 + gid;
       query_fragments8(qrot, r < R ? global_row(r) : 0, r < R, lane, bh, bl);
@@ -270,7 +339,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const
       const int r = r0 + (gid & 3);
       query_fragments(qrot, r < R ? global_row(r) : 0, r < R, lane, bq);
     }
-    // four rows: after the shuffle in score_block this lane finishes ONE key (gid for t < 2, gid + 8 otherwise) and the
+    // four rows: after the shuffle below this lane finishes ONE key (gid for t < 2, gid + 8 otherwise) and the
     // two query rows r0 + 2 (t & 1) + {0, 1}
     const int ra = r0 + 2 * (kEight ? t : t & 1);
     const bool ok_a = ra < R, ok_b = ra + 1 < R;
@@ -294,21 +363,23 @@ __global__ void __launch_bounds__(kThreads, 2) k_score_mma(TqScoreJob job, const
         const float la = ca * nv, lb = cb * nv;
         if (ok_a) out_a[key] = la;
         if (ok_b) out_b[key] = lb;
-        if (la > m_a) { s_a *= __expf(m_a - la); m_a = la; }
-        if (lb > m_b) { s_b *= __expf(m_b - lb); m_b = lb; }
-        s_a += __expf(la - m_a);
-        s_b += __expf(lb - m_b);
+        if (la > m_a) { s_a *= exp_neg(m_a - la); m_a = la; }
+        if (lb > m_b) { s_b *= exp_neg(m_b - lb); m_b = lb; }
+        s_a += exp_neg(la - m_a);
+        s_b += exp_neg(lb - m_b);
       }
     };
     auto score = [&](const uint32_t (&a0)[CW], const uint32_t (&a1)[CW], int kb, uint32_t nb) {
       float c[4];
       if constexpr (kEight) {
-        score_block8<BITS>(a0, a1, bh, bl, lut_base, c);
+        score_block8<BITS>(a0, a1, bh, bl, table, lane_off, c);
         finish_key(kb + my, c[0], c[1], nb & 0xFFFFu);
         finish_key(kb + my + 8, c[2], c[3], nb >> 16);
       } else {
-        score_block<BITS>(a0, a1, bq, lut_base, c);
-        finish_key(kb + my, t < 2 ? c[0] : c[2], t < 2 ? c[1] : c[3], nb);
+        score_block<BITS>(a0, a1, bq, table, lane_off, c);
+        // lane t ^ 2 holds the other query piece of the same rows and finishes the other key: each sends what the other needs
+        const float xa = __shfl_xor_sync(0xffffffffu, t < 2 ? c[2] : c[0], 2), xb = __shfl_xor_sync(0xffffffffu, t < 2 ? c[3] : c[1], 2);
+        finish_key(kb + my, (t < 2 ? c[0] : c[2]) + xa, (t < 2 ? c[1] : c[3]) + xb, nb);
       }
     };
     int kb = warp * 16;
@@ -391,14 +462,6 @@ __device__ __forceinline__ void load_eighth(const uint8_t* row, int e, uint32_t 
   }
 }
 
-// table entry (hi | lo << 16) of local coordinate v (0..15) of a thread's eighth row
-template <int BITS>
-__device__ __forceinline__ uint32_t value_entry(const uint32_t (&w)[PackedV<BITS>::CW], int v, uint32_t lut_base) {
-  constexpr int CPW = 4 * PackedV<BITS>::IPB;
-  const WordAddr<BITS> wa(w[v / CPW], lut_base);
-  return lds_u32(wa(v % CPW));
-}
-
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
   uint32_t y;
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
@@ -422,33 +485,28 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
   pdl_trigger();
   constexpr int GK = Packed<KBITS>::G, KW = Packed<KBITS>::CW;
   constexpr int GV = PackedV<VBITS>::G, VW = PackedV<VBITS>::CW;
-  __shared__ __align__(1024) uint32_t lut_k[256];
-  __shared__ __align__(1024) uint32_t lut_v[256];
+  extern __shared__ __align__(128) uint8_t tables[];
+  uint8_t* table_k = tables;
+  uint8_t* table_v = tables + ByteTable<KBITS>::kBytes;
   __shared__ float sm_m[kWarps][kRows], sm_l[kWarps][kRows];
   __shared__ float sm_acc[kWarps][kRows][kDimA];          // 16 KB
-  {
-    const float ck = __ldg(P.k_codebook + kCentroidOff + threadIdx.x);
-    const __half hk = __float2half_rn(ck);
-    lut_k[threadIdx.x] = (uint32_t)__half_as_ushort(hk) | ((uint32_t)__half_as_ushort(__float2half_rn(ck - __half2float(hk))) << 16);
-    const float cv = __ldg(P.v_codebook + kCentroidOff + threadIdx.x);
-    const __half hv = __float2half_rn(cv);
-    lut_v[threadIdx.x] = (uint32_t)__half_as_ushort(hv) | ((uint32_t)__half_as_ushort(__float2half_rn(cv - __half2float(hv))) << 16);
-  }
-  const uint32_t lutk = (uint32_t)__cvta_generic_to_shared(lut_k);
-  const uint32_t lutv = (uint32_t)__cvta_generic_to_shared(lut_v);
+  build_table<KBITS, true>(table_k, P.k_codebook);
+  build_table<VBITS, false>(table_v, P.v_codebook);
   const int blk = blockIdx.x % P.nblk;
   const int64_t bh = blockIdx.x / P.nblk;
   const int64_t b = bh / P.Hkv, hkv = bh % P.Hkv;
   const int rep = (int)(P.Hq / P.Hkv);
   const int R = rep * (int)P.Sq;
+  // this CTA's keys count from s_begin; a lane's own parts of the rows
   const int64_t s_begin = (int64_t)blk * P.keys_per_block;
-  const int64_t s_end = min(s_begin + (int64_t)P.keys_per_block, P.Sk);
-  const uint8_t* keys = P.k_idx + bh * P.Sk * GK;
-  const uint8_t* vals = P.v_idx + bh * P.Sk * GV;
-  const uint16_t* k_norms = P.k_norms + bh * P.Sk;
-  const uint16_t* v_norms = P.v_norms + bh * P.Sk;
+  const int n_keys = (int)min((int64_t)P.keys_per_block, P.Sk - s_begin);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, t = lane & 3;
+  const uint8_t* keys = P.k_idx + (bh * P.Sk + s_begin) * GK + t * Packed<KBITS>::CB;
+  const uint8_t* vals = P.v_idx + (bh * P.Sk + s_begin) * GV + gid * PackedV<VBITS>::CB;
+  const uint16_t* k_norms = P.k_norms + bh * P.Sk + s_begin;
+  const uint16_t* v_norms = P.v_norms + bh * P.Sk + s_begin;
+  const uint32_t off_k = ByteTable<KBITS>::lane_offset(lane), off_v = ByteTable<VBITS>::lane_offset(lane);
   __syncthreads();
   auto global_row = [&](int r) -> int64_t {
     const int64_t hq = hkv * rep + r / P.Sq, sq = r % P.Sq;
@@ -456,7 +514,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
   };
   pdl_wait();                                    // the rotated queries come from the launch before
   for (int r0 = 0; r0 < R; r0 += kRows) {
-    uint32_t bq[8][4];
+    uint32_t bq[8][2];
     {
       const int r = r0 + (gid & 3);
       query_fragments(P.qrot, r < R ? global_row(r) : 0, r < R, lane, bq);
@@ -467,40 +525,57 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
     float acc[8][4];
 #pragma unroll
     for (int mb = 0; mb < 8; ++mb) acc[mb][0] = acc[mb][1] = acc[mb][2] = acc[mb][3] = 0.f;
-    uint32_t w0[KW], w1[KW], n0[KW], n1[KW];
-    uint32_t vw[4][VW], vx[4][VW];                                   // value rows of this block and of the next
-    uint32_t kn_bits = 0, kn_next = 0, vn_bits = 0, vn_next = 0;      // norms of keys gid (low half) and gid + 8 (high half)
-    // keys, value rows and norms of a block: fetched one block ahead of their use (fetching the value rows at the
-    // start of their own block left most of a memory latency exposed in every round)
-    auto fetch = [&](int64_t kb, uint32_t (&a0)[KW], uint32_t (&a1)[KW], uint32_t (&av)[4][VW], uint32_t& kn, uint32_t& vn) {
-      const int64_t k_lo = kb + gid, k_hi = kb + 8 + gid;
-      const int64_t c_lo = k_lo < s_end ? k_lo : s_begin, c_hi = k_hi < s_end ? k_hi : s_begin;
-      load_quarter<KBITS>(keys + c_lo * GK, t, a0);
-      load_quarter<KBITS>(keys + c_hi * GK, t, a1);
+    // Two blocks of 16 keys a round where their rows fit the registers: one maximum, one rescaling and two independent
+    // chains of look-ups and products.  The next round's lines are fetched into L1 meanwhile; keeping them in registers took
+    // the room of the second block, and K6/V4 and wider spilled (131072 tokens x 8 heads, with projection and finish: K4/V2
+    // 84 -> 70 us, K4/V4 90 -> 79, K8/V8 153 -> 104; two blocks with 4-bit values spill: 83).
+    constexpr int NB = 4 * KW + 8 * VW <= 24 ? 2 : 1;
+    uint32_t w0[NB][KW], w1[NB][KW], vw[NB][4][VW];
+    uint32_t kn_bits[NB], vn_bits[NB];            // norms of keys gid (low half) and gid + 8 (high half)
+    for (int kb = warp * 16 * NB; kb < n_keys; kb += kWarps * 16 * NB) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int64_t key = kb + 2 * t + (q & 1) + 8 * (q >> 1);         // keys 2t, 2t+1, 2t+8, 2t+9
-        load_eighth<VBITS>(vals + (key < s_end ? key : s_begin) * GV, gid, av[q]);
+      for (int nb = 0; nb < NB; ++nb) {
+        const int k0 = kb + 16 * nb;
+        const int c_lo = k0 + gid < n_keys ? k0 + gid : 0, c_hi = k0 + 8 + gid < n_keys ? k0 + 8 + gid : 0;
+        load_quarter<KBITS>(keys + (uint32_t)(c_lo * GK), 0, w0[nb]);
+        load_quarter<KBITS>(keys + (uint32_t)(c_hi * GK), 0, w1[nb]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int key = k0 + 2 * t + (q & 1) + 8 * (q >> 1);           // keys 2t, 2t+1, 2t+8, 2t+9
+          load_eighth<VBITS>(vals + (uint32_t)((key < n_keys ? key : 0) * GV), 0, vw[nb][q]);
+        }
+        kn_bits[nb] = (uint32_t)__ldg(k_norms + c_lo) | ((uint32_t)__ldg(k_norms + c_hi) << 16);
+        vn_bits[nb] = (uint32_t)__ldg(v_norms + c_lo) | ((uint32_t)__ldg(v_norms + c_hi) << 16);
       }
-      kn = (uint32_t)__ldg(k_norms + c_lo) | ((uint32_t)__ldg(k_norms + c_hi) << 16);
-      vn = (uint32_t)__ldg(v_norms + c_lo) | ((uint32_t)__ldg(v_norms + c_hi) << 16);
-    };
-    int64_t kb = s_begin + warp * 16;
-    if (kb < s_end) fetch(kb, w0, w1, vw, kn_bits, vn_bits);
-    for (; kb < s_end; kb += kWarps * 16) {
-      const int64_t kn = kb + kWarps * 16;
-      if (kn < s_end) fetch(kn, n0, n1, vx, kn_next, vn_next);
-      float c[4];
-      score_block<KBITS>(w0, w1, bq, lutk, c);
-      // logits of keys gid (c[0], c[1]) and gid + 8 (c[2], c[3]) for this lane's two rows
-      const bool in_lo = kb + gid < s_end, in_hi = kb + 8 + gid < s_end;
-      const float nk_lo = __half2float(__ushort_as_half((uint16_t)(kn_bits & 0xFFFFu))) * P.scale;
-      const float nk_hi = __half2float(__ushort_as_half((uint16_t)(kn_bits >> 16))) * P.scale;
-      float l[4];
-      l[0] = in_lo ? c[0] * nk_lo : -INFINITY; l[1] = in_lo ? c[1] * nk_lo : -INFINITY;
-      l[2] = in_hi ? c[2] * nk_hi : -INFINITY; l[3] = in_hi ? c[3] * nk_hi : -INFINITY;
-      // block maximum per row over the 16 keys (lanes that differ in gid)
-      float bm[2] = {fmaxf(l[0], l[2]), fmaxf(l[1], l[3])};
+      {
+        const int row = kb + kWarps * 16 * NB + (lane & (16 * NB - 1));
+        if (row < n_keys) {
+          if (NB == 2 || lane < 16) asm volatile("prefetch.global.L1 [%0];" ::"l"(keys - t * Packed<KBITS>::CB + (uint32_t)(row * GK)));
+          if (NB == 2 || lane >= 16) asm volatile("prefetch.global.L1 [%0];" ::"l"(vals - gid * PackedV<VBITS>::CB + (uint32_t)(row * GV)));
+          if (lane < 2) asm volatile("prefetch.global.L1 [%0];" ::"l"((lane ? v_norms : k_norms) + row));
+        }
+      }
+      float l[NB][4];
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) {
+        float c[4];
+        score_block<KBITS>(w0[nb], w1[nb], bq, table_k, off_k, c);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] += __shfl_xor_sync(0xffffffffu, c[j], 2);       // lanes t and t ^ 2 both hold the full sums
+        // logits of keys gid (c[0], c[1]) and gid + 8 (c[2], c[3]) for this lane's two rows
+        const bool in_lo = kb + 16 * nb + gid < n_keys, in_hi = kb + 16 * nb + 8 + gid < n_keys;
+        const float nk_lo = __half2float(__ushort_as_half((uint16_t)(kn_bits[nb] & 0xFFFFu))) * P.scale;
+        const float nk_hi = __half2float(__ushort_as_half((uint16_t)(kn_bits[nb] >> 16))) * P.scale;
+        l[nb][0] = in_lo ? c[0] * nk_lo : -INFINITY; l[nb][1] = in_lo ? c[1] * nk_lo : -INFINITY;
+        l[nb][2] = in_hi ? c[2] * nk_hi : -INFINITY; l[nb][3] = in_hi ? c[3] * nk_hi : -INFINITY;
+      }
+      // maximum per row over the round's keys (lanes that differ in gid)
+      float bm[2] = {fmaxf(l[0][0], l[0][2]), fmaxf(l[0][1], l[0][3])};
+#pragma unroll
+      for (int nb = 1; nb < NB; ++nb) {
+        bm[0] = fmaxf(bm[0], fmaxf(l[nb][0], l[nb][2]));
+        bm[1] = fmaxf(bm[1], fmaxf(l[nb][1], l[nb][3]));
+      }
 #pragma unroll
       for (int o = 4; o <= 16; o <<= 1) {
         bm[0] = fmaxf(bm[0], __shfl_xor_sync(0xffffffffu, bm[0], o));
@@ -509,31 +584,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
       float alpha[2];
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const float nm = fmaxf(run_m[j], bm[j]);              // the block holds at least one valid key: finite
-        alpha[j] = run_m[j] == -INFINITY ? 0.f : __expf(run_m[j] - nm);
+        const float nm = fmaxf(run_m[j], bm[j]);              // the round holds at least one valid key: finite
+        alpha[j] = run_m[j] == -INFINITY ? 0.f : exp_neg(run_m[j] - nm);
         run_m[j] = nm;
+        run_l[j] *= alpha[j];
       }
-      float p[4];
-      p[0] = __expf(l[0] - run_m[0]); p[1] = __expf(l[1] - run_m[1]);
-      p[2] = __expf(l[2] - run_m[0]); p[3] = __expf(l[3] - run_m[1]);
-      // row sums: every (row, key) pair is counted by exactly one of the lanes t and t ^ 2
-      if (t < 2) { run_l[0] = run_l[0] * alpha[0] + p[0]; run_l[1] = run_l[1] * alpha[1] + p[1]; }
-      else       { run_l[0] = run_l[0] * alpha[0] + p[2]; run_l[1] = run_l[1] * alpha[1] + p[3]; }
-      // P' = p * norm_v as fp16 pieces; this lane contributes the high (t < 2) or low (t >= 2) piece
-      const float nv_lo = __half2float(__ushort_as_half((uint16_t)(vn_bits & 0xFFFFu)));
-      const float nv_hi = __half2float(__ushort_as_half((uint16_t)(vn_bits >> 16)));
-      uint32_t x0, x1;
-      {
-        uint32_t h, lo2;
-        split2(p[0] * nv_lo, p[1] * nv_lo, h, lo2);
-        x0 = t < 2 ? h : lo2;
-        split2(p[2] * nv_hi, p[3] * nv_hi, h, lo2);
-        x1 = t < 2 ? h : lo2;
-      }
-      const uint32_t pb0 = movmatrix_trans(x0);               // keys 2t, 2t+1  x column gid
-      const uint32_t pb1 = movmatrix_trans(x1);               // keys 2t+8, 2t+9 x column gid
-      const uint32_t p0 = __byte_perm(pb0, 0u, 0x1010), p1 = __byte_perm(pb0, 0u, 0x3232);     // each value in both halves
-      const uint32_t p2 = __byte_perm(pb1, 0u, 0x1010), p3 = __byte_perm(pb1, 0u, 0x3232);
       // rescale the accumulators when a maximum moved (columns 2t, 2t+1 are this lane's two rows in both halves)
       if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
 #pragma unroll
@@ -541,27 +596,44 @@ __global__ void __launch_bounds__(kThreads, 2) k_decode_attn(DecodeParams P) {
           acc[mb][0] *= alpha[0]; acc[mb][1] *= alpha[1]; acc[mb][2] *= alpha[0]; acc[mb][3] *= alpha[1];
         }
       }
-      // acc^T += V^T P' for 8 blocks of 16 coordinates; this thread's rows are coordinates 16 gid + 2 mb + {0, 1}
 #pragma unroll
-      for (int mb = 0; mb < 8; ++mb) {
-        uint32_t e[4][2];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          e[q][0] = value_entry<VBITS>(vw[q], 2 * mb, lutv);
-          e[q][1] = value_entry<VBITS>(vw[q], 2 * mb + 1, lutv);
+      for (int nb = 0; nb < NB; ++nb) {
+        float p[4];
+        p[0] = exp_neg(l[nb][0] - run_m[0]); p[1] = exp_neg(l[nb][1] - run_m[1]);
+        p[2] = exp_neg(l[nb][2] - run_m[0]); p[3] = exp_neg(l[nb][3] - run_m[1]);
+        // row sums: every (row, key) pair is counted by exactly one of the lanes t and t ^ 2
+        run_l[0] += t < 2 ? p[0] : p[2];
+        run_l[1] += t < 2 ? p[1] : p[3];
+        // P' = p * norm_v as fp16 pieces; this lane contributes the high (t < 2) or low (t >= 2) piece
+        const float nv_lo = __half2float(__ushort_as_half((uint16_t)(vn_bits[nb] & 0xFFFFu)));
+        const float nv_hi = __half2float(__ushort_as_half((uint16_t)(vn_bits[nb] >> 16)));
+        uint32_t x0, x1;
+        {
+          uint32_t h, lo2;
+          split2(p[0] * nv_lo, p[1] * nv_lo, h, lo2);
+          x0 = t < 2 ? h : lo2;
+          split2(p[2] * nv_hi, p[3] * nv_hi, h, lo2);
+          x1 = t < 2 ? h : lo2;
         }
-        // an entry is the operand's two neighbouring k, the pieces of one value; rows gid, gid + 8 are the two coordinates,
-        // the k pairs t, t + 4 the keys 2t, 2t + 1 (first MMA) and 2t + 8, 2t + 9 (second)
-        mma_16816(acc[mb], e[0][0], e[0][1], e[1][0], e[1][1], p0, p1);
-        mma_16816(acc[mb], e[2][0], e[2][1], e[3][0], e[3][1], p2, p3);
+        const uint32_t pb0 = movmatrix_trans(x0);               // keys 2t, 2t+1  x column gid
+        const uint32_t pb1 = movmatrix_trans(x1);               // keys 2t+8, 2t+9 x column gid
+        const uint32_t p0 = __byte_perm(pb0, 0u, 0x1010), p1 = __byte_perm(pb0, 0u, 0x3232);     // each value in both halves
+        const uint32_t p2 = __byte_perm(pb1, 0u, 0x1010), p3 = __byte_perm(pb1, 0u, 0x3232);
+        // acc^T += V^T P' for 8 blocks of 16 coordinates; this thread's rows are coordinates 16 gid + 2 mb + {0, 1}
+#pragma unroll
+        for (int m2 = 0; m2 < 4; ++m2) {
+          uint32_t e[4][4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) entries4<VBITS>(vw[nb][q], m2, table_v, off_v, e[q]);
+          // an entry is the operand's two neighbouring k, the pieces of one value; rows gid, gid + 8 are the two coordinates,
+          // the k pairs t, t + 4 the keys 2t, 2t + 1 (first MMA) and 2t + 8, 2t + 9 (second)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            mma_16816(acc[2 * m2 + h], e[0][2 * h], e[0][2 * h + 1], e[1][2 * h], e[1][2 * h + 1], p0, p1);
+            mma_16816(acc[2 * m2 + h], e[2][2 * h], e[2][2 * h + 1], e[3][2 * h], e[3][2 * h + 1], p2, p3);
+          }
+        }
       }
-#pragma unroll
-      for (int k = 0; k < KW; ++k) { w0[k] = n0[k]; w1[k] = n1[k]; }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int k = 0; k < VW; ++k) vw[q][k] = vx[q][k];
-      kn_bits = kn_next; vn_bits = vn_next;
     }
     // ---- fold the warp: sums over the lanes that share (t & 1), pieces hi + lo two lanes apart
 #pragma unroll
@@ -797,34 +869,27 @@ size_t decode_attention_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk,
   return q + (size_t)rows * nblk * kPartStride * sizeof(float);
 }
 
-template <int KB>
-static int launch_decode_v(const DecodeParams& P, int vbits, unsigned blocks, cudaStream_t st) {
-  switch (vbits) {
-    case 1: launch_after(k_decode_attn<KB, 1>, dim3(blocks), dim3(kThreads), 0, st, P); break;
-    case 2: launch_after(k_decode_attn<KB, 2>, dim3(blocks), dim3(kThreads), 0, st, P); break;
-    case 3: launch_after(k_decode_attn<KB, 3>, dim3(blocks), dim3(kThreads), 0, st, P); break;
-    case 4: launch_after(k_decode_attn<KB, 4>, dim3(blocks), dim3(kThreads), 0, st, P); break;
-    case 5: launch_after(k_decode_attn<KB, 5>, dim3(blocks), dim3(kThreads), 0, st, P); break;
-    case 6: launch_after(k_decode_attn<KB, 6>, dim3(blocks), dim3(kThreads), 0, st, P); break;
-    case 7: launch_after(k_decode_attn<KB, 7>, dim3(blocks), dim3(kThreads), 0, st, P); break;
-    default: launch_after(k_decode_attn<KB, 8>, dim3(blocks), dim3(kThreads), 0, st, P); break;
-  }
+template <int KB, int VB>
+static int launch_decode_kv(const DecodeParams& P, unsigned blocks, cudaStream_t st) {
+  constexpr int smem = (int)(ByteTable<KB>::kBytes + ByteTable<VB>::kBytes);
+  const cudaError_t e = cudaFuncSetAttribute(k_decode_attn<KB, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return refused(e);
+  launch_after(k_decode_attn<KB, VB>, dim3(blocks), dim3(kThreads), (size_t)smem, st, P);
   return check_launch();
 }
 
-// Keys per CTA such that the CTAs fill whole waves of `slots` resident CTAs: at least min_keys (the scratch is
-// sized for blocks of min_keys), a multiple of 16.  With 8 KV heads and 131 072 keys, blocks of 2048 keys are
-// 512 CTAs = 3.46 waves of 148, i.e. four rounds of which the last is half empty; 55 blocks of 2384 keys per head
-// are 2.97 waves.
-static int wave_keys_per_block(int64_t units, int64_t Sk, int min_keys, int slots) {
-  const int64_t nblk_max = (Sk + min_keys - 1) / min_keys;
-  if (units <= 0 || slots <= 0 || units * nblk_max <= slots) return min_keys;
-  const int64_t waves = units * nblk_max / slots;
-  int64_t nblk = waves * slots / units;
-  if (nblk < 1) nblk = 1;
-  int64_t kpb = (Sk + nblk - 1) / nblk;
-  kpb = (kpb + 15) / 16 * 16;
-  return (int)(kpb < min_keys ? min_keys : kpb);
+template <int KB>
+static int launch_decode_v(const DecodeParams& P, int vbits, unsigned blocks, cudaStream_t st) {
+  switch (vbits) {
+    case 1: return launch_decode_kv<KB, 1>(P, blocks, st);
+    case 2: return launch_decode_kv<KB, 2>(P, blocks, st);
+    case 3: return launch_decode_kv<KB, 3>(P, blocks, st);
+    case 4: return launch_decode_kv<KB, 4>(P, blocks, st);
+    case 5: return launch_decode_kv<KB, 5>(P, blocks, st);
+    case 6: return launch_decode_kv<KB, 6>(P, blocks, st);
+    case 7: return launch_decode_kv<KB, 7>(P, blocks, st);
+    default: return launch_decode_kv<KB, 8>(P, blocks, st);
+  }
 }
 
 static int device_sm_count() {
@@ -838,14 +903,16 @@ static int device_sm_count() {
 }
 
 // Blocks of keys per (batch, KV head): fewer keys per CTA fill the chip sooner, and every CTA pays a fixed cost
-// (table, query pieces, first loads, folding its warps) worth about kFixedKeys keys of its loop.  The count with the
+// (tables, query pieces, first loads, folding its warps) worth about kFixedKeys keys of its loop.  The count with the
 // smallest  waves x (keys per CTA + kFixedKeys)  is taken, at most `most` (what the scratch holds) and never blocks
-// of fewer than kDecodeMinKeys keys (two rounds of the CTA's eight warps).
-// 8 KV heads x 32640 tokens, K4/V2: 36 us as 128 CTAs of 2048 keys with one CTA per SM, 30 us as 296 CTAs with two.
-constexpr int kDecodeMinKeys = 256;
-static int decode_blocks(int64_t units, int64_t Sk, int64_t most, int slots) {
+// of fewer than min_keys keys.
+// Decode attention, 8 KV heads x 32640 tokens, K4/V2: 36 us as 128 CTAs of 2048 keys with one CTA per SM, 30 us as 296 CTAs with
+// two.
+constexpr int kDecodeMinKeys = 256;               // two rounds of the CTA's eight warps
+constexpr int kScoreMinKeys = 128;                // one
+static int key_blocks(int64_t units, int64_t Sk, int min_keys, int64_t most, int slots) {
   constexpr int64_t kFixedKeys = 256;
-  int64_t cap = (Sk + kDecodeMinKeys - 1) / kDecodeMinKeys;
+  int64_t cap = (Sk + min_keys - 1) / min_keys;
   if (cap > most) cap = most;
   if (cap > 1024) cap = 1024;
   int64_t best = 1, best_cost = -1;
@@ -878,7 +945,7 @@ int decode_attention(const TqDecodeAttnJob& job, cudaStream_t st) {
   if (job.Sk > 0) {
     const size_t q = ((size_t)rows * kDimA * sizeof(float) + 255) / 256 * 256;
     const int64_t most = (int64_t)((job.workspace_bytes - q) / ((size_t)rows * kPartStride * sizeof(float)));
-    nblk = decode_blocks(job.B * job.Hkv, job.Sk, most, 2 * device_sm_count());
+    nblk = key_blocks(job.B * job.Hkv, job.Sk, kDecodeMinKeys, most, 2 * device_sm_count());
     kKeysPerBlock = (int)(((job.Sk + nblk - 1) / nblk + 15) / 16 * 16);
     nblk = (int)((job.Sk + kKeysPerBlock - 1) / kKeysPerBlock);
   }
@@ -946,11 +1013,14 @@ bool mma_score_eligible(const TqScoreJob& job) {
   return job.D == kDimA && (((uintptr_t)job.idx_bytes) & 15u) == 0 && (((uintptr_t)job.norms) & 1u) == 0;
 }
 
-// logits (and the per-block softmax partials when stats != NULL) for a job whose queries are already rotated
-int mma_score_keys_per_block(const TqScoreJob& job, int min_keys) {
-  return wave_keys_per_block(job.B * job.Hkv, job.Sk, min_keys, 2 * device_sm_count());      // two CTAs per SM
+// Keys per CTA of the call below, `most` blocks at most.  131072 4-bit keys x 8 heads with four query rows: 888 CTAs of 1184 keys (three
+// waves) 59 us a call, one wave of 296 45 us (with the byte tables).  Blocks of 1024 keys and more, as it was, left a short call on few SMs.
+int mma_score_keys_per_block(const TqScoreJob& job, int64_t most) {
+  const int nblk = key_blocks(job.B * job.Hkv, job.Sk, kScoreMinKeys, most, 2 * device_sm_count());      // two CTAs per SM
+  return (int)(((job.Sk + nblk - 1) / nblk + 15) / 16 * 16);
 }
 
+// logits (and the per-block softmax partials when stats != NULL) for a job whose queries are already rotated
 int mma_score_packed(const TqScoreJob& job, const float* qrot, float* stats, int nblk, int keys_per_block, cudaStream_t st) {
   const int64_t blocks = job.B * job.Hkv * nblk;
   const bool eight = job.Hq / job.Hkv * job.Sq > 4;      // more than four query rows per KV head: one pass serves eight

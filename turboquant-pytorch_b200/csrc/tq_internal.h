@@ -23,7 +23,8 @@ int simt_dequantize(const TqDequantizeJob& job, cudaStream_t st);
 // `followed`: the caller launches the next kernel with launch_after()
 int simt_project(const void* x, int x_dtype, int64_t n, int K, const float* m, int N, float* out, cudaStream_t st,
                  bool followed = false);
-size_t simt_score_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int D);
+size_t simt_score_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int D);          // the least
+size_t score_workspace_wanted(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int D);
 int simt_score_packed(const TqScoreJob& job, cudaStream_t st);
 int simt_qjl_compress(const TqQjlCompressJob& job, cudaStream_t st);
 size_t simt_qjl_scores_workspace(int64_t BH, int64_t Sq, int D);
@@ -44,8 +45,8 @@ int few_dequantize(const TqDequantizeJob* jobs, int n_jobs, cudaStream_t st);
 // packed-key logits on the tensor cores, mma.sync (tq_attn_mma.cu); queries already rotated
 bool mma_score_eligible(const TqScoreJob& job);
 int mma_score_packed(const TqScoreJob& job, const float* qrot, float* stats, int nblk, int keys_per_block, cudaStream_t st);
-// keys per CTA (>= min_keys, for which the caller's scratch is sized) that makes the CTAs fill whole waves
-int mma_score_keys_per_block(const TqScoreJob& job, int min_keys);
+// keys per CTA, for at most `most` blocks of keys (what the caller's scratch holds)
+int mma_score_keys_per_block(const TqScoreJob& job, int64_t most);
 
 // decode attention on packed keys and packed values (tq_attn_mma.cu)
 size_t decode_attention_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int keys_per_block);

@@ -1301,17 +1301,31 @@ size_t simt_score_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int D
   return q + (size_t)rows * (nblk > 0 ? nblk : 1) * 2 * sizeof(float);
 }
 
+// Room for the partials of blocks of 128 keys, with which a short call fills the chip, up to a megabyte; never less than
+// simt_score_workspace(), which every caller brings.
+size_t score_workspace_wanted(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int D) {
+  const size_t least = simt_score_workspace(B, Hq, Sq, Sk, D);
+  if (D != 128) return least;
+  const int64_t rows = B * Hq * Sq;
+  const size_t q = ((size_t)rows * D * sizeof(float) + 255) / 256 * 256;
+  const size_t part = (size_t)rows * 2 * sizeof(float);
+  size_t blocks = (size_t)((Sk + 127) / 128);
+  if (blocks * part > ((size_t)1 << 20)) blocks = part > 0 ? ((size_t)1 << 20) / part : 0;
+  const size_t want = q + blocks * part;
+  return want > least && want <= TQ_SCORE_NOALLOC_SCRATCH_BYTES ? want : least;
+}
+
 int simt_score_packed(const TqScoreJob& job, cudaStream_t st) {
   const int64_t rows = job.B * job.Hq * job.Sq;
   if (rows == 0 || job.Sk == 0) return TQ_OK;
-  // the tensor-core kernel takes its block size as a parameter: blocks of at least SCORE_KEYS_PER_BLOCK keys (the
-  // scratch is sized for that) chosen so that the CTAs fill whole waves
+  // the tensor-core kernel takes its block size as a parameter, with as many blocks as the scratch has room for
   const bool use_mma = mma_score_eligible(job);
-  const int kpb = use_mma ? mma_score_keys_per_block(job, SCORE_KEYS_PER_BLOCK) : SCORE_KEYS_PER_BLOCK;
-  const int nblk = (int)((job.Sk + kpb - 1) / kpb);
   float* qrot = reinterpret_cast<float*>(job.workspace);
-  size_t qbytes = ((size_t)rows * job.D * sizeof(float) + 255) / 256 * 256;
+  const size_t qbytes = ((size_t)rows * job.D * sizeof(float) + 255) / 256 * 256;
   float* stats = reinterpret_cast<float*>(reinterpret_cast<char*>(job.workspace) + qbytes);
+  const int64_t most = (int64_t)((job.workspace_bytes - qbytes) / ((size_t)rows * 2 * sizeof(float)));
+  const int kpb = use_mma ? mma_score_keys_per_block(job, most) : SCORE_KEYS_PER_BLOCK;
+  const int nblk = (int)((job.Sk + kpb - 1) / kpb);
   int rc = simt_project(job.q, job.q_dtype, rows, job.D, job.rotation_t, job.D, qrot, st, use_mma);
   if (rc != TQ_OK) return rc;
   const int64_t blocks = job.B * job.Hkv * nblk;
