@@ -489,7 +489,7 @@ def run_side_workload(args, dev):
                                    "k_qjl_score_packed straight from the packed rows (bytes = packed key + 64 fp32 scores)"},
                    roofline={"bound": "tensor", "achieved": n * 393216 * steps / t1 / 1e12, "peak": tpeak,
                              "unit": "TFLOP/s", "frac": n * 393216 * steps / t1 / 1e12 / tpeak, "traffic": None,
-                             "note": "compress = three tcgen05 contraction launches (k_umma_v2_stage); flops are "
+                             "note": "compress = three tcgen05 contractions in one launch (k_umma_v2_stage); flops are "
                                      "the algorithmic 6 D^2 per vector, the hi/lo passes execute 2.7x that; the "
                                      "score kernel is HBM-bound, see scores.frac_of_hbm_peak"})
     else:  # decode

@@ -1,7 +1,7 @@
 // Tensor-core (tcgen05 / TMEM / TMA) path for the MSE + QJL compress stage (K4), fp16 vectors,
 // head_dim 128 or 256.  The reference's three chained D x D contractions
-// (turboquant/compressors.py:83-120) run as three launches of one contraction kernel with a
-// different epilogue each; operands that are fp32 in the reference are carried as fp16 pieces
+// (turboquant/compressors.py:83-120) run as three stages of one persistent kernel, each with its own
+// epilogue; operands that are fp32 in the reference are carried as fp16 pieces
 // hi + lo (lo reaches into fp16 subnormals), so products match an fp32 matmul to ~2^-21:
 //
 //   stage 1  y = x Pi^T            A = x (exact fp16), B = Pi hi/lo.  Epilogue: ||y|| = ||x||, scale,
@@ -11,12 +11,18 @@
 //                                  k_mse (fp16 out), residual r = x - k, ||r|| (out), residual pieces -> scratch
 //   stage 3  p = r S^T             A = residual pieces, B = S hi/lo.  Epilogue: signs (int8 out)
 //
-// A persistent CTA per SM walks 128-vector tiles.  warp 0: TMA loads of the tile's A chunks
-// (128 rows x 64 columns, 128-byte swizzle, one slot per k-chunk and piece) and bulk copies of
-// B chunks (128 output columns x 64 k, 16 KB, pre-swizzled image in global memory, L2-resident)
-// through a ring; warp 1: tcgen05.mma M=128 N=128 K=16 into one 128-column accumulator per
-// block of 128 output columns; the other warps: per tile in flight (two) one epilogue warpgroup
-// per block of 128 columns, thread = vector.  Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, records a
+// A CTA per SM walks its 128-vector tiles two at a time: stage 1 of both, stage 2 of both, stage 3 of both.  A stage of one tile
+// needs nothing but the stage before of the same tile, so while one tile is in its epilogue the other is on the tensor
+// core, whatever their stages, and the scratch between the stages is the two tiles' own (it stays in L2: as three launches
+// over all vectors, stages 2 and 3 moved 866 MB through DRAM for 262144 vectors of head_dim 256, of which 540 MB were
+// residual pieces written and read again, and each stage waited for its own bottleneck: nearest centroids in stage 1,
+// memory in 2, the operand images in 3.  That call takes 399 -> 322 us where it runs on and on, under the power cap, and 290 in a
+// short burst; 445 000 clocks, of which the tensor core's own are 228 000.  What bounds it then is the shared-memory data path: an
+// MMA of N = 256 reads 12 KB in its 129 clocks and B arrives at 64 bytes a clock, which leaves the epilogues little).
+//
+// Warps: 0 the A side's TMA loads (128 rows x 64 columns, 128-byte swizzle) and the index bytes; 1 issues tcgen05.mma M=128 N=D
+// K=16 into one accumulator per tile; four epilogue warpgroups; two expander warps.  Warp 0 also issues the
+// bulk copies of B chunks (pre-swizzled image in global memory, L2-resident) through a ring of their own.  Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, records a
 // status word and leaves through the normal exit.
 
 #include <cuda.h>
@@ -37,7 +43,8 @@ namespace {
 
 constexpr int kRowsT = 128;                    // vectors per tile (MMA M)
 constexpr uint32_t kChunk = 128 * 128;         // 128 rows x 64 fp16 = 16 KB (an A chunk or a B chunk)
-constexpr int kNB = 4;                         // B ring stages
+constexpr int kNB = 3;                         // B ring stages
+constexpr int kNA = 3;                         // A ring slots
 constexpr uint32_t kRawChunk = 128 * 64;       // index bytes of a k-chunk: 128 rows x 64
 constexpr int kExpandThreads = 64;             // stage 2: two expander warps, thread = two rows
 
@@ -45,18 +52,21 @@ template <int D>
 struct VCfg {
   static constexpr int KC = D / 64;            // k chunks
   static constexpr int NBLK = D / 128;         // blocks of 128 output columns
-  // A: two k-chunk slots per piece (chunk kc lands in slot kc & 1 and is released as soon as its MMAs are done), so
+  // A: slots of one k-chunk (both pieces), released as soon as its MMAs are done, so
   // that the B ring can hold stages of ALL output columns: one MMA of N = D per k-step instead of one per block of
   // 128 columns, which reads the A operand once (M = 128 takes 65 clocks at N = 128 and 129 at N = 256)
-  static constexpr int kASlots = 2;
   static constexpr uint32_t kBStage = NBLK * kChunk;                     // one k-chunk of B for all D output columns
-  static constexpr uint32_t kOffA = 0;                                   // [piece 2][slot 2] chunks
-  static constexpr uint32_t kOffB = kOffA + 2u * kASlots * kChunk;       // ring
+  static constexpr uint32_t kOffA = 0;                                   // [slot][piece] chunks
+  static constexpr uint32_t kOffB = kOffA + 2u * kNA * kChunk;           // ring
   static constexpr uint32_t kOffRaw = kOffB + kNB * kBStage;             // stage 2: index bytes of two k-chunks
-  static constexpr uint32_t kOffTab = kOffRaw + 2u * kRawChunk;          // thresholds, centroid piece pairs, cell table, partial sums
-  static constexpr uint32_t kOffBar = kOffTab + 6144;
-  static constexpr int kThreads = 64 + 2 * NBLK * 128;                   // two tiles in flight, one warpgroup per 128 columns
-  static constexpr int threads(int stage) { return kThreads + (stage == 2 ? kExpandThreads : 0); }
+  static constexpr uint32_t kOffTab = kOffRaw + 2u * kRawChunk;          // thresholds, centroid piece pairs, cell table, partial sums, norms
+  static constexpr uint32_t kOffBar = kOffTab + 9216;
+  // Epilogue: four warpgroups, one per 64 columns of a tile: all four on every tile at head_dim 256, two on each of the two
+  // tiles in flight at head_dim 128.
+  static constexpr int kWgs = D / 64;                                    // warpgroups of a tile
+  static constexpr int kEpiThreads = 512;
+  static constexpr int kExpandBegin = 64 + kEpiThreads;
+  static constexpr int kThreads = kExpandBegin + kExpandThreads;
   static constexpr uint32_t kUsedBytes = kOffBar + 256;
   static constexpr uint32_t kSmemBytes = kUsedBytes + 1024;
   static constexpr uint32_t kImageBytes = 2u * KC * NBLK * kChunk;       // [piece][kc][nb] chunks of one operand
@@ -64,17 +74,18 @@ struct VCfg {
 };
 static_assert(VCfg<256>::kSmemBytes <= 232448 && VCfg<128>::kSmemBytes <= 232448, "shared memory budget");
 
-struct V2Stage {
-  CUtensorMap a_hi_map;      // fp16 (D, n), box 64 x 128, 128-byte swizzle
-  CUtensorMap a_lo_map;      // second piece of A (stages 2 and 3)
-  const uint8_t* b_image;    // [piece][kc][nb][128 rows x 128 bytes swizzled]
-  const float* codebook;     // stage 1
-  const uint16_t* x;         // stage 2: the original vectors (n, D) fp16
-  uint16_t* p_hi;            // scratch (n, D): after stage 1 (156 -> 124 us for the call below with one byte per coordinate
-                             // instead of four of centroid pieces) the first D bytes of a row are the vector's index bytes, after
+struct V2Args {
+  CUtensorMap x_map;         // fp16 (D, n), box 64 x 128, 128-byte swizzle
+  CUtensorMap idx_map;       // index bytes: rows of D bytes, 2 D bytes apart, at the head of the rows of p_hi
+  CUtensorMap hi_map;        // the residual's pieces
+  CUtensorMap lo_map;
+  const uint8_t* images;     // three operand images [piece][kc][nb][128 rows x 128 bytes swizzled]
+  const float* codebook;
+  const uint16_t* x;         // the vectors (n, D) fp16
+  uint16_t* p_hi;            // scratch rows (D): after stage 1 the first D bytes of a row are the vector's index bytes, after
                              // stage 2 (which reads a tile's bytes before it writes the tile's rows) the residual's pieces
   uint16_t* p_lo;
-  float* norms;              // scratch (n): ||x||
+  float* vec_norms_out;      // optional, ||x||
   uint8_t* idx_u8_out;       // stage 1: optional, one index per byte (n, D)
   uint8_t* idx_packed_out;   // stage 1: optional, bit-packed rows (n, G), first index in the high bits
   uint8_t* sign_bits_out;    // stage 3: optional, one bit per sign (n, D / 8), coordinate j in bit 7 - j % 8, set for +1
@@ -87,7 +98,7 @@ struct V2Stage {
   int32_t bits;
 };
 
-__device__ int g_v2_status;    // 0 = ok; otherwise (stage << 20) | (code << 16) | block
+__device__ int g_v2_status;    // 0 = ok; otherwise (code << 16) | block
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
@@ -112,9 +123,9 @@ __global__ void k_v2_operand_image(const float* __restrict__ rotation, const flo
   const int64_t ld_n = blockIdx.y == 0 ? D : 1, ld_k = blockIdx.y == 0 ? 1 : blockIdx.y == 1 ? D : M;
   uint8_t* image = images + (size_t)blockIdx.y * VCfg<D>::kImageBytes;
   const int n = e / D, k = e % D;
-  // operand row (= accumulator column) n of Pi^T holds output column 16 t + 2 r + j of its 64, where n = 8 r + 2 t + j: the
-  // stage's TMEM loads give thread t of a quad the accumulator columns 8 r + 2 t + {0, 1}, which are then 16 in a row
-  const int col = blockIdx.y == 1 ? (n & ~63) + 16 * ((n >> 1) & 3) + 2 * ((n >> 3) & 7) + (n & 1) : n;
+  // operand row (= accumulator column) n holds output column 16 t + 2 r + j of its 64, where n = 8 r + 2 t + j: the
+  // epilogues' TMEM loads give thread t of a quad the accumulator columns 8 r + 2 t + {0, 1}, which are then 16 in a row
+  const int col = (n & ~63) + 16 * ((n >> 1) & 3) + 2 * ((n >> 3) & 7) + (n & 1);
   const float v = __ldg(src + (int64_t)col * ld_n + (int64_t)k * ld_k);
   const __half hi = __float2half_rn(v);
   const __half lo = __float2half_rn(v - __half2float(hi));
@@ -176,16 +187,225 @@ __device__ __forceinline__ void tmem_ld_quads(uint32_t taddr, uint32_t (&r)[32])
                : "memory");
 }
 
-template <int D, int STAGE>
-__global__ void __launch_bounds__(VCfg<D>::kThreads + (STAGE == 2 ? kExpandThreads : 0), 1) k_umma_v2_stage(const __grid_constant__ V2Stage p) {
+// Quantiser of a row's 16 accumulator columns: four index bytes a word.  The search shortcut of a codebook with at most 31
+// thresholds (see tq_umma.cu: a candidate from a cubic, its threshold from a lane, one saturating compare), or any codebook.
+struct V2Quantiser {
+  float s, c1, c2, c3, thr_lane_h;      // shortcut; threshold[lane] * 2^40
+  float t0, t1, t2;                     // the first three thresholds * 2^40
+  float s_inv, h_inv;                   // per vector: s / (norm + 1e-8) and 2^40 / (norm + 1e-8)
+};
+// Row hh of the two whose 16 columns each a thread holds: a[4 j + 2 hh + {0, 1}] are columns 2 j, 2 j + 1.  COUNT: up to three thresholds
+// (1- and 2-bit codes) are all compared, from registers; a shuffle per coordinate takes as much of the shared-memory data
+// path as the tensor core's operands leave.
+template <bool COUNT, bool LINEAR>
+__device__ __forceinline__ void index_bytes_fast(const uint32_t (&a)[32], int hh, const V2Quantiser& q, uint32_t (&ib)[4]) {
+  constexpr uint32_t kMagic = 0x4B000000u;     // bits of 2^23, which ride along with every index
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    uint32_t acc = 0u - (kMagic + (kMagic << 8) + (kMagic << 16) + (kMagic << 24));
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const float r = __uint_as_float(a[4 * (2 * w + (b >> 1)) + 2 * hh + (b & 1)]);
+      float t, pf, u;
+      if constexpr (COUNT) {
+        float p1, p2;
+        asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(pf) : "f"(r), "f"(q.h_inv), "f"(-q.t0));
+        asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(p1) : "f"(r), "f"(q.h_inv), "f"(-q.t1));
+        asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(p2) : "f"(r), "f"(q.h_inv), "f"(-q.t2));
+        u = p1 + (p2 + 8388608.0f);
+      } else {
+        asm("fma.rn.sat.f32 %0, %1, %2, 0f3F000000;" : "=f"(t) : "f"(r), "f"(q.s_inv));
+        if constexpr (LINEAR) u = fmaf(q.c1, t, 8388608.0f);
+        else u = fmaf(fmaf(fmaf(q.c3, t, q.c2), t, q.c1), t, 8388608.0f);
+        const float thr_h = __shfl_sync(0xffffffffu, q.thr_lane_h, __float_as_int(u));
+        asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(pf) : "f"(r), "f"(q.h_inv), "f"(-thr_h));
+      }
+      acc = __float_as_uint(u + pf) * (1u << (8 * b)) + acc;
+    }
+    ib[w] = acc;
+  }
+}
+// Out of line, its arguments by value: cold, and nothing of it weighs on the path that runs.
+__device__ __noinline__ uint4 index_bytes_any(uint4 v0, uint4 v1, uint4 v2, uint4 v3, float inv, const float* codebook, const float* thr,
+                                              const uint8_t* cells, int bits) {
+  const int mode = (int)__ldg(codebook + 512);
+  const float s = __ldg(codebook + 513), c1 = __ldg(codebook + 514), c2 = __ldg(codebook + 515), c3 = __ldg(codebook + 516);
+  const uint32_t v[16] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y, v2.z, v2.w, v3.x, v3.y, v3.z, v3.w};
+  uint32_t ib[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const float y = __uint_as_float(v[e]) * inv;
+    int idx;
+    if (mode != 0) {
+      // candidate e0 with index in {e0, e0 + 1} (verified on the host for every y), then one exact compare
+      float t;
+      asm("fma.rn.sat.f32 %0, %1, %2, 0f3F000000;" : "=f"(t) : "f"(y), "f"(s));
+      int e0;
+      if (mode == 1) e0 = __float_as_int(fmaf(fmaf(fmaf(c3, t, c2), t, c1), t, 8388608.0f)) & 0xFF;
+      else e0 = cells[__float_as_int(fmaf(t, 1024.0f, 8388608.0f)) & 0x7FF];
+      idx = e0 + (y > thr[e0] ? 1 : 0);
+    } else {
+      int lo = 0, hi = (1 << bits) - 1;
+      for (int step = 0; step < bits; ++step) {
+        const int mid = (lo + hi) >> 1;
+        if (y > thr[mid]) lo = mid + 1; else hi = mid;
+      }
+      idx = lo;
+    }
+    ib[e >> 2] |= (uint32_t)idx << (8 * (e & 3));
+  }
+  return make_uint4(ib[0], ib[1], ib[2], ib[3]);
+}
+
+// 16 index bytes as 16 / ipb bytes of a packed row
+__device__ __forceinline__ void store_packed16(uint8_t* dst, const uint32_t (&ib)[4], int bits) {
+  const int ipb = 8 / bits;
+  if (ipb == 1) {
+    *reinterpret_cast<uint4*>(dst) = make_uint4(ib[0], ib[1], ib[2], ib[3]);
+  } else if (ipb == 2) {           // 3- and 4-bit codes: byte k = idx[2k] << bits | idx[2k+1]
+    uint32_t o[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t a = ib[2 * h], b = ib[2 * h + 1];
+      const uint32_t b0 = (((a >> 0) & 0xFFu) << bits) | ((a >> 8) & 0xFFu), b1 = (((a >> 16) & 0xFFu) << bits) | (a >> 24);
+      const uint32_t b2 = (((b >> 0) & 0xFFu) << bits) | ((b >> 8) & 0xFFu), b3 = (((b >> 16) & 0xFFu) << bits) | (b >> 24);
+      o[h] = b0 | (b1 << 8) | (b2 << 16) | (b3 << 24);
+    }
+    *reinterpret_cast<uint2*>(dst) = make_uint2(o[0], o[1]);
+  } else if (ipb == 4) {           // 2-bit codes
+    uint32_t o = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t a = ib[k];
+      o |= ((((a >> 0) & 3u) << 6) | (((a >> 8) & 3u) << 4) | (((a >> 16) & 3u) << 2) | ((a >> 24) & 3u)) << (8 * k);
+    }
+    *reinterpret_cast<uint32_t*>(dst) = o;
+  } else {                          // 1-bit codes
+    uint32_t o = 0u;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) o |= ((ib[e >> 2] >> (8 * (e & 3))) & 1u) << (8 * (e >> 3) + 7 - (e & 7));
+    *reinterpret_cast<uint16_t*>(dst) = (uint16_t)o;
+  }
+}
+
+// Stage 2's operand from index bytes.  Up to 2 bits the fp16 pieces of all centroids fit two registers each and a byte permute picks
+// those of two coordinates at once, with 2 idx and 2 idx + 1 as its selectors; with 3 bits the low and the high bytes of a
+// piece fit two registers each, and two permutes pair what they pick.  A look-up in shared memory per coordinate, two warps
+// of them, took 2400 clocks per 64 coordinates of a tile where the MMAs take 1550.
+//   pool, up to 2 bits: {hi01, hi23, lo01, lo23};  3 bits: low bytes of hi (2), high bytes of hi (2), the same of lo
+__device__ __forceinline__ void piece_pool(const uint32_t* lut, int bits, uint32_t (&pool)[8]) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    if (bits <= 2) {
+      pool[j] = __byte_perm(lut[2 * j], lut[2 * j + 1], 0x5410);
+      pool[2 + j] = __byte_perm(lut[2 * j], lut[2 * j + 1], 0x7632);
+    } else {
+#pragma unroll
+      for (int byte = 0; byte < 4; ++byte) {
+        uint32_t w = 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w |= ((lut[4 * j + k] >> (8 * byte)) & 0xFFu) << (8 * k);
+        pool[2 * byte + j] = w;
+      }
+    }
+  }
+}
+// 4 index bytes -> operand words of the high and of the low pieces
+template <int BITS>
+__device__ __forceinline__ void pieces_of_four(uint32_t w, const uint32_t (&pool)[8], uint32_t lut, uint32_t* hi, uint32_t* lo) {
+  if constexpr (BITS == 2) {
+    const uint32_t sel = w * 0x22u + 0x10101010u;
+    hi[0] = __byte_perm(pool[0], pool[1], sel & 0xFFFFu);
+    lo[0] = __byte_perm(pool[2], pool[3], sel & 0xFFFFu);
+    hi[1] = __byte_perm(pool[0], pool[1], sel >> 16);
+    lo[1] = __byte_perm(pool[2], pool[3], sel >> 16);
+  } else if constexpr (BITS == 3) {
+    uint32_t sel = (w | (w >> 4)) & 0x00FF00FFu;
+    sel = (sel | (sel >> 8)) & 0x7777u;
+    const uint32_t h0 = __byte_perm(pool[0], pool[1], sel), h1 = __byte_perm(pool[2], pool[3], sel);
+    const uint32_t l0 = __byte_perm(pool[4], pool[5], sel), l1 = __byte_perm(pool[6], pool[7], sel);
+    hi[0] = __byte_perm(h0, h1, 0x5140); hi[1] = __byte_perm(h0, h1, 0x7362);
+    lo[0] = __byte_perm(l0, l1, 0x5140); lo[1] = __byte_perm(l0, l1, 0x7362);
+  } else {
+    uint32_t e[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t off = u == 0 ? ((w << 2) & 0x3FCu) : ((w >> (8 * u - 2)) & 0x3FCu);
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e[u]) : "r"(lut + off));
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      hi[j] = __byte_perm(e[2 * j], e[2 * j + 1], 0x5410);
+      lo[j] = __byte_perm(e[2 * j], e[2 * j + 1], 0x7632);
+    }
+  }
+}
+template <int BITS>
+__device__ __forceinline__ void expand_chunk(uint32_t raw, uint32_t dst0, int et, const uint32_t (&pool)[8], uint32_t lut) {
+#pragma unroll 1
+  for (int row = et; row < kRowsT; row += kExpandThreads) {
+    const uint32_t r1 = (uint32_t)(row >> 1) & 1u, r2 = (uint32_t)(row >> 2) & 1u;
+    const uint32_t g = ((r2 ^ r1) << 1) | r2;
+    const uint32_t src = raw + (uint32_t)row * 64u, dst = dst0 + (uint32_t)row * 128u;
+    uint4 x[4];
+#pragma unroll
+    for (uint32_t c = 0; c < 4; ++c) x[c] = ld_shared_v4(src + (c ^ g) * 16u);
+#pragma unroll
+    for (uint32_t c = 0; c < 4; ++c) {
+      const uint32_t xw[4] = {x[c].x, x[c].y, x[c].z, x[c].w};
+#pragma unroll
+      for (uint32_t h = 0; h < 2; ++h) {                  // 8 coordinates: one 16-byte operand chunk per piece
+        uint32_t hi[4], lo[4];
+        pieces_of_four<BITS>(xw[2 * h], pool, lut, hi, lo);
+        pieces_of_four<BITS>(xw[2 * h + 1], pool, lut, hi + 2, lo + 2);
+        const uint32_t at = dst + (((2u * (c ^ g) + h) ^ (uint32_t)(row & 7)) << 4);
+        st_shared_v4(at, hi[0], hi[1], hi[2], hi[3]);
+        st_shared_v4(at + kChunk, lo[0], lo[1], lo[2], lo[3]);
+      }
+    }
+  }
+}
+
+// two fused multiply-adds in one instruction (sm_100): the same IEEE results per half as fmaf
+__device__ __forceinline__ unsigned long long square2(uint32_t lo, uint32_t hi, unsigned long long sum) {
+  unsigned long long v, d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(v), "l"(sum));
+  return d;
+}
+
+// The CTA's walk: item (stage, tile), the tiles in pairs, a pair's stages one after the other, tile slot 0 before slot 1.  Every
+// role goes through the same items.
+struct Walk {
+  int n_local, i0 = 0, stage = 1, slot = 0;
+  __device__ __forceinline__ explicit Walk(int n) : n_local(n) {}
+  __device__ __forceinline__ bool done() const { return i0 >= n_local; }
+  __device__ __forceinline__ int tile() const { return i0 + slot; }
+  __device__ __forceinline__ int use() const { return (i0 >> 1) * 3 + stage - 1; }     // the slot's items before this one
+  __device__ __forceinline__ void next() {
+    if (slot == 0 && i0 + 1 < n_local) { slot = 1; return; }
+    slot = 0;
+    if (++stage > 3) { stage = 1; i0 += 2; }
+  }
+};
+template <typename F>
+__device__ __forceinline__ bool walk_items(int n_local, F&& f) {      // f(tile, slot, stage, use) returns false to leave
+#pragma unroll 1
+  for (Walk w(n_local); !w.done(); w.next())
+    if (!f(w.tile(), w.slot, w.stage, w.use())) return false;
+  return true;
+}
+
+// STAGE: the last stage that the launch runs; only the whole walk is launched.
+template <int D, int STAGE = 3>
+__global__ void __launch_bounds__(VCfg<D>::kThreads, 1) k_umma_v2_stage(const __grid_constant__ V2Args p) {
   // The wait comes before the TMEM allocation: a dependent that held TMEM while its predecessor still had to allocate some
-  // on the same SM would wait for good.  For the same reason the last stage does not let a dependent start: what follows it
-  // is not this library's, and may allocate TMEM before it waits.
+  // on the same SM would wait for good.  For the same reason the last kernel of the call does not let a dependent start: what
+  // follows it is not this library's, and may allocate TMEM before it waits.
   if constexpr (STAGE != 3) pdl_trigger();
   pdl_wait();
   using C = VCfg<D>;
   constexpr int KC = C::KC, NBLK = C::NBLK;
-  constexpr int PA = STAGE == 1 ? 1 : 2;       // pieces of A
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
@@ -193,53 +413,62 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads + (STAGE == 2 ? kExpandThrea
     uint32_t dyn_bytes;
     asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
     if (base - smem_u32(smem_raw) + C::kUsedBytes > dyn_bytes) {     // the layout does not fit: report, do nothing
-      if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, (STAGE << 20) | (9 << 16) | (int)blockIdx.x);
+      if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, (9 << 16) | (int)blockIdx.x);
       return;
     }
   }
-  const uint32_t a_smem = base + C::kOffA;
+  const uint32_t a_smem = base + C::kOffA;      // slot s: its high (or only) piece, then its low piece
   const uint32_t b_smem = base + C::kOffB;
+  const uint32_t raw_smem = base + C::kOffRaw;
   float* thr_s = reinterpret_cast<float*>(gbase + C::kOffTab);
   uint32_t* lut_s = reinterpret_cast<uint32_t*>(gbase + C::kOffTab + 1024);
   uint8_t* cells_s = gbase + C::kOffTab + 2048;                        // 1028 bytes
-  float* part_s = reinterpret_cast<float*>(gbase + C::kOffTab + 4096); // [slot 2][block 2][row 128] partial sums of the residual norms
-  const uint32_t bar0 = base + C::kOffBar;
-  const uint32_t bar_afull = bar0;                          // [kASlots] TMA -> MMA (all pieces of a k-chunk)
-  const uint32_t bar_aempty = bar_afull + 8 * 4;            // [kASlots] MMA commit -> producer
-  const uint32_t bar_bfull = bar_aempty + 8 * 4;            // [kNB] bulk copy -> MMA
-  const uint32_t bar_bempty = bar_bfull + 8 * kNB;          // [kNB] MMA commit -> producer
+  float* part_s = reinterpret_cast<float*>(gbase + C::kOffTab + 4096); // [slot 2][warpgroup 4][row 128] partial sums of the norms
+  float* norm_s = reinterpret_cast<float*>(gbase + C::kOffTab + 8192); // [slot 2][row 128] vector norms, stage 1 -> 2
+  const uint32_t bar_afull = base + C::kOffBar;             // [kNA] TMA or expanders -> MMA (all pieces of a k-chunk)
+  const uint32_t bar_aempty = bar_afull + 8 * kNA;          // [kNA] MMA commit -> producer, expanders
+  const uint32_t bar_bfull = bar_aempty + 8 * kNA;          // [kNB] bulk copy -> MMA
+  const uint32_t bar_bempty = bar_bfull + 8 * kNB;          // [kNB] MMA commit -> B producer
   const uint32_t bar_tfull = bar_bempty + 8 * kNB;          // [2] MMA commit -> epilogue
-  const uint32_t bar_tempty = bar_tfull + 16;               // [2] epilogue (4 arrivals) -> MMA
-  const uint32_t bar_rfull = bar_tempty + 16;               // [2] stage 2: TMA -> expanders (index bytes)
+  const uint32_t bar_tempty = bar_tfull + 16;               // [2] epilogue (a warp each) -> MMA
+  const uint32_t bar_ready = bar_tempty + 16;               // [2] epilogue (a warp each): the scratch of the next stage is written
+  const uint32_t bar_rfull = bar_ready + 16;                // [2] stage 2: TMA -> expanders (index bytes)
   const uint32_t bar_rempty = bar_rfull + 16;               // [2] stage 2: expanders -> producer
-  const uint32_t raw_smem = base + C::kOffRaw;
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + C::kOffBar + 200);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + C::kOffBar + 208);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + C::kOffBar + 216);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + C::kOffBar + 224);
+  static_assert(16 * (kNA + kNB) + 80 <= 216, "barriers");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total = p.tiles;
   const int t0 = (int)((int64_t)total * blockIdx.x / gridDim.x);
   const int t1 = (int)((int64_t)total * (blockIdx.x + 1) / gridDim.x);
   const int n_local = t1 - t0;
+  auto failed = [&](int code) {
+    *abort_flag = 1;
+    if (p.status != nullptr) atomicCAS(p.status, 0, (code << 16) | (int)blockIdx.x);
+  };
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < C::kASlots; ++i) { mbar_init(bar_afull + 8 * i, STAGE == 2 ? kExpandThreads : 1); mbar_init(bar_aempty + 8 * i, 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(bar_rfull + 8 * i, 1); mbar_init(bar_rempty + 8 * i, kExpandThreads); }
+    for (int i = 0; i < kNA; ++i) { mbar_init(bar_afull + 8 * i, 1); mbar_init(bar_aempty + 8 * i, 1); }
     for (int i = 0; i < kNB; ++i) { mbar_init(bar_bfull + 8 * i, 1); mbar_init(bar_bempty + 8 * i, 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(bar_tfull + 8 * i, 1); mbar_init(bar_tempty + 8 * i, 4 * NBLK); }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar_tfull + 8 * i, 1);
+      mbar_init(bar_tempty + 8 * i, 4 * C::kWgs);
+      mbar_init(bar_ready + 8 * i, 4 * C::kWgs);
+      mbar_init(bar_rfull + 8 * i, 1);
+      mbar_init(bar_rempty + 8 * i, 1);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if constexpr (STAGE != 3) {
-    if (threadIdx.x >= 64 && threadIdx.x < 64 + 256) {
-      const int e = threadIdx.x - 64;
-      thr_s[e] = __ldg(p.codebook + kThresholdOff + e);
-      const float c = __ldg(p.codebook + kCentroidOff + e);
-      const __half h = __float2half_rn(c);
-      const __half l = __float2half_rn(c - __half2float(h));
-      lut_s[e] = (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
-      for (int w = e; w < 257; w += 256) reinterpret_cast<uint32_t*>(cells_s)[w] = __float_as_uint(__ldg(p.codebook + 528 + w));
-    }
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + 256) {
+    const int e = threadIdx.x - 64;
+    thr_s[e] = __ldg(p.codebook + kThresholdOff + e);
+    const float c = __ldg(p.codebook + kCentroidOff + e);
+    const __half h = __float2half_rn(c);
+    const __half l = __float2half_rn(c - __half2float(h));
+    lut_s[e] = (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
+    for (int w = e; w < 257; w += 256) reinterpret_cast<uint32_t*>(cells_s)[w] = __float_as_uint(__ldg(p.codebook + 528 + w));
   }
   if (warp == 1) tmem_alloc(smem_u32((const void*)tmem_slot), C::kTmemCols);
   tc_fence_before();
@@ -248,45 +477,71 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads + (STAGE == 2 ? kExpandThrea
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    // ------------------------------------------------------------ producer
+    // ------------------------------------------------------------ producer.  The A side and B have a position each and
+    // whichever has room goes on: B's chunks of a stage are there when its A is, which may have to wait for an epilogue.
     if (lane == 0) {
+      int ac = 0, kc = 0;                                   // A: running chunk counter (slot ac % kNA, use ac / kNA), chunk of the item
+      int rc = 0;                                           // running count of index chunks
+      int loads = 0;                                        // bit s: the last use of A slot s was a load of ours
+      int bc = 0, kp = 0;                                   // B: running chunk counter, chunk and piece of the item
+      bool ready = false;                                   // what the stage before wrote is there
+      Walk wa(n_local), wb(n_local);
+      long long start = 0;
       bool ok = true;
-      int bc = 0;                                           // running B chunk counter
-      int ac = 0;                                           // running A chunk counter: slot ac & 1, use ac / 2
-      for (int i = 0; i < n_local && ok; ++i) {
-        const int row0 = (t0 + i) * kRowsT;
-        for (int kc = 0; kc < KC && ok; ++kc, ++ac) {
-          const int as = ac % C::kASlots;
-          if constexpr (STAGE == 2) {                       // the operand itself is written by the expanders
-            ok = mbar_wait(bar_rempty + 8 * as, (uint32_t)(((ac / C::kASlots) & 1) ^ 1), abort_flag);
-            if (!ok) break;
-            mbar_arrive_expect_tx(bar_rfull + 8 * as, kRawChunk);
-            tma_load_2d(raw_smem + as * kRawChunk, &p.a_hi_map, kc * 64, row0, bar_rfull + 8 * as);
-          } else {
-            ok = mbar_wait(bar_aempty + 8 * as, (uint32_t)(((ac / C::kASlots) & 1) ^ 1), abort_flag);
-            if (!ok) break;
-            mbar_arrive_expect_tx(bar_afull + 8 * as, PA * kChunk);
-            tma_load_2d(a_smem + as * kChunk, &p.a_hi_map, kc * 64, row0, bar_afull + 8 * as);
-            if constexpr (PA == 2) tma_load_2d(a_smem + (C::kASlots + as) * kChunk, &p.a_lo_map, kc * 64, row0, bar_afull + 8 * as);
+      for (uint32_t idle = 0; !wa.done() || !wb.done();) {
+        bool moved = false;
+        if (!wb.done() && mbar_try_wait(bar_bempty + 8 * (bc % kNB), (uint32_t)(((bc / kNB) & 1) ^ 1))) {
+          const int s = bc % kNB;
+          mbar_arrive_expect_tx(bar_bfull + 8 * s, C::kBStage);
+          bulk_load(b_smem + s * C::kBStage, p.images + (size_t)(wb.stage - 1) * C::kImageBytes + (size_t)((kp & 1) * KC + (kp >> 1)) * C::kBStage,
+                    C::kBStage, bar_bfull + 8 * s);
+          ++bc;
+          if (++kp == 2 * KC) { kp = 0; wb.next(); }
+          moved = true;
+        }
+        if (!wa.done()) {
+          if (!ready) {
+            ready = wa.stage == 1 || mbar_try_wait(bar_ready + 8 * wa.slot, (uint32_t)(wa.stage & 1));
           }
-          for (int pb = 0; pb < 2; ++pb) {
-            const int s = bc % kNB;
-            ok = mbar_wait(bar_bempty + 8 * s, (uint32_t)(((bc / kNB) & 1) ^ 1), abort_flag);
-            if (!ok) break;
-            mbar_arrive_expect_tx(bar_bfull + 8 * s, C::kBStage);
-            bulk_load(b_smem + s * C::kBStage, p.b_image + (size_t)(pb * KC + kc) * C::kBStage, C::kBStage, bar_bfull + 8 * s);
-            ++bc;
+          const bool raw = wa.stage == 2;                   // the operand itself is written by the expanders
+          if (ready && (raw ? mbar_try_wait(bar_rempty + 8 * (rc & 1), (uint32_t)(((rc >> 1) & 1) ^ 1))
+                            : mbar_try_wait(bar_aempty + 8 * (ac % kNA), (uint32_t)(((ac / kNA) & 1) ^ 1)))) {
+            // the scratch rows are those of the CTA's first two tiles
+            const int row0 = wa.stage == 1 ? (t0 + wa.tile()) * kRowsT : (t0 + wa.slot) * kRowsT;
+            const int as = ac % kNA;
+            if (raw) {
+              mbar_arrive_expect_tx(bar_rfull + 8 * (rc & 1), kRawChunk);
+              tma_load_2d(raw_smem + (rc & 1) * kRawChunk, &p.idx_map, kc * 64, row0, bar_rfull + 8 * (rc & 1));
+              ++rc;
+              loads &= ~(1 << as);
+            } else {
+              const uint32_t dst = a_smem + 2u * as * kChunk;
+              mbar_arrive_expect_tx(bar_afull + 8 * as, wa.stage == 1 ? kChunk : 2 * kChunk);
+              tma_load_2d(dst, wa.stage == 1 ? &p.x_map : &p.hi_map, kc * 64, row0, bar_afull + 8 * as);
+              if (wa.stage == 3) tma_load_2d(dst + kChunk, &p.lo_map, kc * 64, row0, bar_afull + 8 * as);
+              loads |= 1 << as;
+            }
+            ++ac;
+            if (++kc == KC) { kc = 0; ready = false; wa.next(); }
+            moved = true;
           }
         }
+        if (moved) { idle = 0; start = 0; continue; }
+        if ((++idle & 255u) == 0u) {                        // bounded, as mbar_wait
+          const long long now = clock64();
+          if (start == 0) start = now;
+          if (*abort_flag || now - start > kWaitLimitCycles) { ok = false; break; }
+        }
       }
-      if (!ok) {
-        *abort_flag = 1;
-        if (p.status != nullptr) atomicCAS(p.status, 0, (STAGE << 20) | (1 << 16) | (int)blockIdx.x);
-      }
+      if (!ok) failed(1);
       // none of this CTA's own copies may still be in flight when it exits
-      for (int k = 0; k < C::kASlots && k < ac; ++k) {
+      for (int k = 0; k < kNA && k < ac; ++k) {
         const int j = ac - 1 - k;
-        mbar_wait((STAGE == 2 ? bar_rfull : bar_afull) + 8 * (j % C::kASlots), (uint32_t)((j / C::kASlots) & 1), abort_flag);
+        if (loads & (1 << (j % kNA))) mbar_wait(bar_afull + 8 * (j % kNA), (uint32_t)((j / kNA) & 1), abort_flag);
+      }
+      for (int k = 0; k < 2 && k < rc; ++k) {
+        const int j = rc - 1 - k;
+        mbar_wait(bar_rfull + 8 * (j & 1), (uint32_t)((j >> 1) & 1), abort_flag);
       }
       for (int k = 0; k < kNB && k < bc; ++k) {
         const int j = bc - 1 - k;
@@ -295,360 +550,285 @@ __global__ void __launch_bounds__(VCfg<D>::kThreads + (STAGE == 2 ? kExpandThrea
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (converged warp, one elected lane issues)
-    bool ok = true;
-    int bc = 0;
+    int ac = 0, bc = 0;
     // M = 128, N = D (all output columns in one instruction: rows 128.. of the B stage are the second block), fp16
-    const uint32_t idesc = (idesc_f16(false) & ~(0x3Fu << 17)) | ((uint32_t)(D >> 3) << 17);
-    int ac = 0;
-    for (int i = 0; i < n_local && ok; ++i) {
-      const int slot = i & 1;
-      ok = mbar_wait(bar_tempty + 8 * slot, (uint32_t)(((i >> 1) & 1) ^ 1), abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+    const uint32_t idesc = idesc_f16(false, (uint32_t)D);
+    const bool ok = walk_items(n_local, [&](int i, int slot, int stage, int use) {
+      bool go = mbar_wait(bar_tempty + 8 * slot, (uint32_t)((use & 1) ^ 1), abort_flag);
+      if (!__all_sync(0xffffffffu, go)) return false;
+      const uint32_t d_tmem = tmem_base + (uint32_t)(slot * NBLK * 128);
 #pragma unroll 1
-      for (int kc = 0; kc < KC && ok; ++kc, ++ac) {
-        const int as = ac % C::kASlots;
-        ok = mbar_wait(bar_afull + 8 * as, (uint32_t)((ac / C::kASlots) & 1), abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        const uint64_t a_hi = smem_desc_sw128(a_smem + as * kChunk);
-        const uint64_t a_lo = smem_desc_sw128(a_smem + (C::kASlots + as) * kChunk);
-        {
-          const uint32_t d_tmem = tmem_base + (uint32_t)(slot * NBLK * 128);
+      for (int kc = 0; kc < KC; ++kc, ++ac) {
+        const int as = ac % kNA;
+        go = mbar_wait(bar_afull + 8 * as, (uint32_t)((ac / kNA) & 1), abort_flag);
+        if (!__all_sync(0xffffffffu, go)) return false;
+        const uint64_t a_hi = smem_desc_sw128(a_smem + 2u * as * kChunk);
+        const uint64_t a_lo = smem_desc_sw128(a_smem + 2u * as * kChunk + kChunk);
 #pragma unroll 1
-          for (int pb = 0; pb < 2; ++pb) {
-            const int s = bc % kNB;
-            ok = mbar_wait(bar_bfull + 8 * s, (uint32_t)((bc / kNB) & 1), abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after();
-            const uint64_t b_desc = smem_desc_sw128(b_smem + s * C::kBStage);
-            if (elect_one()) {
-              if (pb == 0) {
+        for (int pb = 0; pb < 2; ++pb, ++bc) {
+          const int s = bc % kNB;
+          go = mbar_wait(bar_bfull + 8 * s, (uint32_t)((bc / kNB) & 1), abort_flag);
+          if (!__all_sync(0xffffffffu, go)) return false;
+          tc_fence_after();
+          const uint64_t b_desc = smem_desc_sw128(b_smem + s * C::kBStage);
+          if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_f16(d_tmem, a_hi + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kc | k) != 0 ? 1u : 0u);
-                if constexpr (PA == 2) {
+            for (int k = 0; k < 4; ++k)
+              umma_f16(d_tmem, a_hi + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kc | k | pb) != 0 ? 1u : 0u);
+            if (pb == 0 && stage != 1) {
 #pragma unroll
-                  for (int k = 0; k < 4; ++k) umma_f16(d_tmem, a_lo + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, 1u);
-                }
-              } else {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) umma_f16(d_tmem, a_hi + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, 1u);
-              }
-              umma_commit(bar_bempty + 8 * s);              // the ring stage is free once these MMAs are done
-              if (pb == 1) {
-                umma_commit(bar_aempty + 8 * as);           // last use of this k-chunk of A
-                if (kc == KC - 1) umma_commit(bar_tfull + 8 * slot);
-              }
+              for (int k = 0; k < 4; ++k) umma_f16(d_tmem, a_lo + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, 1u);
             }
-            __syncwarp();
-            ++bc;
+            umma_commit(bar_bempty + 8 * s);                // the ring stage is free once these MMAs are done
+            if (pb == 1) {
+              umma_commit(bar_aempty + 8 * as);             // last use of this k-chunk of A
+              if (kc == KC - 1) umma_commit(bar_tfull + 8 * slot);
+            }
           }
+          __syncwarp();
         }
       }
-    }
-    if (!ok && lane == 0) {
-      *abort_flag = 1;
-      if (p.status != nullptr) atomicCAS(p.status, 0, (STAGE << 20) | (2 << 16) | (int)blockIdx.x);
-    }
-  } else if (STAGE == 2 && warp >= C::kThreads / 32) {
+      return true;
+    });
+    if (!ok && lane == 0) failed(2);
+  } else if (threadIdx.x >= C::kExpandBegin) {
     // ------------------------------------------------------------ expanders (stage 2): index bytes of a k-chunk -> centroid
     // pieces hi and lo in operand layout, thread = two rows.  The thread walks its four 16-byte pieces in an order XOR-ed with
     // `g`, a linear map of the row's bits 1 and 2 for which the map and its sum with the identity are both one-to-one:
     // the eight rows of a quarter warp then read eight different bank groups of the raw chunk and write eight different
     // ones of the operand.
     const uint32_t lut = smem_u32(lut_s);
-    bool ok = true;
-    int ac = 0;
-    for (int i = 0; i < n_local && ok; ++i) {
-      for (int kc = 0; kc < KC && ok; ++kc, ++ac) {
-        const int as = ac % C::kASlots;
-        const uint32_t parity = (uint32_t)((ac / C::kASlots) & 1);
-        ok = mbar_wait(bar_rfull + 8 * as, parity, abort_flag) && mbar_wait(bar_aempty + 8 * as, parity ^ 1u, abort_flag);
-        if (!ok) break;
-#pragma unroll 1
-        for (int row = threadIdx.x - C::kThreads; row < kRowsT; row += kExpandThreads) {
-        const uint32_t r1 = (uint32_t)(row >> 1) & 1u, r2 = (uint32_t)(row >> 2) & 1u;
-        const uint32_t g = ((r2 ^ r1) << 1) | r2;
-        const uint32_t src = raw_smem + as * kRawChunk + (uint32_t)row * 64u;
-        const uint32_t dst = a_smem + as * kChunk + (uint32_t)row * 128u;
-#pragma unroll
-        for (uint32_t c = 0; c < 4; ++c) {
-          const uint32_t cc = c ^ g;
-          const uint4 x = ld_shared_v4(src + cc * 16u);
-          const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-          for (uint32_t h = 0; h < 2; ++h) {                // 8 coordinates: one 16-byte operand chunk per piece
-            uint32_t e[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const uint32_t w = xw[2 * h + (u >> 2)];
-              const int sh = 8 * (u & 3);
-              const uint32_t off = sh == 0 ? ((w << 2) & 0x3FCu) : ((w >> (sh - 2)) & 0x3FCu);
-              asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e[u]) : "r"(lut + off));
-            }
-            const uint32_t at = dst + (((2u * cc + h) ^ (uint32_t)(row & 7)) << 4);
-            st_shared_v4(at, __byte_perm(e[0], e[1], 0x5410), __byte_perm(e[2], e[3], 0x5410), __byte_perm(e[4], e[5], 0x5410),
-                         __byte_perm(e[6], e[7], 0x5410));
-            st_shared_v4(at + C::kASlots * kChunk, __byte_perm(e[0], e[1], 0x7632), __byte_perm(e[2], e[3], 0x7632),
-                         __byte_perm(e[4], e[5], 0x7632), __byte_perm(e[6], e[7], 0x7632));
-          }
-        }
-        }
+    const int et = threadIdx.x - C::kExpandBegin;
+    uint32_t pool[8];
+    piece_pool(lut_s, p.bits, pool);
+    int ac = 0, rc = 0;
+    const bool ok = walk_items(n_local, [&](int i, int slot, int stage, int use) {
+      if (stage != 2) { ac += KC; return true; }
+      for (int kc = 0; kc < KC; ++kc, ++ac, ++rc) {
+        const int as = ac % kNA, rs = rc & 1;
+        bool go = mbar_wait(bar_rfull + 8 * rs, (uint32_t)((rc >> 1) & 1), abort_flag) &&
+                  mbar_wait(bar_aempty + 8 * as, (uint32_t)(((ac / kNA) & 1) ^ 1), abort_flag);
+        go = bar_red_and(5, kExpandThreads, go);            // leave together: the two warps meet at a barrier below
+        if (!go) return false;
+        const uint32_t raw = raw_smem + rs * kRawChunk, dst = a_smem + 2u * as * kChunk;
+        if (p.bits <= 2) expand_chunk<2>(raw, dst, et, pool, lut);
+        else if (p.bits == 3) expand_chunk<3>(raw, dst, et, pool, lut);
+        else expand_chunk<8>(raw, dst, et, pool, lut);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // operand writes -> visible to the tensor core
-        mbar_arrive(bar_afull + 8 * as);
-        mbar_arrive(bar_rempty + 8 * as);
+        asm volatile("bar.sync 6, %0;" ::"n"(kExpandThreads) : "memory");
+        if (et == 0) {
+          mbar_arrive(bar_afull + 8 * as);
+          mbar_arrive(bar_rempty + 8 * rs);
+        }
       }
-    }
-    if (!ok) {
-      *abort_flag = 1;
-      if (p.status != nullptr) atomicCAS(p.status, 0, (STAGE << 20) | (4 << 16) | (int)blockIdx.x);
-    }
+      return true;
+    });
+    if (!ok && lane == 0) failed(4);
   } else {
-    // ------------------------------------------------------------ epilogue: per tile in flight one warpgroup per block
-    // of 128 output columns, thread = vector
+    // ------------------------------------------------------------ epilogue: a warpgroup per 64 columns of a tile, thread = vector.
+    // What bounds a tile is the chain of its stages (contraction, epilogue, the way through the scratch), so
+    // as many warps as there are share one epilogue: with a warpgroup per 128 columns and two of the four for each tile,
+    // stage 2's took 15 400 clocks of the 24 500 between its contraction's start and the next one's.
+    constexpr int kWgs = C::kWgs;
     const int ew = warp - 2;
     const int wgi = ew >> 2;
-    const int slot = wgi / NBLK, blk = wgi % NBLK;
+    const int group = wgi / kWgs, part = wgi % kWgs;
     const int quarter = warp & 3;                 // TMEM lanes this warp may touch: 32*quarter ..
     const int rloc = quarter * 32 + lane;
-    bool ok = true;
-    // search shortcut of the codebook (stage 1): 1 = polynomial, 2 = cell table, 0 = binary search
-    int mode = 0;
-    float sc_s = 0.f, sc_c1 = 0.f, sc_c2 = 0.f, sc_c3 = 0.f;
-    if constexpr (STAGE == 1) {
-      mode = (int)__ldg(p.codebook + 512);
-      sc_s = __ldg(p.codebook + 513);
-      sc_c1 = __ldg(p.codebook + 514);
-      sc_c2 = __ldg(p.codebook + 515);
-      sc_c3 = __ldg(p.codebook + 516);
-    }
-    for (int i = slot; i < n_local && ok; i += 2) {
+    const int col0 = part * 64;
+    V2Quantiser q;
+    q.s = __ldg(p.codebook + 513);
+    q.c1 = __ldg(p.codebook + 514);
+    q.c2 = __ldg(p.codebook + 515);
+    q.c3 = __ldg(p.codebook + 516);
+    q.thr_lane_h = thr_s[lane] * 1099511627776.0f;
+    q.t0 = thr_s[0] * 1099511627776.0f;
+    q.t1 = thr_s[1] * 1099511627776.0f;
+    q.t2 = thr_s[2] * 1099511627776.0f;
+    const bool fast = (int)__ldg(p.codebook + 512) == 1 && p.bits <= 5;             // up to 31 thresholds: one per lane
+    const bool linear = __ldg(p.codebook + 518) == 1.0f;
+    const bool x_wide = ((uintptr_t)p.x & 31u) == 0, k_wide = ((uintptr_t)p.k_mse_out & 31u) == 0;
+    const bool ok = walk_items(n_local, [&](int i, int slot, int stage, int use) {
+      if (kWgs == 2 && slot != group) return true;
+      const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(slot * NBLK * 128 + col0);
       const int64_t row = (int64_t)(t0 + i) * kRowsT + rloc;
+      const int64_t srow = (int64_t)(t0 + slot) * kRowsT + rloc;      // its row of the scratch
       const bool valid = row < p.n;
       // stage 2: a quad of lanes holds 64 columns of a row, 16 each, so that its accesses to x, k_mse and the pieces are whole
-      // 128-byte lines (see below).  The norms and the first coordinates are in flight while the tile's contraction runs.
+      // 128-byte lines (see below).  The first coordinates are in flight while the tile's contraction runs.
       const int quad = lane & 3, r8 = lane >> 2;
       const int64_t qrow = (int64_t)(t0 + i) * kRowsT + quarter * 32 + r8;        // rows qrow + {0, 8, 16, 24}
-      const bool x_wide = ((uintptr_t)p.x & 31u) == 0;
-      uint32_t xn[8];
-      float nv4[4];
-      if constexpr (STAGE == 2) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) nv4[u] = qrow + 8 * u < p.n ? p.norms[qrow + 8 * u] : 0.f;
-        load_row32(p.x + (qrow < p.n ? qrow : 0) * D + blk * 128 + 16 * quad, xn, x_wide);
-      }
-      // The exit decision is made uniform before anything collective: per warp (the TMEM loads are
-      // warp-collective) and, where the two warpgroups of a tile later meet at a named barrier (stage 2,
-      // head_dim 256), over those 256 threads, so that nobody waits at that barrier for a warp that left.
-      ok = __all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * slot, (uint32_t)((i >> 1) & 1), abort_flag));
-      if constexpr (STAGE == 2 && NBLK == 2) ok = bar_red_and(3 + slot, 256, ok);
-      if (!ok) break;
+      uint32_t xn[2][8];
+      auto x_load = [&](int step) {                 // step = (16 rows rg, 8 rows hh)
+        const int64_t r = qrow + 8 * step;
+        load_row32(p.x + (r < p.n ? r : 0) * D + col0 + 16 * quad, xn[step & 1], x_wide);
+      };
+      if (stage == 2) { x_load(0); x_load(1); }
+      // The exit decision is made uniform before anything collective, over all the warps that meet at named barriers below, so
+      // that nobody waits at a barrier for a warp that left (the TMEM loads are collective over a warp).
+      const bool go = bar_red_and(3 + group, 128 * kWgs, mbar_wait(bar_tfull + 8 * slot, (uint32_t)(use & 1), abort_flag));
+      if (!go) return false;
       tc_fence_after();
-      const uint32_t tile_acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(slot * NBLK * 128);
-      const uint32_t tacc = tile_acc + (uint32_t)(blk * 128);     // this warpgroup's block of columns
-      const int col0 = blk * 128;
-      uint32_t v[16];
-      if constexpr (STAGE == 1) {
-        float ssq = 0.f;                         // the norm needs every column: both warpgroups sweep the whole row
-        uint32_t v2[16];                         // two buffers: a TMEM load is in flight behind the arithmetic
-        tmem_issue16(tile_acc, v);
+      float* parts = part_s + slot * 4 * 128;
+      if (stage == 1) {
 #pragma unroll 1
-        for (int c = 0; c < D / 16; c += 2) {
-          tmem_wait16(v);
-          tmem_issue16(tile_acc + (c + 1) * 16, v2);
+        for (int rg = 0; rg < 2; ++rg) {
+          uint32_t a[32];
+          tmem_ld_quads(tacc + ((uint32_t)(rg * 16) << 16), a);
 #pragma unroll
-          for (int e = 0; e < 16; ++e) ssq = fmaf(__uint_as_float(v[e]), __uint_as_float(v[e]), ssq);
-          tmem_wait16(v2);
-          tmem_issue16(c + 2 < D / 16 ? tile_acc + (c + 2) * 16 : tacc, v);      // after the last step: step 0 of the sweep below
+          for (int hh = 0; hh < 2; ++hh) {
+            unsigned long long ssq2 = 0ull, ssq3 = 0ull;
 #pragma unroll
-          for (int e = 0; e < 16; ++e) ssq = fmaf(__uint_as_float(v2[e]), __uint_as_float(v2[e]), ssq);
+            for (int j = 0; j < 8; j += 2) {
+              ssq2 = square2(a[4 * j + 2 * hh], a[4 * j + 2 * hh + 1], ssq2);
+              ssq3 = square2(a[4 * j + 4 + 2 * hh], a[4 * j + 4 + 2 * hh + 1], ssq3);
+            }
+            float sq = (__uint_as_float((uint32_t)ssq2) + __uint_as_float((uint32_t)(ssq2 >> 32))) +
+                       (__uint_as_float((uint32_t)ssq3) + __uint_as_float((uint32_t)(ssq3 >> 32)));
+            sq += __shfl_xor_sync(0xffffffffu, sq, 1);          // the quad's four parts of the row
+            sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+            if (quad == 0) parts[part * 128 + quarter * 32 + r8 + 16 * rg + 8 * hh] = sq;
+          }
         }
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(128 * kWgs) : "memory");
+        float ssq = 0.f;                           // lane = row
+#pragma unroll
+        for (int w = 0; w < kWgs; ++w) ssq += parts[w * 128 + rloc];
         const float norm = __fsqrt_rn(ssq);
         const float inv = __fdiv_rn(1.0f, norm + 1e-8f);
-        if (valid && blk == 0) p.norms[row] = norm;
-        const int bits = p.bits;
-        uint32_t ib0[4] = {0u, 0u, 0u, 0u};       // index bytes of the even step
+        if (part == 0) {
+          norm_s[slot * 128 + rloc] = norm;
+          if (valid && p.vec_norms_out != nullptr) p.vec_norms_out[row] = norm;
+        }
 #pragma unroll 1
-        for (int c = 0; c < 8; ++c) {
-          tmem_wait16(v);
-          uint32_t ib[4] = {0u, 0u, 0u, 0u};
+        for (int rg = 0; rg < 2; ++rg) {
+          uint32_t a[32];
+          tmem_ld_quads(tacc + ((uint32_t)(rg * 16) << 16), a);
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const float y = __uint_as_float(v[e]) * inv;
-            int idx;
-            if (mode != 0) {
-              // candidate e0 with index in {e0, e0 + 1} (verified on the host for every y), then one exact compare
-              float t;
-              asm("fma.rn.sat.f32 %0, %1, %2, 0f3F000000;" : "=f"(t) : "f"(y), "f"(sc_s));
-              int e0;
-              if (mode == 1) {
-                float q = fmaf(sc_c3, t, sc_c2);
-                q = fmaf(q, t, sc_c1);
-                e0 = __float_as_int(fmaf(q, t, 8388608.0f)) & 0xFF;
-              } else {
-                e0 = cells_s[__float_as_int(fmaf(t, 1024.0f, 8388608.0f)) & 0x7FF];
-              }
-              idx = e0 + (y > thr_s[e0] ? 1 : 0);
-            } else {
-              int lo = 0, hi = (1 << bits) - 1;
-              for (int step = 0; step < bits; ++step) {
-                const int mid = (lo + hi) >> 1;
-                if (y > thr_s[mid]) lo = mid + 1; else hi = mid;
-              }
-              idx = lo;
+          for (int hh = 0; hh < 2; ++hh) {
+            const int step = 2 * rg + hh;
+            const int64_t r = qrow + 8 * step;
+            const float inv_r = __shfl_sync(0xffffffffu, inv, r8 + 8 * step);
+            q.s_inv = q.s * inv_r;
+            q.h_inv = 1099511627776.0f * inv_r;    // 2^40: exact scaling
+            uint32_t ib[4];
+            if (fast && p.bits <= 2) index_bytes_fast<true, false>(a, hh, q, ib);
+            else if (fast && linear) index_bytes_fast<false, true>(a, hh, q, ib);
+            else if (fast) index_bytes_fast<false, false>(a, hh, q, ib);
+            else {
+              auto four = [&](int j) { return make_uint4(a[4 * j + 2 * hh], a[4 * j + 2 * hh + 1], a[4 * j + 4 + 2 * hh], a[4 * j + 5 + 2 * hh]); };
+              const uint4 o = index_bytes_any(four(0), four(2), four(4), four(6), inv_r, p.codebook, thr_s, cells_s, p.bits);
+              ib[0] = o.x; ib[1] = o.y; ib[2] = o.z; ib[3] = o.w;
             }
-            ib[e >> 2] |= (uint32_t)idx << (8 * (e & 3));
-          }
-          if (c + 1 < 8) tmem_issue16(tacc + (c + 1) * 16, v);
-          if (valid && p.idx_u8_out != nullptr)
-            *reinterpret_cast<uint4*>(p.idx_u8_out + row * D + col0 + c * 16) = make_uint4(ib[0], ib[1], ib[2], ib[3]);
-          if (valid && p.idx_packed_out != nullptr) {
-            // the 16 indices of this step as 16 / ipb packed bytes of the row
-            const int ipb = 8 / bits;
-            uint8_t* dst = p.idx_packed_out + row * (int64_t)(D / ipb) + (col0 + c * 16) / ipb;
-            if (ipb == 1) {
-              *reinterpret_cast<uint4*>(dst) = make_uint4(ib[0], ib[1], ib[2], ib[3]);
-            } else if (ipb == 2) {           // 3- and 4-bit codes: byte k = idx[2k] << bits | idx[2k+1]
-              uint32_t o[2];
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const uint32_t a = ib[2 * h], b = ib[2 * h + 1];
-                const uint32_t b0 = (((a >> 0) & 0xFFu) << bits) | ((a >> 8) & 0xFFu), b1 = (((a >> 16) & 0xFFu) << bits) | (a >> 24);
-                const uint32_t b2 = (((b >> 0) & 0xFFu) << bits) | ((b >> 8) & 0xFFu), b3 = (((b >> 16) & 0xFFu) << bits) | (b >> 24);
-                o[h] = b0 | (b1 << 8) | (b2 << 16) | (b3 << 24);
-              }
-              *reinterpret_cast<uint2*>(dst) = make_uint2(o[0], o[1]);
-            } else if (ipb == 4) {           // 2-bit codes
-              uint32_t o = 0u;
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const uint32_t a = ib[k];
-                o |= ((((a >> 0) & 3u) << 6) | (((a >> 8) & 3u) << 4) | (((a >> 16) & 3u) << 2) | ((a >> 24) & 3u)) << (8 * k);
-              }
-              *reinterpret_cast<uint32_t*>(dst) = o;
-            } else {                          // 1-bit codes
-              uint32_t o = 0u;
-#pragma unroll
-              for (int e = 0; e < 16; ++e) o |= ((ib[e >> 2] >> (8 * (e & 3))) & 1u) << (8 * (e >> 3) + 7 - (e & 7));
-              *reinterpret_cast<uint16_t*>(dst) = (uint16_t)o;
+            if (r < p.n) {
+              const int col = col0 + 16 * quad;
+              const uint4 bytes = make_uint4(ib[0], ib[1], ib[2], ib[3]);
+              *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.p_hi + (srow - lane + r8 + 8 * step) * D) + col) = bytes;
+              if (p.idx_u8_out != nullptr) *reinterpret_cast<uint4*>(p.idx_u8_out + r * D + col) = bytes;
+              if (p.idx_packed_out != nullptr)
+                store_packed16(p.idx_packed_out + r * (int64_t)(D / (8 / p.bits)) + col / (8 / p.bits), ib, p.bits);
             }
-          }
-          if ((c & 1) == 0) {                     // two steps leave as one access
-#pragma unroll
-            for (int j = 0; j < 4; ++j) ib0[j] = ib[j];
-          } else if (valid) {
-            const uint32_t both[8] = {ib0[0], ib0[1], ib0[2], ib0[3], ib[0], ib[1], ib[2], ib[3]};
-            store_row32(reinterpret_cast<uint8_t*>(p.p_hi + row * D) + col0 + (c - 1) * 16, both, true);
           }
         }
-      } else if constexpr (STAGE == 2) {
+      } else if (stage == 2) {
         // Rows x 32 bytes per access cost the load/store unit a slot per row (see store_row32), and the operand traffic of the
-        // MMAs and the expanders runs through the same data path: thread = row took 199 us here for the call above, of
-        // which 16 400 of 26 600 clocks per tile were such slots.  tcgen05.ld.16x256b spreads a row over a quad of lanes
-        // instead: thread (r8, quad) gets rows r8 and r8 + 8 of 16, 16 columns each, and a warp's access is 8 lines: 133 us.
-        const bool k_wide = ((uintptr_t)p.k_mse_out & 31u) == 0;
+        // MMAs and the expanders runs through the same data path: thread = row took 199 us here for 262144 vectors of head_dim
+        // 256 in a launch of its own, of which 16 400 of 26 600 clocks per tile were such slots.  tcgen05.ld.16x256b spreads a
+        // row over a quad of lanes instead: thread (r8, quad) gets rows r8 and r8 + 8 of 16, 16 columns each, and a warp's
+        // access is 8 lines: 133 us.
+        float nv4[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) nv4[u] = norm_s[slot * 128 + quarter * 32 + r8 + 8 * u];
 #pragma unroll
         for (int rg = 0; rg < 2; ++rg) {            // 16 rows
-          float sq[2] = {0.f, 0.f};
+          uint32_t a[32];
+          tmem_ld_quads(tacc + ((uint32_t)(rg * 16) << 16), a);
 #pragma unroll
-          for (int cg = 0; cg < 2; ++cg) {          // 64 columns
-            uint32_t a[32];
-            tmem_ld_quads(tacc + ((uint32_t)(rg * 16) << 16) + (uint32_t)(cg * 64), a);
+          for (int hh = 0; hh < 2; ++hh) {          // row r8 or r8 + 8 of them
+            const int step = 2 * rg + hh;
+            const int64_t r = qrow + 8 * step;
+            const int64_t col = col0 + 16 * quad;
+            const int64_t sat = (srow - lane + r8 + 8 * step) * D + col;        // the scratch row of r
+            uint32_t xw[8];
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              const int64_t r = qrow + 16 * rg + 8 * hh;
-              const int64_t at = r * D + col0 + 64 * cg + 16 * quad;
-              uint32_t xw[8];
+            for (int j = 0; j < 8; ++j) xw[j] = xn[hh][j];
+            if (step + 2 < 4) x_load(step + 2);
+            float sq = 0.f;
+            if (r < p.n) {
+              const float nv = nv4[step];
+              uint32_t kq[8], rh[8], rl[8];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) xw[j] = xn[j];
-              const int nxt = 4 * rg + 2 * cg + hh + 1;                // the next (rg, cg, hh)
-              if (nxt < 8) {
-                const int64_t rn = qrow + 16 * (nxt >> 2) + 8 * (nxt & 1);
-                load_row32(p.x + (rn < p.n ? rn : 0) * D + col0 + 64 * ((nxt >> 1) & 1) + 16 * quad, xn, x_wide);
+              for (int j = 0; j < 8; ++j) {
+                const float k0 = __uint_as_float(a[4 * j + 2 * hh]) * nv, k1 = __uint_as_float(a[4 * j + 2 * hh + 1]) * nv;
+                const __half2 xh = *reinterpret_cast<const __half2*>(&xw[j]);
+                const float r0 = __low2float(xh) - k0, r1 = __high2float(xh) - k1;
+                sq = fmaf(r0, r0, sq);
+                sq = fmaf(r1, r1, sq);
+                const __half2 kh = __floats2half2_rn(k0, k1);
+                kq[j] = *reinterpret_cast<const uint32_t*>(&kh);
+                const __half2 h2 = __floats2half2_rn(r0, r1);
+                rh[j] = *reinterpret_cast<const uint32_t*>(&h2);
+                const __half2 l2 = __floats2half2_rn(r0 - __low2float(h2), r1 - __high2float(h2));
+                rl[j] = *reinterpret_cast<const uint32_t*>(&l2);
               }
-              if (r < p.n) {
-                const float nv = nv4[2 * rg + hh];
-                uint32_t kq[8], rh[8], rl[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  const float k0 = __uint_as_float(a[4 * j + 2 * hh]) * nv, k1 = __uint_as_float(a[4 * j + 2 * hh + 1]) * nv;
-                  const __half2 xh = *reinterpret_cast<const __half2*>(&xw[j]);
-                  const float r0 = __low2float(xh) - k0, r1 = __high2float(xh) - k1;
-                  sq[hh] = fmaf(r0, r0, sq[hh]);
-                  sq[hh] = fmaf(r1, r1, sq[hh]);
-                  const __half2 kh = __floats2half2_rn(k0, k1);
-                  kq[j] = *reinterpret_cast<const uint32_t*>(&kh);
-                  const __half2 h2 = __floats2half2_rn(r0, r1);
-                  rh[j] = *reinterpret_cast<const uint32_t*>(&h2);
-                  const __half2 l2 = __floats2half2_rn(r0 - __low2float(h2), r1 - __high2float(h2));
-                  rl[j] = *reinterpret_cast<const uint32_t*>(&l2);
-                }
-                if (p.k_mse_out != nullptr) store_row32(p.k_mse_out + at, kq, k_wide);
-                store_row32(p.p_hi + at, rh, true);
-                store_row32(p.p_lo + at, rl, true);
-              }
+              store_row32(p.p_hi + sat, rh, true);
+              store_row32(p.p_lo + sat, rl, true);
+              if (p.k_mse_out != nullptr) store_row32(p.k_mse_out + r * D + col, kq, k_wide);
             }
-          }
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {          // the quad's four parts of a row
-            sq[hh] += __shfl_xor_sync(0xffffffffu, sq[hh], 1);
-            sq[hh] += __shfl_xor_sync(0xffffffffu, sq[hh], 2);
-            const int64_t r = qrow + 16 * rg + 8 * hh;
-            if constexpr (NBLK == 2) {
-              // the residual norm spans both blocks: each warpgroup leaves its part
-              if (quad == 0) part_s[(slot * 2 + blk) * 128 + quarter * 32 + r8 + 16 * rg + 8 * hh] = sq[hh];
-            } else {
-              if (quad == 0 && r < p.n) p.rnorm_out[r] = __half_as_ushort(__float2half_rn(__fsqrt_rn(sq[hh])));
-            }
+            sq += __shfl_xor_sync(0xffffffffu, sq, 1);          // the quad's four parts of the row
+            sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+            if (quad == 0) parts[part * 128 + quarter * 32 + r8 + 8 * step] = sq;
           }
         }
-        if constexpr (NBLK == 2) {
-          asm volatile("bar.sync %0, 256;" ::"r"(1 + slot) : "memory");
-          if (blk == 0 && valid)
-            p.rnorm_out[row] = __half_as_ushort(__float2half_rn(__fsqrt_rn(part_s[slot * 2 * 128 + rloc] + part_s[(slot * 2 + 1) * 128 + rloc])));
-          asm volatile("bar.sync %0, 256;" ::"r"(1 + slot) : "memory");     // part_s is reused by the next tile
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(128 * kWgs) : "memory");
+        if (part == 0 && valid) {
+          float ssq = 0.f;
+#pragma unroll
+          for (int w = 0; w < kWgs; ++w) ssq += parts[w * 128 + rloc];
+          p.rnorm_out[row] = __half_as_ushort(__float2half_rn(__fsqrt_rn(ssq)));
         }
+        // the parts are written again after the barrier that opens the tile's next stage
       } else {
-        const bool s_wide = ((uintptr_t)p.signs_out & 31u) == 0;
 #pragma unroll 1
-        for (int c = 0; c < 8; c += 2) {
-          uint32_t v2[16];
-          tmem_issue16(tacc + c * 16, v);
-          tmem_issue16(tacc + (c + 1) * 16, v2);
-          tmem_wait16(v);
-          tmem_wait16(v2);
-          if (valid && p.signs_out != nullptr) {
-            uint32_t sw[8];
+        for (int rg = 0; rg < 2; ++rg) {
+          uint32_t a[32];
+          tmem_ld_quads(tacc + ((uint32_t)(rg * 16) << 16), a);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              uint32_t x = 0u;
+          for (int hh = 0; hh < 2; ++hh) {
+            const int64_t r = qrow + 16 * rg + 8 * hh;
+            const int col = col0 + 16 * quad;
+            if (r < p.n && p.signs_out != nullptr) {
+              uint32_t sw[4];
 #pragma unroll
-              for (int b = 0; b < 4; ++b) {
-                const uint32_t s8 = __uint_as_float(j < 4 ? v[4 * j + b] : v2[4 * (j - 4) + b]) >= 0.f ? 0x01u : 0xFFu;
-                x |= s8 << (8 * b);
+              for (int w = 0; w < 4; ++w) {
+                uint32_t x = 0u;
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                  x |= (__uint_as_float(a[4 * (2 * w + (b >> 1)) + 2 * hh + (b & 1)]) >= 0.f ? 0x01u : 0xFFu) << (8 * b);
+                sw[w] = x;
               }
-              sw[j] = x;
+              *reinterpret_cast<uint4*>(p.signs_out + r * D + col) = make_uint4(sw[0], sw[1], sw[2], sw[3]);
             }
-            store_row32(p.signs_out + row * D + col0 + c * 16, sw, s_wide);
-          }
-          if (valid && p.sign_bits_out != nullptr) {
-            uint32_t o = 0u;
+            if (r < p.n && p.sign_bits_out != nullptr) {
+              uint32_t o = 0u;
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
-              o |= (__uint_as_float(e < 16 ? v[e] : v2[e - 16]) >= 0.f ? 1u : 0u) << (8 * (e >> 3) + 7 - (e & 7));
-            *reinterpret_cast<uint32_t*>(p.sign_bits_out + row * (D / 8) + (col0 + c * 16) / 8) = o;
+              for (int e = 0; e < 16; ++e)
+                o |= (__uint_as_float(a[4 * (e >> 1) + 2 * hh + (e & 1)]) >= 0.f ? 1u : 0u) << (8 * (e >> 3) + 7 - (e & 7));
+              *reinterpret_cast<uint16_t*>(p.sign_bits_out + r * (D / 8) + col / 8) = (uint16_t)o;
+            }
           }
         }
       }
       tc_fence_before();
+      if (stage < 3) asm volatile("fence.proxy.async.global;" ::: "memory");   // the scratch is read by the copy engine
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_tempty + 8 * slot);
-    }
-    if (!ok && lane == 0) {
-      *abort_flag = 1;
-      if (p.status != nullptr) atomicCAS(p.status, 0, (STAGE << 20) | (3 << 16) | (int)blockIdx.x);
-    }
+      if (lane == 0) {
+        mbar_arrive(bar_tempty + 8 * slot);
+        if (stage < 3) mbar_arrive(bar_ready + 8 * slot);
+      }
+      return true;
+    });
+    if (!ok && lane == 0) failed(3);
   }
   tc_fence_before();
   __syncthreads();
@@ -683,15 +863,6 @@ int encode_index_rows(TensorMapEncodeFn enc, CUtensorMap* map, const void* ptr, 
   return TQ_OK;
 }
 
-template <int D, int STAGE>
-int launch_stage(const V2Stage& p, int grid, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(k_umma_v2_stage<D, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)VCfg<D>::kSmemBytes);
-  if (e != cudaSuccess) return refused(e);
-  launch_after(k_umma_v2_stage<D, STAGE>, dim3(grid), dim3(VCfg<D>::threads(STAGE)), VCfg<D>::kSmemBytes, st, p);
-  return check_launch();
-}
-
 template <int D>
 int run(const TqQjlCompressJob& job, cudaStream_t st) {
   TensorMapEncodeFn enc = tensor_map_encoder();
@@ -699,29 +870,20 @@ int run(const TqQjlCompressJob& job, cudaStream_t st) {
   const int64_t n = job.B * job.H * job.S;
   const int64_t tiles = (n + kRowsT - 1) / kRowsT;
   if (tiles >= ((int64_t)1 << 30)) return TQ_ETOOBIG;
-  // workspace: three operand images, then the two piece arrays, then the norms
+  // workspace: three operand images, then the two piece arrays
   uint8_t* ws = reinterpret_cast<uint8_t*>(((uintptr_t)job.workspace + 1023u) & ~(uintptr_t)1023u);
   const size_t img = VCfg<D>::kImageBytes;
-  uint8_t* img1 = ws;
-  uint8_t* img2 = ws + img;
-  uint8_t* img3 = ws + 2 * img;
   const size_t piece = ((size_t)n * D * 2 + 1023) / 1024 * 1024;
-  uint16_t* p_hi = reinterpret_cast<uint16_t*>(ws + 3 * img);
-  uint16_t* p_lo = reinterpret_cast<uint16_t*>(ws + 3 * img + piece);
-  float* norms = reinterpret_cast<float*>(ws + 3 * img + 2 * piece);
-  const int ib = (D * D + 255) / 256;
-  k_v2_operand_image<D><<<dim3(ib, 3), 256, 0, st>>>(job.rotation, job.qjl_t, job.M, img1);
-  int rc = check_launch();
-  if (rc != TQ_OK) return rc;
-  static thread_local V2Stage p;
+  V2Args p;
+  p.images = ws;
+  p.p_hi = reinterpret_cast<uint16_t*>(ws + 3 * img);
+  p.p_lo = reinterpret_cast<uint16_t*>(ws + 3 * img + piece);
   void* status_ptr = nullptr;
   cudaGetSymbolAddress(&status_ptr, g_v2_status);
   p.status = reinterpret_cast<int32_t*>(status_ptr);
   p.codebook = job.codebook;
   p.x = reinterpret_cast<const uint16_t*>(job.x);
-  p.p_hi = p_hi;
-  p.p_lo = p_lo;
-  p.norms = job.vec_norms_out != nullptr ? job.vec_norms_out : norms;
+  p.vec_norms_out = job.vec_norms_out;
   p.idx_u8_out = job.idx_mode == TQ_IDX_PACKED ? nullptr : reinterpret_cast<uint8_t*>(job.idx_out);
   p.idx_packed_out = job.idx_mode == TQ_IDX_PACKED ? reinterpret_cast<uint8_t*>(job.idx_out) : nullptr;
   p.k_mse_out = job.k_mse_out;
@@ -731,24 +893,21 @@ int run(const TqQjlCompressJob& job, cudaStream_t st) {
   p.n = n;
   p.tiles = (int32_t)tiles;
   p.bits = job.bits;
+  int rc;
+  if ((rc = encode_rows(enc, &p.x_map, job.x, n, D)) != TQ_OK) return rc;
+  if ((rc = encode_index_rows(enc, &p.idx_map, p.p_hi, n, D)) != TQ_OK) return rc;
+  if ((rc = encode_rows(enc, &p.hi_map, p.p_hi, n, D)) != TQ_OK) return rc;
+  if ((rc = encode_rows(enc, &p.lo_map, p.p_lo, n, D)) != TQ_OK) return rc;
+  const cudaError_t e = cudaFuncSetAttribute(k_umma_v2_stage<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VCfg<D>::kSmemBytes);
+  if (e != cudaSuccess) return refused(e);        // before the first launch, which lets a dependent start
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int grid = (int)(tiles < sms ? tiles : sms);
-  // stage 1: A = x
-  if ((rc = encode_rows(enc, &p.a_hi_map, job.x, n, D)) != TQ_OK) return rc;
-  p.a_lo_map = p.a_hi_map;
-  p.b_image = img1;
-  if ((rc = launch_stage<D, 1>(p, grid, st)) != TQ_OK) return rc;
-  // stage 2: A from the index bytes at the head of the rows of p_hi
-  if ((rc = encode_index_rows(enc, &p.a_hi_map, p_hi, n, D)) != TQ_OK) return rc;
-  p.b_image = img2;
-  if ((rc = launch_stage<D, 2>(p, grid, st)) != TQ_OK) return rc;
-  // stage 3: A = the piece arrays
-  if ((rc = encode_rows(enc, &p.a_hi_map, p_hi, n, D)) != TQ_OK) return rc;
-  if ((rc = encode_rows(enc, &p.a_lo_map, p_lo, n, D)) != TQ_OK) return rc;
-  p.b_image = img3;
-  return launch_stage<D, 3>(p, grid, st);
+  k_v2_operand_image<D><<<dim3((D * D + 255) / 256, 3), 256, 0, st>>>(job.rotation, job.qjl_t, job.M, ws);
+  if ((rc = check_launch()) != TQ_OK) return rc;
+  launch_after(k_umma_v2_stage<D>, dim3(grid), dim3(VCfg<D>::kThreads), VCfg<D>::kSmemBytes, st, p);
+  return check_launch();
 }
 
 }  // namespace
