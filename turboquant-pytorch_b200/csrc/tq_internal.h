@@ -88,7 +88,7 @@ size_t umma_qjl_scores_image_bytes(int64_t BH, int64_t Sq, int D);
 int umma_qjl_scores(const TqQjlScoreJob& job, void* images, cudaStream_t st);
 int simt_project_two(const void* x, int x_dtype, int64_t n, int D, const float* m0, const float* m1, float* out0, float* out1,
                      cudaStream_t st);
-int simt_qjl_query_operand(const TqQjlScoreJob& job, void* images, cudaStream_t st);
+int simt_qjl_query_operand(const TqQjlScoreJob& job, void* images, int per_unit, cudaStream_t st);      // per_unit: 16 or 64 queries
 int umma_qjl_device_status();
 
 }  // namespace tq

@@ -15,11 +15,16 @@
 //                swizzle: already the operand layout) and of raw sign chunks (128 x 64 bytes);
 //                the unit's query image (all chunks, hi and lo) by bulk copy on unit change
 //   warps 2..9   expanders: signs -> fp16 +-||r|| written in the swizzled operand layout
-//   warp 1       issues tcgen05.mma kind::f16, M=128 N=128 K=16: columns 0..63 are the queries' high pieces, 64..127 their
-//                low pieces, 4 k-steps per chunk.  An MMA of N = 64 takes as long as one of N = 128 (66 and 65 clocks), so
-//                a pass per piece over the same keys cost twice the tensor time and read every key operand twice (70 us
-//                for 16 heads x 16384 keys of head_dim 256, 66 so)
-//   warps 10..13 drain: TMEM -> high + low -> 128-byte rows of scores[q][key0 .. key0+31]
+//   warp 1       issues tcgen05.mma kind::f16, M=128 N=128 K=16 (N=32 for up to 16 queries): columns 0..63 are the queries'
+//                high pieces, 64..127 their low pieces, 4 k-steps per chunk.  An MMA of N = 64 takes as long as one of N = 128
+//                (66 and 65 clocks), so
+//                a pass per piece over the same keys cost twice the tensor time and read every key operand twice
+//   warps 10..17 drain, two groups on alternate tiles: TMEM -> high + low -> 128-byte rows of scores[q][key0 .. key0+31].  One
+//                group took longer over a tile of head_dim 128 than its keys take to arrive
+// What bounds it is how much of the keys is in flight: k_mse and sign chunks are consumed in turn and their rings take all the
+// room that the query image leaves.  The call with 16 heads x 16384 keys: head_dim 256, 64 queries 82 -> 75 us, 16 queries 74 -> 57;
+// head_dim 128, 64 queries 57 -> 45 (the second drain group), one query 45 -> 35.  Expanded signs in tensor memory instead of
+// shared memory: 61 us where 57 is said, 48 for 45.
 // Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, records a status
 // word and leaves through the normal exit.
 
@@ -39,38 +44,44 @@ namespace {
 #include "tq_tc_ptx.cuh"
 
 constexpr int kKeys = 128;                     // keys per tile (MMA M)
-constexpr int kQ = 64;                         // queries per unit (MMA N)
 constexpr uint32_t kChunkA = kKeys * 128;      // one operand chunk: 128 rows x 64 fp16 = 16 KB
 constexpr uint32_t kChunkRaw = kKeys * 64;     // raw signs of a chunk: 128 rows x 64 int8 = 8 KB
-constexpr uint32_t kChunkB = kQ * 128;         // one query chunk: 64 rows x 64 fp16 = 8 KB
-constexpr int kNSK = 3, kNSG = 2, kNSR = 2, kNT = 4;
-constexpr int kExpWarps = 8, kDrainWarps = 4;
-constexpr int kThreadsQ = 64 + 32 * (kExpWarps + kDrainWarps);   // 448
+constexpr int kNT = 4;
+constexpr int kExpWarps = 8, kDrainWarps = 8;
+constexpr int kThreadsQ = 64 + 32 * (kExpWarps + kDrainWarps);   // 576
 
-template <int D>
+// QN: queries per unit (half of the MMA's N).  16 where there are no more: the operand image is a quarter, its room goes to the rings that
+// the keys come through, and the drain has a quarter of the columns.
+template <int D, int QN>
 struct QCfg {
   static constexpr int kHalfChunks = D / 64;                     // chunks per operand half (k_mse | signs)
   static constexpr int kChunks = 2 * kHalfChunks;                // contraction length 2D in chunks of 64
-  static constexpr uint32_t kImageBytes = 2u * kChunks * kChunkB;   // per chunk the high pieces of 64 queries, then the low ones
+  static constexpr uint32_t kChunkB = QN * 128;                  // one query chunk: QN rows x 64 fp16
+  static constexpr uint32_t kImageBytes = 2u * kChunks * kChunkB;   // per chunk the high pieces of the queries, then the low ones
+  // Rings: k_mse chunks, expanded signs, raw signs.  What is in flight is what they hold.
+  static constexpr bool kTight = D == 256 && QN == 64;
+  static constexpr int kNSK = kTight ? 3 : QN == 64 ? 6 : D == 256 ? 7 : 8;
+  static constexpr int kNSG = QN == 64 ? 2 : 3;
+  static constexpr int kNSR = kTight ? 2 : 4;
   static constexpr uint32_t kOffImg = 0;
   static constexpr uint32_t kOffK = kOffImg + kImageBytes;
   static constexpr uint32_t kOffG = kOffK + kNSK * kChunkA;
   static constexpr uint32_t kOffR = kOffG + kNSG * kChunkA;
   static constexpr uint32_t kOffBar = kOffR + kNSR * kChunkRaw;
-  static constexpr uint32_t kUsedBytes = kOffBar + 256;
+  static constexpr uint32_t kUsedBytes = kOffBar + 512;
   static constexpr uint32_t kSmemBytes = kUsedBytes + 1024;      // + slack for aligning the base to 1024 bytes
+  static_assert(8 * (2 * (kNSK + kNSG + kNSR + kNT) + 2) <= 400 && kSmemBytes <= 232448, "shared memory budget");
 };
-static_assert(QCfg<256>::kSmemBytes <= 232448 && QCfg<128>::kSmemBytes <= 232448, "shared memory budget");
 
 struct QjlBatch {
   CUtensorMap kmse_map;      // fp16 (D, Sk, BH), box 64 x 128, 128-byte swizzle
   CUtensorMap sign_map;      // uint8 (D, Sk, BH), box 64 x 128, no swizzle
   const uint16_t* rnorm;     // fp16 bits (BH, Sk)
-  const uint8_t* images;     // [unit][chunk][hi | lo][64 rows x 128 bytes swizzled]
+  const uint8_t* images;     // [unit][chunk][hi | lo][QN rows x 128 bytes swizzled]
   float* scores;             // (BH, Sq, Sk)
   int32_t* status;
   int64_t Sq, Sk;
-  int32_t n_qblocks;         // ceil(Sq / 64)
+  int32_t n_qblocks;         // ceil(Sq / QN)
   int32_t tiles_per_unit;    // ceil(Sk / 128)
   int32_t total_tiles;
   int32_t pad_;
@@ -90,11 +101,12 @@ __device__ __forceinline__ uint32_t idesc_f16_n(uint32_t n) {
   return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
-template <int D>
+template <int D, int QN>
 __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_constant__ QjlBatch batch) {
   pdl_wait();                                    // before the TMEM allocation: see tq_v2_umma.cu
-  using C = QCfg<D>;
-  constexpr int kHalfChunks = C::kHalfChunks, kChunks = C::kChunks;
+  using C = QCfg<D, QN>;
+  constexpr int kHalfChunks = C::kHalfChunks, kChunks = C::kChunks, kNSK = C::kNSK, kNSG = C::kNSG, kNSR = C::kNSR;
+  constexpr int kTmemCols = 2 * QN * kNT;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
@@ -121,8 +133,8 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
   const uint32_t bar_tempty = bar_tfull + 8 * kNT;         // [kNT] drain (4 arrivals) -> MMA
   const uint32_t bar_imgfull = bar_tempty + 8 * kNT;
   const uint32_t bar_imgfree = bar_imgfull + 8;
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + C::kOffBar + 200);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + C::kOffBar + 208);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + C::kOffBar + 400);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + C::kOffBar + 408);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total = batch.total_tiles;
@@ -141,7 +153,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(smem_u32((const void*)tmem_slot), 2 * kQ * kNT);
+  if (warp == 1) tmem_alloc(smem_u32((const void*)tmem_slot), kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -200,7 +212,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
     bool ok = true;
     int img_uses = 0, cur_unit = -1;
     int kc = 0, gc = 0;
-    const uint32_t idesc = idesc_f16_n(2 * kQ);
+    const uint32_t idesc = idesc_f16_n(2 * QN);
     const uint64_t b_base = smem_desc_sw128(img_smem);
     for (int i = 0; i < n_local && ok; ++i) {
       const int t = t0 + i;
@@ -214,12 +226,13 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
       ok = ok && mbar_wait(bar_tempty + 8 * b, (uint32_t)(((i / kNT) & 1) ^ 1), abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      const uint32_t d_tmem = tmem_base + (uint32_t)(b * 2 * kQ);
+      const uint32_t d_tmem = tmem_base + (uint32_t)(b * 2 * QN);
       const bool last_of_unit = i + 1 >= n_local || (t + 1) / tpu != unit;
 #pragma unroll 1
       for (int c = 0; c < kChunks; ++c) {
-        // chunks 0 .. D/64-1 come from the k_mse ring, the others from the expanded sign ring
-        const bool from_k = c < kHalfChunks;
+        // k_mse and expanded signs in turn, so that both rings are refilled at the same pace: with all of a tile's k_mse
+        // chunks first, the loads in flight were those of one ring most of the time
+        const bool from_k = (c & 1) == 0;
         uint32_t a_addr, full_bar, empty_bar, parity;
         if (from_k) {
           const int s = kc % kNSK;
@@ -237,7 +250,7 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
         if (!ok) break;
         tc_fence_after();
         const uint64_t a_base = smem_desc_sw128(a_addr);
-        const uint64_t b_off = (uint64_t)((uint32_t)c * 2u * kChunkB / 16);
+        const uint64_t b_off = (uint64_t)((uint32_t)((c & 1) * kHalfChunks + (c >> 1)) * 2u * C::kChunkB / 16);
         if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < 4; ++k)
@@ -305,30 +318,30 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
     bool ok = true;
-    for (int i = 0; i < n_local && ok; ++i) {
+    for (int i = (warp - 2 - kExpWarps) >> 2; i < n_local && ok; i += kDrainWarps / 4) {
       const int t = t0 + i;
       const int unit = t / tpu, kt = t - unit * tpu;
       const int64_t bh = unit / batch.n_qblocks;
-      const int q0 = (unit % batch.n_qblocks) * kQ;
+      const int q0 = (unit % batch.n_qblocks) * QN;
       const int64_t key = (int64_t)kt * kKeys + row;
       const int b = i % kNT;
       ok = __all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * b, (uint32_t)((i / kNT) & 1), abort_flag));   // warp-collective TMEM loads follow
       if (!ok) break;
       tc_fence_after();
-      const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * 2 * kQ);
+      const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * 2 * QN);
       float* out = batch.scores + (bh * batch.Sq + q0) * batch.Sk + key;
-      const bool key_ok = key < batch.Sk;
+      const int rows = key < batch.Sk ? (int)(batch.Sq - q0 < QN ? batch.Sq - q0 : QN) : 0;      // queries that this lane stores
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < QN / 16; ++c) {
         uint32_t cur[16], low[16];
         tmem_issue16(tacc + c * 16, cur);
-        tmem_issue16(tacc + kQ + c * 16, low);
+        tmem_issue16(tacc + QN + c * 16, low);
         tmem_wait16(cur);
         tmem_wait16(low);
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-          const int q = c * 16 + e;
-          if (key_ok && q0 + q < batch.Sq) out[(int64_t)q * batch.Sk] = __uint_as_float(cur[e]) + __uint_as_float(low[e]);
+          if (c * 16 + e < rows) *out = __uint_as_float(cur[e]) + __uint_as_float(low[e]);
+          out += batch.Sk;
         }
       }
       tc_fence_before();
@@ -344,16 +357,16 @@ __global__ void __launch_bounds__(kThreadsQ, 1) k_umma_qjl_scores(const __grid_c
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 2 * kQ * kNT);
+    tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
-template <int D>
+template <int D, int QN>
 int launch(const TqQjlScoreJob& job, uint8_t* images, cudaStream_t st) {
   TensorMapEncodeFn enc = tensor_map_encoder();
   if (enc == nullptr) return TQ_ELAUNCH;
   static thread_local QjlBatch batch;
-  const int n_qblocks = (int)((job.Sq + kQ - 1) / kQ);
+  const int n_qblocks = (int)((job.Sq + QN - 1) / QN);
   const int64_t tpu = (job.Sk + kKeys - 1) / kKeys;
   const int64_t units = job.BH * n_qblocks;
   const int64_t total = units * tpu;
@@ -371,7 +384,7 @@ int launch(const TqQjlScoreJob& job, uint8_t* images, cudaStream_t st) {
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { note_cuda_error(100000 + (int)r); return TQ_ELAUNCH; }
-  int rc = simt_qjl_query_operand(job, images, st);
+  int rc = simt_qjl_query_operand(job, images, QN, st);
   if (rc != TQ_OK) return rc;
   batch.rnorm = job.rnorm;
   batch.images = images;
@@ -389,10 +402,10 @@ int launch(const TqQjlScoreJob& job, uint8_t* images, cudaStream_t st) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int grid = (int)(total < sms ? total : sms);
-  cudaError_t e = cudaFuncSetAttribute(k_umma_qjl_scores<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)QCfg<D>::kSmemBytes);
+  cudaError_t e = cudaFuncSetAttribute(k_umma_qjl_scores<D, QN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)QCfg<D, QN>::kSmemBytes);
   if (e != cudaSuccess) return refused(e);
-  launch_after(k_umma_qjl_scores<D>, dim3(grid), dim3(kThreadsQ), QCfg<D>::kSmemBytes, st, batch);
+  launch_after(k_umma_qjl_scores<D, QN>, dim3(grid), dim3(kThreadsQ), QCfg<D, QN>::kSmemBytes, st, batch);
   return check_launch();
 }
 
@@ -409,14 +422,15 @@ bool umma_qjl_scores_eligible(const TqQjlScoreJob& job) {
 
 size_t umma_qjl_scores_image_bytes(int64_t BH, int64_t Sq, int D) {
   if (D != 128 && D != 256) return 0;
-  const int64_t units = BH * ((Sq + kQ - 1) / kQ);
-  return (size_t)units * (D == 256 ? QCfg<256>::kImageBytes : QCfg<128>::kImageBytes) + 1024;
+  const int64_t units = BH * ((Sq + 63) / 64);
+  return (size_t)units * (D == 256 ? QCfg<256, 64>::kImageBytes : QCfg<128, 64>::kImageBytes) + 1024;
 }
 
 // images: scratch for the query operands
 int umma_qjl_scores(const TqQjlScoreJob& job, void* images, cudaStream_t st) {
   uint8_t* img = reinterpret_cast<uint8_t*>(((uintptr_t)images + 1023u) & ~(uintptr_t)1023u);
-  return job.D == 256 ? launch<256>(job, img, st) : launch<128>(job, img, st);
+  if (job.Sq <= 16) return job.D == 256 ? launch<256, 16>(job, img, st) : launch<128, 16>(job, img, st);
+  return job.D == 256 ? launch<256, 64>(job, img, st) : launch<128, 64>(job, img, st);
 }
 
 int umma_qjl_device_status() {

@@ -1015,24 +1015,25 @@ __global__ void __launch_bounds__(NT) k_qjl_scores(TqQjlScoreJob job, const floa
 }
 
 // Query operand of the tensor-core score kernel (tq_qjl_umma.cu), head_dim a multiple of 64: per unit (head, block of
-// 64 queries) the rows [Q | corr * Q S^T] as fp16 pieces hi + lo, laid out [chunk of 64 columns][piece][row][64], rows of
-// 128 bytes with 16-byte chunk c at c ^ (row & 7); rows past Sq are zero.  A CTA takes 32 rows and 64 columns: the
+// 16 or 64 queries) the rows [Q | corr * Q S^T] as fp16 pieces hi + lo, laid out [chunk of 64 columns][piece][row][64], rows of
+// 128 bytes with 16-byte chunk c at c ^ (row & 7); rows past Sq are zero.  A CTA takes 16 or 32 rows and 64 columns: the
 // projection (one sequential chain per output, as tq_project), then the query's own columns and the projected ones.
 // 1024 queries of head_dim 256 took 27 us as projection, upcast and image kernels (the projection read the whole matrix
 // for every four rows).
-template <int QDT>
-__global__ void __launch_bounds__(NT) k_qjl_query_operand(const void* q, int D, int64_t Sq, int n_qblocks,
+template <int QDT, int RI>
+__global__ void __launch_bounds__(NT) k_qjl_query_operand(const void* q, int D, int64_t Sq, int n_qblocks, int per_unit,
                                                          const float* __restrict__ qjl_t, float corr, uint8_t* __restrict__ images) {
-  constexpr int RI = 2, ROWS = 16 * RI;
+  constexpr int ROWS = 16 * RI;
   pdl_trigger();
   extern __shared__ __align__(16) float smem[];
   const int lda = lda_for(D);
   float* As = smem;
   float* Bs = As + ROWS * lda;
   const int chunks = D / 64;
-  const int cb = blockIdx.x % chunks, half = (blockIdx.x / chunks) & 1, unit = blockIdx.x / (2 * chunks);
+  const int groups = per_unit / ROWS;
+  const int cb = blockIdx.x % chunks, group = (blockIdx.x / chunks) % groups, unit = blockIdx.x / (groups * chunks);
   const int64_t bh = unit / n_qblocks;
-  const int64_t q0 = (int64_t)(unit % n_qblocks) * 64 + half * ROWS;       // first query of this CTA, of head bh
+  const int64_t q0 = (int64_t)(unit % n_qblocks) * per_unit + group * ROWS;       // first query of this CTA, of head bh
   b_begin<1, B_KN>(D, qjl_t + cb * 64, D, 64, Bs);
   // rows past the end of this head read as zero, so the row limit is the head's own end
   load_tile_rows<QDT, RI>(q, bh * Sq + q0, (bh + 1) * Sq, D, 1, (bh + 1) * Sq, 0, 0, D, As, lda, nullptr);
@@ -1040,11 +1041,11 @@ __global__ void __launch_bounds__(NT) k_qjl_query_operand(const void* q, int D, 
   zero_acc<RI, 1>(acc);
   tile_gemm<RI, 1, B_KN>(As, lda, D, qjl_t + cb * 64, D, 64, Bs, acc);
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  constexpr size_t piece = 64 * 64;                                        // elements of one piece of a chunk
+  const size_t piece = (size_t)per_unit * 64;                              // elements of one piece of a chunk
   uint16_t* img = reinterpret_cast<uint16_t*>(images) + (size_t)unit * 2 * chunks * 2 * piece;
 #pragma unroll
   for (int ri = 0; ri < RI; ++ri) {
-    const int r = ty * RI + ri, n = half * ROWS + r;
+    const int r = ty * RI + ri, n = group * ROWS + r;
 #pragma unroll
     for (int part = 0; part < 2; ++part) {                                 // the query's columns, then the projected ones
       uint16_t hi[4], lo[4];
@@ -1379,16 +1380,17 @@ size_t simt_qjl_scores_workspace(int64_t BH, int64_t Sq, int D) {
   return (size_t)2 * BH * Sq * D * sizeof(float);   // projected queries + room for upcast queries
 }
 
-int simt_qjl_query_operand(const TqQjlScoreJob& job, void* images, cudaStream_t st) {
-  const int n_qblocks = (int)((job.Sq + 63) / 64);
-  const int64_t blocks = job.BH * n_qblocks * 2 * (job.D / 64);
-  const size_t smem = sizeof(float) * (32 * lda_for(job.D) + b_ring_floats(1));
+int simt_qjl_query_operand(const TqQjlScoreJob& job, void* images, int per_unit, cudaStream_t st) {
+  const int n_qblocks = (int)((job.Sq + per_unit - 1) / per_unit);
+  const int rows = per_unit == 16 ? 16 : 32;
+  const int64_t blocks = job.BH * n_qblocks * (per_unit / rows) * (job.D / 64);
+  const size_t smem = sizeof(float) * (rows * lda_for(job.D) + b_ring_floats(1));
   const float corr = (float)(1.2533141373155001 / (double)job.D);   // sqrt(pi/2) / m with m = D
   int rc = TQ_OK;
   TQ_DISPATCH_DT(job.q_dtype, {
-    auto kern = k_qjl_query_operand<DT_>;
+    auto kern = rows == 16 ? k_qjl_query_operand<DT_, 1> : k_qjl_query_operand<DT_, 2>;
     rc = set_smem(kern, smem);
-    if (rc == TQ_OK) kern<<<(unsigned)blocks, NT, smem, st>>>(job.q, job.D, job.Sq, n_qblocks, job.qjl_t, corr, reinterpret_cast<uint8_t*>(images));
+    if (rc == TQ_OK) kern<<<(unsigned)blocks, NT, smem, st>>>(job.q, job.D, job.Sq, n_qblocks, per_unit, job.qjl_t, corr, reinterpret_cast<uint8_t*>(images));
   });
   return rc != TQ_OK ? rc : check_launch();
 }
