@@ -59,8 +59,14 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// flat vector number -> element offset of its first coordinate
+// flat vector number -> element offset of its first coordinate.  A 64-bit division is a subroutine of a hundred instructions, so
+// numbers that fit take 32-bit ones.
 __device__ __forceinline__ int64_t vec_offset(int64_t n, int64_t H, int64_t S, int64_t sb, int64_t sh, int64_t ss) {
+  if (((n | H | S) >> 32) == 0) {
+    const uint32_t un = (uint32_t)n, uS = (uint32_t)S, uH = (uint32_t)H;
+    const uint32_t t = un / uS, b = t / uH;
+    return (int64_t)b * sb + (int64_t)(t - b * uH) * sh + (int64_t)(un - t * uS) * ss;
+  }
   int64_t s = n % S;
   int64_t t = n / S;
   int64_t h = t % H;

@@ -21,14 +21,19 @@ constexpr int TM = 64;    // vectors per tile of the large form (RI = 4)
 constexpr int KC = 16;    // k rows of B staged per step
 constexpr int NT = 256;   // threads per CTA
 constexpr int BPAD = 4;
-constexpr int BST = 3;    // stages of the ring that B travels through
+// Stages of the ring that B travels through, for 64 * nj columns.  A fifth leaves room for one CTA fewer per SM.
+__host__ __device__ constexpr int b_stages(int nj) { return nj <= 2 ? 4 : 3; }
 
 enum { B_KN = 0, B_NK = 1 };
+
+// A thread's place in the 16 x 16 grid over a tile; a warp is 4 rows of it by 8 columns.
+__device__ __forceinline__ int tile_tx() { return (threadIdx.x & 7) | ((threadIdx.x >> 2) & 8); }
+__device__ __forceinline__ int tile_ty() { return ((threadIdx.x >> 3) & 3) | ((threadIdx.x >> 4) & 12); }
 
 __host__ __device__ inline int lda_for(int K) { return round_up(K, KC) + 4; }
 __host__ __device__ inline int ldb_for(int N) { return round_up(N, 64) + BPAD; }
 // floats of shared memory for the ring of a contraction with 64 * nj columns
-__host__ __device__ inline int b_ring_floats(int nj) { return BST * KC * (64 * nj + BPAD); }
+__host__ __device__ inline int b_ring_floats(int nj) { return b_stages(nj) * KC * (64 * nj + BPAD); }
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool ok) {
   const int bytes = ok ? 4 : 0;                          // 0: the word is filled with zero, nothing is read
@@ -39,13 +44,13 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool ok
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
-// One k-chunk of B (rows k0 .. k0 + KC) into ring stage k0 / KC % BST, as one group of asynchronous copies.  A chunk
+// One k-chunk of B (rows k0 .. k0 + KC) into its ring stage, as one group of asynchronous copies.  A chunk
 // past the end of B commits an empty group, so that groups and chunks keep step.
 template <int NJ, int BL>
 __device__ __forceinline__ void b_stage(int k0, int K, const float* __restrict__ Bg, int64_t ldg, int N, float* ring) {
   constexpr int npad = 64 * NJ;
   constexpr int ldb = npad + BPAD;
-  float* Bs = ring + (k0 / KC) % BST * (KC * ldb);
+  float* Bs = ring + (k0 / KC) % b_stages(NJ) * (KC * ldb);
   if (k0 < round_up(K, KC)) {
     if (BL == B_KN && (N & 3) == 0 && (ldg & 3) == 0 && ((uintptr_t)Bg & 15u) == 0) {
       for (int e = threadIdx.x; e < KC * (npad / 4); e += NT) {
@@ -67,12 +72,12 @@ __device__ __forceinline__ void b_stage(int k0, int K, const float* __restrict__
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// The first BST - 1 chunks of B: issued before whatever the kernel does ahead of the contraction, so that their
+// The first chunks of B: issued before whatever the kernel does ahead of the contraction, so that their
 // latency runs beside it.  The previous contraction's readers must be past their last barrier.
 template <int NJ, int BL>
 __device__ __forceinline__ void b_begin(int K, const float* __restrict__ Bg, int64_t ldg, int N, float* ring) {
 #pragma unroll
-  for (int c = 0; c < BST - 1; ++c) b_stage<NJ, BL>(c * KC, K, Bg, ldg, N, ring);
+  for (int c = 0; c < b_stages(NJ) - 1; ++c) b_stage<NJ, BL>(c * KC, K, Bg, ldg, N, ring);
 }
 
 // acc[ri][4*j+c] += sum_k As[(ty*RI+ri)*lda + k] * B[k][tx*4 + 64*j + c]
@@ -80,41 +85,68 @@ __device__ __forceinline__ void b_begin(int K, const float* __restrict__ Bg, int
 // [N][K] row-major with row stride ldg (B_NK).  Columns >= N and rows >= K read
 // as zero.  As must hold zeros in columns [K, round_up(K,16)).  b_begin() with the same B comes first.
 //
-// B goes through a ring of three chunks of 16 rows by asynchronous copies: one barrier per chunk, and a chunk's L2
-// latency passes under the two before it (staged through registers with two barriers, each chunk cost that latency:
+// B goes through a ring of chunks of 16 rows by asynchronous copies: one barrier per chunk, and a chunk's L2
+// latency passes under those before it (staged through registers with two barriers, each chunk cost that latency:
 // 40 us for 4096 vectors of head_dim 128 on 64 SMs).  Every output is one chain of fused multiply-adds in
 // ascending k, whatever RI is.
+//
+// What bounds it is what the shared-memory loads return: 128 bytes a clock into the registers, broadcast or not, that is
+// RI + 4 NJ floats a thread and k (80 clocks of a 32 x 128 tile's k, 96 of a 64 x 128 tile's) against RI x 4 NJ / 128 lanes of
+// multiply-adds (32 and 64).  So with one tile per SM the small tile is faster, with two the large one.  With RI = 2 the
+// operands of the next four k are loaded while the last four are multiplied; two columns share one packed multiply-add
+// (fma.rn.f32x2: the same IEEE result in each half).
+__device__ __forceinline__ void fma2_acc(float& c0, float& c1, float a, float b0, float b1) {
+  unsigned long long av, bv, cv;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(av) : "f"(a));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(bv) : "f"(b0), "f"(b1));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(cv) : "f"(c0), "f"(c1));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(cv) : "l"(av), "l"(bv), "l"(cv));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(c0), "=f"(c1) : "l"(cv));
+}
+// volatile: the compiler otherwise moves the loads back to their uses
+__device__ __forceinline__ float4 lds4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 template <int RI, int NJ, int BL>
 __device__ __forceinline__ void tile_gemm(const float* As, int lda, int K, const float* __restrict__ Bg, int64_t ldg,
                                           int N, float* ring, float (&acc)[RI][4 * NJ]) {
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
+  const int tx = tile_tx(), ty = tile_ty();
   constexpr int ldb = 64 * NJ + BPAD;
   const int kpad = round_up(K, KC);
+  const uint32_t Ar = (uint32_t)__cvta_generic_to_shared(As + ty * RI * lda);
   for (int k0 = 0; k0 < kpad; k0 += KC) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(BST - 2) : "memory");
+    asm volatile("cp.async.wait_group %0;" ::"n"(b_stages(NJ) - 2) : "memory");
     __syncthreads();                            // chunk k0 is there for everyone; the stage of chunk k0 - KC is free
-    b_stage<NJ, BL>(k0 + (BST - 1) * KC, K, Bg, ldg, N, ring);
-    const float* Bs = ring + (k0 / KC) % BST * (KC * ldb);
+    b_stage<NJ, BL>(k0 + (b_stages(NJ) - 1) * KC, K, Bg, ldg, N, ring);
+    const uint32_t Bs = (uint32_t)__cvta_generic_to_shared(ring + (k0 / KC) % b_stages(NJ) * (KC * ldb) + tx * 4);
+    constexpr int BUF = RI <= 2 ? 2 : 1;        // the large tile has no registers for a second set
+    float4 a[BUF][RI], b[BUF][4][NJ];
+    auto load = [&](int g) {
 #pragma unroll
-    for (int kk = 0; kk < KC; kk += 4) {
-      float4 a[RI];
+      for (int ri = 0; ri < RI; ++ri) a[g % BUF][ri] = lds4(Ar + 4u * (uint32_t)(ri * lda + k0 + 4 * g));
 #pragma unroll
-      for (int ri = 0; ri < RI; ++ri) a[ri] = *reinterpret_cast<const float4*>(As + (ty * RI + ri) * lda + k0 + kk);
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) b[g % BUF][u][j] = lds4(Bs + 4u * (uint32_t)((4 * g + u) * ldb + 64 * j));
+    };
+    if (BUF == 2) load(0);
+#pragma unroll
+    for (int g = 0; g < KC / 4; ++g) {
+      if (BUF == 1) load(g);
+      else if (g + 1 < KC / 4) load(g + 1);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        float4 b[NJ];
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) b[j] = *reinterpret_cast<const float4*>(Bs + (kk + u) * ldb + tx * 4 + 64 * j);
 #pragma unroll
         for (int ri = 0; ri < RI; ++ri) {
-          float av = (u == 0) ? a[ri].x : (u == 1) ? a[ri].y : (u == 2) ? a[ri].z : a[ri].w;
+          const float4 af = a[g % BUF][ri];
+          const float av = (u == 0) ? af.x : (u == 1) ? af.y : (u == 2) ? af.z : af.w;
 #pragma unroll
           for (int j = 0; j < NJ; ++j) {
-            acc[ri][4 * j + 0] = fmaf(av, b[j].x, acc[ri][4 * j + 0]);
-            acc[ri][4 * j + 1] = fmaf(av, b[j].y, acc[ri][4 * j + 1]);
-            acc[ri][4 * j + 2] = fmaf(av, b[j].z, acc[ri][4 * j + 2]);
-            acc[ri][4 * j + 3] = fmaf(av, b[j].w, acc[ri][4 * j + 3]);
+            const float4 bf = b[g % BUF][u][j];
+            fma2_acc(acc[ri][4 * j + 0], acc[ri][4 * j + 1], av, bf.x, bf.y);
+            fma2_acc(acc[ri][4 * j + 2], acc[ri][4 * j + 3], av, bf.z, bf.w);
           }
         }
       }
@@ -134,7 +166,7 @@ __device__ __forceinline__ void zero_acc(float (&acc)[RI][4 * NJ]) {
 // registers -> Cs[r*ldc + n] for n < ncols (a multiple of 4, at most ldc); caller syncs around it
 template <int RI, int NJ>
 __device__ __forceinline__ void acc_to_smem(const float (&acc)[RI][4 * NJ], float* Cs, int ldc, int ncols) {
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = tile_tx(), ty = tile_ty();
 #pragma unroll
   for (int ri = 0; ri < RI; ++ri)
 #pragma unroll
@@ -147,33 +179,36 @@ __device__ __forceinline__ void acc_to_smem(const float (&acc)[RI][4 * NJ], floa
 }
 
 // Load a tile of vectors as fp32 into Xs (zero padded to kpad columns, zero rows
-// past n_total); per-row L2 norms into nrm[] when wanted.
-// A warp loads two of its rows at a time, so that up to eight of a lane's loads are in flight.
+// past n_total); per-row L2 norms into nrm[] when wanted, and As = x / (norm + 1e-8) of the warp's own rows.
+// A warp loads up to four of its rows at a time, so that sixteen of a lane's loads are in flight.
 template <int XDT, int RI>
 __device__ __forceinline__ void load_tile_rows(const void* x, int64_t row0, int64_t n_total, int D, int64_t H, int64_t S,
-                                               int64_t sb, int64_t sh, int64_t ss, float* Xs, int ld, float* nrm) {
+                                               int64_t sb, int64_t sh, int64_t ss, float* Xs, int ld, float* nrm,
+                                               float* As = nullptr) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kpad = round_up(D, KC);
+  constexpr int R = RI == 1 ? 2 : 4;
 #pragma unroll
-  for (int r0 = warp; r0 < 16 * RI; r0 += 2 * (NT / 32)) {
-    float ssq[2] = {0.f, 0.f};
-    int64_t off[2];
+  for (int r0 = warp; r0 < 16 * RI; r0 += R * (NT / 32)) {
+    float ssq[R];
+    int64_t off[R];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < R; ++h) {
+      ssq[h] = 0.f;
       const int64_t n = row0 + r0 + h * (NT / 32);
       off[h] = n < n_total ? vec_offset(n, H, S, sb, sh, ss) : -1;
     }
     for (int k0 = 0; k0 < kpad; k0 += 128) {
-      float v[2][4];
+      float v[R][4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
+      for (int h = 0; h < R; ++h)
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int k = k0 + 32 * u + lane;
           v[h][u] = (off[h] >= 0 && k < D) ? load_elem<XDT>(x, off[h] + k) : 0.f;
         }
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
+      for (int h = 0; h < R; ++h)
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int k = k0 + 32 * u + lane;
@@ -185,9 +220,20 @@ __device__ __forceinline__ void load_tile_rows(const void* x, int64_t row0, int6
     }
     if (nrm != nullptr) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float s = warp_sum(ssq[h]);
-        if (lane == 0) nrm[r0 + h * (NT / 32)] = __fsqrt_rn(s);
+      for (int h = 0; h < R; ++h) ssq[h] = __fsqrt_rn(warp_sum(ssq[h]));
+#pragma unroll
+      for (int h = 0; h < R; ++h)
+        if (lane == 0) nrm[r0 + h * (NT / 32)] = ssq[h];
+    }
+    if (As != nullptr) {                          // each lane its own columns
+      for (int k0 = lane; k0 < kpad; k0 += 128) {
+#pragma unroll
+        for (int h = 0; h < R; ++h)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int at = (r0 + h * (NT / 32)) * ld + k0 + 32 * u;
+            if (k0 + 32 * u < kpad) As[at] = nrm != nullptr ? __fdiv_rn(Xs[at], ssq[h] + 1e-8f) : Xs[at];
+          }
       }
     }
   }
@@ -267,6 +313,76 @@ __device__ __forceinline__ void emit_indices_row(const float* row, int D, int bi
   }
 }
 
+// The same for the rows warp + 8 i of a tile, four at a time where there are as many: a search is `bits` dependent look-ups,
+// which the other rows' hide.
+template <int R, int IPB, int NB>
+__device__ __forceinline__ void emit_packed_rows(const float* Cs, int ldc, int D, int bits, const float* thr_s, uint8_t* out, int64_t row0,
+                                                 int64_t n_total, int r0, int lane) {
+  const int G = (D + IPB - 1) / IPB;
+  for (int g0 = lane; g0 < G; g0 += 32 * NB) {
+    float y[R * IPB * NB];
+    int q[R * IPB * NB];
+#pragma unroll
+    for (int h = 0; h < R; ++h)
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int i = 0; i < IPB; ++i) {
+          const int c = (g0 + 32 * b) * IPB + i;
+          y[(h * NB + b) * IPB + i] = c < D ? Cs[(r0 + 8 * h) * ldc + c] : -INFINITY;      // past the end: index 0
+        }
+    quantize_many<R * IPB * NB>(y, thr_s, bits, q);
+#pragma unroll
+    for (int h = 0; h < R; ++h)
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        unsigned byte = 0;
+#pragma unroll
+        for (int i = 0; i < IPB; ++i) byte |= (unsigned)q[(h * NB + b) * IPB + i] << (bits * (IPB - 1 - i));
+        const int64_t n = row0 + r0 + 8 * h;
+        if (g0 + 32 * b < G && n < n_total) out[n * G + g0 + 32 * b] = (uint8_t)byte;
+      }
+  }
+}
+template <int RI>
+__device__ __forceinline__ void emit_indices_tile(const float* Cs, int ldc, int D, int bits, int mode, const float* thr_s, void* out,
+                                                  int64_t row0, int64_t n_total) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int R = RI == 1 ? 2 : 4;
+#pragma unroll 1
+  for (int r0 = warp; r0 < 16 * RI; r0 += 8 * R) {
+    if (mode == TQ_IDX_PACKED) {
+      const int ipb = 8 / bits;
+      uint8_t* o = reinterpret_cast<uint8_t*>(out);
+      if (ipb == 1) emit_packed_rows<R, 1, 4>(Cs, ldc, D, bits, thr_s, o, row0, n_total, r0, lane);
+      else if (ipb == 2) emit_packed_rows<R, 2, 2>(Cs, ldc, D, bits, thr_s, o, row0, n_total, r0, lane);
+      else if (ipb == 4) emit_packed_rows<R, 4, 1>(Cs, ldc, D, bits, thr_s, o, row0, n_total, r0, lane);
+      else emit_packed_rows<R, 8, 1>(Cs, ldc, D, bits, thr_s, o, row0, n_total, r0, lane);
+      continue;
+    }
+    for (int c0 = lane; c0 < D; c0 += 128) {
+      float y[4 * R];
+      int q[4 * R];
+#pragma unroll
+      for (int h = 0; h < R; ++h)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) y[4 * h + u] = c0 + 32 * u < D ? Cs[(r0 + 8 * h) * ldc + c0 + 32 * u] : 0.f;
+      quantize_many<4 * R>(y, thr_s, bits, q);
+#pragma unroll
+      for (int h = 0; h < R; ++h) {
+        const int64_t n = row0 + r0 + 8 * h;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = c0 + 32 * u;
+          if (c >= D || n >= n_total) continue;
+          if (mode == TQ_IDX_U8) reinterpret_cast<uint8_t*>(out)[n * (int64_t)D + c] = (uint8_t)q[4 * h + u];
+          else reinterpret_cast<int64_t*>(out)[n * (int64_t)D + c] = (int64_t)q[4 * h + u];
+        }
+      }
+    }
+  }
+}
+
 __device__ __forceinline__ int fetch_index(const void* idx, int mode, int64_t n, int c, int D, int bits) {
   if (mode == TQ_IDX_PACKED) {
     const int ipb = 8 / bits;
@@ -317,16 +433,11 @@ __global__ void __launch_bounds__(NT) k_quantize(TqQuantizeJob job) {
     __syncthreads();
     b_begin<NJ, B_KN>(D, job.rotation_t, D, D, Bs);
     load_tile_rows<XDT, RI>(job.x, row0, n_total, D, job.H, job.S, job.stride_b, job.stride_h, job.stride_s, As, lda,
-                        job.normalize ? nrm : nullptr);
+                        job.normalize ? nrm : nullptr, job.normalize ? As : nullptr);
     if (job.normalize) {
-      __syncwarp();
-      for (int r = warp; r < TM; r += NT / 32) {
-        float nv = nrm[r];
-        int64_t n = row0 + r;
-        if (lane == 0 && n < n_total) job.norms_out[n] = __half_as_ushort(__float2half_rn(nv));
-        float den = nv + 1e-8f;
-        for (int k = lane; k < kpad; k += 32) As[r * lda + k] = __fdiv_rn(As[r * lda + k], den);
-      }
+      __syncwarp();                               // a warp's rows are warp + 8 i
+      const int r = warp + 8 * lane;
+      if (r < TM && row0 + r < n_total) job.norms_out[row0 + r] = __half_as_ushort(__float2half_rn(nrm[r]));
     }
     float acc[RI][4 * NJ];
     zero_acc<RI, NJ>(acc);
@@ -334,10 +445,7 @@ __global__ void __launch_bounds__(NT) k_quantize(TqQuantizeJob job) {
     __syncthreads();
     acc_to_smem<RI, NJ>(acc, As, lda, kpad);
     __syncthreads();
-    for (int r = warp; r < TM; r += NT / 32) {
-      int64_t n = row0 + r;
-      if (n < n_total) emit_indices_row(As + r * lda, D, job.bits, job.idx_mode, thr_s, job.idx_out, n, lane);
-    }
+    emit_indices_tile<RI>(As, lda, D, job.bits, job.idx_mode, thr_s, job.idx_out, row0, n_total);
   }
 }
 
@@ -358,7 +466,7 @@ __global__ void __launch_bounds__(NT) k_dequantize(TqDequantizeJob job) {
   const int64_t n_total = job.B * job.H * job.S;
   const int64_t tiles = (n_total + TM - 1) / TM;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = tile_tx(), ty = tile_ty();
   const int kpad = round_up(D, KC);
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t row0 = tile * TM;
@@ -412,7 +520,7 @@ __global__ void __launch_bounds__(NT) k_project(const void* x, int64_t n_total, 
   float* As = smem;
   float* Bs = As + TM * lda;
   const int64_t tiles = (n_total + TM - 1) / TM;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = tile_tx(), ty = tile_ty();
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t row0 = tile * TM;
     __syncthreads();
@@ -831,20 +939,14 @@ __global__ void __launch_bounds__(NT) k_qjl_compress(TqQjlCompressJob job) {
   const int64_t n_total = job.B * job.H * job.S;
   const int64_t tiles = (n_total + TM - 1) / TM;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = tile_tx(), ty = tile_ty();
   const int kpad = round_up(D, KC);
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t row0 = tile * TM;
     __syncthreads();
     b_begin<NJ, B_KN>(D, job.rotation_t, D, D, Bs);
     load_tile_rows<XDT, RI>(job.x, row0, n_total, D, job.H, job.S, job.stride_b, job.stride_h, job.stride_s, Xs, lda,
-                        job.normalize ? nrm : nullptr);
-    __syncwarp();
-    for (int r = warp; r < TM; r += NT / 32) {
-      float den = job.normalize ? nrm[r] + 1e-8f : 1.f;
-      for (int k = lane; k < kpad; k += 32)
-        As[r * lda + k] = job.normalize ? __fdiv_rn(Xs[r * lda + k], den) : Xs[r * lda + k];
-    }
+                        job.normalize ? nrm : nullptr, As);
     {
       float acc[RI][4 * NJ];
       zero_acc<RI, NJ>(acc);
@@ -855,22 +957,23 @@ __global__ void __launch_bounds__(NT) k_qjl_compress(TqQjlCompressJob job) {
     }
     __syncthreads();
     // quantise in place: As <- centroid of the nearest level
-    for (int r = warp; r < TM; r += NT / 32) {
-      int64_t n = row0 + r;
+#pragma unroll 1
+    for (int r = warp; r < TM; r += 4 * (NT / 32)) {
       for (int c0 = lane; c0 < kpad; c0 += 128) {
-        float y[4];
-        int q[4];
+        float y[16];
+        int q[16];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) y[u] = c0 + 32 * u < D ? As[r * lda + c0 + 32 * u] : 0.f;
-        quantize_many<4>(y, thr_s, job.bits, q);
+        for (int u = 0; u < 16; ++u) y[u] = c0 + 32 * (u & 3) < D ? As[(r + 8 * (u >> 2)) * lda + c0 + 32 * (u & 3)] : 0.f;
+        quantize_many<16>(y, thr_s, job.bits, q);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int c = c0 + 32 * u;
+        for (int u = 0; u < 16; ++u) {
+          const int c = c0 + 32 * (u & 3), rr = r + 8 * (u >> 2);
+          const int64_t n = row0 + rr;
           if (c < D && job.idx_out != nullptr && n < n_total) {
             if (job.idx_mode == TQ_IDX_I64) reinterpret_cast<int64_t*>(job.idx_out)[n * D + c] = q[u];
             else if (job.idx_mode == TQ_IDX_U8) reinterpret_cast<uint8_t*>(job.idx_out)[n * D + c] = (uint8_t)q[u];
           }
-          if (c < kpad) As[r * lda + c] = c < D ? cent_s[q[u]] : 0.f;
+          if (c < kpad) As[rr * lda + c] = c < D ? cent_s[q[u]] : 0.f;
         }
       }
     }
@@ -958,7 +1061,7 @@ __global__ void __launch_bounds__(NT) k_qjl_scores(TqQjlScoreJob job, const floa
   const int64_t key_tiles = (job.Sk + TM - 1) / TM;
   const int64_t total = job.BH * key_tiles;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = tile_tx(), ty = tile_ty();
   const int kpad = round_up(D, KC);
   for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
     const int64_t bh = t / key_tiles;
@@ -1040,7 +1143,7 @@ __global__ void __launch_bounds__(NT) k_qjl_query_operand(const void* q, int D, 
   float acc[RI][4];
   zero_acc<RI, 1>(acc);
   tile_gemm<RI, 1, B_KN>(As, lda, D, qjl_t + cb * 64, D, 64, Bs, acc);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = tile_tx(), ty = tile_ty();
   const size_t piece = (size_t)per_unit * 64;                              // elements of one piece of a chunk
   uint16_t* img = reinterpret_cast<uint16_t*>(images) + (size_t)unit * 2 * chunks * 2 * piece;
 #pragma unroll
@@ -1194,11 +1297,11 @@ static int set_smem(K kernel, size_t bytes) {
 
 static inline int nj_for(int n) { return (n + 63) / 64; }
 
-// Vectors per tile: 64 (RI = 4) reads the matrix once for more vectors, 32 (RI = 2) gives twice the CTAs and half the
-// work behind each barrier.  Below two tiles of 64 per SM the chip is not full either way and the small tile wins.
-// With the ring, head_dim 128 in fp32: 4096 vectors quantised in 40 -> 19 us; 8192 vectors quantised in 32 -> 22 us, rebuilt in
-// 37 -> 26 us, MSE + QJL compressed in 78 -> 50 us (single launches, cold caches).
-static inline bool small_tiles(int64_t n) { return n < (int64_t)2 * TM * sm_count(); }
+// Vectors per tile: 64 (RI = 4) where an SM would get two tiles of 32 (RI = 2), which load more from shared memory per multiply-add
+// (see tile_gemm).  One contraction of head_dim 128: 12 300 clocks for one tile of 32 on an SM, 20 000 for two, 15 700 for one of 64.
+// Head_dim 128 in fp32: 4096 vectors quantised in 16.6 -> 14.4 us, 8192 in 22.7 -> 18.6 (32-vector tiles before), 16384 in 41 -> 27
+// and 100 000 in 160 -> 130 (operands of 64-vector tiles loaded four k at a time, two columns an instruction).
+static inline bool small_tiles(int64_t n) { return n <= (int64_t)(TM / 2) * sm_count(); }
 
 #define TQ_DISPATCH_NJ(nj, ...)                              \
   switch (nj) {                                              \
