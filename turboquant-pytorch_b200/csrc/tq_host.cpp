@@ -29,6 +29,14 @@ struct Api {
   decltype(&tq_qjl_compress) qjl_compress = nullptr;
   decltype(&tq_qjl_compress_workspace_bytes) qjl_compress_ws = nullptr;
   decltype(&tq_prod_inner_product) prod_inner = nullptr;
+  decltype(&tq_score_packed) score_packed = nullptr;
+  decltype(&tq_score_workspace_bytes) score_ws = nullptr;
+  decltype(&tq_decode_attention) decode_attention = nullptr;
+  decltype(&tq_decode_attention_workspace_bytes) decode_attention_ws = nullptr;
+  decltype(&tq_qjl_scores) qjl_scores = nullptr;
+  decltype(&tq_qjl_scores_workspace_bytes) qjl_scores_ws = nullptr;
+  decltype(&tq_qjl_scores_packed) qjl_scores_packed = nullptr;
+  decltype(&tq_qjl_scores_packed_workspace_bytes) qjl_scores_packed_ws = nullptr;
   PyObject* check = nullptr;               // Python: check(rc, what) raises for rc != 0
   // the classes' own job methods, as functions: MSECompressor.compress_job, decompress_job, TurboQuantV3.compress_jobs, decompress_jobs
   PyObject* jobs = nullptr;
@@ -114,6 +122,13 @@ at::Tensor make(at::IntArrayRef sizes, at::ScalarType type, int dev) {
 }
 
 void* stream_of(int dev) { return (void*)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream(); }
+
+// tokens [start, start + length) of a (B, H, S, D) tensor: what narrow(2, ...) gives, for half its host time (1.4 -> 0.76 us; a
+// generation step of 32 layers hands out 64 of them)
+at::Tensor tokens(const at::Tensor& t, int64_t start, int64_t length) {
+  const int64_t sizes[4] = {t.size(0), t.size(1), length, t.size(3)};
+  return at::as_strided(t, sizes, t.strides(), t.storage_offset() + start * t.stride(2));
+}
 
 // runs a call of the C ABI without the interpreter lock; false with a Python exception set when it fails
 template <typename F>
@@ -230,7 +245,7 @@ PyObject* compress_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor& x = i ? v : k;
     Ref dict(PyDict_New());
     if (!dict || !set_item(dict.p, k_comp, packed_dict(idx[i], norms[i], b, h, cut, d, i ? cv.bits : ck.bits)) ||
-        !set_item(dict.p, k_fp16, THPVariable_Wrap(x.narrow(2, cut, window))) || !set_item(dict.p, k_shape, shape_tuple(b, h, s, d)) ||
+        !set_item(dict.p, k_fp16, THPVariable_Wrap(tokens(x, cut, window))) || !set_item(dict.p, k_shape, shape_tuple(b, h, s, d)) ||
         !set_item(dict.p, k_split, PyLong_FromLongLong(cut)))
       return nullptr;
     PyTuple_SET_ITEM(out.p, i, dict.release());
@@ -283,7 +298,7 @@ PyObject* decompress_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int n_copies = 0;
   for (int i = 0; i < 2; ++i) {
     if (windows[i].numel() == 0) continue;
-    const at::Tensor dst = full[i].narrow(2, inner[i][2], windows[i].size(2));
+    const at::Tensor dst = tokens(full[i], inner[i][2], windows[i].size(2));
     const int64_t eb = dst.element_size();
     if (!copy_fits(windows[i], eb) || !copy_fits(dst, eb)) { const_cast<at::Tensor&>(dst).copy_(windows[i]); continue; }
     TqCopyJob& c = copies[n_copies++];
@@ -414,7 +429,8 @@ PyObject* prod_inner(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // ---------------------------------------------------------------- MSE + QJL
 // qjl_compress(x (B,H,S,D), pi, pi_t, codebook, qjl_t, bits, form) -> tuple | None.  form 0: the V2 dict's tensors
 // (k_mse, signs, rnorm); 1: packed (rows, sign bits, rnorm, norms), only where the tensor-core path takes it; 2: the
-// first generation's (indices, signs, rnorm) in int64 and fp32, vectors taken as they are
+// first generation's (indices, signs, rnorm) in int64 and fp32, vectors taken as they are; 3 and 4: forms 0 and 1 with the
+// vectors' own leading dimensions instead of rows
 PyObject* qjl_compress(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const int dev = c10::cuda::current_device();
@@ -422,7 +438,7 @@ PyObject* qjl_compress(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int i = 1; i < 5; ++i)
     if (!plain(a[i], dev)) return none();
   const at::Tensor &x = THPVariable_Unpack(a[0]), &qt = THPVariable_Unpack(a[4]);
-  const int64_t bits = PyLong_AsLongLong(a[5]), form = PyLong_AsLongLong(a[6]);
+  const int64_t bits = PyLong_AsLongLong(a[5]), asked = PyLong_AsLongLong(a[6]), form = asked >= 3 ? asked - 3 : asked;
   if (x.dim() != 4 || x.numel() == 0 || x.stride(3) != 1 || bits < 1 || bits > 8 || qt.dim() != 2) return none();
   const int64_t b = x.size(0), h = x.size(1), s = x.size(2), d = x.size(3), m = qt.size(1), rows = b * h * s;
   if (d > 256 || m > 256 || qt.size(0) != d || THPVariable_Unpack(a[1]).size(0) != d) return none();
@@ -438,13 +454,16 @@ PyObject* qjl_compress(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (bytes) { ws = make({(int64_t)bytes}, at::kByte, dev); j.workspace = ws.data_ptr(); j.workspace_bytes = bytes; }
   }
   at::Tensor first, signs, rnorm, norms;
+  const bool shaped = asked >= 3;
+  auto rows_of = [&](int64_t width, at::ScalarType type) { return shaped ? make({b, h, s, width}, type, dev) : make({rows, width}, type, dev); };
+  auto one_of = [&](at::ScalarType type) { return shaped ? make({b, h, s}, type, dev) : make({rows}, type, dev); };
   if (form == 0) {
-    first = make({rows, d}, at::kHalf, dev); signs = make({rows, m}, at::kChar, dev); rnorm = make({rows}, at::kHalf, dev);
+    first = rows_of(d, at::kHalf); signs = rows_of(m, at::kChar); rnorm = one_of(at::kHalf);
     j.k_mse_out = (uint16_t*)first.data_ptr(); j.idx_mode = TQ_IDX_U8; j.rnorm_dtype = TQ_F16;
   } else if (form == 1) {
     if (!ws.defined() || !x.is_contiguous() || m != d || (d != 128 && d != 256) || ((uintptr_t)x.data_ptr() & 15u)) return none();
-    first = make({rows, row_bytes(d, bits)}, at::kByte, dev); signs = make({rows, d / 8}, at::kByte, dev);
-    rnorm = make({rows}, at::kHalf, dev); norms = make({rows}, at::kFloat, dev);
+    first = rows_of(row_bytes(d, bits), at::kByte); signs = rows_of(d / 8, at::kByte);
+    rnorm = one_of(at::kHalf); norms = one_of(at::kFloat);
     j.idx_out = first.data_ptr(); j.idx_mode = TQ_IDX_PACKED; j.signs_dtype = 2; j.rnorm_dtype = TQ_F16; j.vec_norms_out = (float*)norms.data_ptr();
   } else {
     first = make({rows, d}, at::kLong, dev); signs = make({rows, m}, at::kFloat, dev); rnorm = make({rows}, at::kFloat, dev);
@@ -464,6 +483,168 @@ PyObject* qjl_compress(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Ref r3(THPVariable_Wrap(norms));
   if (!r3) return nullptr;
   return PyTuple_Pack(4, r0.p, r1.p, r2.p, r3.p);
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------- attention from packed keys
+bool is(const at::Tensor& t, at::ScalarType type, at::IntArrayRef sizes) { return t.scalar_type() == type && t.sizes() == sizes && t.is_contiguous(); }
+bool bit_width(PyObject* o, int64_t* bits) {
+  if (!PyLong_Check(o)) return false;
+  *bits = PyLong_AsLongLong(o);
+  if (*bits == -1 && PyErr_Occurred()) { PyErr_Clear(); return false; }
+  return *bits >= 1 && *bits <= 8;
+}
+// a float argument; false for anything that is not a plain number
+bool number(PyObject* o, float* v) {
+  if (!PyFloat_CheckExact(o) && !PyLong_CheckExact(o)) return false;
+  const double d = PyFloat_AsDouble(o);
+  if (d == -1.0 && PyErr_Occurred()) { PyErr_Clear(); return false; }
+  *v = (float)d;
+  return true;
+}
+at::Tensor scratch(size_t bytes, int dev) { return make({(int64_t)(bytes > 256 ? bytes : 256)}, at::kByte, dev); }
+
+// score_packed(q, idx_bytes, norms, pi_t, codebook, bits, scale, softmax) -> logits | (logits, probs) | None
+PyObject* score_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const int dev = c10::cuda::current_device();
+  int64_t bits;
+  float scale;
+  if (n != 8 || !float_plain(a[0], dev) || !bit_width(a[5], &bits) || !number(a[6], &scale) || !PyBool_Check(a[7])) return none();
+  for (int i = 1; i < 5; ++i)
+    if (!plain(a[i], dev)) return none();
+  const at::Tensor &q = THPVariable_Unpack(a[0]), &idx = THPVariable_Unpack(a[1]), &norms = THPVariable_Unpack(a[2]),
+                   &pi_t = THPVariable_Unpack(a[3]), &cb = THPVariable_Unpack(a[4]);
+  if (q.dim() != 4 || idx.dim() != 4 || !q.is_contiguous()) return none();
+  const int64_t b = q.size(0), hq = q.size(1), sq = q.size(2), d = q.size(3), hkv = idx.size(1), sk = idx.size(2);
+  if (d < 1 || d > 256 || hkv < 1 || hq % hkv != 0 || !is(idx, at::kByte, {b, hkv, sk, row_bytes(d, bits)}) || !is(norms, at::kHalf, {b, hkv, sk}) ||
+      !is(pi_t, at::kFloat, {d, d}) || cb.scalar_type() != at::kFloat || cb.numel() != TQ_CODEBOOK_FLOATS || !cb.is_contiguous())
+    return none();
+  c10::AutoGradMode no_grad(false);
+  at::Tensor logits = make({b, hq, sq, sk}, at::kFloat, dev), probs;
+  if (a[7] == Py_True) probs = make({b, hq, sq, sk}, at::kFloat, dev);
+  at::Tensor ws = scratch(api.score_ws(b, hq, sq, sk, (int)d), dev);
+  TqScoreJob j{};
+  j.q = q.data_ptr(); j.q_dtype = dtype_of(q); j.D = (int32_t)d; j.bits = (int32_t)bits;
+  j.B = b; j.Hq = hq; j.Sq = sq; j.Hkv = hkv; j.Sk = sk;
+  j.idx_bytes = (const uint8_t*)idx.data_ptr(); j.norms = (const uint16_t*)norms.data_ptr();
+  j.rotation_t = (const float*)pi_t.data_ptr(); j.codebook = (const float*)cb.data_ptr(); j.scale = scale;
+  j.logits = (float*)logits.data_ptr(); j.probs = probs.defined() ? (float*)probs.data_ptr() : nullptr;
+  j.workspace = ws.data_ptr(); j.workspace_bytes = (size_t)ws.numel();
+  void* st = stream_of(dev);
+  if (!call("tq_score_packed", [&] { return api.score_packed(&j, st); })) return nullptr;
+  Ref l(THPVariable_Wrap(logits));
+  if (!l || !probs.defined()) return l.release();
+  Ref p(THPVariable_Wrap(probs));
+  return p ? PyTuple_Pack(2, l.p, p.p) : nullptr;
+  END_HANDLE_TH_ERRORS
+}
+
+// decode_attention(q, k dict, v dict, key_codec, value_codec, k_window, v_window, scale) -> fp32 of q's shape | None
+PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TQ_NAME(k_idx, "idx_bytes"); TQ_NAME(k_norms, "vec_norms");
+  const int dev = c10::cuda::current_device();
+  float scale;
+  if (n != 8 || !float_plain(a[0], dev) || !PyDict_CheckExact(a[1]) || !PyDict_CheckExact(a[2]) || !float_plain(a[5], dev) ||
+      !float_plain(a[6], dev) || !number(a[7], &scale))
+    return none();
+  const at::Tensor &q = THPVariable_Unpack(a[0]), &kw = THPVariable_Unpack(a[5]), &vw = THPVariable_Unpack(a[6]);
+  if (q.dim() != 4 || q.size(3) != 128 || !q.is_contiguous()) return none();
+  const int64_t b = q.size(0), hq = q.size(1), sq = q.size(2);
+  Codec codec[2];
+  at::Tensor idx[2], norms[2];                        // held until the launch is out
+  for (int i = 0; i < 2; ++i) {
+    PyObject *io = PyDict_GetItem(a[1 + i], k_idx), *no = PyDict_GetItem(a[1 + i], k_norms);
+    if (io == nullptr || no == nullptr || !plain(io, dev) || !plain(no, dev) || !read_codec(a[3 + i], dev, &codec[i]) || codec[i].dim != 128) return none();
+    idx[i] = THPVariable_Unpack(io);
+    norms[i] = THPVariable_Unpack(no);
+    if (idx[i].dim() != 4 || norms[i].dim() != 3) return none();
+  }
+  const int64_t hkv = idx[0].size(1), sk = idx[0].size(2);
+  if (hkv < 1 || hq % hkv != 0) return none();
+  for (int i = 0; i < 2; ++i)
+    if (!is(idx[i], at::kByte, {b, hkv, sk, row_bytes(128, codec[i].bits)}) || !is(norms[i], at::kHalf, {b, hkv, sk})) return none();
+  if (kw.dim() != 4 || kw.sizes() != vw.sizes() || kw.scalar_type() != vw.scalar_type() || kw.strides() != vw.strides()) return none();
+  const int64_t w = kw.size(2);
+  if (w > 0 && (kw.size(0) != b || kw.size(1) != hkv || kw.size(3) != 128 || kw.stride(3) != 1)) return none();
+  c10::AutoGradMode no_grad(false);
+  at::Tensor out = make({b, hq, sq, 128}, at::kFloat, dev);
+  at::Tensor ws = scratch(api.decode_attention_ws(b, hq, sq, sk), dev);
+  TqDecodeAttnJob j{};
+  j.q = q.data_ptr(); j.q_dtype = dtype_of(q); j.D = 128; j.key_bits = (int32_t)codec[0].bits; j.value_bits = (int32_t)codec[1].bits;
+  j.B = b; j.Hq = hq; j.Sq = sq; j.Hkv = hkv; j.Sk = sk;
+  j.k_idx = (const uint8_t*)idx[0].data_ptr(); j.k_norms = (const uint16_t*)norms[0].data_ptr();
+  j.v_idx = (const uint8_t*)idx[1].data_ptr(); j.v_norms = (const uint16_t*)norms[1].data_ptr();
+  j.k_rotation_t = (const float*)codec[0].pi_t; j.v_rotation = (const float*)codec[1].pi;
+  j.k_codebook = (const float*)codec[0].cb; j.v_codebook = (const float*)codec[1].cb;
+  j.window_dtype = w > 0 ? dtype_of(kw) : TQ_F16;
+  if (w > 0) {
+    j.k_window = kw.data_ptr(); j.v_window = vw.data_ptr(); j.W = w;
+    j.wstride_b = kw.stride(0); j.wstride_h = kw.stride(1); j.wstride_s = kw.stride(2);
+  }
+  j.scale = scale;
+  j.out = (float*)out.data_ptr(); j.workspace = ws.data_ptr(); j.workspace_bytes = (size_t)ws.numel();
+  void* st = stream_of(dev);
+  if (!call("tq_decode_attention", [&] { return api.decode_attention(&j, st); })) return nullptr;
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// qjl_scores(q, k_mse, signs, rnorm, qjl_t) -> fp32 (B, H, Sq, Sk) | None
+PyObject* qjl_scores(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const int dev = c10::cuda::current_device();
+  if (n != 5 || !float_plain(a[0], dev)) return none();
+  for (int i = 1; i < 5; ++i)
+    if (!plain(a[i], dev)) return none();
+  const at::Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &signs = THPVariable_Unpack(a[2]), &rn = THPVariable_Unpack(a[3]),
+                   &qt = THPVariable_Unpack(a[4]);
+  if (q.dim() != 4 || k.dim() != 4 || !q.is_contiguous()) return none();
+  const int64_t b = q.size(0), h = q.size(1), sq = q.size(2), d = q.size(3), sk = k.size(2);
+  if (d < 1 || d > 256 || !is(k, at::kHalf, {b, h, sk, d}) || !is(signs, at::kChar, {b, h, sk, d}) || !is(rn, at::kHalf, {b, h, sk}) ||
+      !is(qt, at::kFloat, {d, d}))
+    return none();
+  c10::AutoGradMode no_grad(false);
+  at::Tensor out = make({b, h, sq, sk}, at::kFloat, dev);
+  at::Tensor ws = scratch(api.qjl_scores_ws(b * h, sq, (int)d), dev);
+  TqQjlScoreJob j{};
+  j.q = q.data_ptr(); j.q_dtype = dtype_of(q); j.D = (int32_t)d; j.BH = b * h; j.Sq = sq; j.Sk = sk;
+  j.k_mse = (const uint16_t*)k.data_ptr(); j.signs = (const int8_t*)signs.data_ptr(); j.rnorm = (const uint16_t*)rn.data_ptr();
+  j.qjl_t = (const float*)qt.data_ptr(); j.scores = (float*)out.data_ptr(); j.workspace = ws.data_ptr(); j.workspace_bytes = (size_t)ws.numel();
+  void* st = stream_of(dev);
+  if (!call("tq_qjl_scores", [&] { return api.qjl_scores(&j, st); })) return nullptr;
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// qjl_scores_packed(q, rows, sign_bits, vec_norms, rnorm, pi_t, qjl_t, codebook, bits) -> fp32 (B, H, Sq, Sk) | None
+PyObject* qjl_scores_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const int dev = c10::cuda::current_device();
+  int64_t bits;
+  if (n != 9 || !float_plain(a[0], dev) || !bit_width(a[8], &bits)) return none();
+  for (int i = 1; i < 8; ++i)
+    if (!plain(a[i], dev)) return none();
+  const at::Tensor &q = THPVariable_Unpack(a[0]), &rows = THPVariable_Unpack(a[1]), &sb = THPVariable_Unpack(a[2]), &vn = THPVariable_Unpack(a[3]),
+                   &rn = THPVariable_Unpack(a[4]), &pi_t = THPVariable_Unpack(a[5]), &qt = THPVariable_Unpack(a[6]), &cb = THPVariable_Unpack(a[7]);
+  if (q.dim() != 4 || rows.dim() != 4 || !q.is_contiguous()) return none();
+  const int64_t b = q.size(0), h = q.size(1), sq = q.size(2), d = q.size(3), sk = rows.size(2);
+  if ((d != 128 && d != 256) || !is(rows, at::kByte, {b, h, sk, row_bytes(d, bits)}) || !is(sb, at::kByte, {b, h, sk, d / 8}) ||
+      !is(vn, at::kFloat, {b, h, sk}) || !is(rn, at::kHalf, {b, h, sk}) || !is(pi_t, at::kFloat, {d, d}) || !is(qt, at::kFloat, {d, d}) ||
+      cb.scalar_type() != at::kFloat || cb.numel() != TQ_CODEBOOK_FLOATS || !cb.is_contiguous())
+    return none();
+  c10::AutoGradMode no_grad(false);
+  at::Tensor out = make({b, h, sq, sk}, at::kFloat, dev);
+  at::Tensor ws = scratch(api.qjl_scores_packed_ws(b * h, sq, (int)d), dev);
+  TqQjlPackedScoreJob j{};
+  j.q = q.data_ptr(); j.q_dtype = dtype_of(q); j.D = (int32_t)d; j.bits = (int32_t)bits; j.BH = b * h; j.Sq = sq; j.Sk = sk;
+  j.idx_packed = (const uint8_t*)rows.data_ptr(); j.sign_bits = (const uint8_t*)sb.data_ptr(); j.vec_norms = (const float*)vn.data_ptr();
+  j.rnorm = (const uint16_t*)rn.data_ptr(); j.rotation_t = (const float*)pi_t.data_ptr(); j.qjl_t = (const float*)qt.data_ptr();
+  j.codebook = (const float*)cb.data_ptr(); j.scores = (float*)out.data_ptr(); j.workspace = ws.data_ptr(); j.workspace_bytes = (size_t)ws.numel();
+  void* st = stream_of(dev);
+  if (!call("tq_qjl_scores_packed", [&] { return api.qjl_scores_packed(&j, st); })) return nullptr;
+  return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
 
@@ -624,8 +805,8 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (views) {
       Ref k(PyObject_GetAttr(lay, n_k)), v(PyObject_GetAttr(lay, n_v));
       if (!k || !v) return nullptr;
-      Ref kv(THPVariable_Wrap(THPVariable_Unpack(k.p).narrow(2, 0, total[l] + s_new)));
-      Ref vv(THPVariable_Wrap(THPVariable_Unpack(v.p).narrow(2, 0, total[l] + s_new)));
+      Ref kv(THPVariable_Wrap(tokens(THPVariable_Unpack(k.p), 0, total[l] + s_new)));
+      Ref vv(THPVariable_Wrap(tokens(THPVariable_Unpack(v.p), 0, total[l] + s_new)));
       if (!kv || !vv) return nullptr;
       PyObject* pair = PyTuple_Pack(2, kv.p, vv.p);
       if (pair == nullptr) return nullptr;
@@ -636,32 +817,38 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(addresses of the six C functions in the order of Api, check, the four job methods)
+// bind(addresses of the C functions in the order of Api, check, the four job methods)
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  void* p[6];
-  if (n != 8 || !PyTuple_Check(a[7]) || PyTuple_GET_SIZE(a[7]) != 4) {
-    PyErr_SetString(PyExc_TypeError, "bind takes six addresses, a function and a tuple of four");
+  constexpr int kFns = 14;
+  void* p[kFns];
+  if (n != kFns + 2 || !PyTuple_Check(a[kFns + 1]) || PyTuple_GET_SIZE(a[kFns + 1]) != 4) {
+    PyErr_SetString(PyExc_TypeError, "bind takes fourteen addresses, a function and a tuple of four");
     return nullptr;
   }
-  for (int i = 0; i < 6; ++i) {
+  for (int i = 0; i < kFns; ++i) {
     p[i] = PyLong_AsVoidPtr(a[i]);
     if (p[i] == nullptr) { if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address"); return nullptr; }
   }
   api.quantize = (decltype(api.quantize))p[0]; api.dequantize = (decltype(api.dequantize))p[1];
   api.copy_rows = (decltype(api.copy_rows))p[2]; api.qjl_compress = (decltype(api.qjl_compress))p[3];
   api.qjl_compress_ws = (decltype(api.qjl_compress_ws))p[4]; api.prod_inner = (decltype(api.prod_inner))p[5];
-  Py_INCREF(a[6]);
+  api.score_packed = (decltype(api.score_packed))p[6]; api.score_ws = (decltype(api.score_ws))p[7];
+  api.decode_attention = (decltype(api.decode_attention))p[8]; api.decode_attention_ws = (decltype(api.decode_attention_ws))p[9];
+  api.qjl_scores = (decltype(api.qjl_scores))p[10]; api.qjl_scores_ws = (decltype(api.qjl_scores_ws))p[11];
+  api.qjl_scores_packed = (decltype(api.qjl_scores_packed))p[12]; api.qjl_scores_packed_ws = (decltype(api.qjl_scores_packed_ws))p[13];
+  Py_INCREF(a[kFns]);
   Py_XDECREF(api.check);
-  api.check = a[6];
-  Py_INCREF(a[7]);
+  api.check = a[kFns];
+  Py_INCREF(a[kFns + 1]);
   Py_XDECREF(api.jobs);
-  api.jobs = a[7];
+  api.jobs = a[kFns + 1];
   Py_RETURN_NONE;
 }
 
 #define TQ_FN(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {TQ_FN(bind), TQ_FN(compress_kv), TQ_FN(decompress_kv), TQ_FN(compress), TQ_FN(decompress),
-                         TQ_FN(quantize_rows), TQ_FN(dequantize_rows), TQ_FN(prod_inner), TQ_FN(qjl_compress),
+                         TQ_FN(quantize_rows), TQ_FN(dequantize_rows), TQ_FN(prod_inner), TQ_FN(qjl_compress), TQ_FN(score_packed),
+                         TQ_FN(decode_attention), TQ_FN(qjl_scores), TQ_FN(qjl_scores_packed),
                          TQ_FN(step_plan), TQ_FN(step), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_tq_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

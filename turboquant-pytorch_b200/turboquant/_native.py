@@ -201,7 +201,9 @@ def host():
         else:
             H.bind(*(C.cast(getattr(L, n), C.c_void_p).value for n in
                      ("tq_quantize", "tq_dequantize", "tq_copy_rows", "tq_qjl_compress", "tq_qjl_compress_workspace_bytes",
-                      "tq_prod_inner_product")), check, JOB_METHODS)
+                      "tq_prod_inner_product", "tq_score_packed", "tq_score_workspace_bytes", "tq_decode_attention",
+                      "tq_decode_attention_workspace_bytes", "tq_qjl_scores", "tq_qjl_scores_workspace_bytes",
+                      "tq_qjl_scores_packed", "tq_qjl_scores_packed_workspace_bytes")), check, JOB_METHODS)
         _host = H
     return _host
 

@@ -29,7 +29,6 @@ class TurboQuantCompressorV2:
         self._s_t = self.S.T.contiguous()
         self._cb = N.codebook_block(self.centroids, self.mse_bits).to(device)
 
-    @torch.no_grad()
     def compress(self, states: torch.Tensor, packed: bool = False) -> dict:
         """The reference's dict ("k_mse" fp16, "qjl_signs" int8, "residual_norm" fp16, "shape"), or with packed=True
         the packed form of the same information (not in the reference, whose stored form is larger than the 16-bit
@@ -39,6 +38,18 @@ class TurboQuantCompressorV2:
           "vec_norms"     (B,H,S) fp32      ||x||: k_mse = (centroids[idx] @ Pi) * vec_norms
           "residual_norm" (B,H,S) fp16, "shape", "packed": True
         asymmetric_attention_scores takes either form; unpack() turns the packed one into the reference's."""
+        if states.is_cuda and states.dim() == 4:
+            done = N.host().qjl_compress(states, self.Pi, self.PiT, self._cb, self._s_t, self.mse_bits, 4 if packed else 3)
+            if done is not None:
+                shape = tuple(states.shape)
+                if not packed:
+                    return {"k_mse": done[0], "qjl_signs": done[1], "residual_norm": done[2], "shape": shape}
+                return {"mse_idx_bytes": done[0], "sign_bits": done[1], "vec_norms": done[3], "residual_norm": done[2],
+                        "shape": shape, "packed": True}
+        return self._compress_general(states, packed)
+
+    @torch.no_grad()
+    def _compress_general(self, states: torch.Tensor, packed: bool) -> dict:
         B, H, S, D = states.shape
         if not packed:
             k_mse, _idx, signs, rnorm = _ops.qjl_compress(states, self.Pi, self.PiT, self._cb, self._s_t, self.mse_bits,
