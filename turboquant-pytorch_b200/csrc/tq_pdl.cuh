@@ -3,9 +3,10 @@
 // kernel of the stream wrote is there already, because the first kernel of the chain is an ordinary launch.  The
 // predecessor lets it start with pdl_trigger at its own beginning: by then all its CTAs are running, so the dependent
 // takes no place from it.  Only a kernel that a launch_after() of the same call follows may trigger: the last kernel of a call
-// would let another library's dependent kernel start beside it.  Packed scores of 131072 keys x 8 heads with softmax 64 -> 59.5 us, decode attention of 32640 tokens
-// 41 -> 35 us, three launches each; MSE + QJL: compress and
-// scores of 8 x 4096 packed keys 64 -> 58 us, scores of 16 x 16384 keys 84 -> 81 us.
+// would let another library's dependent kernel start beside it.  Against ordinary launches of the same kernels, packed
+// scores of 131072 keys x 8 heads with softmax took 59.5 instead of 64 us (46 now, the kernels being faster), decode attention of 32640 tokens
+// 35 instead of 41 (31 now), three launches each; MSE + QJL: compress and
+// scores of 8 x 4096 packed keys 58 instead of 64 (37 now), scores of 16 x 16384 keys 81 instead of 84 (76 now).
 #pragma once
 
 #include <cuda_runtime.h>
