@@ -117,3 +117,14 @@ def test_native_steps_are_read_where_they_are_recorded():
         assert c._entries(1) == [(0, 2, "first", (64, 80, 96, 112)), (2, 1, "second", (0, 16, 32, 48))]
         assert c._entries(2) == [(0, 1, "second", (64, 80, 96, 112))]
     assert len(c._step_log) == 2 and len(c._layers[0].packed) == 2 and not hasattr(c, "_file_steps")
+
+
+@pytest.mark.parametrize("entry", ["tq_score_workspace_bytes", "tq_decode_attention_workspace_bytes", "tq_qjl_scores_workspace_bytes",
+                                   "tq_qjl_scores_packed_workspace_bytes"])
+def test_a_replaced_scratch_size_is_asked(monkeypatch, entry):
+    """The extension holds the library's own size entries; a call whose entry was replaced takes the path that asks it."""
+    assert N.attention_host(entry) is N.host()
+    with monkeypatch.context() as m:
+        m.setattr(N.lib(), entry, lambda *a: 0)
+        assert isinstance(N.attention_host(entry), N._GeneralPath)
+    assert N.attention_host(entry) is N.host()

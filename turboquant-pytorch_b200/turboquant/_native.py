@@ -153,6 +153,8 @@ def lib():
     for name in ("tq_packed_row_bytes", "tq_build_codebook", "tq_quantize_rotated", "tq_quantize", "tq_dequantize",
                  "tq_project", "tq_copy_rows", "tq_score_packed", "tq_score_packed_noalloc", "tq_qjl_compress", "tq_qjl_scores", "tq_prod_inner_product"):
         getattr(L, name).restype = i32
+    _SIZE_ENTRIES.update((n, getattr(L, n)) for n in ("tq_score_workspace_bytes", "tq_decode_attention_workspace_bytes",
+                                                     "tq_qjl_scores_workspace_bytes", "tq_qjl_scores_packed_workspace_bytes"))
     _lib = L
     return L
 
@@ -206,6 +208,17 @@ def host():
                       "tq_qjl_scores_packed", "tq_qjl_scores_packed_workspace_bytes")), check, JOB_METHODS)
         _host = H
     return _host
+
+
+# the attention calls' scratch-size entries as lib() bound them
+_SIZE_ENTRIES: dict = {}
+_general = _GeneralPath()
+
+
+def attention_host(size_entry: str):
+    """host(), unless the scratch-size entry of the call has been replaced on lib() (to give the call less scratch, say): the
+    extension holds the library's own, so such a call takes the general path, which asks the one that is there."""
+    return host() if getattr(lib(), size_entry) is _SIZE_ENTRIES[size_entry] else _general
 
 
 def check(rc: int, what: str):

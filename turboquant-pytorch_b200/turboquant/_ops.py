@@ -131,7 +131,7 @@ def score_packed(q: torch.Tensor, idx_bytes: torch.Tensor, norms: torch.Tensor, 
                  codebook: torch.Tensor, bits: int, scale: float = 1.0, softmax: bool = False):
     """q (B,Hq,Sq,D); packed keys (B,Hkv,Sk,G) + norms (B,Hkv,Sk) -> logits (B,Hq,Sq,Sk) [, probs]."""
     if q.is_cuda:
-        done = N.host().score_packed(q, idx_bytes, norms, pi_t, codebook, bits, scale, softmax)
+        done = N.attention_host("tq_score_workspace_bytes").score_packed(q, idx_bytes, norms, pi_t, codebook, bits, scale, softmax)
         if done is not None:
             return done
     q = q.contiguous()
@@ -184,7 +184,8 @@ def decode_attention(q: torch.Tensor, k_comp: Optional[dict], v_comp: Optional[d
     the windows are (B, Hkv, W, 128) tensors (views are fine, unit last stride) or None.  Returns fp32 (B, Hq, Sq, 128).
     """
     N.require_cuda(q, "decode_attention")
-    done = N.host().decode_attention(q, k_comp, v_comp, key_codec, val_codec, k_window, v_window, scale)
+    done = N.attention_host("tq_decode_attention_workspace_bytes").decode_attention(q, k_comp, v_comp, key_codec, val_codec, k_window,
+                                                                                    v_window, scale)
     if done is not None:
         return done
     B, Hq, Sq, D = q.shape
@@ -353,7 +354,8 @@ def qjl_scores_packed(q: torch.Tensor, idx_packed: torch.Tensor, sign_bits: torc
     """q (B,H,Sq,D) against the packed MSE+QJL form ((B,H,Sk,G) index rows, (B,H,Sk,D/8) sign bits, fp32 vector norms,
     fp16 residual norms) -> (B,H,Sq,Sk) fp32."""
     N.require_cuda(q, "qjl_scores_packed")
-    done = N.host().qjl_scores_packed(q, idx_packed, sign_bits, vec_norms, rnorm, pi_t, qjl_t, codebook, bits)
+    done = N.attention_host("tq_qjl_scores_packed_workspace_bytes").qjl_scores_packed(q, idx_packed, sign_bits, vec_norms, rnorm, pi_t,
+                                                                                       qjl_t, codebook, bits)
     if done is not None:
         return done
     B, H, Sq, D = q.shape
@@ -385,7 +387,7 @@ def qjl_scores(q: torch.Tensor, k_mse: torch.Tensor, signs: torch.Tensor, rnorm:
                qjl_t: torch.Tensor) -> torch.Tensor:
     """q (B,H,Sq,D) against the compressed dict tensors -> (B,H,Sq,Sk) fp32."""
     N.require_cuda(q, "qjl_scores")
-    done = N.host().qjl_scores(q, k_mse, signs, rnorm, qjl_t)
+    done = N.attention_host("tq_qjl_scores_workspace_bytes").qjl_scores(q, k_mse, signs, rnorm, qjl_t)
     if done is not None:
         return done
     B, H, Sq, D = q.shape
