@@ -119,8 +119,7 @@ def test_native_steps_are_read_where_they_are_recorded():
     assert len(c._step_log) == 2 and len(c._layers[0].packed) == 2 and not hasattr(c, "_file_steps")
 
 
-@pytest.mark.parametrize("entry", ["tq_score_workspace_bytes", "tq_decode_attention_workspace_bytes", "tq_qjl_scores_workspace_bytes",
-                                   "tq_qjl_scores_packed_workspace_bytes"])
+@pytest.mark.parametrize("entry", ["tq_score_workspace_bytes", "tq_decode_attention_workspace_bytes", "tq_qjl_scores_packed_workspace_bytes"])
 def test_a_replaced_scratch_size_is_asked(monkeypatch, entry):
     """The extension holds the library's own size entries; a call whose entry was replaced takes the path that asks it."""
     assert N.attention_host(entry) is N.host()

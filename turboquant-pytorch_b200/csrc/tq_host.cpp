@@ -33,8 +33,6 @@ struct Api {
   decltype(&tq_score_workspace_bytes) score_ws = nullptr;
   decltype(&tq_decode_attention) decode_attention = nullptr;
   decltype(&tq_decode_attention_workspace_bytes) decode_attention_ws = nullptr;
-  decltype(&tq_qjl_scores) qjl_scores = nullptr;
-  decltype(&tq_qjl_scores_workspace_bytes) qjl_scores_ws = nullptr;
   decltype(&tq_qjl_scores_packed) qjl_scores_packed = nullptr;
   decltype(&tq_qjl_scores_packed_workspace_bytes) qjl_scores_packed_ws = nullptr;
   PyObject* check = nullptr;               // Python: check(rc, what) raises for rc != 0
@@ -591,33 +589,6 @@ PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// qjl_scores(q, k_mse, signs, rnorm, qjl_t) -> fp32 (B, H, Sq, Sk) | None
-PyObject* qjl_scores(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
-  const int dev = c10::cuda::current_device();
-  if (n != 5 || !float_plain(a[0], dev)) return none();
-  for (int i = 1; i < 5; ++i)
-    if (!plain(a[i], dev)) return none();
-  const at::Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &signs = THPVariable_Unpack(a[2]), &rn = THPVariable_Unpack(a[3]),
-                   &qt = THPVariable_Unpack(a[4]);
-  if (q.dim() != 4 || k.dim() != 4 || !q.is_contiguous()) return none();
-  const int64_t b = q.size(0), h = q.size(1), sq = q.size(2), d = q.size(3), sk = k.size(2);
-  if (d < 1 || d > 256 || !is(k, at::kHalf, {b, h, sk, d}) || !is(signs, at::kChar, {b, h, sk, d}) || !is(rn, at::kHalf, {b, h, sk}) ||
-      !is(qt, at::kFloat, {d, d}))
-    return none();
-  c10::AutoGradMode no_grad(false);
-  at::Tensor out = make({b, h, sq, sk}, at::kFloat, dev);
-  at::Tensor ws = scratch(api.qjl_scores_ws(b * h, sq, (int)d), dev);
-  TqQjlScoreJob j{};
-  j.q = q.data_ptr(); j.q_dtype = dtype_of(q); j.D = (int32_t)d; j.BH = b * h; j.Sq = sq; j.Sk = sk;
-  j.k_mse = (const uint16_t*)k.data_ptr(); j.signs = (const int8_t*)signs.data_ptr(); j.rnorm = (const uint16_t*)rn.data_ptr();
-  j.qjl_t = (const float*)qt.data_ptr(); j.scores = (float*)out.data_ptr(); j.workspace = ws.data_ptr(); j.workspace_bytes = (size_t)ws.numel();
-  void* st = stream_of(dev);
-  if (!call("tq_qjl_scores", [&] { return api.qjl_scores(&j, st); })) return nullptr;
-  return THPVariable_Wrap(out);
-  END_HANDLE_TH_ERRORS
-}
-
 // qjl_scores_packed(q, rows, sign_bits, vec_norms, rnorm, pi_t, qjl_t, codebook, bits) -> fp32 (B, H, Sq, Sk) | None
 PyObject* qjl_scores_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -819,10 +790,10 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // bind(addresses of the C functions in the order of Api, check, the four job methods)
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  constexpr int kFns = 14;
+  constexpr int kFns = 12;
   void* p[kFns];
   if (n != kFns + 2 || !PyTuple_Check(a[kFns + 1]) || PyTuple_GET_SIZE(a[kFns + 1]) != 4) {
-    PyErr_SetString(PyExc_TypeError, "bind takes fourteen addresses, a function and a tuple of four");
+    PyErr_SetString(PyExc_TypeError, "bind takes twelve addresses, a function and a tuple of four");
     return nullptr;
   }
   for (int i = 0; i < kFns; ++i) {
@@ -834,8 +805,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   api.qjl_compress_ws = (decltype(api.qjl_compress_ws))p[4]; api.prod_inner = (decltype(api.prod_inner))p[5];
   api.score_packed = (decltype(api.score_packed))p[6]; api.score_ws = (decltype(api.score_ws))p[7];
   api.decode_attention = (decltype(api.decode_attention))p[8]; api.decode_attention_ws = (decltype(api.decode_attention_ws))p[9];
-  api.qjl_scores = (decltype(api.qjl_scores))p[10]; api.qjl_scores_ws = (decltype(api.qjl_scores_ws))p[11];
-  api.qjl_scores_packed = (decltype(api.qjl_scores_packed))p[12]; api.qjl_scores_packed_ws = (decltype(api.qjl_scores_packed_ws))p[13];
+  api.qjl_scores_packed = (decltype(api.qjl_scores_packed))p[10]; api.qjl_scores_packed_ws = (decltype(api.qjl_scores_packed_ws))p[11];
   Py_INCREF(a[kFns]);
   Py_XDECREF(api.check);
   api.check = a[kFns];
@@ -848,7 +818,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
 #define TQ_FN(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {TQ_FN(bind), TQ_FN(compress_kv), TQ_FN(decompress_kv), TQ_FN(compress), TQ_FN(decompress),
                          TQ_FN(quantize_rows), TQ_FN(dequantize_rows), TQ_FN(prod_inner), TQ_FN(qjl_compress), TQ_FN(score_packed),
-                         TQ_FN(decode_attention), TQ_FN(qjl_scores), TQ_FN(qjl_scores_packed),
+                         TQ_FN(decode_attention), TQ_FN(qjl_scores_packed),
                          TQ_FN(step_plan), TQ_FN(step), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_tq_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -154,7 +154,7 @@ def lib():
                  "tq_project", "tq_copy_rows", "tq_score_packed", "tq_score_packed_noalloc", "tq_qjl_compress", "tq_qjl_scores", "tq_prod_inner_product"):
         getattr(L, name).restype = i32
     _SIZE_ENTRIES.update((n, getattr(L, n)) for n in ("tq_score_workspace_bytes", "tq_decode_attention_workspace_bytes",
-                                                     "tq_qjl_scores_workspace_bytes", "tq_qjl_scores_packed_workspace_bytes"))
+                                                     "tq_qjl_scores_packed_workspace_bytes"))
     _lib = L
     return L
 
@@ -204,7 +204,7 @@ def host():
             H.bind(*(C.cast(getattr(L, n), C.c_void_p).value for n in
                      ("tq_quantize", "tq_dequantize", "tq_copy_rows", "tq_qjl_compress", "tq_qjl_compress_workspace_bytes",
                       "tq_prod_inner_product", "tq_score_packed", "tq_score_workspace_bytes", "tq_decode_attention",
-                      "tq_decode_attention_workspace_bytes", "tq_qjl_scores", "tq_qjl_scores_workspace_bytes",
+                      "tq_decode_attention_workspace_bytes",
                       "tq_qjl_scores_packed", "tq_qjl_scores_packed_workspace_bytes")), check, JOB_METHODS)
         _host = H
     return _host

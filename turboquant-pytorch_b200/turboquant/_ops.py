@@ -387,9 +387,6 @@ def qjl_scores(q: torch.Tensor, k_mse: torch.Tensor, signs: torch.Tensor, rnorm:
                qjl_t: torch.Tensor) -> torch.Tensor:
     """q (B,H,Sq,D) against the compressed dict tensors -> (B,H,Sq,Sk) fp32."""
     N.require_cuda(q, "qjl_scores")
-    done = N.attention_host("tq_qjl_scores_workspace_bytes").qjl_scores(q, k_mse, signs, rnorm, qjl_t)
-    if done is not None:
-        return done
     B, H, Sq, D = q.shape
     Sk = k_mse.shape[2]
     q = q.contiguous()
